@@ -237,8 +237,10 @@ Params make_dev_params(const n4_params_t *p) {
   return r;
 }
 
-// Workspace layout for a group of K CTAs over the given fitting grids.
-Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool grid) {
+// Workspace layout for a group of K CTAs over the given fitting grids;
+// max_smem: shared memory per CTA (whole-GPU path, whose volume takes what is
+// left beside the tables).
+Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool grid, int max_smem = 0) {
   Plan pl{};
   pl.levels = (int)p->NumberOfFittingLevels;
   pl.nc0x = (int)p->NumberOfControlPoints_x;
@@ -257,57 +259,77 @@ Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool 
     pl.Ymax = std::max(pl.Ymax, d.Y);
     pl.Zmax = std::max(pl.Zmax, d.Z);
     const long long rows = (long long)d.X * d.Y;
-    // grid: contiguous rows; cluster: whole x-planes, ceil(X / K) per CTA
-    const long long rpc = grid ? (rows + K - 1) / K : ((long long)d.X + K - 1) / K * d.Y;
-    rows_max = std::max(rows_max, rpc);
-    slab = std::max(slab, rpc * d.Z);
-    // the y contraction spans every x-plane a CTA touches: all of them when
-    // rows are interleaved (cluster), a contiguous range otherwise (grid)
-    nvxl = std::max(nvxl, grid ? (rpc - 1) / d.Y + 2 : ((long long)d.X + K - 1) / K);
+    if (grid) {   // rows dealt out by weight, in contiguous ranges
+      rows_max = std::max(rows_max, grid_rows_bound(rows, d.Z, K));
+      slab = std::max(slab, grid_voxels_bound(rows, d.Z, K));
+      // x-planes whose sums are held at a time
+      nvxl = std::max(nvxl, ((rows + K - 1) / K - 1) / d.Y + 2);
+    } else {      // whole x-planes, ceil(X / K) per CTA
+      const long long planes = ((long long)d.X + K - 1) / K;
+      rows_max = std::max(rows_max, planes * d.Y);
+      slab = std::max(slab, planes * d.Y * d.Z);
+      nvxl = std::max(nvxl, planes);
+    }
   }
   pl.slab_floats = (int)slab;
   pl.rows_max = (int)rows_max;
   pl.nvxl = (int)nvxl;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t r = o; o = align_up(o + bytes, 16); return (int)r; };
-  pl.o_ax = take(axis_bytes(pl.Xmax, pl.NCX - 3));
-  pl.o_ay = take(axis_bytes(pl.Ymax, pl.NCY - 3));
-  pl.o_az = take(axis_bytes(pl.Zmax, pl.NCZ - 3));
+  pl.o_ax = take(eaxis_bytes(pl.Xmax, pl.NCX - 3));
+  pl.o_ay = take(eaxis_bytes(pl.Ymax, pl.NCY - 3));
+  pl.o_az = take(eaxis_bytes(pl.Zmax, pl.NCZ - 3));
   pl.o_L = take((size_t)pl.NLAT * 4);
   pl.o_D = take((size_t)pl.NLAT * 4);
   pl.o_den = take((size_t)pl.NLAT * 4);
   pl.o_tmp = take((size_t)pl.NLAT * 4);
   pl.o_aux = take((size_t)pl.NLAT * 4);
-  // cluster path: the histogram copies and the two FFT work buffers share
-  // the Gd region (see Plan::alias_sharpen); grid path: shared memory
-  const size_t hist_bytes = (size_t)kHistCopies * pl.bins * 4, fft_bytes = (size_t)pl.npad * 16;
-  pl.alias_sharpen = grid ? 0 : 1;
-  if (grid) {
-    pl.o_hist = take(hist_bytes);
-    pl.o_fa = take(fft_bytes);
-    pl.o_fb = take(fft_bytes);
-  }
   pl.o_H64 = take((size_t)pl.bins * 8);
   pl.o_R2 = take((size_t)pl.bins * 8);   // the residual's per-bin linear form
   pl.o_E = take((size_t)pl.bins * 8);
   pl.o_tw = take((size_t)pl.npad * 16);
-  pl.o_ff = grid ? take((size_t)pl.npad * 8) : 0;   // cluster: in the Gd region
   pl.o_red = take(160 * 8);
-  pl.o_misc = take(64);
-  pl.sm_bytes = (int)align_up(o, 128);
-  o = 0;
-  pl.b_imlog = take(((size_t)pl.slab_floats + 8) * 4);   // logU (cluster: the staged rows first)
+  // the histogram copies and the two FFT work buffers share the Gd region
+  const size_t hist_bytes = (size_t)kHistCopies * pl.bins * 4, fft_bytes = (size_t)pl.npad * 16;
+  const size_t alias_bytes = 2 * fft_bytes + std::max(hist_bytes, (size_t)pl.npad * 8);
   pl.a_fa = 0;
   pl.a_fb = (int)fft_bytes;
   pl.a_hist = (int)(2 * fft_bytes);
   pl.a_ff = pl.a_hist;   // written by the sharpening after the histogram copies are merged
-  const size_t ff_bytes = (size_t)pl.npad * 8;
-  pl.b_Gd = take(std::max((size_t)pl.rows_max * pl.NCZ * 4, grid ? 0 : 2 * fft_bytes + std::max(hist_bytes, ff_bytes)));
-  pl.b_T2 = take((size_t)pl.nvxl * pl.NCY * pl.NCZ * 4);
+  const size_t gd = (size_t)pl.rows_max * pl.NCZ * 4, t2 = (size_t)pl.nvxl * pl.NCY * pl.NCZ * 4,
+               yt = (size_t)pl.nvxl * (pl.NCY - 2) * 4;
+  if (grid) {
+    // Gd: 24 KB hold the rows of a CTA's share of a 256x256x160 grid (280 of
+    // 11 control points); T2 of six 11x11 planes; both fall back to global
+    // memory.  The row list and the volume take the rest.
+    pl.gd_bytes = (int)align_up(std::max<size_t>(alias_bytes, 24 << 10), 128);
+    pl.o_gd = take(pl.gd_bytes);
+    pl.t2_bytes = 4 << 10;
+    pl.o_t2 = take(pl.t2_bytes);
+    pl.o_ytab = take(pl.t2_bytes);
+    o = align_up(o, 128);
+    pl.o_pool = (int)o;
+    const long long rest = (long long)max_smem - kStaticSmemReserve - (long long)o;
+    pl.pool_bytes = (int)std::max<long long>(0, rest / 128 * 128);
+    o += pl.pool_bytes;
+  } else {
+    pl.o_rows = take((size_t)pl.rows_max * 8);
+    pl.o_ytab = take(yt);
+  }
+  pl.sm_bytes = (int)align_up(o, 128);
+  o = 0;
+  pl.b_imlog = take(((size_t)pl.slab_floats + 8) * 4);   // logU (cluster: the staged rows first)
+  pl.b_Gd = take(grid ? gd : std::max(gd, alias_bytes));
+  pl.b_T2 = take(t2);
   pl.b_slotA = take(sizeof(Stats));
-  pl.b_slotB = take((size_t)pl.bins * 8);
-  pl.b_slotC = take((size_t)pl.NLAT * 4);
-  pl.b_slice = take(std::max((size_t)(pl.NLAT + K - 1) / K * 4, (size_t)(pl.bins + K - 1) / K * 8));
+  if (grid) {
+    pl.b_ytab = take(yt);
+    pl.b_rows = take((size_t)pl.rows_max * 16);
+    pl.b_slotB = take(8);
+  } else {
+    pl.b_slotB = take((size_t)pl.bins * 8);
+    pl.b_slotC = take((size_t)pl.NLAT * 4);
+  }
   pl.big_bytes = (int)align_up(o, 128);
   return pl;
 }
@@ -474,13 +496,18 @@ struct RunVol {
   Dims d;
 };
 
-// Workspaces of the whole-GPU path for one volume (sized before any capture).
+// Words of one accumulator set of the whole-GPU path.
+int grid_acc_len(const Plan &pl) { return std::max(pl.bins, pl.NLAT) + 1; }
+
+// Workspaces of the whole-GPU path for one volume (sized before any capture):
+// the CTAs' slices; the accumulator sets and the barrier, zero at launch;
+// the rows' ranges.
 n4_status_t ensure_grid_workspace(n4_context *ctx, const n4_params_t *p, const Dims &d) {
   std::vector<Dims> one{d};
-  Plan pl = make_plan(p, ctx->nsm, one, true);
+  Plan pl = make_plan(p, ctx->nsm, one, true, ctx->max_smem);
   TRY(ctx->big.ensure((size_t)pl.big_bytes * ctx->nsm, "grid workspace"));
-  TRY(ctx->red.ensure(std::max((size_t)pl.bins * 8, (size_t)pl.NLAT * 4) + 64, "grid reduction"));
-  TRY(ctx->bar.ensure(64, "grid barrier"));
+  TRY(ctx->red.ensure((size_t)3 * grid_acc_len(pl) * 8 + 64, "grid reduction"));
+  TRY(ctx->bar.ensure((size_t)d.X * d.Y * 4, "grid rows"));
   return N4_OK;
 }
 
@@ -500,26 +527,26 @@ n4_status_t launch_grid_path(n4_context *ctx, const n4_params_t *p, const Params
                              const VolJob &job0, int nt, cudaStream_t st) {
   std::vector<Dims> one{rv.d};
   int nblk = ctx->nsm;
-  Plan pl = make_plan(p, nblk, one, true);
+  Plan pl = make_plan(p, nblk, one, true, ctx->max_smem);
   if (pl.sm_bytes + kStaticSmemReserve > ctx->max_smem)
     return fail(N4_ERR_TOO_LARGE, "histogram/lattice workspace exceeds shared memory");
-  if ((long long)pl.rows_max * rv.d.Z >= (1ll << 22))
+  if (((long long)rv.d.X * rv.d.Y + nblk - 1) / nblk * rv.d.Z >= (1ll << 22))
     return fail(N4_ERR_TOO_LARGE, "fitting grid too large for one GPU (raise ShrinkFactor)");
-  TRY(ctx->big.ensure((size_t)pl.big_bytes * nblk, "grid workspace"));
-  TRY(ctx->red.ensure(std::max((size_t)pl.bins * 8, (size_t)pl.NLAT * 4) + 64, "grid reduction"));
-  TRY(ctx->bar.ensure(64, "grid barrier"));
-  CK(cudaMemsetAsync(ctx->bar.p, 0, 64, st));
+  TRY(ensure_grid_workspace(ctx, p, rv.d));
+  const size_t acc_bytes = (size_t)3 * grid_acc_len(pl) * 8;
+  CK(cudaMemsetAsync(ctx->red.p, 0, acc_bytes + 64, st));
   GridArgs a{};
   a.pl = pl;
   a.pr = pr;
   a.job = job0;
   a.big_base = ctx->big.as<char>();
   a.big_stride = pl.big_bytes;
-  a.bar.count = ctx->bar.as<unsigned>();
-  a.bar.gen = ctx->bar.as<unsigned>() + 1;
-  a.bar.err = (int *)ctx->bar.as<unsigned>() + 2;
+  a.acc = ctx->red.as<unsigned long long>();
+  a.acc_len = grid_acc_len(pl);
+  a.bar.count = (unsigned *)(ctx->red.as<char>() + acc_bytes);
+  a.bar.err = (int *)(a.bar.count + 8);
   a.bar.nblocks = nblk;
-  a.red_global = ctx->red.as<float>();
+  a.ext = ctx->bar.as<unsigned>();
   const int smem = pl.sm_bytes;
   if (nt == 1024) return launch_grid_kernel<1024>(a, nblk, smem, st);
   if (nt == 768) return launch_grid_kernel<768>(a, nblk, smem, st);
@@ -571,13 +598,25 @@ TuneKey tune_key(const n4_params_t *p, const std::vector<Dims> &vols) {
   return k;
 }
 
+// Threads per CTA of the whole-GPU path: 512 where a CTA's share is small (its
+// time is the latency of barriers and FFTs, which more warps lengthen: 1.33
+// against 1.59 ms for 40 iterations of 80x84x88 voxels, 4000 per CTA), 1024
+// where it is large (42 iterations of 256x256x160, 71000 per CTA: 7.3 against
+// 7.5 million cycles; 20 of 181x217x181, 48000 per CTA: 2.86 against 2.93).
+int grid_threads(const n4_context *ctx, const n4_params_t *p, const Dims &d) {
+  if (p->flags & N4_FLAG_CTA_512) return 512;
+  return (long long)d.X * d.Y * d.Z / ctx->nsm < 16384 ? 512 : 1024;
+}
+
 n4_status_t choose_path(n4_context *ctx, const n4_params_t *p, const std::vector<Dims> &vols, bool batch,
                         Choice &c) {
   const Dims &d0 = vols[0];
-  c.nt = (p->flags & N4_FLAG_CTA_512) ? 512 : 1024;
+  // clusters of 512 threads per CTA: 128 registers a thread, no spills; 1024
+  // (64 registers) took 1.18 ms against 1.06 for 36 iterations of a 64x64x48
+  // volume and 2.35 against 2.26 ms at 320x320x320, shrink 4
+  c.nt = 512;
   c.grid = false;
   c.K = 0;
-  (void)d0;
   (void)batch;
   const int forced_k = (int)((p->flags >> 8) & 31u);
   if (forced_k) {
@@ -606,6 +645,7 @@ n4_status_t choose_path(n4_context *ctx, const n4_params_t *p, const std::vector
   if (c.K == 0) {
     if (p->flags & N4_FLAG_FORCE_CLUSTER) return fail(N4_ERR_TOO_LARGE, "volume does not fit a thread-block cluster");
     c.grid = true;
+    c.nt = grid_threads(ctx, p, d0);
   }
   return N4_OK;
 }
@@ -694,10 +734,10 @@ n4_status_t plan_run(n4_context *ctx, const n4_params_t *p, const std::vector<Ru
       for (int i : P.in_cluster) sub.push_back(dims[i]);
       const Plan pl = make_plan(p, 16, sub, false);
       int cap = 0;
-      TRY(capacity(ctx, 1024, 16, pl.sm_bytes + pl.big_bytes, &cap));
+      TRY(capacity(ctx, 512, 16, pl.sm_bytes + pl.big_bytes, &cap));
       if (cap > 0) {
         ch.grid = false;
-        ch.nt = 1024;
+        ch.nt = 512;
         ch.K = 16;
       } else {
         for (int i : P.in_cluster) P.in_grid.push_back(i);
@@ -1106,7 +1146,8 @@ n4_status_t enqueue_run(n4_context *ctx, const n4_params_t *p, const Prepared &P
   }
   for (int i : P.in_grid) {
     VolJob j = B.hp<VolJob>(P.o_job)[i];
-    TRY(launch_grid_path(ctx, p, P.pr, P.rvs[i], j, P.ch.nt ? P.ch.nt : 1024, st));
+    const int nt = P.ch.grid && P.ch.nt ? P.ch.nt : grid_threads(ctx, p, P.dims[i]);
+    TRY(launch_grid_path(ctx, p, P.pr, P.rvs[i], j, nt, st));
     ++launches;
   }
   if (profile) TRY(prof_mark(ctx, 2, st));

@@ -3,7 +3,7 @@
 // * per-axis cubic B-spline tables (span index, weights, fit weights),
 //   computed in FP64 with the reference's formulas (N4.py:174-181,
 //   N4.py:210-222) and stored in FP32;
-// * a CTA-level Stockham radix-8/4/2 FFT in shared memory and the Gaussian
+// * a CTA-level Stockham radix-4/2 FFT in shared memory and the Gaussian
 //   Wiener-deconvolution sharpening map built on it (N4.py:32-101,
 //   cudaN4.cu:733-817);
 // * fractional-histogram binning and the piecewise-linear remap
@@ -21,7 +21,7 @@ constexpr int kMaxThreads = 1024;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kHistCopies = 8;                   // shared histogram copies per CTA
 constexpr int kHistMaxShift = 24;                // fixed-point weight 2^shift, shift <= 24
-constexpr unsigned long long kSpinLimit = 1ull << 25;   // bounded waits (~2-4 s)
+constexpr unsigned long long kSpinLimit = 1ull << 23;   // bounded waits (a few seconds)
 
 // ---------------------------------------------------------------- tables
 // One axis of the fitting grid at one level.  Arrays live in shared or
@@ -72,41 +72,51 @@ __device__ __forceinline__ int span_of(int i, double span, int nsp) {
   return s < 0 ? 0 : (s >= nsp ? nsp - 1 : s);
 }
 
+// Weights of voxel i along an axis of `nsp` spans of `span` voxels: the cubic
+// weights w = B0..B3, the fit's numerator weights p = w^3 / sum w^2 and
+// denominator weights q = w^2, formed in FP64.  Returns the span index.
+__device__ __forceinline__ int axis_voxel(int i, double span, int nsp, float4 &w, float4 &p, float4 &q) {
+  const int s = span_of(i, span, nsp);
+  const double u = __dadd_rn((double)i, 0.5);
+  const double t = __ddiv_rn(__dsub_rn(u, __dmul_rn((double)s, span)), span);
+  const double t2 = t * t, t3 = t * t * t, tm = 1.0 - t;
+  const double w0 = tm * tm * tm / 6.0;
+  const double w1 = (3.0 * t3 - 6.0 * t2 + 4.0) / 6.0;
+  const double w2 = (-3.0 * t3 + 3.0 * t2 + 3.0 * t + 1.0) / 6.0;
+  const double w3 = t3 / 6.0;
+  const double S = w0 * w0 + w1 * w1 + w2 * w2 + w3 * w3;
+  w = make_float4((float)w0, (float)w1, (float)w2, (float)w3);
+  p = make_float4((float)(w0 * w0 * w0 / S), (float)(w1 * w1 * w1 / S), (float)(w2 * w2 * w2 / S),
+                  (float)(w3 * w3 * w3 / S));
+  q = make_float4((float)(w0 * w0), (float)(w1 * w1), (float)(w2 * w2), (float)(w3 * w3));
+  return s;
+}
+
+// Voxel range of every span by binary search on the monotone span index.
+__device__ __forceinline__ void axis_ranges(int n, int nsp, double span, int *lo_out, int *hi_out) {
+  for (int sp = threadIdx.x; sp < nsp; sp += blockDim.x) {
+    int lo = 0, hi = n;                // first voxel with span >= sp
+    while (lo < hi) { int m = (lo + hi) >> 1; if (span_of(m, span, nsp) >= sp) hi = m; else lo = m + 1; }
+    int l2 = lo, h2 = n;               // first voxel with span >= sp + 1
+    while (l2 < h2) { int m = (l2 + h2) >> 1; if (span_of(m, span, nsp) >= sp + 1) h2 = m; else l2 = m + 1; }
+    lo_out[sp] = lo;
+    hi_out[sp] = l2;
+  }
+}
+
 // Fill one axis table with the CTA's threads (caller synchronises).
 __device__ void build_axis(const Axis &a) {
   const double span = __ddiv_rn((double)a.n, (double)a.nsp);
   for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
-    int s = span_of(i, span, a.nsp);
-    double u = __dadd_rn((double)i, 0.5);
-    double t = __ddiv_rn(__dsub_rn(u, __dmul_rn((double)s, span)), span);
-    double t2 = t * t, t3 = t * t * t, tm = 1.0 - t;
-    double w0 = tm * tm * tm / 6.0;
-    double w1 = (3.0 * t3 - 6.0 * t2 + 4.0) / 6.0;
-    double w2 = (-3.0 * t3 + 3.0 * t2 + 3.0 * t + 1.0) / 6.0;
-    double w3 = t3 / 6.0;
-    double S = w0 * w0 + w1 * w1 + w2 * w2 + w3 * w3;
-    a.s[i] = s;
-    a.w[i] = make_float4((float)w0, (float)w1, (float)w2, (float)w3);
-    a.p[0 * a.n + i] = (float)(w0 * w0 * w0 / S);
-    a.p[1 * a.n + i] = (float)(w1 * w1 * w1 / S);
-    a.p[2 * a.n + i] = (float)(w2 * w2 * w2 / S);
-    a.p[3 * a.n + i] = (float)(w3 * w3 * w3 / S);
-    a.q[0 * a.n + i] = (float)(w0 * w0);
-    a.q[1 * a.n + i] = (float)(w1 * w1);
-    a.q[2 * a.n + i] = (float)(w2 * w2);
-    a.q[3 * a.n + i] = (float)(w3 * w3);
-    a.p4[i] = make_float4(a.p[i], a.p[a.n + i], a.p[2 * a.n + i], a.p[3 * a.n + i]);
-    a.q4[i] = make_float4(a.q[i], a.q[a.n + i], a.q[2 * a.n + i], a.q[3 * a.n + i]);
+    float4 w, p, q;
+    a.s[i] = axis_voxel(i, span, a.nsp, w, p, q);
+    a.w[i] = w;
+    a.p4[i] = p;
+    a.q4[i] = q;
+    a.p[0 * a.n + i] = p.x; a.p[1 * a.n + i] = p.y; a.p[2 * a.n + i] = p.z; a.p[3 * a.n + i] = p.w;
+    a.q[0 * a.n + i] = q.x; a.q[1 * a.n + i] = q.y; a.q[2 * a.n + i] = q.z; a.q[3 * a.n + i] = q.w;
   }
-  // voxel range of every span by binary search on the monotone span index
-  for (int sp = threadIdx.x; sp < a.nsp; sp += blockDim.x) {
-    int lo = 0, hi = a.n;              // first voxel with span >= sp
-    while (lo < hi) { int m = (lo + hi) >> 1; if (span_of(m, span, a.nsp) >= sp) hi = m; else lo = m + 1; }
-    int l2 = lo, h2 = a.n;             // first voxel with span >= sp + 1
-    while (l2 < h2) { int m = (l2 + h2) >> 1; if (span_of(m, span, a.nsp) >= sp + 1) h2 = m; else l2 = m + 1; }
-    a.lo[sp] = lo;
-    a.hi[sp] = l2;
-  }
+  axis_ranges(a.n, a.nsp, span, a.lo, a.hi);
 }
 
 // b = sum_j w_j g[j] with a fixed association (identical in every pass).
@@ -117,14 +127,6 @@ __device__ __forceinline__ float dot4(float4 w, const float *g) {
   b = __fmaf_rn(w.w, g[3], b);
   return b;
 }
-
-// Exact floor(i / d) for 0 <= i < 2^22 and 1 <= d <= 2^10 via a 32-bit magic.
-struct FastDiv {
-  unsigned d, m;
-  __host__ __device__ FastDiv() : d(1), m(0) {}
-  __host__ __device__ explicit FastDiv(unsigned dd) : d(dd), m((unsigned)((0x100000000ull + dd - 1) / dd)) {}
-  __device__ __forceinline__ unsigned div(unsigned i) const { return d == 1 ? i : __umulhi(i, m); }
-};
 
 // GPU global timer (ns) and the SM this thread runs on.
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -224,21 +226,6 @@ __device__ __forceinline__ void dft4(double2 &v0, double2 &v1, double2 &v2, doub
   double2 t0 = cadd(v0, v2), t1 = csub(v0, v2), t2 = cadd(v1, v3), t3 = mul_mi(csub(v1, v3));
   v0 = cadd(t0, t2); v2 = csub(t0, t2); v1 = cadd(t1, t3); v3 = csub(t1, t3);
 }
-__device__ __forceinline__ void dft8(double2 *v) {
-  const double c = 0.70710678118654752440;
-  double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
-  double2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-  dft4(e0, e1, e2, e3);
-  dft4(o0, o1, o2, o3);
-  o1 = make_double2(c * (o1.x + o1.y), c * (o1.y - o1.x));   // * e^{-i pi/4}
-  o2 = mul_mi(o2);                                            // * e^{-i pi/2}
-  o3 = make_double2(c * (o3.y - o3.x), -c * (o3.x + o3.y));  // * e^{-3i pi/4}
-  v[0] = cadd(e0, o0); v[4] = csub(e0, o0);
-  v[1] = cadd(e1, o1); v[5] = csub(e1, o1);
-  v[2] = cadd(e2, o2); v[6] = csub(e2, o2);
-  v[3] = cadd(e3, o3); v[7] = csub(e3, o3);
-}
-
 // tw[m] = exp(-2 pi i m / N), m in [0, N).
 __device__ void fft_twiddles(double2 *tw, int N) {
   for (int m = threadIdx.x; m < N; m += blockDim.x) {
@@ -248,10 +235,16 @@ __device__ void fft_twiddles(double2 *tw, int N) {
   }
 }
 
+template <int R> __device__ __forceinline__ void dft_r(double2 *v);
+template <> __device__ __forceinline__ void dft_r<2>(double2 *v) { dft2(v); }
+template <> __device__ __forceinline__ void dft_r<4>(double2 *v) { dft4(v[0], v[1], v[2], v[3]); }
+
 // One Stockham pass of radix R (Govindaraju et al., SC'08, "High performance
-// discrete Fourier transforms on graphics processors"): x -> y.
-template <int R>
-__device__ void stockham_pass(const double2 *x, double2 *y, int N, int Ns, const double2 *tw) {
+// discrete Fourier transforms on graphics processors"): in(0..N) -> y.  The
+// input is a function, so that an elementwise step before an FFT can be part
+// of its first pass (Ns = 1, where every twiddle is 1).
+template <int R, class In>
+__device__ __forceinline__ void stockham_pass(const In &in, double2 *y, int N, int Ns, const double2 *tw) {
   const int T = N / R;
   const int tstep = N / (Ns * R);
   for (int j = threadIdx.x; j < T; j += blockDim.x) {
@@ -259,101 +252,87 @@ __device__ void stockham_pass(const double2 *x, double2 *y, int N, int Ns, const
     double2 v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      v[r] = x[j + r * T];
-      if (r) v[r] = cmul(v[r], tw[(r * k * tstep) & (N - 1)]);
+      v[r] = in(j + r * T);
+      if (r && Ns > 1) v[r] = cmul(v[r], tw[(r * k * tstep) & (N - 1)]);
     }
-    if (R == 8) dft8(v);
-    else if (R == 4) dft4(v[0], v[1], v[2], v[3]);
-    else dft2(v);
+    dft_r<R>(v);
     const int base = (j - k) * R + k;
 #pragma unroll
     for (int r = 0; r < R; ++r) y[base + r * Ns] = v[r];
   }
-}
-
-template <int R> __device__ __forceinline__ void dft_r(double2 *v);
-template <> __device__ __forceinline__ void dft_r<2>(double2 *v) { dft2(v); }
-template <> __device__ __forceinline__ void dft_r<4>(double2 *v) { dft4(v[0], v[1], v[2], v[3]); }
-template <> __device__ __forceinline__ void dft_r<8>(double2 *v) { dft8(v); }
-
-// Largest radix used by the FFT passes (4: five passes for N = 512).
-#ifndef N4_FFT_MAX_RADIX
-#define N4_FFT_MAX_RADIX 4
-#endif
-__device__ __forceinline__ int fft_radix(int rem) {
-  return (N4_FFT_MAX_RADIX >= 8 && rem % 8 == 0) ? 8 : (rem % 4 == 0 ? 4 : 2);
-}
-
-// First Stockham pass (Ns = 1: every twiddle is 1) of an FFT whose input
-// x[i] = in(i) is produced on the fly, so that the elementwise step before an
-// FFT needs no pass and no barrier of its own.
-template <int R, class In>
-__device__ void stockham_first(const In &in, double2 *y, int N) {
-  const int T = N / R;
-  for (int j = threadIdx.x; j < T; j += blockDim.x) {
-    double2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = in(j + r * T);
-    dft_r<R>(v);
-#pragma unroll
-    for (int r = 0; r < R; ++r) y[j * R + r] = v[r];
-  }
-}
-
-// Forward FFT (length N = 2^m, 4 <= N <= 4096) of in(0..N): first pass into
-// a, then the remaining passes ping-ponging a and b, each ending with a CTA
-// barrier.  Returns the buffer that holds the result.
-template <class In>
-__device__ double2 *fft_from(const In &in, double2 *a, double2 *b, int N, const double2 *tw) {
-  const int R0 = fft_radix(N);
-  if (R0 == 8) stockham_first<8>(in, a, N);
-  else if (R0 == 4) stockham_first<4>(in, a, N);
-  else stockham_first<2>(in, a, N);
   __syncthreads();
-  int Ns = R0, rem = N / R0;
-  while (rem > 1) {
-    const int R = fft_radix(rem);
-    if (R == 8) stockham_pass<8>(a, b, N, Ns, tw);
-    else if (R == 4) stockham_pass<4>(a, b, N, Ns, tw);
-    else stockham_pass<2>(a, b, N, Ns, tw);
-    __syncthreads();
-    double2 *t = a; a = b; b = t;
-    Ns *= R;
-    rem /= R;
+}
+
+// Forward FFT (length N = 2^m, 4 <= N <= 4096) of in(0..N): radix 4, the last
+// pass radix 2 where N is no power of 4; the first pass goes to a, the others
+// ping-pong a and b, each ending with a CTA barrier.  Returns the buffer that
+// holds the result.  (Radix 8 needs more registers than the engine's kernels
+// have left.)  NC: N where it is known at compile time (512, up to 256 bins:
+// the passes' strides and twiddle steps become constants), else 0.
+template <int NC, class In>
+__device__ __forceinline__ double2 *fft_from(const In &in, double2 *a, double2 *b, int N, const double2 *tw) {
+  auto from = [](const double2 *x) { return [x](int i) { return x[i]; }; };
+  if constexpr (NC == 512) {
+    stockham_pass<4>(in, a, 512, 1, tw);
+    stockham_pass<4>(from(a), b, 512, 4, tw);
+    stockham_pass<4>(from(b), a, 512, 16, tw);
+    stockham_pass<4>(from(a), b, 512, 64, tw);
+    stockham_pass<2>(from(b), a, 512, 256, tw);
+    return a;
+  } else {
+    const int R0 = N % 4 == 0 ? 4 : 2;
+    if (R0 == 4) stockham_pass<4>(in, a, N, 1, tw);
+    else stockham_pass<2>(in, a, N, 1, tw);
+    for (int Ns = R0, rem = N / R0; rem > 1;) {
+      const int R = rem % 4 == 0 ? 4 : 2;
+      if (R == 4) stockham_pass<4>(from(a), b, N, Ns, tw);
+      else stockham_pass<2>(from(a), b, N, Ns, tw);
+      double2 *t = a; a = b; b = t;
+      Ns *= R;
+      rem /= R;
+    }
+    return a;
   }
-  return a;
 }
 
 // ---------------------------------------------------------------- sharpening
 struct SharpenBufs {
   double2 *a, *b;    // [N] work buffers
   double2 *tw;       // [N] twiddles (filled by the caller once)
-  double *Ff;        // [N] real Fourier transform of the Gaussian
+  double *Ff;        // [N/2 + 1] the Gaussian, then its real Fourier transform
 };
 
-// E[0..bins) from the fractional histogram (bin b's weight hv(b)) (N4.py:32-101,
-// cudaN4.cu:733-817), all in FP64; all threads of the CTA call it.  Four FFTs;
-// each elementwise step is folded into the first pass of the FFT after it.
-// R2 (optional): the residual table of residual_lin, R2[b] for b < bins - 1.
-template <class HistF>
-__device__ void sharpen_map(const HistF &hv, int bins, int N, int off, double binMin, double slope,
-                            double wiener, double fwhm, const SharpenBufs &sb, double *E, float2 *R2 = nullptr) {
+// The Gaussian's height and exponent per squared bin for a bin width `slope`.
+struct Gauss {
+  double scale, exponent;
+};
+__device__ __forceinline__ Gauss gauss_of(double slope, double fwhm) {
   const double ln2 = 0.69314718055994530942;
   const double scaledFWHM = fwhm / slope;
-  const double expFactor = 4.0 * ln2 / (scaledFWHM * scaledFWHM);
-  const double scaleFactor = 2.0 * sqrt(ln2 / 3.14159265358979323846) / scaledFWHM;
+  return Gauss{2.0 * sqrt(ln2 / 3.14159265358979323846) / scaledFWHM, 4.0 * ln2 / (scaledFWHM * scaledFWHM)};
+}
+
+// E[0..bins) from the fractional histogram (bin b's weight hv(b)) (N4.py:32-101,
+// cudaN4.cu:733-817), all in FP64; all threads of the CTA call it.  Four FFTs.
+// The steps with an exponential or a division go over all threads of the CTA,
+// one value each, and use the symmetry of real inputs (index k stands for
+// N - k too): inside an FFT's first pass, on its N/4 threads, four of them
+// would follow one another in every thread.  R2 (optional): the residual table
+// of residual_lin, R2[b] for b < bins - 1.
+template <int NC, class HistF>
+__device__ __forceinline__ void sharpen_map_n(const HistF &hv, int bins, int N, int off, double binMin, double slope,
+                                              double wiener, const Gauss &ga, const SharpenBufs &sb, double *E,
+                                              float2 *R2) {
   const double invN = 1.0 / (double)N;
-  // the periodic Gaussian's N/2 + 1 distinct values, one per thread of the
-  // CTA (the first FFT pass has only N/4 threads busy), held in sb.Ff until
-  // the second FFT overwrites it with the transform
+  // the periodic Gaussian's N/2 + 1 distinct values, held in sb.Ff until the
+  // transform takes their place
   for (int d = threadIdx.x; d <= N / 2; d += blockDim.x)
-    sb.Ff[d] = scaleFactor * exp(-(double)d * (double)d * expFactor);
+    sb.Ff[d] = ga.scale * exp(-(double)d * (double)d * ga.exponent);
   __syncthreads();
   // z = V + i F : the padded histogram and the periodic Gaussian in one FFT
-  double2 *Z = fft_from(
+  double2 *Z = fft_from<NC>(
       [&](int i) {
-        const int d = i <= N / 2 ? i : N - i;
-        const double F = sb.Ff[d];
+        const double F = sb.Ff[i <= N / 2 ? i : N - i];
         const double V = (i >= off && i < off + bins) ? hv(i - off) : 0.0;
         return make_double2(V, F);
       },
@@ -361,19 +340,21 @@ __device__ void sharpen_map(const HistF &hv, int bins, int N, int off, double bi
   double2 *W = (Z == sb.a) ? sb.b : sb.a;
   // split the packed transform; Wiener filter Re(conj(Ff)/(|Ff|^2 + w)) with
   // Ff real; conj(Uf), so that the forward FFT inverts
-  double2 *Y = fft_from(
-      [&](int k) {
-        const double2 zk = Z[k], zn = Z[(N - k) & (N - 1)];
-        const double2 Vf = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
-        const double Ff = 0.5 * (zk.y + zn.y);
-        const double g = Ff / (Ff * Ff + wiener);
-        sb.Ff[k] = Ff;
-        return make_double2(Vf.x * g, -Vf.y * g);
-      },
-      W, Z, N, sb.tw);
+  for (int k = threadIdx.x; k <= N / 2; k += blockDim.x) {
+    const int kn = (N - k) & (N - 1);
+    const double2 zk = Z[k], zn = Z[kn];
+    const double2 Vf = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
+    const double Ff = 0.5 * (zk.y + zn.y);
+    const double g = Ff / (Ff * Ff + wiener);
+    sb.Ff[k] = Ff;
+    W[kn] = make_double2(Vf.x * g, Vf.y * g);
+    W[k] = make_double2(Vf.x * g, -Vf.y * g);
+  }
+  __syncthreads();
+  double2 *Y = fft_from<NC>([&](int k) { return W[k]; }, Z, W, N, sb.tw);
   double2 *Y2 = (Y == W) ? Z : W;
   // U = max(Re(ifft(Uf)), 0); pack the numerator c_i U_i (real) and U (imaginary)
-  double2 *P = fft_from(
+  double2 *P = fft_from<NC>(
       [&](int i) {
         const double U = fmax(Y[i].x * invN, 0.0);
         const double c = binMin + (double)(i - off) * slope;
@@ -382,25 +363,34 @@ __device__ void sharpen_map(const HistF &hv, int bins, int N, int off, double bi
       Y2, Y, N, sb.tw);
   double2 *P2 = (P == Y2) ? Y : Y2;
   // Gaussian smoothing of both: multiply by the (real) Ff, inverse transform
-  double2 *S = fft_from(
+  double2 *S = fft_from<NC>(
       [&](int k) {
         const double2 v = P[k];
-        const double f = sb.Ff[k];
+        const double f = sb.Ff[k <= N / 2 ? k : N - k];
         return make_double2(v.x * f, -v.y * f);
       },
       P2, P, N, sb.tw);
-  auto e_at = [&](int b) {
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) {
     const double2 v = S[off + b];
     const double nu = v.x * invN, de = -v.y * invN;
-    return (de != 0.0) ? nu / de : 0.0;
-  };
-  for (int b = threadIdx.x; b < bins; b += blockDim.x) {
-    const double e = e_at(b);
-    E[b] = e;
-    if (R2 && b + 1 < bins)
-      R2[b] = make_float2((float)(binMin + (double)b * slope - e), (float)(slope - (e_at(b + 1) - e)));
+    E[b] = (de != 0.0) ? nu / de : 0.0;
   }
   __syncthreads();
+  if (R2) {
+    for (int b = threadIdx.x; b + 1 < bins; b += blockDim.x) {
+      const double e = E[b];
+      R2[b] = make_float2((float)(binMin + (double)b * slope - e), (float)(slope - (E[b + 1] - e)));
+    }
+    __syncthreads();
+  }
+}
+
+template <class HistF>
+__device__ __forceinline__ void sharpen_map(const HistF &hv, int bins, int N, int off, double binMin, double slope,
+                                            double wiener, const Gauss &ga, const SharpenBufs &sb, double *E,
+                                            float2 *R2 = nullptr) {
+  if (N == 512) sharpen_map_n<512>(hv, bins, 512, off, binMin, slope, wiener, ga, sb, E, R2);
+  else sharpen_map_n<0>(hv, bins, N, off, binMin, slope, wiener, ga, sb, E, R2);
 }
 
 // Float-float arithmetic (a value as the unevaluated sum of two floats, ~48
@@ -420,11 +410,11 @@ __device__ __forceinline__ float two_sum(float a, float b, float &err) {
 // itself is taken, because there one ulp decides whether the reference
 // counts or drops the maximum voxel (N4.py:27).
 //
-// coord_ff gives the same coordinate from float-float arithmetic as a bin k
-// and a fraction f (|error| < 2^-24, the resolution of the histogram's fixed
-// point): d = x - binMin exactly by TwoSum (binMin is the minimum of FP32
-// values, a float), times 1/slope held as a float-float.  It declines values
-// within two bins of the top, which take the FP64 path.
+// coord_split (below) gives the same coordinate from float-float arithmetic
+// as a bin k and a fraction f (|error| < 2^-24, the resolution of the
+// histogram's fixed point): d = x - binMin exactly by TwoSum (binMin is the
+// minimum of FP32 values, a float), times 1/slope held as a float-float.  It
+// declines values within two bins of the top, which take the FP64 path.
 struct BinMap {
   double binMin, slope, inv_slope, top;
   float fmin, ih, il, ff_limit;
@@ -436,22 +426,29 @@ struct BinMap {
     const double c = d * inv_slope;
     return c > top ? d / slope : c;
   }
-  __device__ __forceinline__ bool coord_ff(float x, int &k, float &f) const {
-    float dl;
-    const float dh = two_sum(x, -fmin, dl);                  // x - binMin = dh + dl exactly
-    const float p = __fmul_rn(dh, ih);
-    const float pe = __fmaf_rn(dh, ih, -p);                  // p + pe = dh * ih exactly
-    const float cl = __fadd_rn(pe, __fmaf_rn(dh, il, __fmul_rn(dl, ih)));
-    if (!(p < ff_limit)) return false;                       // near the top bin (or NaN)
-    const float kf = floorf(p);
-    f = __fadd_rn(__fsub_rn(p, kf), cl);                     // p - kf is exact
-    k = (int)kf;
-    if (f < 0.0f) { f = __fadd_rn(f, 1.0f); --k; }
-    else if (f >= 1.0f) { f = __fsub_rn(f, 1.0f); ++k; }
-    if (k < 0) { k = 0; f = 0.0f; }                          // x >= binMin: only rounding reaches here
-    return true;
-  }
 };
+
+// The same coordinate in float-float arithmetic, from the map's fields fmin,
+// ih + il and ff_limit: the bin k and the fraction f of x, or false within
+// two bins of the top and for a NaN (k = 0, f = 0: in range of every table).
+// Branch-free, so that several voxels' chains overlap.
+__device__ __forceinline__ bool coord_split(float x, float fmin, float ih, float il, float limit, int &k, float &f) {
+  float dl;
+  const float dh = two_sum(x, -fmin, dl);                  // x - binMin = dh + dl exactly
+  const float p = __fmul_rn(dh, ih);
+  const float pe = __fmaf_rn(dh, ih, -p);                  // p + pe = dh * ih exactly
+  const float cl = __fadd_rn(pe, __fmaf_rn(dh, il, __fmul_rn(dl, ih)));
+  const bool in = p < limit;                               // not near the top bin (or NaN)
+  const float kf = floorf(p);
+  float fr = __fadd_rn(__fsub_rn(p, kf), cl);              // p - kf is exact
+  int kk = (int)kf;
+  if (fr < 0.0f) { fr = __fadd_rn(fr, 1.0f); --kk; }
+  else if (fr >= 1.0f) { fr = __fsub_rn(fr, 1.0f); ++kk; }
+  const bool ok = in && kk >= 0;                           // x >= binMin: only rounding gives kk < 0
+  k = ok ? kk : 0;
+  f = ok ? fr : 0.0f;
+  return in;
+}
 
 // exp(x) - 1 of a convergence term (N4.py:121-126): for |x| < 1/4 its Taylor
 // series through x^7 / 7! in Horner form, x + x^2 (1/2! + x (1/3! + ...)),
@@ -489,29 +486,12 @@ __device__ __forceinline__ int hist_bin(double c, int bins, double scale, unsign
   return -1;                                             // the reference drops it
 }
 
-// hist_bin from a coordinate given as bin k (< bins - 1) and fraction f.
-__device__ __forceinline__ int hist_bin_ff(int k, float f, double scale, unsigned &qlo, unsigned &qhi) {
-  const unsigned one = (unsigned)scale;
-  if (f == 0.0f) { qlo = one; qhi = 0u; return k; }
-  qhi = min(__float2uint_rn(__fmul_rn(f, (float)scale)), one);
-  qlo = one - qhi;
-  return k;
-}
-
 // The FP64 path of a value near the top bin, out of line: inlined, the
-// compiler may evaluate it for every value under a predicate.
-__device__ __noinline__ int hist_bin_top(const BinMap &bm, float x, int bins, double scale, unsigned &qlo,
+// compiler may evaluate it for every value under a predicate.  `bm` is in
+// shared memory.
+__device__ __noinline__ int hist_bin_top(const BinMap *bm, float x, int bins, double scale, unsigned &qlo,
                                          unsigned &qhi) {
-  return hist_bin(bm.coord(x), bins, scale, qlo, qhi);
-}
-
-// Histogram contribution of one value: float-float below the top two bins.
-__device__ __forceinline__ int hist_bin_of(const BinMap &bm, float x, int bins, double scale, unsigned &qlo,
-                                           unsigned &qhi) {
-  int k;
-  float f;
-  if (bm.coord_ff(x, k, f)) return hist_bin_ff(k, f, scale, qlo, qhi);
-  return hist_bin_top(bm, x, bins, scale, qlo, qhi);
+  return hist_bin(bm->coord(x), bins, scale, qlo, qhi);
 }
 
 // Largest shift <= 24 for which `n` voxels cannot overflow a 32-bit bin.
@@ -560,23 +540,12 @@ __device__ __forceinline__ float residual_lin(int k, float f, const float2 *R2) 
   return __fmaf_rn(f, t.y, t.x);
 }
 
-// The FP64 residual of a value near the top bin, out of line: inlined, the
-// compiler may evaluate it for every value under a predicate.
-__device__ __noinline__ float residual_top(const BinMap &bm, float x, const double *E, int bins) {
-  return (float)((double)x - sharpened_value(bm.coord(x), E, bins));
-}
-
-// Residual x - E(x) of a masked value (N4.py:107-113): the bin and fraction
-// from the float-float coordinate, then the bin's linear form; FP64 in the
-// top two bins.  (An FP32 coordinate, error ~2^-24 c, moved the lattice of a
+// The FP64 residual of a value near the top bin, out of line as above.  (An
+// FP32 coordinate for the others, error ~2^-24 c, moved the lattice of a
 // 32x32x24 volume after 2 x 4 iterations by 1.4e-4 relative, measured with
 // the oracle: the bound is 1e-4.)
-__device__ __forceinline__ float residual_of(const BinMap &bm, float x, const float2 *R2, const double *E,
-                                             int bins) {
-  int k;
-  float f;
-  if (bm.coord_ff(x, k, f)) return residual_lin(k, f, R2);
-  return residual_top(bm, x, E, bins);
+__device__ __noinline__ float residual_top(const BinMap *bm, float x, const double *E, int bins) {
+  return (float)((double)x - sharpened_value(bm->coord(x), E, bins));
 }
 
 // Refined lattice value at output index (ox, oy, oz) (array indices), from
@@ -618,39 +587,36 @@ __device__ void refine_lattice(const float *L, int ncx, int ncy, int ncz, float 
 }
 
 // ---------------------------------------------------------------- grid barrier
-// Sense-counting barrier over all CTAs of a cooperative launch.  Every wait
+// Barrier over all CTAs of a cooperative launch: arrivals are counted up
+// from zero, and a CTA waits until the count reaches the end of its own
+// round.  One release-add and one acquire-poll per CTA and round.  Every wait
 // is bounded: on timeout (or when another CTA already failed) it records
 // N4_ERR_TIMEOUT in *err and returns false.
 struct GridBarrier {
   unsigned *count;
-  unsigned *gen;
   int *err;
   unsigned nblocks;
 
   __device__ bool sync() const {
-    __syncthreads();
     __shared__ int s_ok;
+    __syncthreads();
     if (threadIdx.x == 0) {
-      volatile unsigned *vgen = gen;
-      volatile int *verr = err;
-      int ok = (*verr == 0);
-      unsigned g0 = *vgen;
+      unsigned t;
       __threadfence();
-      unsigned t = atomicAdd(count, 1u);
-      if (t == nblocks - 1) {
-        atomicExch(count, 0u);
-        __threadfence();
-        atomicAdd(gen, 1u);
-      } else {
-        unsigned long long spins = 0;
-        while (*vgen == g0) {
-          if (*verr != 0) { ok = 0; break; }
-          if (++spins > kSpinLimit) { atomicExch(err, (int)N4_ERR_TIMEOUT); ok = 0; break; }
-          __nanosleep(64);
-        }
+      asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(count) : "memory");
+      const unsigned end = t / nblocks * nblocks + nblocks;   // the round this arrival belongs to
+      unsigned long long spins = 0;
+      int ok = 1;
+      for (;;) {
+        unsigned c;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+        if ((int)(c - end) >= 0) break;
+        ++spins;
+        if ((spins & 255u) == 0 && *(volatile int *)err != 0) { ok = 0; break; }
+        if (spins > kSpinLimit) { atomicExch(err, (int)N4_ERR_TIMEOUT); ok = 0; break; }
       }
       __threadfence();
-      s_ok = ok && (*verr == 0);
+      s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;

@@ -4,9 +4,10 @@
 // A group is either a thread-block cluster (the volume lives in the
 // cluster's distributed shared memory; partials are exchanged through DSMEM;
 // hardware cluster barriers) or the whole grid of a cooperative launch (the
-// volume lives in global memory/L2; partials are exchanged through global
-// memory; a bounded software barrier).  The algorithm below is written once
-// for both.
+// masked part of the volume lives in the SMs' shared memory as far as it
+// fits, the rest in global memory/L2; partials are exchanged by integer
+// atomics in global memory; a bounded software barrier).  The algorithm below
+// is written once for both.
 //
 // Per level, with L the control lattice, D its last update and Gd = rows(D)
 // the per-row partial evaluation of D (x/y contracted, one value per z
@@ -22,10 +23,17 @@
 // logU follows L by the same updates, applied per voxel: eval is linear, so
 // logU = im_log - eval(rows(L)) up to FP32 rounding, which the reset at every
 // level start clears.
+//
+// Rows.  A row of the fitting grid is kept as the range [z0, z1) from its
+// first to its last masked voxel; a CTA works on the list of its rows that
+// have one (an ellipsoid mask leaves 36 % of the rows out and fills 60 % of
+// the others).  2^sg lanes share a row; in the passes that follow the
+// lattice's spans along z, a lane takes one span of the row or, with fewer
+// spans than lanes, an equal part of it, so that a row's voxels are taken a
+// few per lane instead of one after the other in one thread.
 #pragma once
 #include <cooperative_groups.h>
 #include <new>
-#include <type_traits>
 
 #include "n4_device.cuh"
 
@@ -33,44 +41,69 @@ namespace cg = cooperative_groups;
 
 namespace n4 {
 
-// Fixed-point scale 2^shift of one volume's histogram: the largest shift
-// (<= 24) for which no 32-bit bin of a histogram copy can overflow.  A copy
-// (one per 8th warp) receives at most an 8th of a CTA's voxels plus 160.  It
-// depends on the volume and the group size alone (not on the other volumes of
-// a batch), so a volume gets bitwise the same result in any batch.
-__host__ __device__ inline int volume_hist_shift(int X, int Y, int Z, int K, bool grid) {
-  const long long rows = (long long)X * Y;
-  const long long rpc = grid ? (rows + K - 1) / K : ((long long)X + K - 1) / K * Y;
-  return hist_shift_for((rpc * Z + 7) / 8 + 160);
-}
-
-// Voxels (or rows) whose loads a thread issues together in the voxel passes:
-// 4 on the whole-GPU path, whose rows are read from L2/HBM; 1 on the cluster
-// path, whose rows are in shared memory (measured: batching there only adds
-// registers and instructions).
-template <bool Grid> struct RowBatch { static constexpr int n = Grid ? 4 : 1; };
 #define kNaN __int_as_float(0x7fc00000)
 
+// Work of one row in the whole-GPU path's partition: its voxels and what it
+// costs beside them.  The floor keeps a CTA of many short rows within the
+// row buffers (grid_rows_bound).
+__host__ __device__ inline int grid_row_overhead(int Z) { return Z / 8 > 16 ? Z / 8 : 16; }
+// Most rows, and most voxels, the partition gives one of K CTAs.
+__host__ __device__ inline long long grid_rows_bound(long long rows, int Z, int K) {
+  const int c = grid_row_overhead(Z);
+  return (rows * (Z + c) / K + Z + c) / (1 + c) + 2;
+}
+__host__ __device__ inline long long grid_voxels_bound(long long rows, int Z, int K) {
+  const int c = grid_row_overhead(Z);
+  return rows * (Z + c) / K + 2ll * (Z + c);
+}
+// log2 of the lanes that share a row outside the span passes (the histogram)
+__host__ __device__ inline int row_lanes_log2(int Z) { return Z <= 64 ? 3 : (Z <= 256 ? 4 : 5); }
+
 // ------------------------------------------------------------------ layout
-// Byte offsets of one CTA's workspace.  "sm" offsets are always in shared
-// memory; "big" offsets are in shared memory for the cluster path and in a
-// per-CTA slice of global memory for the grid path.
+// One axis of the fitting grid at one level, in the CTA's dynamic shared
+// memory: byte offsets of the span index and the weights of every voxel
+// (B0..B3, the fit's numerator weights w^3 / sum w^2 and denominator weights
+// w^2) and of the spans' voxel ranges.
+struct EAxis {
+  int n, nc, nsp;
+  int o_s, o_w, o_p, o_q, o_lo, o_hi;
+};
+__host__ __device__ inline size_t eaxis_bytes(int n, int nsp) {
+  return ((size_t)n * 4 + 15) / 16 * 16 + (size_t)n * 48 + ((size_t)nsp * 8 + 15) / 16 * 16;
+}
+__host__ __device__ inline EAxis eaxis_at(int off, int n, int nc) {
+  EAxis a;
+  a.n = n; a.nc = nc; a.nsp = nc - 3;
+  a.o_w = off;
+  a.o_p = a.o_w + n * 16;
+  a.o_q = a.o_p + n * 16;
+  a.o_s = a.o_q + n * 16;
+  a.o_lo = a.o_s + (n * 4 + 15) / 16 * 16;
+  a.o_hi = a.o_lo + a.nsp * 4;
+  return a;
+}
+
+// Byte offsets of one CTA's workspace: "o_" offsets in dynamic shared memory;
+// "b_" offsets in dynamic shared memory behind sm_bytes (cluster path) or in
+// a per-CTA slice of global memory (whole-GPU path).
 struct Plan {
   // limits
   int levels, nc0x, nc0y, nc0z, NCX, NCY, NCZ, NLAT;
   int Xmax, Ymax, Zmax, slab_floats, rows_max, nvxl;
   int bins, npad, hoff;
   // shared
-  int o_ax, o_ay, o_az, o_L, o_D, o_den, o_tmp, o_aux, o_hist, o_H64, o_R2, o_E;
-  int o_fa, o_fb, o_tw, o_ff, o_red, o_misc;
+  int o_ax, o_ay, o_az, o_L, o_D, o_den, o_tmp, o_aux, o_H64, o_R2, o_E;
+  int o_tw, o_red, o_rows, o_ytab;
+  // whole-GPU path: the shared homes of Gd (also the FFT's), of T2 and of the
+  // row list and slab, used as far as a volume fits them
+  int o_gd, gd_bytes, o_t2, t2_bytes, o_pool, pool_bytes;
   int sm_bytes;
   // big
-  int b_imlog, b_Gd, b_T2, b_slotA, b_slotB, b_slotC, b_slice, big_bytes;
-  // cluster path: the FFT work buffers, the histogram copies and the
-  // Gaussian's transform (which the sharpening writes after the copies are
-  // merged, over them) live in the Gd region, dead from the end of pass A
-  // until the update, at these offsets
-  int alias_sharpen, a_fa, a_fb, a_hist, a_ff;
+  int b_imlog, b_Gd, b_T2, b_ytab, b_rows, b_slotA, b_slotB, b_slotC, big_bytes;
+  // the FFT work buffers, the histogram copies and the Gaussian's transform
+  // (which the sharpening writes after the copies are merged, over them) live
+  // in the Gd region, dead from the end of pass A until the fit, at these offsets
+  int a_fa, a_fb, a_hist, a_ff;
 };
 
 struct Params {
@@ -92,6 +125,17 @@ struct VolJob {
 // Statistics exchanged after pass A: min, max, sum y, sum y^2.
 struct Stats { double v[4]; };
 
+// What the passes of one iteration need from the statistics, in the CTA's
+// shared memory (o_red, after the reduction scratch).
+struct Iter {
+  double st[4];     // group min, max, sum y, sum y^2
+  BinMap bm;
+  double scale;     // 2^hshift
+  Gauss gauss;
+  int degenerate;   // no bin range: nothing to fit
+  float cv;
+};
+
 // ------------------------------------------------------------------ groups
 struct ClusterGroup {
   __device__ int rank() const { return (int)cg::this_cluster().block_rank(); }
@@ -100,14 +144,20 @@ struct ClusterGroup {
   template <class T> __device__ const T *peer(const T *p, int r) const {
     return cg::this_cluster().map_shared_rank(const_cast<T *>(p), r);
   }
-  template <class T> __device__ T load(const T *p) const { return *p; }
   static constexpr bool kGrid = false;
 };
 
+// Accumulators of the whole-GPU path in global memory, zero at launch: three
+// sets used in turn (one is cleared while the next is in use), each `len`
+// words for the histogram or the lattice sums, the last word a count of
+// partials that are not numbers.
 struct GridGroup {
   GridBarrier bar;
   char *big_base;      // per-CTA big regions, stride big_stride
   size_t big_stride;
+  unsigned long long *acc;   // [3][len]
+  int len;
+  unsigned *ext;       // [X*Y] row ranges z0 | z1 << 16 (0: no masked voxel)
   __device__ int rank() const { return (int)blockIdx.x; }
   __device__ int size() const { return (int)gridDim.x; }
   __device__ bool sync() const { return bar.sync(); }
@@ -115,7 +165,6 @@ struct GridGroup {
     const char *mine = big_base + (size_t)blockIdx.x * big_stride;
     return (const T *)(big_base + (size_t)r * big_stride + ((const char *)p - mine));
   }
-  template <class T> __device__ T load(const T *p) const { return __ldcg(p); }
   static constexpr bool kGrid = true;
 };
 
@@ -136,7 +185,7 @@ struct GridGroup {
 #else
 #define N4_MARK(k) do { } while (0)
 #endif
-enum { PH_SETUP, PH_A, PH_B, PH_SHARP, PH_C, PH_FIT, PH_UPDATE, PH_A_LOOP, PH_A_RED, PH_B_ZERO, PH_B_LOOP, PH_B_MERGE,
+enum { PH_SETUP, PH_A, PH_SHARP, PH_UPDATE, PH_A_LOOP, PH_A_RED, PH_B_LOOP, PH_B_MERGE,
        PH_B_RED, PH_F_T1, PH_F_T2, PH_F_P, PH_F_RED, PH_N };
 #ifdef N4_PHASE_TIMERS
 __shared__ long long ph_acc[PH_N + 1];   // per-phase cycles, then the last mark
@@ -146,15 +195,12 @@ __shared__ long long ph_acc[PH_N + 1];   // per-phase cycles, then the last mark
 // The Engine's fields are uniform over the CTA.  Whole-GPU path: one object
 // per CTA in shared memory (EngineSlot), its fields written by thread 0 only
 // (construction, run, set_level, each followed by a barrier); held in
-// registers, the ~50 fields (pointers of the axis tables and work arrays)
-// stay live through every pass and push the voxel loops into local-memory
-// spills (measured: 512x512x320 in 6.2 ms instead of 6.5).  Cluster path: one
-// object per thread, every thread writing its own copy (measured: the shared
-// object made the 256x256x176 batch 11 % slower, its loops reloading fields
-// after every shared-memory store or atomic).
+// registers, the fields stay live through every pass and push the voxel loops
+// into local-memory spills.  Cluster path: one object per thread, every thread
+// writing its own copy (a shared object made the loops reload fields after
+// every shared-memory store or atomic).
 template <class Group>
 struct Engine {
-  static constexpr int kRB = RowBatch<Group::kGrid>::n;
   static constexpr bool kShared = Group::kGrid;   // the object lives in shared memory
   // the threads that write the fields, and the barrier that publishes them
   __device__ __forceinline__ bool writer() const { return !kShared || threadIdx.x == 0; }
@@ -162,50 +208,104 @@ struct Engine {
   Group g;
   const Plan &pl;
   const Params &pr;
-  char *sm;
-  char *big;
-  float *red_global;   // grid path: [NLAT] / [bins] slice-reduction buffer
+  char *big;           // whole-GPU path: this CTA's slice of global memory
   // volume
-  int X, Y, Z, nrow, rank, K;
-  // rows of this CTA: grid path, contiguous rows r0 + rl; cluster path,
-  // whole x-planes vx = rank + m * K (m = rl / Y), interleaved over the group
-  int r0, nplane;
-  int hshift;   // fixed-point scale of this volume's histogram
-  FastDiv divZ;
-  float *logu;         // [nrow][Z] logU of the local rows (NaN outside the mask)
+  int X, Y, Z, rank, K;
+  int nact;            // rows of this CTA with a masked voxel
+  int vx0, np;         // its x-planes: cluster, vx = rank + m * K; whole-GPU path, vx = vx0 + m; m < np
+  int hshift;          // fixed-point scale of this volume's histogram
+  int seq;             // whole-GPU path: group sums so far
+  double nfg;          // masked voxels of the volume
   const float *src;    // the job's log volume (global memory), read by reset
   // level
   int ncx, ncy, ncz, nlat;
-  Axis ax, ay, az;
-  // smem views
-  float *L, *D, *den, *tmp, *aux;
-  double *E, *Ff;
-  float2 *R2;          // the residual's per-bin linear form (residual_lin)
-  unsigned *hist;
-  unsigned long long *H64;
-  double2 *fa, *fb, *tw;
-  double *red;
-  float *Gd, *T2, *slotC;
-  Stats *slotA;
-  unsigned long long *slotB;
+  int sg, sh;          // pass A: log2 of the lanes per row and per span of it
+  int sz, szh;         // z contraction: the same
+  int tp;              // x-planes T2 holds at a time
+  EAxis ax, ay, az;
+  // whole-GPU path: where the volume's buffers are (shared memory or the slice)
+  float *gdp, *t2p, *slab_g;
+  int *ytabp;
+  int4 *rowsp;
+  int slab_off, slab_cap;
 
-  __device__ Engine(const Group &g_, const Plan &p, const Params &r, char *sm_, char *big_, float *rg)
-      : g(g_), pl(p), pr(r), sm(sm_), big(big_), red_global(rg) {
-    L = (float *)(sm + pl.o_L); D = (float *)(sm + pl.o_D); den = (float *)(sm + pl.o_den);
-    tmp = (float *)(sm + pl.o_tmp); aux = (float *)(sm + pl.o_aux);
-    hist = (unsigned *)(sm + pl.o_hist); H64 = (unsigned long long *)(sm + pl.o_H64);
-    R2 = (float2 *)(sm + pl.o_R2); E = (double *)(sm + pl.o_E);
-    fa = (double2 *)(sm + pl.o_fa); fb = (double2 *)(sm + pl.o_fb); tw = (double2 *)(sm + pl.o_tw);
-    Ff = (double *)(sm + pl.o_ff); red = (double *)(sm + pl.o_red);
-    Gd = (float *)(big + pl.b_Gd); T2 = (float *)(big + pl.b_T2);
-    logu = (float *)(big + pl.b_imlog);
-    if (pl.alias_sharpen) {
-      fa = (double2 *)(big + pl.b_Gd + pl.a_fa); fb = (double2 *)(big + pl.b_Gd + pl.a_fb);
-      hist = (unsigned *)(big + pl.b_Gd + pl.a_hist);
-      Ff = (double *)(big + pl.b_Gd + pl.a_ff);
+  __device__ Engine(const Group &g_, const Plan &p, const Params &r, char *big_) : g(g_), pl(p), pr(r), big(big_) {
+    seq = 0;
+  }
+
+  // ---- memory
+  static __device__ __forceinline__ char *dyn() {
+    extern __shared__ __align__(128) char smem[];
+    return smem;
+  }
+  template <class T> static __device__ __forceinline__ T *at(int off) { return (T *)(dyn() + off); }
+  __device__ __forceinline__ float *L() const { return at<float>(pl.o_L); }
+  __device__ __forceinline__ float *D() const { return at<float>(pl.o_D); }
+  __device__ __forceinline__ float *den() const { return at<float>(pl.o_den); }
+  __device__ __forceinline__ float *tmp() const { return at<float>(pl.o_tmp); }
+  __device__ __forceinline__ float *aux() const { return at<float>(pl.o_aux); }
+  __device__ __forceinline__ double *red() const { return at<double>(pl.o_red); }
+  __device__ __forceinline__ Iter &iter() const { return *at<Iter>(pl.o_red + 144 * 8); }
+  __device__ __forceinline__ double *E() const { return at<double>(pl.o_E); }
+  __device__ __forceinline__ float2 *R2() const { return at<float2>(pl.o_R2); }
+  __device__ __forceinline__ unsigned long long *H64() const { return at<unsigned long long>(pl.o_H64); }
+  __device__ __forceinline__ int alias0() const { return Group::kGrid ? pl.o_gd : pl.sm_bytes + pl.b_Gd; }
+  __device__ __forceinline__ unsigned *hist() const { return at<unsigned>(alias0() + pl.a_hist); }
+  __device__ __forceinline__ float *Gd() const {
+    if constexpr (Group::kGrid) return gdp;
+    else return at<float>(pl.sm_bytes + pl.b_Gd);
+  }
+  __device__ __forceinline__ float *T2() const {
+    if constexpr (Group::kGrid) return t2p;
+    else return at<float>(pl.sm_bytes + pl.b_T2);
+  }
+  __device__ __forceinline__ int *ytab() const {
+    if constexpr (Group::kGrid) return ytabp;
+    else return at<int>(pl.o_ytab);
+  }
+  __device__ __forceinline__ Stats *slotA() const {
+    if constexpr (Group::kGrid) return (Stats *)(big + pl.b_slotA);
+    else return at<Stats>(pl.sm_bytes + pl.b_slotA);
+  }
+  __device__ __forceinline__ unsigned long long *slotB() const {
+    if constexpr (Group::kGrid) return (unsigned long long *)(big + pl.b_slotB);
+    else return at<unsigned long long>(pl.sm_bytes + pl.b_slotB);
+  }
+  __device__ __forceinline__ float *slotC() const { return at<float>(pl.sm_bytes + pl.b_slotC); }   // cluster path
+
+  // ---- rows.  Row r of the CTA: its voxels [z0, z1), voxel z at p[z]; its
+  // plane m and y.
+  struct Row {
+    int z0, z1, m, vy;
+    float *p;
+  };
+  __device__ __forceinline__ Row row(int r) const {
+    Row o;
+    if constexpr (Group::kGrid) {
+      const int4 d = rowsp[r];
+      o.z0 = d.y & 0xffff; o.z1 = (int)((unsigned)d.y >> 16); o.m = d.z; o.vy = d.w;
+      o.p = (d.x + o.z1 <= slab_cap ? at<float>(slab_off) : slab_g) + d.x;
+    } else {
+      const uint2 d = at<uint2>(pl.o_rows)[r];
+      o.z0 = (int)(d.x & 0xffffu); o.z1 = (int)(d.x >> 16);
+      o.m = (int)(d.y >> 16); o.vy = (int)(d.y & 0xffffu);
+      o.p = at<float>(pl.sm_bytes + pl.b_imlog) + (o.m * Y + o.vy) * Z;
     }
-    slotA = (Stats *)(big + pl.b_slotA); slotB = (unsigned long long *)(big + pl.b_slotB);
-    slotC = (float *)(big + pl.b_slotC);
+    return o;
+  }
+  __device__ __forceinline__ int plane_vx(int m) const { return Group::kGrid ? vx0 + m : rank + m * K; }
+  __device__ __forceinline__ const float *src_row(const Row &r) const {
+    return src + ((size_t)plane_vx(r.m) * Y + r.vy) * Z;
+  }
+
+  // The part of row `r` that lane (sp, h) takes in a span pass: its span's
+  // voxels inside the row's range, cut into 2^sh equal pieces.
+  static __device__ __forceinline__ void piece(const Row &r, int lo, int hi, int h, int sh, int &a, int &b) {
+    a = max(lo, r.z0);
+    b = min(hi, r.z1);
+    const int c = (b - a + (1 << sh) - 1) >> sh;   // <= 0 when the span misses the row
+    a += h * c;
+    b = min(b, a + c);
   }
 
   // ---- level geometry
@@ -215,38 +315,90 @@ struct Engine {
       ncy = ((pl.nc0y - 3) << level) + 3;
       ncz = ((pl.nc0z - 3) << level) + 3;
       nlat = ncx * ncy * ncz;
-      ax = axis_at(sm + pl.o_ax, X, ncx);
-      ay = axis_at(sm + pl.o_ay, Y, ncy);
-      az = axis_at(sm + pl.o_az, Z, ncz);
+      ax = eaxis_at(pl.o_ax, X, ncx);
+      ay = eaxis_at(pl.o_ay, Y, ncy);
+      az = eaxis_at(pl.o_az, Z, ncz);
+      // lanes per row: 8, or enough for one per span (16 or 32 lanes of a
+      // 160-voxel row hold too little each: the z contraction at 512x512x320
+      // took 68k and 109k cycles per iteration against 48k)
+      sg = 3;
+      while (sg < 5 && (1 << sg) < az.nsp) ++sg;
+      sh = 0;
+      while (sh < sg && (az.nsp << (sh + 1)) <= (1 << sg)) ++sh;
+      // z contraction: the whole-GPU path's long rows the same way; on the
+      // cluster path a lane takes a whole span
+      sz = sg;
+      szh = sh;
+      if constexpr (!Group::kGrid) {
+        sz = szh = 0;
+        while (sz < 5 && (1 << sz) < az.nsp) ++sz;
+      }
+      if constexpr (Group::kGrid) {
+        const int slice = ncy * ncz;
+        tp = pl.t2_bytes / 4 / slice;
+        t2p = at<float>(pl.o_t2);
+        ytabp = at<int>(pl.o_ytab);
+        if (tp < 1) {
+          tp = pl.nvxl;
+          t2p = (float *)(big + pl.b_T2);
+          ytabp = (int *)(big + pl.b_ytab);
+        }
+      } else {
+        tp = max(np, 1);
+      }
     }
     publish();
-    build_axis(ax);
-    build_axis(ay);
-    build_axis(az);
+    build_eaxis(ax);
+    build_eaxis(ay);
+    build_eaxis(az);
+    __syncthreads();
+    if (np <= tp) build_ytab(0, np);
     __syncthreads();
   }
 
-  __device__ __forceinline__ void row_xy(int rl, int &vx, int &vy) const {
-    if (Group::kGrid) {
-      const int row = r0 + rl;
-      vx = row / Y;
-      vy = row - vx * Y;
-    } else {
-      const int m = rl / Y;
-      vx = rank + m * K;
-      vy = rl - m * Y;
+  static __device__ void build_eaxis(const EAxis &a) {
+    const double span = __ddiv_rn((double)a.n, (double)a.nsp);
+    for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
+      float4 w, p, q;
+      at<int>(a.o_s)[i] = axis_voxel(i, span, a.nsp, w, p, q);
+      at<float4>(a.o_w)[i] = w;
+      at<float4>(a.o_p)[i] = p;
+      at<float4>(a.o_q)[i] = q;
+    }
+    axis_ranges(a.n, a.nsp, span, at<int>(a.o_lo), at<int>(a.o_hi));
+  }
+
+  // ytab[m][sp]: first row of the CTA's list at or after the first voxel of
+  // y-span sp in plane m0 + m (sp = nspy: after the plane), so that a span's
+  // rows of a plane are ytab[m][sp] .. ytab[m][sp + 1] - 1.
+  __device__ void build_ytab(int m0, int cnt) {
+    const int w = ay.nsp + 1;
+    for (int t = threadIdx.x; t < cnt * w; t += blockDim.x) {
+      const int m = m0 + t / w, sp = t % w;
+      const int vy = sp < ay.nsp ? at<int>(ay.o_lo)[sp] : Y;
+      int lo = 0, hi = nact;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const Row r = row(mid);
+        if (r.m > m || (r.m == m && r.vy >= vy)) hi = mid;
+        else lo = mid + 1;
+      }
+      ytab()[t] = lo;
     }
   }
 
-  // ---- rows(lat) -> Gt: x/y contraction of the lattice for every local row
-  __device__ void rowtab(const float *lat, float *Gt) {
-    const int ntask = nrow * ncz;
-    for (int t = threadIdx.x; t < ntask; t += blockDim.x) {
-      const int rl = t / ncz, cz = t - rl * ncz;
-      int vx, vy;
-      row_xy(rl, vx, vy);
-      const int sx = ax.s[vx], sy = ay.s[vy];
-      const float4 wx = ax.w[vx], wy = ay.w[vy];
+  // ---- rows(lat) -> Gd: x/y contraction of the lattice for every row of the list
+  __device__ __forceinline__ int ncz_log2() const { return 32 - __clz(max(ncz - 1, 1)); }
+  __device__ void rowtab(const float *lat) {
+    const int lsh = ncz_log2();
+    float *Gt = Gd();
+    for (int t = threadIdx.x; t < (nact << lsh); t += blockDim.x) {
+      const int r = t >> lsh, cz = t & ((1 << lsh) - 1);
+      if (cz >= ncz) continue;
+      const Row o = row(r);
+      const int vx = plane_vx(o.m);
+      const int sx = at<int>(ax.o_s)[vx], sy = at<int>(ay.o_s)[o.vy];
+      const float4 wx = at<float4>(ax.o_w)[vx], wy = at<float4>(ay.o_w)[o.vy];
       const float wxa[4] = {wx.x, wx.y, wx.z, wx.w};
       const float wya[4] = {wy.x, wy.y, wy.z, wy.w};
       float acc = 0.0f;
@@ -258,483 +410,564 @@ struct Engine {
         for (int jy = 0; jy < 4; ++jy) s = __fmaf_rn(wya[jy], lp[jy * ncz], s);
         acc = __fmaf_rn(wxa[jx], s, acc);
       }
-      Gt[t] = acc;
+      Gt[r * ncz + cz] = acc;
     }
   }
 
-  // x-planes this CTA holds rows of: cluster, vx = rank + m*K for m < nplane
-  // (local rows m*Y .. m*Y + Y - 1); grid, the planes r0/Y .. (r0+nrow-1)/Y
-  __device__ __forceinline__ int nplanes_local() const {
-    if (Group::kGrid) return nrow > 0 ? (r0 + nrow - 1) / Y - r0 / Y + 1 : 0;
-    return nplane;
-  }
-  __device__ __forceinline__ int plane_vx(int m) const { return Group::kGrid ? r0 / Y + m : rank + m * K; }
-
-  // rowtab(lat, Gt) after a lattice update, through the x-contracted planes:
+  // rowtab(lat) after a lattice update, through the x-contracted planes:
   // per local x-plane, X[cy][cz] = sum_jx wx lat[sx+jx][cy][cz] (into aux,
-  // free outside the warm-start trial), then per row Gt[cz] = sum_jy wy
+  // free outside the warm-start trial), then per row Gd[cz] = sum_jy wy
   // X[sy+jy][cz]: 8 loads and multiply-adds per entry instead of 32.  Falls
   // back to rowtab when the planes' slices do not fit in a lattice-sized
   // buffer.  The caller synchronises.
-  __device__ void rowtab_planes(const float *lat, float *Gt) {
-    const int np = nplanes_local(), slice = ncy * ncz;
-    if ((long long)np * slice > pl.NLAT) { rowtab(lat, Gt); return; }
-    float *Xp = aux;
+  __device__ void rowtab_planes(const float *lat) {
+    const int slice = ncy * ncz;
+    if ((long long)np * slice > pl.NLAT) { rowtab(lat); return; }
+    float *Xp = aux();
     for (int t = threadIdx.x; t < np * slice; t += blockDim.x) {
       const int m = t / slice, c = t - m * slice;
       const int vx = plane_vx(m);
-      const int sx = ax.s[vx];
-      const float4 wx = ax.w[vx];
-      const float *pa = lat + (size_t)sx * slice + c;
+      const float4 wx = at<float4>(ax.o_w)[vx];
+      const float *pa = lat + at<int>(ax.o_s)[vx] * slice + c;
       float a = __fmul_rn(wx.x, pa[0]);
       a = __fmaf_rn(wx.y, pa[slice], a);
       a = __fmaf_rn(wx.z, pa[2 * slice], a);
       Xp[t] = __fmaf_rn(wx.w, pa[3 * slice], a);
     }
     __syncthreads();
-    const int vx0 = Group::kGrid ? r0 / Y : 0;
-    for (int t = threadIdx.x; t < nrow * ncz; t += blockDim.x) {
-      const int rl = t / ncz, cz = t - rl * ncz;
-      int vx, vy;
-      row_xy(rl, vx, vy);
-      const int m = Group::kGrid ? vx - vx0 : rl / Y;
-      const int sy = ay.s[vy];
-      const float4 wy = ay.w[vy];
-      const float *xa = Xp + m * slice + sy * ncz + cz;
+    const int lsh = ncz_log2();
+    float *Gt = Gd();
+    for (int t = threadIdx.x; t < (nact << lsh); t += blockDim.x) {
+      const int r = t >> lsh, cz = t & ((1 << lsh) - 1);
+      if (cz >= ncz) continue;
+      const Row o = row(r);
+      const float4 wy = at<float4>(ay.o_w)[o.vy];
+      const float *xa = Xp + o.m * slice + at<int>(ay.o_s)[o.vy] * ncz + cz;
       float a = __fmul_rn(wy.x, xa[0]);
       a = __fmaf_rn(wy.y, xa[ncz], a);
       a = __fmaf_rn(wy.z, xa[2 * ncz], a);
-      Gt[t] = __fmaf_rn(wy.w, xa[3 * ncz], a);
+      Gt[r * ncz + cz] = __fmaf_rn(wy.w, xa[3 * ncz], a);
     }
   }
 
-  // First voxel of local row rl in the job's log volume: grid, contiguous
-  // rows r0 + rl; cluster, plane vx = rank + m*K, row vy of it
-  __device__ __forceinline__ const float *src_row(int rl) const {
-    if (Group::kGrid) return src + (size_t)(r0 + rl) * Z;
-    const int m = rl / Y;
-    return src + ((size_t)(rank + m * K) * Y + (rl - m * Y)) * Z;
+  // Calls body(row, its index, a, b, sp) for every (row, span) piece of this
+  // lane.  Rows go to warps in list order; with more spans than lanes the
+  // spans are taken in rounds.
+  template <class Body>
+  __device__ __forceinline__ void span_pass(Body &&body) const {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int l = lane & ((1 << sg) - 1), sub = lane >> sg, rs = 5 - sg;
+    const int per = (1 << sg) >> sh;   // spans per round
+    const int ntask = (nact + (1 << rs) - 1) >> rs;
+    for (int sp0 = 0; sp0 < az.nsp; sp0 += per) {
+      const int sp = sp0 + (l >> sh), h = l & ((1 << sh) - 1);
+      const bool on = sp < az.nsp;
+      const int lo = on ? at<int>(az.o_lo)[sp] : 0, hi = on ? at<int>(az.o_hi)[sp] : 0;
+      for (int task = warp; task < ntask; task += nw) {
+        const int r = (task << rs) + sub;
+        if (r >= nact) continue;
+        const Row o = row(r);
+        int a, b;
+        piece(o, lo, hi, h, sh, a, b);
+        body(o, r, a, b, sp);
+      }
+    }
   }
 
-  // logU = im_log - eval(rows(lat)) for every local voxel, im_log read from
-  // the slab itself when `staged` (the cluster kernel's bulk copy of the
+  // logU = im_log - eval(rows(lat)) for every voxel of the rows, im_log read
+  // from the slab itself when `staged` (the cluster kernel's bulk copy of the
   // volume, before the first reset), else from the job's log volume in
   // global memory; rows(lat) goes through the Gd region (free at every
   // reset: level start, warm-start trial).
   __device__ void reset(const float *lat, bool staged = false) {
-    rowtab(lat, Gd);
+    rowtab(lat);
     __syncthreads();
-    const int n = nrow * Z;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const int rl = (int)divZ.div((unsigned)i), vz = i - rl * Z;
-      const float v = staged ? logu[i] : src_row(rl)[vz];
-      logu[i] = isnan(v) ? v : __fsub_rn(v, eval(Gd, rl, vz));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s;
+    for (int r = (warp << rs) + sub; r < nact; r += nw << rs) {
+      const Row o = row(r);
+      const float *im = staged ? o.p : src_row(o);
+      const float *g0 = Gd() + r * ncz;
+      for (int z = o.z0 + l; z < o.z1; z += 1 << s) {
+        const float v = im[z];
+        o.p[z] = isnan(v) ? v : __fsub_rn(v, dot4(at<float4>(az.o_w)[z], g0 + at<int>(az.o_s)[z]));
+      }
     }
     __syncthreads();
-  }
-
-  __device__ __forceinline__ float eval(const float *Gt, int rl, int vz) const {
-    return dot4(az.w[vz], Gt + rl * ncz + az.s[vz]);
   }
 
   // ---- group reductions
-  // Stats: every CTA reads all K slots in the same order.
-  __device__ bool reduce_stats(const double in[4], double out[4]) {
-    if (threadIdx.x == 0) { for (int i = 0; i < 4; ++i) slotA->v[i] = in[i]; }
+  // Masked min/max and the convergence sums of the group, then what the
+  // iteration takes from them (Iter), the same in every CTA.  idle() runs on
+  // the CTA's other warps while the first one reduces.
+  static __device__ __forceinline__ int fkey(float v) {   // order of floats as order of ints (an involution)
+    const int k = __float_as_int(v);
+    return k ^ ((k >> 31) & 0x7fffffff);
+  }
+  static __device__ __forceinline__ float funkey(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+  template <class Idle>
+  __device__ bool reduce_stats(float vmin, float vmax, double s0, double s1, bool need_cv, Idle &&idle) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double *sc = red();
+    vmin = funkey(__reduce_min_sync(kFull, fkey(vmin)));
+    vmax = funkey(__reduce_max_sync(kFull, fkey(vmax)));
+    if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
+    if (lane == 0) { sc[warp] = vmin; sc[32 + warp] = vmax; sc[64 + warp] = s0; sc[96 + warp] = s1; }
+    __syncthreads();
+    if (warp == 0) {
+      const bool in = lane < nw;
+      vmin = funkey(__reduce_min_sync(kFull, fkey(in ? (float)sc[lane] : INFINITY)));
+      vmax = funkey(__reduce_max_sync(kFull, fkey(in ? (float)sc[32 + lane] : -INFINITY)));
+      s0 = in ? sc[64 + lane] : 0.0;
+      s1 = in ? sc[96 + lane] : 0.0;
+      if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
+      if (lane == 0) { Stats *a = slotA(); a->v[0] = vmin; a->v[1] = vmax; a->v[2] = s0; a->v[3] = s1; }
+    }
+    N4_MARK(PH_A_LOOP);
     if (!g.sync()) return false;
-    if (threadIdx.x < 32) {
+    if (warp == 0) {
       float mn = INFINITY, mx = -INFINITY;
-      double s0 = 0.0, s1 = 0.0;
-      for (int k = threadIdx.x; k < K; k += 32) {
-        const Stats *p = g.peer(slotA, k);
-        mn = fminf(mn, (float)g.load(&p->v[0]));
-        mx = fmaxf(mx, (float)g.load(&p->v[1]));
-        s0 += g.load(&p->v[2]);
-        s1 += g.load(&p->v[3]);
+      s0 = 0.0;
+      s1 = 0.0;
+      for (int k = lane; k < K; k += 32) {
+        const Stats *p = g.peer(slotA(), k);
+        double v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = Group::kGrid ? __ldcg(&p->v[i]) : p->v[i];
+        mn = fminf(mn, (float)v[0]);
+        mx = fmaxf(mx, (float)v[1]);
+        s0 += v[2];
+        s1 += v[3];
       }
-      mn = warp_min(mn); mx = warp_max(mx); s0 = warp_sum(s0); s1 = warp_sum(s1);
-      if (threadIdx.x == 0) { red[0] = mn; red[1] = mx; red[2] = s0; red[3] = s1; }
+      mn = funkey(__reduce_min_sync(kFull, fkey(mn)));
+      mx = funkey(__reduce_max_sync(kFull, fkey(mx)));
+      if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
+      if (lane == 0) {
+        Iter &it = iter();
+        it.st[0] = mn; it.st[1] = mx; it.st[2] = s0; it.st[3] = s1;
+        // bin range of the masked logU (N4.py:14-15); st holds FP32 values
+        const double slope = ((double)mx - (double)mn) / (double)(pr.bins - 1);
+        it.degenerate = !(slope > 0.0) || !isfinite(slope);
+        it.bm = BinMap(mn, it.degenerate ? 1.0 : slope, pr.bins);
+        it.scale = ldexp(1.0, hshift);
+        it.gauss = gauss_of(it.bm.slope, pr.fwhm);
+        if (need_cv) it.cv = cv_from(it.st);
+      }
+    } else {
+      idle();
     }
-    __syncthreads();
-    for (int i = 0; i < 4; ++i) out[i] = red[i];
     __syncthreads();
     return true;
   }
 
-  // Sum of every CTA's `mine[0..n)` into `out` (shared), identical in all
-  // CTAs, each entry summed over the CTAs in rank order.  Cluster: after one
-  // barrier every CTA reads all K partials through DSMEM (a partial is written
-  // again only after later barriers of the iteration, by which time every
-  // peer has read it).  Grid: each CTA reduces one slice over all peers, then
-  // every CTA gathers the slices; slices live in a buffer of their own, so a
-  // CTA may modify `out` while slower peers are still gathering.
-  // Sum over the group's K partials of entry c, in rank order: exact for the
-  // integer histogram, Kahan-compensated for the fit's float partials.
-  struct Acc64 {
-    unsigned long long s = 0;
-    __device__ __forceinline__ void add(unsigned long long x) { s += x; }
-    __device__ __forceinline__ unsigned long long value() const { return s; }
-  };
-  template <class T> using AccOf = typename std::conditional<std::is_same<T, float>::value, KahanSum, Acc64>::type;
-
-  template <class T>
-  __device__ bool allreduce(const T *mine, T *out, int n) {
-    if (!g.sync()) return false;
-    if (!Group::kGrid) {
-      for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        AccOf<T> acc;
-#pragma unroll 4
-        for (int k = 0; k < K; ++k) acc.add(*(g.peer(mine, k) + c));
-        out[c] = acc.value();
-      }
-      __syncthreads();
-      return true;
-    }
-    const int per = (n + K - 1) / K;
-    const int c0 = rank * per, c1 = min(n, c0 + per);
-    T *slice = Group::kGrid ? (T *)red_global : (T *)(big + pl.b_slice);
-    // one warp per entry of the slice: lane l sums the partials of CTAs
-    // l, l + 32, ... (compensated for floats), then a fixed shuffle tree adds
-    // the lanes, so that the K loads of an entry are in flight together
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int c = c0 + warp; c < c1; c += nwarp) {
-      AccOf<T> acc;
-      for (int k = lane; k < K; k += 32) acc.add(g.load(g.peer(mine, k) + c));
-      T v = acc.value();
-#pragma unroll
-      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-      if (lane == 0) slice[Group::kGrid ? c : c - c0] = v;
-    }
-    if (!g.sync()) return false;
+  // Sum of every CTA's partial entries over the group; fin(c, sum) for every
+  // entry c of [0, n) on one thread of each CTA, the same sum in all of them.
+  // Cluster path: the partials are in `mine` (shared memory), read through
+  // DSMEM in rank order, eight loads in flight; exact for the integer
+  // histogram, Kahan-compensated for the fit's float partials.  A partial is
+  // written again only after later barriers of the iteration, by which time
+  // every peer has read it.
+  template <class T, class Fin>
+  __device__ __forceinline__ void peers_sum(const T *mine, int n, Fin &&fin) const {
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
-      if (Group::kGrid) {
-        out[c] = __ldcg(slice + c);
-      } else {
-        const int owner = c / per;
-        out[c] = *(g.peer(slice, owner) + (c - owner * per));
+      SumOf<T> acc;
+      for (int k0 = 0; k0 < K; k0 += 8) {
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = k0 + u < K ? *(g.peer(mine, k0 + u) + c) : T(0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (k0 + u < K) acc.add(v[u]);
+      }
+      fin(c, acc.value());
+    }
+  }
+  template <class T> struct SumOf;
+
+  // Whole-GPU path: the accumulator set of the current sum, and, after its
+  // barrier, the set that may be cleared (the one read at the previous sum).
+  __device__ __forceinline__ unsigned long long *acc_set(int s) const {
+    if constexpr (Group::kGrid) return g.acc + (size_t)(s % 3) * g.len;
+    else return nullptr;
+  }
+  __device__ __forceinline__ void acc_clear() const {
+    if constexpr (Group::kGrid) {
+      if (rank == 0) {
+        unsigned long long *a = acc_set(seq + 2);
+        for (int i = threadIdx.x; i < g.len; i += blockDim.x) a[i] = 0ull;
       }
     }
+  }
+  __device__ __forceinline__ void acc_next() {
     __syncthreads();
-    return true;
+    if (writer()) ++seq;
+    publish();
   }
 
-  // ---- separable fit contraction of the local rows into slotC (full lattice)
-  // num: the residuals left by pass C with weights w^3/sum w^2; den: the mask
-  // with weights w^2 (N4.py:224-236).
-  //   T1[row][cz]   z contraction: one thread per (row, z-span) accumulates
-  //                 the span's 4 targets in registers; spans s = phi mod 4
-  //                 never share a target, so 4 phases add without atomics in
-  //                 a fixed order
-  //   T2[vx][cy][cz] y contraction over the CTA's rows of each x-plane
-  //   slotC[c]       x contraction (the CTA's partial lattice)
-  // then the group all-reduce of the partial lattices.  The sums across rows
-  // (y, x and over the CTAs) are Kahan-compensated: a control point of the
-  // 256x256x160 grid gathers ~5e5 voxels through them.  The sum within a row
-  // covers one span (at most Z / spans voxels, fixed order) and is plain FP32.
-  __device__ void contract(bool num_mode, const BinMap *bm = nullptr, bool degenerate = false) {
-    float *T1 = Gd;   // Gd is dead between pass A and the next update
-    const int nt1 = nrow * ncz;
-    // whole-GPU path, few spans per row (coarse levels): the (row, span) tasks
-    // leave most of the CTA's threads idle (443 rows of 160 voxels for 1024
-    // threads at 512x512x320), so each span is cut in two halves, summed by
-    // two threads into two tables (the second after the first in Gd, when it
-    // fits) that are added at the end.  (On the cluster path, rows of ~44
-    // voxels, the extra tasks and the final pass cost more than they save.)
-    const int gd_floats = (pl.b_T2 - pl.b_Gd) / 4;
-    const int halves = (Group::kGrid && az.nsp <= 4 && 2 * nt1 <= gd_floats) ? 2 : 1;
-    float *T1b = T1 + nt1;
-    for (int t = threadIdx.x; t < halves * nt1; t += blockDim.x) T1[t] = 0.0f;
+  // Fixed-point scale of the lattice sums of the whole-GPU path: `bound` is at
+  // least the sum of the magnitudes of all terms, so that the 64-bit integer
+  // sum cannot overflow; integer sums are exact and the same in any order.
+  static __device__ __forceinline__ int sum_shift(double bound) {
+    return min(61 - ilogb(fmin(fmax(bound, 1e-30), 1e300)), 52);
+  }
+
+  // ---- separable fit contraction of the rows into the group's lattice sums
+  // num: the residuals with weights w^3/sum w^2; den: the mask with weights
+  // w^2 (N4.py:224-236).
+  //   T1[row][cz]   z contraction: the lane of a (row, span) piece accumulates
+  //                 the span's 4 targets in registers; the pieces of a span
+  //                 are added by shuffles, and target t takes its sums from
+  //                 spans t-3 .. t by shuffles too
+  //   T2[m][cy][cz] y contraction over the CTA's rows of each x-plane
+  //   lattice       x contraction (the CTA's partial lattice)
+  // then the group's sum of the partial lattices, fin(c, sum) per entry.  The
+  // sums across rows (y, x and over the CTAs) are Kahan-compensated or exact:
+  // a control point of the 256x256x160 grid gathers ~5e5 voxels through them.
+  // The sum within a row covers one span and is plain FP32.
+  template <bool Num, class Fin>
+  __device__ bool contract(Fin &&fin) {
+    float *T1 = Gd();   // Gd is dead between pass A and the next update
+    const Iter &it = iter();
+    const bool degenerate = Num && it.degenerate;
+    {
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+      const int l = lane & ((1 << sz) - 1), rs = 5 - sz, d = 1 << szh;
+      const int per = (1 << sz) >> szh;   // spans per round: all of them, up to 32
+      const int ntask = (nact + (1 << rs) - 1) >> rs;
+      for (int sp0 = 0; sp0 < az.nsp; sp0 += per) {
+        const int k = l >> szh, sp = sp0 + k, h = l & (d - 1);
+        const bool in = sp < az.nsp;
+        const int lo = in ? at<int>(az.o_lo)[sp] : 0, hi = in ? at<int>(az.o_hi)[sp] : 0;
+        for (int task = warp; task < ntask; task += nw) {
+          const int r = (task << rs) + (lane >> sz);
+          const bool on = in && r < nact;
+          float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (on && !degenerate) {
+            const Row o = row(r);
+            int a, b;
+            piece(o, lo, hi, h, szh, a, b);
+            span_sums<Num>(o.p, a, b, s);
+          }
+          for (int w = d >> 1; w; w >>= 1) {
+            s.x += __shfl_xor_sync(kFull, s.x, w); s.y += __shfl_xor_sync(kFull, s.y, w);
+            s.z += __shfl_xor_sync(kFull, s.z, w); s.w += __shfl_xor_sync(kFull, s.w, w);
+          }
+          // the sums of the one, two and three spans before
+          const float y1 = __shfl_up_sync(kFull, s.y, d), z1 = __shfl_up_sync(kFull, s.z, d),
+                      w1 = __shfl_up_sync(kFull, s.w, d), z2 = __shfl_up_sync(kFull, s.z, 2 * d),
+                      w2 = __shfl_up_sync(kFull, s.w, 2 * d), w3 = __shfl_up_sync(kFull, s.w, 3 * d);
+          if (on && h == 0) {
+            float *t1 = T1 + r * ncz + sp;
+            const bool p1 = k >= 1, p2 = k >= 2, p3 = k >= 3;
+            // targets in the order of span mod 4; a round finds the last
+            // three targets of the one before open
+            const auto put = [&](int i, float x0, float x1, float x2, float x3) {
+              const float x = rotated_sum(sp & 3, x0, x1, x2, x3);
+              t1[i] = sp0 > 0 && k + i < 3 ? t1[i] + x : x;
+            };
+            put(0, s.x, p1 ? y1 : 0.0f, p2 ? z2 : 0.0f, p3 ? w3 : 0.0f);
+            if (k == per - 1 || sp == az.nsp - 1) {
+              put(1, s.y, p1 ? z1 : 0.0f, p2 ? w2 : 0.0f, 0.0f);
+              put(2, s.z, p1 ? w1 : 0.0f, 0.0f, 0.0f);
+              put(3, s.w, 0.0f, 0.0f, 0.0f);
+            }
+          }
+          __syncwarp();
+        }
+      }
+    }
     __syncthreads();
-    const float4 *W4 = num_mode ? az.p4 : az.q4;
-    for (int phase = 0; phase < 4; ++phase) {
-      const int nsp = phase < az.nsp ? (az.nsp - phase + 3) / 4 : 0;   // spans phase, phase+4, ...
-      const int per_row = nsp * halves;
-      const int ntask = nrow * per_row;
-      for (int t = threadIdx.x; t < ntask; t += blockDim.x) {
-        const int rl = t / per_row, rem = t - rl * per_row;
-        const int sp = phase + 4 * (halves == 2 ? rem >> 1 : rem), h = halves == 2 ? rem & 1 : 0;
-        int lo = az.lo[sp], hi = az.hi[sp];
-        if (halves == 2) {
-          const int mid = (lo + hi) >> 1;
-          if (h) lo = mid;
-          else hi = mid;
-        }
-        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-        if (num_mode) {
-          // residual R = logU - E(logU) of each masked voxel
-          const float *iv = logu + (size_t)rl * Z;
-          if constexpr (kRB == 1) {
-            for (int vz = lo; vz < hi; ++vz) {
-              const float lu = iv[vz];
-              if (isnan(lu)) continue;
-              const float r = degenerate ? 0.0f : residual_of(*bm, lu, R2, E, pr.bins);
-              const float4 w = W4[vz];
-              a0 = __fmaf_rn(w.x, r, a0); a1 = __fmaf_rn(w.y, r, a1);
-              a2 = __fmaf_rn(w.z, r, a2); a3 = __fmaf_rn(w.w, r, a3);
-            }
-          } else
-          // kRB voxels at a time: their loads are issued before the
-          // first is used; the terms are added in voxel order
-          for (int vb = lo; vb < hi; vb += kRB) {
-            float v[kRB];
-#pragma unroll
-            for (int u = 0; u < kRB; ++u) v[u] = vb + u < hi ? iv[vb + u] : kNaN;
-#pragma unroll
-            for (int u = 0; u < kRB; ++u) {
-              if (isnan(v[u])) continue;
-              const int vz = vb + u;
-              const float lu = v[u];
-              const float r = degenerate ? 0.0f : residual_of(*bm, lu, R2, E, pr.bins);
-              const float4 w = W4[vz];
-              a0 = __fmaf_rn(w.x, r, a0); a1 = __fmaf_rn(w.y, r, a1);
-              a2 = __fmaf_rn(w.z, r, a2); a3 = __fmaf_rn(w.w, r, a3);
-            }
-          }
-        } else {
-          const float *iv = logu + (size_t)rl * Z;
-          if constexpr (kRB == 1) {
-            for (int vz = lo; vz < hi; ++vz) {
-              if (isnan(iv[vz])) continue;
-              const float4 w = W4[vz];
-              a0 += w.x; a1 += w.y; a2 += w.z; a3 += w.w;
-            }
-          } else
-          for (int vb = lo; vb < hi; vb += kRB) {
-            float v[kRB];
-#pragma unroll
-            for (int u = 0; u < kRB; ++u) v[u] = vb + u < hi ? iv[vb + u] : kNaN;
-#pragma unroll
-            for (int u = 0; u < kRB; ++u) {
-              if (isnan(v[u])) continue;
-              const float4 w = W4[vb + u];
-              a0 += w.x; a1 += w.y; a2 += w.z; a3 += w.w;
-            }
-          }
-        }
-        float *t1 = (h ? T1b : T1) + rl * ncz + sp;
-        t1[0] += a0; t1[1] += a1; t1[2] += a2; t1[3] += a3;
-      }
-      __syncthreads();
-    }
-    if (halves == 2) {
-      for (int t = threadIdx.x; t < nt1; t += blockDim.x) T1[t] = __fadd_rn(T1[t], T1b[t]);
-      __syncthreads();
-    }
     N4_MARK(PH_F_T1);
-    const float *PY = num_mode ? ay.p : ay.q;
-    const float *PX = num_mode ? ax.p : ax.q;
-    if (Group::kGrid) {
-      // contiguous rows: planes vx0..vx1, partially covered at both ends
-      const int vx0 = r0 / Y, vx1 = (r0 + nrow - 1) / Y;
-      const int nt2 = (vx1 - vx0 + 1) * ncy * ncz;
-      for (int t = threadIdx.x; t < nt2; t += blockDim.x) {
-        const int cz = t % ncz, cy = (t / ncz) % ncy, xl = t / (ncz * ncy);
-        const int rb = (vx0 + xl) * Y - r0;   // local row of (vx, 0)
-        KahanSum acc, acc2;   // two chains (alternate rows), merged at the end
-        for (int j = 0; j < 4; ++j) {
-          const int sp = cy - j;
-          if (sp < 0 || sp >= ay.nsp) continue;
-          const int lo = max(ay.lo[sp], -rb), hi = min(ay.hi[sp], nrow - rb);
-          const float *wy = PY + j * Y;
-          int vy = lo;
-          for (; vy + 1 < hi; vy += 2) {
-            acc.add_prod(wy[vy], T1[(rb + vy) * ncz + cz]);
-            acc2.add_prod(wy[vy + 1], T1[(rb + vy + 1) * ncz + cz]);
-          }
-          if (vy < hi) acc.add_prod(wy[vy], T1[(rb + vy) * ncz + cz]);
-        }
-        acc.merge(acc2);
-        T2[t] = acc.value();
+    double scale = 1.0;
+    if constexpr (Group::kGrid) {
+      const double range = it.st[1] - it.st[0];
+      scale = ldexp(1.0, sum_shift(Num ? nfg * (5.0 * range + fabs(it.st[0]) + fabs(it.st[1])) : nfg));
+    }
+    const int slice = ncy * ncz;
+    for (int m0 = 0; m0 < np || m0 == 0; m0 += tp) {
+      const int cnt = min(tp, np - m0);
+      if (np > tp) {
+        build_ytab(m0, cnt);
+        __syncthreads();
       }
+      plane_sums<Num>(T1, cnt);
       __syncthreads();
       N4_MARK(PH_F_T2);
+      // x contraction of planes m0 .. m0 + cnt - 1
+      const float *T2p = T2();
+      const float *PX = at<float>(Num ? ax.o_p : ax.o_q);
       for (int c = threadIdx.x; c < nlat; c += blockDim.x) {
-        const int cz = c % ncz, cy = (c / ncz) % ncy, cx = c / (ncz * ncy);
+        const int cx = c / slice, cc = c - cx * slice;
         KahanSum acc;
+        bool any = false;
         for (int j = 0; j < 4; ++j) {
           const int sp = cx - j;
           if (sp < 0 || sp >= ax.nsp) continue;
-          const int lo = max(ax.lo[sp], vx0), hi = min(ax.hi[sp], vx1 + 1);
-          const float *wx = PX + j * X;
-          for (int vx = lo; vx < hi; ++vx) acc.add_prod(wx[vx], T2[((vx - vx0) * ncy + cy) * ncz + cz]);
+          const int lo = at<int>(ax.o_lo)[sp], hi = at<int>(ax.o_hi)[sp];
+          int m, vx;
+          const int end = Group::kGrid ? min(hi, vx0 + m0 + cnt) : hi;
+          if constexpr (Group::kGrid) {
+            vx = max(lo, vx0 + m0);
+            m = vx - vx0 - m0;
+          } else {
+            m = lo <= rank ? 0 : (lo - rank + K - 1) / K;
+            vx = rank + m * K;
+          }
+          for (; vx < end; vx += Group::kGrid ? 1 : K, ++m) {
+            acc.add_prod(PX[vx * 4 + j], T2p[m * slice + cc]);
+            any = true;
+          }
         }
-        slotC[c] = acc.value();
+        if constexpr (Group::kGrid) {
+          if (any) {
+            const double v = ((double)acc.s - (double)acc.c) * scale;
+            if (!isfinite(v)) atomicAdd(acc_set(seq) + g.len - 1, 1ull);
+            else if (v != 0.0) {
+              const double lim = 4611686018427387904.0 / K;   // 2^62: the sum of K terms cannot wrap
+              atomicAdd(acc_set(seq) + c, (unsigned long long)__double2ll_rn(fmin(fmax(v, -lim), lim)));
+            }
+          }
+        } else {
+          slotC()[c] = acc.value();
+        }
+      }
+      if (np > tp) __syncthreads();
+    }
+    N4_MARK(PH_F_P);
+    if (!g.sync()) return false;
+    if constexpr (Group::kGrid) {
+      const unsigned long long *a = acc_set(seq);
+      const bool nan = __ldcg(a + g.len - 1) != 0;
+      const double inv = 1.0 / scale;
+      for (int c = threadIdx.x; c < nlat; c += blockDim.x)
+        fin(c, nan ? kNaN : (float)((double)(long long)__ldcg(a + c) * inv));
+      acc_clear();
+      acc_next();
+    } else {
+      peers_sum(slotC(), nlat, fin);
+      __syncthreads();
+    }
+    N4_MARK(PH_F_RED);
+    return true;
+  }
+
+  // x0 + x1 + x2 + x3, the sums of spans s, s - 1, s - 2, s - 3, added in the
+  // order of span mod 4 (m = s mod 4).
+  static __device__ __forceinline__ float rotated_sum(int m, float x0, float x1, float x2, float x3) {
+    const float a = m & 1 ? x1 : x0, b = m & 1 ? x0 : x3, c = m & 1 ? x3 : x2, e = m & 1 ? x2 : x1;
+    const float t0 = m & 2 ? c : a, t1 = m & 2 ? e : b, t2 = m & 2 ? a : c, t3 = m & 2 ? b : e;
+    return __fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3);
+  }
+
+  // The four targets' sums of voxels [a, b) of a row, in voxel order: weights
+  // times the residual R = logU - E(logU) (Num), or the weights of the masked
+  // voxels.  Voxels outside the mask add zeros.  The residuals of U voxels are
+  // formed together, without branches.
+  template <bool Num>
+  __device__ __forceinline__ void span_sums(const float *p, int a, int b, float4 &s) const {
+    constexpr int U = Group::kGrid ? 2 : 4;   // measured best on each path
+    const Iter &it = iter();
+    const float bmin = it.bm.fmin, ih = it.bm.ih, il = it.bm.il, lim = it.bm.ff_limit;
+    const float4 *W = at<float4>(Num ? az.o_p : az.o_q);
+    for (int z = a; z < b; z += U) {
+      float v[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = z + u < b ? p[z + u] : kNaN;
+      unsigned top = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if constexpr (Num) {
+          int k;
+          float f;
+          const bool in = coord_split(v[u], bmin, ih, il, lim, k, f);
+          x[u] = in ? residual_lin(k, f, R2()) : 0.0f;
+          if (!in && !isnan(v[u])) top |= 1u << u;
+        } else {
+          x[u] = isnan(v[u]) ? 0.0f : 1.0f;
+        }
+      }
+      if (Num && top) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (top >> u & 1u) x[u] = residual_top(&it.bm, v[u], E(), pr.bins);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float4 w = W[min(z + u, b - 1)];
+        s.x = __fmaf_rn(w.x, x[u], s.x); s.y = __fmaf_rn(w.y, x[u], s.y);
+        s.z = __fmaf_rn(w.z, x[u], s.z); s.w = __fmaf_rn(w.w, x[u], s.w);
+      }
+    }
+  }
+
+  // T2[m][cy][cz] of `cnt` x-planes.  Cluster path: one thread per entry over
+  // its four spans' rows, Kahan in two chains (rows at even and at odd
+  // distance from the span's start); rows before and after the plane's listed
+  // ones add zeros, which a chain need take only once.  Whole-GPU path, whose
+  // CTAs hold two or three planes: one lane per span, the four sums added in
+  // FP64.
+  template <bool Num>
+  __device__ void plane_sums(const float *T1, int cnt) {
+    float *T2p = T2();
+    const int *yt = ytab();
+    const float *PY = at<float>(Num ? ay.o_p : ay.o_q);
+    const int n = cnt * ncy * ncz, w = ay.nsp + 1;
+    if constexpr (!Group::kGrid) {
+      for (int u = threadIdx.x; u < n; u += blockDim.x) {
+        const int q = u / ncz, cz = u - q * ncz;
+        const int m = q / ncy, cy = q - m * ncy;
+        KahanSum acc, acc2;
+        for (int j = 0; j < 4; ++j) {
+          const int sp = cy - j;
+          if (sp < 0 || sp >= ay.nsp) continue;
+          const int lo = at<int>(ay.o_lo)[sp], hi = at<int>(ay.o_hi)[sp];
+          const int r0 = yt[m * w + sp], r1 = yt[m * w + sp + 1];
+          const int va = r0 < r1 ? row_vy(r0) : hi, vb = va + (r1 - r0);
+          if (va > lo) acc.add(0.0f);
+          if (va > lo + 1) acc2.add(0.0f);
+          const float *t1 = T1 + r0 * ncz + cz, *py = PY + va * 4 + j;
+          int k = r1 - r0;
+          if (k > 0 && ((va - lo) & 1)) {
+            acc2.add_prod(py[0], t1[0]);
+            t1 += ncz;
+            py += 4;
+            --k;
+          }
+          for (; k > 1; k -= 2, t1 += 2 * ncz, py += 8) {
+            acc.add_prod(py[0], t1[0]);
+            acc2.add_prod(py[4], t1[ncz]);
+          }
+          if (k > 0) acc.add_prod(py[0], t1[0]);
+          if (r0 < r1 && vb < hi) {
+            const int even = (vb - lo) & 1 ? vb + 1 : vb, odd = (vb - lo) & 1 ? vb : vb + 1;
+            if (even < hi) acc.add(0.0f);
+            if (odd < hi) acc2.add(0.0f);
+          }
+        }
+        acc.merge(acc2);
+        T2p[u] = acc.value();
       }
       return;
     }
-    // whole planes vx = rank + m*K: y contraction per local plane
-    const int nt2 = nplane * ncy * ncz;
-    for (int t = threadIdx.x; t < nt2; t += blockDim.x) {
-      const int cz = t % ncz, cy = (t / ncz) % ncy, m = t / (ncz * ncy);
-      const float *t1 = T1 + (size_t)m * Y * ncz + cz;
-      KahanSum acc, acc2;   // two chains (alternate rows), merged at the end
-      for (int j = 0; j < 4; ++j) {
-        const int sp = cy - j;
-        if (sp < 0 || sp >= ay.nsp) continue;
-        const float *wy = PY + j * Y;
-        int vy = ay.lo[sp];
-        const int hi = ay.hi[sp];
-        for (; vy + 1 < hi; vy += 2) {
-          acc.add_prod(wy[vy], t1[vy * ncz]);
-          acc2.add_prod(wy[vy + 1], t1[(vy + 1) * ncz]);
+    const int nt = (n * 4 + 31) & ~31;   // whole warps: the lanes of an entry exchange their sums
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) {
+      const int u = t >> 2, j = t & 3;
+      const int q = u / ncz, cz = u - q * ncz;
+      const int m = q / ncy, cy = q - m * ncy, sp = cy - j;
+      double s = 0.0;
+      if (u < n && sp >= 0 && sp < ay.nsp) {
+        KahanSum acc, acc2;
+        int r = yt[m * w + sp];
+        const int end = yt[m * w + sp + 1];
+        for (; r + 1 < end; r += 2) {
+          acc.add_prod(PY[row_vy(r) * 4 + j], T1[r * ncz + cz]);
+          acc2.add_prod(PY[row_vy(r + 1) * 4 + j], T1[(r + 1) * ncz + cz]);
         }
-        if (vy < hi) acc.add_prod(wy[vy], t1[vy * ncz]);
+        if (r < end) acc.add_prod(PY[row_vy(r) * 4 + j], T1[r * ncz + cz]);
+        s = ((double)acc.s - (double)acc.c) + ((double)acc2.s - (double)acc2.c);
       }
-      acc.merge(acc2);
-      T2[t] = acc.value();
+      s += __shfl_xor_sync(kFull, s, 1);
+      s += __shfl_xor_sync(kFull, s, 2);
+      if (u < n && j == 0) T2p[u] = (float)s;
     }
-    __syncthreads();
-    N4_MARK(PH_F_T2);
-    for (int c = threadIdx.x; c < nlat; c += blockDim.x) {
-      const int cz = c % ncz, cy = (c / ncz) % ncy, cx = c / (ncz * ncy);
-      KahanSum acc;
-      for (int j = 0; j < 4; ++j) {
-        const int sp = cx - j;
-        if (sp < 0 || sp >= ax.nsp) continue;
-        const float *wx = PX + j * X;
-        // local planes inside [lo, hi): vx = rank + m*K
-        const int lo = ax.lo[sp], hi = ax.hi[sp];
-        int m = lo <= rank ? 0 : (lo - rank + K - 1) / K;
-        for (int vx = rank + m * K; vx < hi; vx += K, ++m) acc.add_prod(wx[vx], T2[(m * ncy + cy) * ncz + cz]);
-      }
-      slotC[c] = acc.value();
-    }
+  }
+  __device__ __forceinline__ int row_vy(int r) const {
+    if constexpr (Group::kGrid) return rowsp[r].w;
+    else return (int)(at<uint2>(pl.o_rows)[r].y & 0xffffu);
   }
 
   // ---- pass A: the previous update's convergence sums from eval(Gd) (when
   // need_cv), applied to logU (when apply: logU -= eval(Gd)), and the masked
-  // min/max of logU
-  __device__ bool pass_a(bool need_cv, bool apply, double st[4]) {
+  // min/max of logU; clears the histogram copies
+  __device__ bool pass_a(bool need_cv, bool apply) {
     float vmin = INFINITY, vmax = -INFINITY;
     double sy = 0.0, syy = 0.0;
-    const int per = (int)blockDim.x / Z;   // whole rows per sweep: each thread keeps one z
-    if (per > 0) {
-      const int rs = (int)threadIdx.x / Z, vz = (int)threadIdx.x - rs * Z;
-      if (rs < per) {
-        const float4 w = az.w[vz];
-        const int sz = az.s[vz];
-        if constexpr (kRB == 1) {
-          for (int rl = rs; rl < nrow; rl += per) {
-            float lu = logu[rl * Z + vz];
-            if (isnan(lu)) continue;   // outside the mask
-            if (need_cv) {
-              const float ed = dot4(w, Gd + rl * ncz + sz);
-              const float y = expm1_conv(-ed);
-              sy += (double)y;
-              syy += (double)y * (double)y;
-              if (apply) {
-                lu = __fsub_rn(lu, ed);
-                logu[rl * Z + vz] = lu;
+    const float *Gp = Gd();
+    const float4 *W4 = at<float4>(az.o_w);
+    span_pass(
+        [&](const Row &o, int r, int a, int b, int sp) {
+          if (a >= b) return;
+          constexpr int U = 2;
+          if (need_cv) {
+            const float *gp = Gp + r * ncz + sp;
+            const float g[4] = {gp[0], gp[1], gp[2], gp[3]};
+            for (int z = a; z < b; z += U) {
+              float v[U], ed[U], y[U];
+#pragma unroll
+              for (int u = 0; u < U; ++u) v[u] = z + u < b ? o.p[z + u] : kNaN;
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                ed[u] = dot4(W4[min(z + u, b - 1)], g);
+                y[u] = expm1_conv(-ed[u]);
+              }
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const bool in = !isnan(v[u]);
+                const double yd = in ? (double)y[u] : 0.0;
+                sy += yd;
+                syy += yd * yd;
+                if (apply) {
+                  v[u] = __fsub_rn(v[u], ed[u]);
+                  if (in) o.p[z + u] = v[u];
+                }
+                vmin = fminf(vmin, v[u]);   // a NaN operand is passed over
+                vmax = fmaxf(vmax, v[u]);
               }
             }
-            vmin = fminf(vmin, lu);
-            vmax = fmaxf(vmax, lu);
-          }
-        } else
-        // kRB rows at a time: their loads are all issued before the
-        // first of them is used; the values are then taken in row order
-        for (int rb = rs; rb < nrow; rb += kRB * per) {
-          float v[kRB], evd[kRB];
-#pragma unroll
-          for (int u = 0; u < kRB; ++u) {
-            const int rl = rb + u * per;
-            v[u] = rl < nrow ? logu[rl * Z + vz] : kNaN;
-          }
-#pragma unroll
-          for (int u = 0; u < kRB; ++u) {
-            const int rl = rb + u * per;
-            evd[u] = (!isnan(v[u]) && need_cv) ? dot4(w, Gd + rl * ncz + sz) : 0.0f;
-          }
-#pragma unroll
-          for (int u = 0; u < kRB; ++u) {
-            if (isnan(v[u])) continue;   // outside the mask
-            float lu = v[u];
-            if (need_cv) {
-              const float y = expm1_conv(-evd[u]);
-              sy += (double)y;
-              syy += (double)y * (double)y;
-              if (apply) {
-                lu = __fsub_rn(lu, evd[u]);
-                logu[(rb + u * per) * Z + vz] = lu;
-              }
+          } else {
+            for (int z = a; z < b; ++z) {
+              const float v = o.p[z];
+              vmin = fminf(vmin, v);
+              vmax = fmaxf(vmax, v);
             }
-            vmin = fminf(vmin, lu);
-            vmax = fmaxf(vmax, lu);
           }
-        }
-      }
-    } else {
-      const int n = nrow * Z;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        float lu = logu[i];
-        if (isnan(lu)) continue;
-        if (need_cv) {
-          const int rl = (int)divZ.div((unsigned)i), vz = i - rl * Z;
-          const float ed = eval(Gd, rl, vz);
-          const float y = expm1_conv(-ed);
-          sy += (double)y;
-          syy += (double)y * (double)y;
-          if (apply) {
-            lu = __fsub_rn(lu, ed);
-            logu[i] = lu;
-          }
-        }
-        vmin = fminf(vmin, lu);
-        vmax = fmaxf(vmax, lu);
-      }
-    }
-    double loc[4];
-    block_reduce4(vmin, vmax, sy, syy, red + 8, loc);
-    if (threadIdx.x == 0) for (int i = 0; i < 4; ++i) red[4 + i] = loc[i];
-    __syncthreads();
-    for (int i = 0; i < 4; ++i) loc[i] = red[4 + i];
-    __syncthreads();
-    N4_MARK(PH_A_LOOP);
-    const bool ok = reduce_stats(loc, st);
+        });
+    const bool ok = reduce_stats(vmin, vmax, sy, syy, need_cv, [&] {
+      // the copies lie in the Gd region, which every thread has read by now
+      unsigned *h = hist();
+      for (int i = (int)threadIdx.x - 32; i < kHistCopies * pr.bins; i += (int)blockDim.x - 32) h[i] = 0u;
+    });
     N4_MARK(PH_A_RED);
     return ok;
   }
 
   // ---- pass B + sharpening: histogram of logU over the group, then E
-  __device__ bool pass_b(const BinMap &bm) {
-    const int bins = pr.bins, shift = hshift;
-    const double scale = ldexp(1.0, shift);
-    for (int i = threadIdx.x; i < kHistCopies * bins; i += blockDim.x) hist[i] = 0u;
-    __syncthreads();
-    N4_MARK(PH_B_ZERO);
-    unsigned *hc = hist + ((threadIdx.x >> 5) % kHistCopies) * bins;
-    const int n = nrow * Z;   // the local voxels in order: lanes take consecutive voxels
-    if constexpr (kRB == 1) {
-      for (int base = 0; base < n; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        int key = -1;
-        unsigned qlo = 0, qhi = 0;
-        if (i < n) {
-          const float lu = logu[i];
-          if (!isnan(lu)) key = hist_bin_of(bm, lu, bins, scale, qlo, qhi);
-        }
-        if (key >= 0) {
-          atomicAdd(&hc[key], qlo);
-          if (qhi) atomicAdd(&hc[key + 1], qhi);
-        }
-      }
-    } else {
-      // kRB voxels per thread at a time, their loads issued first
-      for (int base = 0; base < n; base += kRB * blockDim.x) {
-        float v[kRB];
+  __device__ bool pass_b() {
+    const int bins = pr.bins;
+    const Iter &it = iter();
+    {
+      const float bmin = it.bm.fmin, ih = it.bm.ih, il = it.bm.il, lim = it.bm.ff_limit;
+      const float scale = (float)it.scale;
+      const unsigned one = (unsigned)scale;
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+      const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s;
+      unsigned *hc = hist() + (warp % kHistCopies) * bins;
+      for (int r = (warp << rs) + sub; r < nact; r += nw << rs) {
+        const Row o = row(r);
+        constexpr int U = 2;
+        for (int z = o.z0 + l; z < o.z1; z += U << s) {
+          float v[U], f[U];
+          int k[U];
+          bool in[U];
 #pragma unroll
-        for (int u = 0; u < kRB; ++u) {
-          const int i = base + u * (int)blockDim.x + (int)threadIdx.x;
-          v[u] = i < n ? logu[i] : kNaN;
-        }
+          for (int u = 0; u < U; ++u) v[u] = z + (u << s) < o.z1 ? o.p[z + (u << s)] : kNaN;
 #pragma unroll
-        for (int u = 0; u < kRB; ++u) {
-          if (isnan(v[u])) continue;
-          unsigned qlo = 0, qhi = 0;
-          const int key = hist_bin_of(bm, v[u], bins, scale, qlo, qhi);
-          if (key >= 0) {
-            atomicAdd(&hc[key], qlo);
-            if (qhi) atomicAdd(&hc[key + 1], qhi);
+          for (int u = 0; u < U; ++u) in[u] = coord_split(v[u], bmin, ih, il, lim, k[u], f[u]);
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (in[u]) {
+              const unsigned qhi = min(__float2uint_rn(__fmul_rn(f[u], scale)), one);
+              atomicAdd(&hc[k[u]], one - qhi);
+              atomicAdd(&hc[k[u] + 1], qhi);
+            } else if (!isnan(v[u])) {
+              unsigned qlo = 0, qhi = 0;
+              const int key = hist_bin_top(&it.bm, v[u], bins, it.scale, qlo, qhi);
+              if (key >= 0) {
+                atomicAdd(&hc[key], qlo);
+                if (qhi) atomicAdd(&hc[key + 1], qhi);
+              }
+            }
           }
         }
       }
@@ -743,70 +976,286 @@ struct Engine {
     N4_MARK(PH_B_LOOP);
     for (int b = threadIdx.x; b < bins; b += blockDim.x) {
       unsigned long long s = 0;
-      for (int c = 0; c < kHistCopies; ++c) s += hist[c * bins + b];
-      slotB[b] = s;
+#pragma unroll
+      for (int c = 0; c < kHistCopies; ++c) s += hist()[c * bins + b];
+      if constexpr (Group::kGrid) {
+        if (s) atomicAdd(acc_set(seq) + b, s);
+      } else {
+        slotB()[b] = s;
+      }
     }
-    __syncthreads();
     N4_MARK(PH_B_MERGE);
-    if (!allreduce(slotB, H64, bins)) return false;
+    if (!g.sync()) return false;
+    if constexpr (Group::kGrid) {
+      const unsigned long long *a = acc_set(seq);
+      for (int b = threadIdx.x; b < bins; b += blockDim.x) H64()[b] = __ldcg(a + b);
+      acc_clear();
+      acc_next();
+    } else {
+      peers_sum(slotB(), bins, [&](int b, unsigned long long s) { H64()[b] = s; });
+      __syncthreads();
+    }
     N4_MARK(PH_B_RED);
-    N4_MARK(PH_B);
-    const double inv = ldexp(1.0, -shift);
-    const unsigned long long *h64 = H64;
-    SharpenBufs sb{fa, fb, tw, Ff};
-    sharpen_map([=](int b) { return (double)h64[b] * inv; }, bins, pl.npad, pl.hoff, bm.binMin, bm.slope,
-                pr.wiener, pr.fwhm, sb, E, R2);
+    const double inv = 1.0 / it.scale;   // exact: a power of two
+    const unsigned long long *h64 = H64();
+    const int a0 = alias0();
+    SharpenBufs sb{at<double2>(a0 + pl.a_fa), at<double2>(a0 + pl.a_fb), at<double2>(pl.o_tw), at<double>(a0 + pl.a_ff)};
+    sharpen_map([=](int b) { return (double)h64[b] * inv; }, bins, pl.npad, pl.hoff, it.bm.binMin, it.bm.slope,
+                pr.wiener, it.gauss, sb, E(), R2());
     N4_MARK(PH_SHARP);
     return true;
   }
 
-  // ---- one sharpen + fit step from the current logU; leaves the update in D
-  __device__ bool fit_step(const double st[4]) {
-    // bin range of the masked logU (N4.py:14-15); st holds FP32 values
-    const double bmin = st[0], bmax = st[1];
-    const double slope = (bmax - bmin) / (double)(pr.bins - 1);
-    const bool degenerate = !(slope > 0.0) || !isfinite(slope);
-    const BinMap bm(bmin, degenerate ? 1.0 : slope, pr.bins);
-    if (!degenerate) { if (!pass_b(bm)) return false; }
-    N4_MARK(PH_C);
-    contract(true, &bm, degenerate);   // the residual is formed inside the z contraction
+  // ---- one sharpen + fit step from the current logU: the update goes to D
+  // and into L, and its rows to Gd (through aux with `planes`)
+  __device__ bool fit_step(bool planes = true) {
+    if (!iter().degenerate) { if (!pass_b()) return false; }
+    float *Dp = D(), *Lp = L();
+    const float *dn = den();
+    const bool zd = pr.zero_den != 0;
+    const float eps = pr.eps;
+    if (!contract<true>([&](int c, float nu) {   // the residual is formed inside the z contraction
+          const float de = dn[c];
+          const float d = zd ? (de != 0.0f ? nu / de : 0.0f) : nu / (de + eps);
+          Dp[c] = d;
+          Lp[c] += d;
+        }))
+      return false;
+    if (planes) rowtab_planes(Dp);
+    else rowtab(Dp);
     __syncthreads();
-    N4_MARK(PH_F_P);
-    if (!allreduce(slotC, D, nlat)) return false;
-    N4_MARK(PH_F_RED);
-    for (int c = threadIdx.x; c < nlat; c += blockDim.x) {
-      const float nu = D[c], de = den[c];
-      D[c] = pr.zero_den ? (de != 0.0f ? nu / de : 0.0f) : nu / (de + pr.eps);
-    }
-    __syncthreads();
+    N4_MARK(PH_UPDATE);
     return true;
   }
 
-  __device__ float cv_from(const double st[4], double nfg) const {
+  __device__ float cv_from(const double st[4]) const {
     const double mean_y = st[2] / nfg;
     double var = st[3] / nfg - mean_y * mean_y;
     if (pr.ddof1) var = nfg > 1.0 ? var * nfg / (nfg - 1.0) : 0.0;
     return (float)(sqrt(var > 0.0 ? var : 0.0) / (1.0 + mean_y));
   }
 
-  // ---- the whole volume (logU of the local rows in the big region's slab;
-  // im_log read from job.imlog; cluster path: the slab holds the local rows
-  // of im_log on entry)
+  // Range of the masked voxels of one row of Z voxels (z0 | z1 << 16, 0 when
+  // there is none) and their number, by one warp.
+  static __device__ unsigned row_range(const float *p, int Z, int &count) {
+    const int lane = threadIdx.x & 31;
+    int z0 = Z, z1 = 0;
+    count = 0;
+    for (int b = 0; b < Z; b += 32) {
+      const unsigned m = __ballot_sync(kFull, b + lane < Z && !isnan(p[b + lane]));
+      if (m) {
+        z0 = min(z0, b + __ffs(m) - 1);
+        z1 = b + 32 - __clz(m);
+        count += __popc(m);
+      }
+    }
+    return z1 > 0 ? (unsigned)z0 | (unsigned)z1 << 16 : 0u;
+  }
+
+  // The rows i of [0, n) with range(i) != 0, in order: put(position, voxels
+  // before it, i, range).  Returns their number; all threads call it.
+  template <class Range, class Put>
+  __device__ int list_rows(int n, Range &&range, Put &&put) {
+    int *sc = (int *)red();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int rows = 0, voxels = 0;
+    for (int b = 0; b < n; b += blockDim.x) {
+      const int i = b + (int)threadIdx.x;
+      const unsigned e = i < n ? range(i) : 0u;
+      const int len = (int)(e >> 16) - (int)(e & 0xffffu);
+      const unsigned m = __ballot_sync(kFull, e != 0);
+      int ps = len;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int q = __shfl_up_sync(kFull, ps, o);
+        if (lane >= o) ps += q;
+      }
+      if (lane == 31) { sc[warp] = __popc(m); sc[32 + warp] = ps; }
+      __syncthreads();
+      int pr_ = rows + __popc(m & ((1u << lane) - 1)), pv = voxels + ps - len, tr = 0, tv = 0;
+      for (int w = 0; w < nw; ++w) {
+        if (w < warp) { pr_ += sc[w]; pv += sc[32 + w]; }
+        tr += sc[w];
+        tv += sc[32 + w];
+      }
+      if (e) put(pr_, pv, i, e);
+      rows += tr;
+      voxels += tv;
+      __syncthreads();
+    }
+    return rows;
+  }
+
+  // First row whose preceding rows weigh at least `target`: prefix[k] is the
+  // weight before CTA k's even share of the rows.  One warp.
+  __device__ int boundary(const long long *prefix, long long target) const {
+    const int lane = threadIdx.x & 31, c = grid_row_overhead(Z);
+    int k = 0;
+    for (int q = lane; q < K; q += 32)
+      if (prefix[q] <= target) k = max(k, q);
+    k = __reduce_max_sync(kFull, k);
+    const long long rows = (long long)X * Y;
+    const int lo = (int)(rows * k / K), hi = (int)(rows * (k + 1) / K);
+    long long run = prefix[k];
+    if constexpr (Group::kGrid) {
+      for (int b = lo; b < hi; b += 32) {
+        const unsigned e = b + lane < hi ? __ldcg(g.ext + b + lane) : 0u;
+        const int w = e ? (int)(e >> 16) - (int)(e & 0xffffu) + c : 0;
+        int ps = w;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int q = __shfl_up_sync(kFull, ps, o);
+          if (lane >= o) ps += q;
+        }
+        const unsigned m = __ballot_sync(kFull, b + lane < hi && run + ps - w >= target);
+        if (m) return b + __ffs(m) - 1;
+        run += __shfl_sync(kFull, ps, 31);
+      }
+    }
+    return hi;
+  }
+
+  // The CTA's row list, the volume's masked voxels and the histogram's scale.
+  __device__ bool find_rows() {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int cnt = 0, rows = 0;   // the warp's masked voxels, the CTA's rows
+    if constexpr (Group::kGrid) {
+      // even shares of the rows are looked over first, then the rows are dealt
+      // out in contiguous ranges of equal weight
+      const long long nrows = (long long)X * Y;
+      const int q0 = (int)(nrows * rank / K), q1 = (int)(nrows * (rank + 1) / K);
+      const int c = grid_row_overhead(Z);
+      long long weight = 0;
+      for (int i = q0 + warp; i < q1; i += nw) {
+        int n;
+        const unsigned e = row_range(src + (size_t)i * Z, Z, n);
+        if (lane == 0) g.ext[i] = e;
+        cnt += n;
+        if (e) weight += (int)(e >> 16) - (int)(e & 0xffffu) + c;
+      }
+      long long *sc = (long long *)red();
+      if (lane == 0) sc[warp] = weight;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < nw; ++w) weight += sc[w];
+        *slotB() = (unsigned long long)weight;
+      }
+      if (!g.sync()) return false;
+      long long *prefix = at<long long>(pl.o_gd);   // K + 1 words, free before the first level
+      for (int k = threadIdx.x; k < K; k += blockDim.x) prefix[k + 1] = (long long)__ldcg(g.peer(slotB(), k));
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        prefix[0] = 0;
+        for (int k = 0; k < K; ++k) prefix[k + 1] += prefix[k];
+      }
+      __syncthreads();
+      int *bd = (int *)(red() + 120);
+      if (warp < 2) {
+        const int b = boundary(prefix, prefix[K] * (rank + warp) / K);
+        if (lane == 0) bd[warp] = b;
+      }
+      __syncthreads();
+      const int r0 = bd[0], r1 = rank == K - 1 ? (int)nrows : bd[1];
+      const unsigned *ext = g.ext;
+      auto range = [=](int i) { return __ldcg(ext + r0 + i); };
+      rows = list_rows(r1 - r0, range, [](int, int, int, unsigned) {});
+      if (threadIdx.x == 0) {
+        nact = rows;
+        const bool in = (long long)rows * 16 <= pl.pool_bytes / 4;
+        const int used = in ? (rows * 16 + 127) / 128 * 128 : 0;
+        rowsp = in ? at<int4>(pl.o_pool) : (int4 *)(big + pl.b_rows);
+        slab_off = pl.o_pool + used;
+        slab_cap = (pl.pool_bytes - used) / 4;
+        slab_g = (float *)(big + pl.b_imlog);
+        gdp = (long long)rows * pl.NCZ * 4 <= pl.gd_bytes ? at<float>(pl.o_gd) : (float *)(big + pl.b_Gd);
+        bd[0] = 0x7fffffff;
+        bd[1] = -1;
+      }
+      __syncthreads();
+      int4 *out = rowsp;
+      const int yy = Y;
+      list_rows(r1 - r0, range, [=](int r, int v, int i, unsigned e) {
+        const int vx = (r0 + i) / yy;
+        out[r] = make_int4(v - (int)(e & 0xffffu), (int)e, vx, r0 + i - vx * yy);
+        if (r == 0) bd[0] = vx;
+        if (r == rows - 1) bd[1] = vx;
+      });
+      if (threadIdx.x == 0) {
+        vx0 = rows ? bd[0] : 0;
+        np = rows ? bd[1] - bd[0] + 1 : 0;
+      }
+      __syncthreads();
+      for (int r = threadIdx.x; r < rows; r += blockDim.x) out[r].z -= vx0;
+    } else {
+      const int nplane = X > rank ? (X - rank + K - 1) / K : 0, nrow = nplane * Y;
+      const float *slab = at<float>(pl.sm_bytes + pl.b_imlog);
+      unsigned *ext = at<unsigned>(pl.sm_bytes + pl.b_Gd);   // free before the first level
+      for (int i = warp; i < nrow; i += nw) {
+        int n;
+        const unsigned e = row_range(slab + (size_t)i * Z, Z, n);
+        if (lane == 0) ext[i] = e;
+        cnt += n;
+      }
+      // a plane's rows are listed from its first to its last row with a masked
+      // voxel, empty ones between them as the empty range [1, 1)
+      int *ya = at<int>(pl.sm_bytes + pl.b_T2), *yb = ya + nplane;
+      for (int m = threadIdx.x; m < nplane; m += blockDim.x) { ya[m] = Y; yb[m] = -1; }
+      __syncthreads();
+      const int yy = Y;
+      for (int i = threadIdx.x; i < nrow; i += blockDim.x)
+        if (ext[i]) {
+          atomicMin(&ya[i / yy], i % yy);
+          atomicMax(&yb[i / yy], i % yy);
+        }
+      __syncthreads();
+      uint2 *out = at<uint2>(pl.o_rows);
+      auto range = [=](int i) {
+        const unsigned e = ext[i];
+        return e || i % yy < ya[i / yy] || i % yy > yb[i / yy] ? e : 0x10001u;
+      };
+      rows = list_rows(nrow, range, [=](int r, int, int i, unsigned e) {
+        const int m = i / yy;
+        out[r] = make_uint2(e, (unsigned)m << 16 | (unsigned)(i - m * yy));
+      });
+      nact = rows;
+      np = nplane;
+      vx0 = 0;
+    }
+    __syncthreads();
+    // most voxels one histogram copy can get: rows go to warps, and so to
+    // copies, in list order (pass_b)
+    int *copies = (int *)(red() + 128);
+    if (threadIdx.x < kHistCopies) copies[threadIdx.x] = 0;
+    __syncthreads();
+    const int rs = 5 - row_lanes_log2(Z);
+    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
+      const Row o = row(r);
+      atomicAdd(&copies[(r >> rs) % kHistCopies], o.z1 - o.z0);
+    }
+    __syncthreads();
+    int most = 0;
+    for (int k = 0; k < kHistCopies; ++k) most = max(most, copies[k]);
+    __syncthreads();
+    // the group's masked voxels and its fullest copy; the copies' sums stay
+    // below 2^32, and the scale does not depend on a batch's other volumes
+    if (!reduce_stats(0.0f, (float)most, lane == 0 ? (double)cnt : 0.0, 0.0, true, [] {})) return false;
+    if (writer()) {
+      nfg = iter().st[2];
+      // an even eighth of a CTA's voxels (its planes whole) and 160 more, or
+      // the fullest copy's voxels where they are more
+      const long long even = Group::kGrid ? 0 : ((long long)(X + K - 1) / K * Y * Z + 7) / 8 + 160;
+      hshift = hist_shift_for(max(even, (long long)(iter().st[1] * 1.000001) + 1));
+    }
+    publish();
+    return true;
+  }
+
+  // ---- the whole volume (im_log read from job.imlog; cluster path: the slab
+  // holds the local rows of im_log on entry)
   __device__ void run(const VolJob &job) {
     if (writer()) {
       X = job.X; Y = job.Y; Z = job.Z;
       rank = g.rank(); K = g.size();
-      if constexpr (Group::kGrid) {  // contiguous rows: the volume lives in global memory
-        r0 = (int)((long long)X * Y * rank / K);
-        nrow = (int)((long long)X * Y * (rank + 1) / K) - r0;
-        nplane = 0;
-      } else {                       // interleaved planes: every CTA samples the whole volume
-        r0 = 0;
-        nplane = X > rank ? (X - rank + K - 1) / K : 0;
-        nrow = nplane * Y;
-      }
-      divZ = FastDiv((unsigned)Z);
-      hshift = volume_hist_shift(X, Y, Z, K, Group::kGrid);
+      nact = 0; np = 0; vx0 = 0; hshift = 0;
+      nfg = 1.0;
       src = job.imlog;
     }
     publish();
@@ -820,23 +1269,8 @@ struct Engine {
       ph_acc[PH_N] = clock64();
     }
 #endif
-    fft_twiddles(tw, pl.npad);
-    // foreground count of the group
-    float cnt = 0.0f;
-    double cntd = 0.0;
-    for (int i = threadIdx.x; i < nrow * Z; i += blockDim.x) {
-      const int rl = (int)divZ.div((unsigned)i);
-      cnt += isnan(Group::kGrid ? src_row(rl)[i - rl * Z] : logu[i]) ? 0.0f : 1.0f;   // cluster: staged
-    }
-    cntd = cnt;
-    double loc[4], st[4];
-    block_reduce4(0.0f, 0.0f, cntd, 0.0, red + 8, loc);
-    if (threadIdx.x == 0) red[4] = loc[2];
-    __syncthreads();
-    loc[0] = 0.0; loc[1] = 0.0; loc[2] = red[4]; loc[3] = 0.0;
-    __syncthreads();
-    if (!reduce_stats(loc, st)) { if (lead) rep->status = N4_ERR_TIMEOUT; return; }
-    const double nfg = st[2];
+    fft_twiddles(at<double2>(pl.o_tw), pl.npad);
+    if (!find_rows()) { if (lead) rep->status = N4_ERR_TIMEOUT; return; }
     if (lead) { rep->foreground = (long long)nfg; rep->levels = 0; rep->warm_start_used = 0; }
     if (nfg < 1.0) {
       if (rank == 0) {
@@ -848,22 +1282,22 @@ struct Engine {
 
     // first-level lattice
     set_level(0);
-    for (int c = threadIdx.x; c < nlat; c += blockDim.x) L[c] = job.warm ? job.warm[c] : 0.0f;
+    for (int c = threadIdx.x; c < nlat; c += blockDim.x) L()[c] = job.warm ? job.warm[c] : 0.0f;
     __syncthreads();
 
     for (int level = 0; level < pl.levels; ++level) {
       if (level > 0) {
         const int pcx = ncx, pcy = ncy, pcz = ncz;
-        refine_lattice(L, pcx, pcy, pcz, tmp);
+        refine_lattice(L(), pcx, pcy, pcz, tmp());
         __syncthreads();
         set_level(level);
-        for (int c = threadIdx.x; c < nlat; c += blockDim.x) L[c] = tmp[c];
+        for (int c = threadIdx.x; c < nlat; c += blockDim.x) L()[c] = tmp()[c];
         __syncthreads();
       }
       // logU of this level's lattice, then the constant denominator of the fit
-      reset(L, level == 0 && !Group::kGrid);
-      contract(false);
-      if (!allreduce(slotC, den, nlat)) goto timeout;
+      reset(L(), level == 0 && !Group::kGrid);
+      float *dn = den();
+      if (!contract<false>([=](int c, float v) { dn[c] = v; })) goto timeout;
       const int maxIt = pr.iters[level];
       int it = 0;
       float cv = 1e10f;
@@ -874,30 +1308,29 @@ struct Engine {
         // behind L, as the main loop expects after an iteration.
         float cvs[2];
         for (int arm = 0; arm < 2; ++arm) {
-          for (int c = threadIdx.x; c < nlat; c += blockDim.x) L[c] = arm == 0 ? job.warm[c] : 0.0f;
+          for (int c = threadIdx.x; c < nlat; c += blockDim.x) L()[c] = arm == 0 ? job.warm[c] : 0.0f;
           __syncthreads();
-          if (arm == 1) reset(L);   // arm 0 starts from the level's reset (L = warm)
-          if (!pass_a(false, false, st)) goto timeout;
-          if (!fit_step(st)) goto timeout;
-          rowtab(D, Gd);
-          for (int c = threadIdx.x; c < nlat; c += blockDim.x) L[c] += D[c];
-          __syncthreads();
-          if (!pass_a(true, false, st)) goto timeout;   // the update's CV; logU not advanced
-          cvs[arm] = cv_from(st, nfg);
+          if (arm == 1) reset(L());   // arm 0 starts from the level's reset (L = warm)
+          if (!pass_a(false, false)) goto timeout;
+          if (!fit_step(false)) goto timeout;
+          if (!pass_a(true, false)) goto timeout;   // the update's CV; logU not advanced
+          cvs[arm] = iter().cv;
           if (arm == 0) {   // keep the warm result in aux, its update in tmp
-            for (int c = threadIdx.x; c < nlat; c += blockDim.x) { aux[c] = L[c]; tmp[c] = D[c]; }
-            __syncthreads();
+            for (int c = threadIdx.x; c < nlat; c += blockDim.x) { aux()[c] = L()[c]; tmp()[c] = D()[c]; }
           }
+          __syncthreads();
         }
         const bool use_warm = cvs[0] <= cvs[1];
         if (use_warm) {
           // logU back to the warm lattice, L and D to the warm arm's update
           reset(job.warm);
-          for (int c = threadIdx.x; c < nlat; c += blockDim.x) { L[c] = aux[c]; D[c] = tmp[c]; }
-          __syncthreads();
-          rowtab_planes(D, Gd);
+          for (int c = threadIdx.x; c < nlat; c += blockDim.x) { L()[c] = aux()[c]; D()[c] = tmp()[c]; }
           __syncthreads();
         }
+        // pass A left the histogram copies in the Gd region
+        if (use_warm) rowtab_planes(D());
+        else rowtab(D());
+        __syncthreads();
         cv = use_warm ? cvs[0] : cvs[1];
         it = 1;
         if (lead) {
@@ -908,36 +1341,47 @@ struct Engine {
       }
       N4_MARK(PH_SETUP);
       for (;;) {
-        if (!pass_a(it > 0, it > 0, st)) goto timeout;   // applies the last update
+        if (!pass_a(it > 0, it > 0)) goto timeout;   // applies the last update
         N4_MARK(PH_A);
-        if (it > 0) cv = cv_from(st, nfg);
+        if (it > 0) cv = iter().cv;
         if (!((double)cv > pr.thr) || it >= maxIt) break;
-        if (!fit_step(st)) goto timeout;
-        for (int c = threadIdx.x; c < nlat; c += blockDim.x) L[c] += D[c];
-        __syncthreads();
-        rowtab_planes(D, Gd);
-        __syncthreads();
-        N4_MARK(PH_UPDATE);
+        if (!fit_step()) goto timeout;
         ++it;
       }
       if (lead) { rep->iterations[level] = it; rep->final_cv[level] = cv; rep->levels = level + 1; }
     }
     if (rank == 0) {
-      for (int c = threadIdx.x; c < nlat; c += blockDim.x) job.lattice_out[c] = L[c];
+      for (int c = threadIdx.x; c < nlat; c += blockDim.x) job.lattice_out[c] = L()[c];
       if (threadIdx.x == 0) { rep->status = N4_OK; rep->device_end_ns = global_ns(); }
     }
 #ifdef N4_PHASE_TIMERS
     if (lead)
-      printf("N4PHASE K=%d nt=%d setup=%lld A=%lld Aloop=%lld Ared=%lld Bzero=%lld Bloop=%lld Bmerge=%lld Bred=%lld "
-             "Bconv=%lld sharp=%lld C=%lld T1=%lld T2=%lld P=%lld Fred=%lld update=%lld\n",
+      printf("N4PHASE K=%d nt=%d setup=%lld A=%lld Aloop=%lld Ared=%lld Bloop=%lld Bmerge=%lld Bred=%lld "
+             "sharp=%lld T1=%lld T2=%lld P=%lld Fred=%lld update=%lld\n",
              K, (int)blockDim.x, ph_acc[PH_SETUP], ph_acc[PH_A], ph_acc[PH_A_LOOP], ph_acc[PH_A_RED],
-             ph_acc[PH_B_ZERO], ph_acc[PH_B_LOOP], ph_acc[PH_B_MERGE], ph_acc[PH_B_RED], ph_acc[PH_B],
-             ph_acc[PH_SHARP], ph_acc[PH_C], ph_acc[PH_F_T1], ph_acc[PH_F_T2], ph_acc[PH_F_P], ph_acc[PH_F_RED],
-             ph_acc[PH_UPDATE]);
+             ph_acc[PH_B_LOOP], ph_acc[PH_B_MERGE], ph_acc[PH_B_RED], ph_acc[PH_SHARP], ph_acc[PH_F_T1],
+             ph_acc[PH_F_T2], ph_acc[PH_F_P], ph_acc[PH_F_RED], ph_acc[PH_UPDATE]);
 #endif
     return;
   timeout:
     if (lead) rep->status = N4_ERR_TIMEOUT;
+  }
+};
+
+// Sum over a cluster's partials of one entry: exact for the integer
+// histogram, Kahan-compensated for the fit's float partials.
+template <class Group>
+template <class T>
+struct Engine<Group>::SumOf {
+  T s = 0;
+  KahanSum k;
+  __device__ __forceinline__ void add(T x) {
+    if constexpr (sizeof(T) == 4) k.add(x);
+    else s += x;
+  }
+  __device__ __forceinline__ T value() const {
+    if constexpr (sizeof(T) == 4) return k.value();
+    else return s;
   }
 };
 
@@ -947,8 +1391,8 @@ template <class Group>
 struct EngineSlot {
   static_assert(Engine<Group>::kShared, "only the whole-GPU path keeps its Engine in shared memory");
   alignas(16) unsigned char raw[sizeof(Engine<Group>)];
-  __device__ Engine<Group> &make(const Group &g, const Plan &p, const Params &r, char *sm, char *big, float *rg) {
-    if (threadIdx.x == 0) new (raw) Engine<Group>(g, p, r, sm, big, rg);
+  __device__ Engine<Group> &make(const Group &g, const Plan &p, const Params &r, char *big) {
+    if (threadIdx.x == 0) new (raw) Engine<Group>(g, p, r, big);
     __syncthreads();
     return *reinterpret_cast<Engine<Group> *>(raw);
   }

@@ -287,8 +287,6 @@ __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ Cl
   }
   __syncthreads();
   ClusterGroup g;
-  char *sm = smem;
-  char *big = smem + s_pl.sm_bytes;
   unsigned phase = 0;
   for (;;) {
     if (g.rank() == 0 && threadIdx.x == 0) s_job = atomicAdd(a.queue, 1);
@@ -299,7 +297,7 @@ __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ Cl
     const VolJob &job = a.jobs[a.order[j]];
     const int rank = g.rank(), K = g.size();
     const int nplane = job.X > rank ? (job.X - rank + K - 1) / K : 0;
-    float *slab = (float *)(big + s_pl.b_imlog);
+    float *slab = (float *)(smem + s_pl.sm_bytes + s_pl.b_imlog);
     // planes rank, rank + K, ... (each Y*Z contiguous floats)
     int ok = stage_rows(job.imlog, rank, K, nplane, job.Y * job.Z, slab, &s_mbar, phase, a.use_tma != 0) ? 1 : 0;
     if (!ok && threadIdx.x == 0) job.report->status = N4_ERR_TIMEOUT;
@@ -316,7 +314,7 @@ __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ Cl
       if (!ok) mbar_wait(&s_mbar, phase ^ 1u);
       break;
     }
-    Engine<ClusterGroup> e(g, s_pl, s_pr, sm, big, nullptr);
+    Engine<ClusterGroup> e(g, s_pl, s_pr, nullptr);
     e.run(job);   // the slab holds the staged rows
   }
 }
@@ -328,20 +326,20 @@ struct GridArgs {
   char *big_base;
   size_t big_stride;
   GridBarrier bar;
-  float *red_global;
+  unsigned long long *acc;   // [3][acc_len], zero
+  int acc_len;
+  unsigned *ext;             // [X*Y]
 };
 
 template <int NT>
 __global__ void __launch_bounds__(NT, 1) k_n4_grid(const __grid_constant__ GridArgs a) {
-  extern __shared__ __align__(128) char smem[];
   __shared__ Plan s_pl;
   __shared__ Params s_pr;
   if (threadIdx.x == 0) { s_pl = a.pl; s_pr = a.pr; }
   __syncthreads();
-  GridGroup g{a.bar, a.big_base, a.big_stride};
-  char *big = a.big_base + (size_t)blockIdx.x * a.big_stride;
+  GridGroup g{a.bar, a.big_base, a.big_stride, a.acc, a.acc_len, a.ext};
   __shared__ EngineSlot<GridGroup> s_eng;
-  Engine<GridGroup> &e = s_eng.make(g, s_pl, s_pr, smem, big, a.red_global);
+  Engine<GridGroup> &e = s_eng.make(g, s_pl, s_pr, a.big_base + (size_t)blockIdx.x * a.big_stride);
   e.run(a.job);
 }
 
@@ -961,8 +959,8 @@ __global__ void k_sharpen(const unsigned long long *hist, const double *stats, i
   if (stats[3] > 0.0) {
     SharpenBufs sb{fa, fb, tw, Ff};
     const double inv = ldexp(1.0, -shift);
-    sharpen_map([=](int b) { return (double)hist[b] * inv; }, bins, npad, hoff, stats[0], stats[2], wiener, fwhm,
-                sb, E);
+    sharpen_map([=](int b) { return (double)hist[b] * inv; }, bins, npad, hoff, stats[0], stats[2], wiener,
+                gauss_of(stats[2], fwhm), sb, E);
     for (int b = threadIdx.x; b < bins; b += blockDim.x) E_out[b] = E[b];
   } else {
     for (int b = threadIdx.x; b < bins; b += blockDim.x) E_out[b] = 0.0;

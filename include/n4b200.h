@@ -48,8 +48,8 @@ typedef enum {
  * overriding the autotuner; N4_ERR_TOO_LARGE when a volume's share does not
  * fit one CTA's shared memory.  0 = choose automatically. */
 #define N4_FLAG_CLUSTER_SIZE(k) (((unsigned int)(k) & 31u) << 8)
-/* Bit 13: 512 threads per CTA instead of 1024 (twice the registers per
- * thread); overrides the autotuner's choice of threads. */
+/* Bit 13: 512 threads per CTA (the cluster path's default; the whole-GPU path
+ * takes 1024 for large volumes); overrides the autotuner's choice of threads. */
 #define N4_FLAG_CTA_512         0x2000u
 /* Bit 14: every mask pointer of a run (n4_run, n4_run_host, n4_run_batched*,
  * n4_batch_graph_create*, n4_warm_inputs, n4_autotune) points to uint8_t
