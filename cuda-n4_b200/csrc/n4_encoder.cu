@@ -56,48 +56,116 @@ struct Div {
   __device__ __forceinline__ int q(int k) const { return (int)(((unsigned long long)(unsigned)k * M) >> 40); }
 };
 
+// Sixteen consecutive k of one operand row, as bf16 pairs (low half first).
+struct Vals {
+  unsigned v[8];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0u;
+  }
+  __device__ __forceinline__ void put(int j, bf16 x) {   // j a constant after unrolling, the word clear before
+    v[j >> 1] |= (unsigned)__bfloat16_as_ushort(x) << (16 * (j & 1));
+  }
+  __device__ __forceinline__ void half(int h, const uint4 &q) {
+    v[4 * h] = q.x; v[4 * h + 1] = q.y; v[4 * h + 2] = q.z; v[4 * h + 3] = q.w;
+  }
+};
+
+// p[j], j < min(nv, 16), the others 0; `vec`: p is 16-byte aligned.
+__device__ __forceinline__ void load_run(Vals &o, const bf16 *p, int nv, bool vec) {
+  o.clear();
+  if (vec && nv >= 16) {
+    o.half(0, *(const uint4 *)p);
+    o.half(1, *(const uint4 *)(p + 8));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < nv) o.put(j, p[j]);
+  }
+}
+// p[j * stride], j < min(nv, 16).
+__device__ __forceinline__ void load_strided(Vals &o, const bf16 *p, size_t stride, int nv) {
+  o.clear();
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (j < nv) o.put(j, p[j * stride]);
+}
+
+// One row of a gather over the 27 taps of a 3x3x3 window: k = 27 c + t reads
+// p[c * stride + tap[t]] when bit t of `mask` is set (the tap meets a voxel),
+// 0 otherwise.  The window's bounds are in the mask, once per row.
+struct TapRow {
+  const bf16 *p;
+  unsigned mask;
+};
+__device__ __forceinline__ void load_taps(Vals &o, const TapRow &r, const int *tap, int stride, int k, int nv) {
+  o.clear();
+  int c = k / 27, t = k - c * 27;
+  const bf16 *q = r.p + (ptrdiff_t)c * stride;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    if (j < nv && (r.mask >> t & 1u)) o.put(j, q[tap[t]]);
+    if (++t == 27) { t = 0; q += stride; }
+  }
+}
+
 // C[m][n] = sum_k A(m,k) B(k,n) over this block's K range; P supplies the
-// sizes, the gathers and the store.  128 threads: 4 warps of 32x32.  Tile
-// staging: each thread owns half a row of the A tile and half a row of the
-// B tile (16 consecutive k), so the row's index decomposition (P::a_row,
-// P::b_row) is done once per block and the k decomposition uses constant
-// divisors or Div; the 16 values go to shared memory as two 16-byte stores.
-template <class P>
+// sizes, the loads of 16 consecutive k of a row (load_a, load_b; the row's
+// index decomposition once per block in a_row, b_row), tap offsets of window
+// gathers (tap, in shared memory) and the store.  128 threads, a 64 x NT tile
+// (NT = 16, 32, 64: the smallest that holds N, so that a layer of 16 channels
+// does not stage and multiply 48 columns of zeros): 4 warps of 16x16, 32x16 or
+// 32x32.  A thread stages half a row of the A tile and, up to 2 NT threads,
+// of the B tile; the next tile is loaded into registers while this one is
+// multiplied.  The sums' order over k does not depend on the tile.
+template <class P, int NT>
 __global__ void __launch_bounds__(128) k_igemm(const P p) {
   __shared__ __align__(16) bf16 As[BM][BK + PAD];
-  __shared__ __align__(16) bf16 Bs[BN][BK + PAD];
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  __shared__ __align__(16) bf16 Bs[NT][BK + PAD];
+  __shared__ int tap[27];
+  constexpr int WX = NT == 16 ? 1 : 2;             // warps along n
+  constexpr int WM = BM / (4 / WX), WN = NT / WX;  // a warp's tile
+  constexpr int MI = WM / 16, NJ = WN / 8;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * NT;
   const int kper = ((p.K + gridDim.z - 1) / gridDim.z + BK - 1) / BK * BK;
   const int kb = blockIdx.z * kper, ke = min(p.K, kb + kper);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const int wm = (warp / WX) * WM, wn = (warp % WX) * WN;
   const int sr = threadIdx.x >> 1, sc = (threadIdx.x & 1) * 16;   // staged row, first column
-  const bool a_ok = m0 + sr < p.M, b_ok = n0 + sr < p.N;
+  if (threadIdx.x < 27) tap[threadIdx.x] = p.tap(threadIdx.x);
+  __syncthreads();
+  const bool a_ok = m0 + sr < p.M, b_ok = sr < NT && n0 + sr < p.N;
   const typename P::ARow ar = p.a_row(a_ok ? m0 + sr : 0);
   const typename P::BRow br = p.b_row(b_ok ? n0 + sr : 0);
-  float acc[2][4][4] = {};
-  const bf16 zero = __float2bfloat16(0.0f);
-  for (int k0 = kb; k0 < ke; k0 += BK) {
-    unsigned pa[8], pb[8];   // bf16 pairs, low half first
-#pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-      const int k = k0 + sc + j;
-      const bf16 a0 = (a_ok && k < ke) ? p.a(ar, k) : zero, a1 = (a_ok && k + 1 < ke) ? p.a(ar, k + 1) : zero;
-      const bf16 b0 = (b_ok && k < ke) ? p.b(br, k) : zero, b1 = (b_ok && k + 1 < ke) ? p.b(br, k + 1) : zero;
-      pa[j / 2] = (unsigned)__bfloat16_as_ushort(a0) | ((unsigned)__bfloat16_as_ushort(a1) << 16);
-      pb[j / 2] = (unsigned)__bfloat16_as_ushort(b0) | ((unsigned)__bfloat16_as_ushort(b1) << 16);
+  float acc[MI][NJ][4] = {};
+  Vals va, vb;
+  va.clear();
+  vb.clear();
+  const auto load = [&](int k0) {
+    const int k = k0 + sc, nv = ke - k;
+    if (a_ok && nv > 0) p.load_a(va, ar, tap, k, nv);
+    else va.clear();
+    if (sr < NT) {
+      if (b_ok && nv > 0) p.load_b(vb, br, tap, k, nv);
+      else vb.clear();
     }
-    *(uint4 *)&As[sr][sc] = make_uint4(pa[0], pa[1], pa[2], pa[3]);
-    *(uint4 *)&As[sr][sc + 8] = make_uint4(pa[4], pa[5], pa[6], pa[7]);
-    *(uint4 *)&Bs[sr][sc] = make_uint4(pb[0], pb[1], pb[2], pb[3]);
-    *(uint4 *)&Bs[sr][sc + 8] = make_uint4(pb[4], pb[5], pb[6], pb[7]);
+  };
+  if (kb < ke) load(kb);
+  for (int k0 = kb; k0 < ke; k0 += BK) {
+    *(uint4 *)&As[sr][sc] = make_uint4(va.v[0], va.v[1], va.v[2], va.v[3]);
+    *(uint4 *)&As[sr][sc + 8] = make_uint4(va.v[4], va.v[5], va.v[6], va.v[7]);
+    if (sr < NT) {
+      *(uint4 *)&Bs[sr][sc] = make_uint4(vb.v[0], vb.v[1], vb.v[2], vb.v[3]);
+      *(uint4 *)&Bs[sr][sc + 8] = make_uint4(vb.v[4], vb.v[5], vb.v[6], vb.v[7]);
+    }
     __syncthreads();
+    if (k0 + BK < ke) load(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 16) {
-      unsigned af[2][4], bfr[4][2];
+      unsigned af[MI][4], bfr[NJ][2];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
+      for (int i = 0; i < MI; ++i) {
         const int r = wm + 16 * i + g;
         af[i][0] = *(const unsigned *)&As[r][kk + 2 * tig];
         af[i][1] = *(const unsigned *)&As[r + 8][kk + 2 * tig];
@@ -105,22 +173,22 @@ __global__ void __launch_bounds__(128) k_igemm(const P p) {
         af[i][3] = *(const unsigned *)&As[r + 8][kk + 2 * tig + 8];
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < NJ; ++j) {
         const int c = wn + 8 * j + g;
         bfr[j][0] = *(const unsigned *)&Bs[c][kk + 2 * tig];
         bfr[j][1] = *(const unsigned *)&Bs[c][kk + 2 * tig + 8];
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
+        for (int j = 0; j < NJ; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MI; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int m = m0 + wm + 16 * i + g + (e >= 2 ? 8 : 0);
@@ -151,22 +219,27 @@ struct ConvFwd {
   const float *bias;
   bf16 *y;
   int relu;
-  struct ARow { const bf16 *xb; int id0, ih0, iw0; };   // batch image, corner of the 3x3x3 window
+  using ARow = TapRow;                 // the corner of the window; taps inside the image
   struct BRow { const bf16 *wn; };
+  __device__ int tap(int t) const { return (t / 9 * s.H + t / 3 % 3) * s.W + t % 3; }
   __device__ ARow a_row(int m) const {
     const int op = s.out_pos();
     const int b = m / op, r = m - b * op;
-    const int od = r / (s.Ho * s.Wo), oh = (r / s.Wo) % s.Ho, ow = r % s.Wo;
-    return ARow{x + (size_t)b * s.Ci * s.in_pos(), 2 * od - 1, 2 * oh - 1, 2 * ow - 1};
+    const int id = 2 * (r / (s.Ho * s.Wo)) - 1, ih = 2 * (r / s.Wo % s.Ho) - 1, iw = 2 * (r % s.Wo) - 1;
+    unsigned mask = 0;
+    for (int t = 0; t < 27; ++t) {
+      const int d = id + t / 9, h = ih + t / 3 % 3, w2 = iw + t % 3;
+      if (d >= 0 && d < s.D && h >= 0 && h < s.H && w2 >= 0 && w2 < s.W) mask |= 1u << t;
+    }
+    return ARow{x + (ptrdiff_t)b * s.Ci * s.in_pos() + ((ptrdiff_t)id * s.H + ih) * s.W + iw, mask};
   }
-  __device__ bf16 a(const ARow &R, int k) const {
-    const int ci = k / 27, t = k - ci * 27;
-    const int id = R.id0 + t / 9, ih = R.ih0 + (t / 3) % 3, iw = R.iw0 + t % 3;
-    if (id < 0 || id >= s.D || ih < 0 || ih >= s.H || iw < 0 || iw >= s.W) return __float2bfloat16(0.0f);
-    return R.xb[((size_t)ci * s.D + id) * s.H * s.W + ih * s.W + iw];
+  __device__ void load_a(Vals &o, const ARow &R, const int *tp, int k, int nv) const {
+    load_taps(o, R, tp, s.in_pos(), k, nv);
   }
   __device__ BRow b_row(int n) const { return BRow{w + (size_t)n * K}; }
-  __device__ bf16 b(const BRow &R, int k) const { return R.wn[k]; }
+  __device__ void load_b(Vals &o, const BRow &R, const int *, int k, int nv) const {
+    load_run(o, R.wn + k, nv, (((uintptr_t)w | (unsigned)K * 2u) & 15u) == 0);
+  }
   __device__ void store(int m, int n, int, float v) const {
     const int op = s.out_pos();
     const int b = m / op, r = m - b * op;
@@ -176,76 +249,243 @@ struct ConvFwd {
   }
 };
 
-// dy masked by the ReLU of the forward output
-__device__ __forceinline__ float dact(const bf16 *dy, const bf16 *y, size_t i, int relu) {
-  const float g = __bfloat162float(dy[i]);
-  return (relu && __bfloat162float(y[i]) <= 0.0f) ? 0.0f : g;
+// The gradient of a ReLU's input: g where its output `y` is positive.
+__device__ __forceinline__ bf16 relu_grad(float g, bf16 y) {
+  return __bfloat162float(y) <= 0.0f ? __float2bfloat16(0.0f) : __float2bfloat16(g);
 }
 
-// dx = conv_transpose(dy', w): M = B*inpos, N = Ci, K = Co*27
+// dx = conv_transpose(dy, w) masked by the ReLU that made x: a GEMM of the
+// input positions (rows) by Ci, over K = Co*27.  Input position i meets output
+// (i + 1 - kd) / 2 where that is whole: with f = floor((i + 1) / 2) it is
+// f - (kd >> 1), for kd = 1 when i is even and kd = 0, 2 when it is odd.  So of
+// the 27 taps of a channel only 1, 2, 4 or 8 meet an output, the same ones for
+// all positions of one parity class (8 classes).
 struct ConvDgrad {
-  int M, N, K;
   Shape s;
-  const bf16 *dy, *y, *w;
+  const bf16 *dy, *x, *w;
   bf16 *dx;
-  int relu;
-  struct ARow { size_t base; int pd0, ph0, pw0; };   // batch offset in dy, input position + 1
-  struct BRow { int n; };
-  __device__ ARow a_row(int m) const {
-    const int ip = s.in_pos();
-    const int b = m / ip, r = m - b * ip;
-    const int id = r / (s.H * s.W), ih = (r / s.W) % s.H, iw = r % s.W;
-    return ARow{(size_t)b * s.Co * s.out_pos(), id + 1, ih + 1, iw + 1};
-  }
-  __device__ bf16 a(const ARow &R, int k) const {
-    const int co = k / 27, t = k - co * 27;
-    const int pd = R.pd0 - t / 9, ph = R.ph0 - (t / 3) % 3, pw = R.pw0 - t % 3;
-    if ((pd | ph | pw) & 1) return __float2bfloat16(0.0f);   // also rejects odd negatives
-    const int od = pd >> 1, oh = ph >> 1, ow = pw >> 1;
-    if (pd < 0 || ph < 0 || pw < 0 || od >= s.Do || oh >= s.Ho || ow >= s.Wo) return __float2bfloat16(0.0f);
-    const size_t i = R.base + (size_t)co * s.out_pos() + (od * s.Ho + oh) * s.Wo + ow;
-    return __float2bfloat16(dact(dy, y, i, relu));
-  }
-  __device__ BRow b_row(int n) const { return BRow{n}; }
-  __device__ bf16 b(const BRow &R, int k) const {
-    const int co = k / 27, t = k - co * 27;
-    return w[((size_t)co * s.Ci + R.n) * 27 + t];
-  }
-  __device__ void store(int m, int n, int, float v) const {
-    const int ip = s.in_pos();
-    const int b = m / ip, r = m - b * ip;
-    dx[((size_t)b * s.Ci + n) * ip + r] = __float2bfloat16(v);
+  // positions of one axis with parity p, and rows of class c (parities of d,
+  // h, w in bits 2, 1, 0) over the batch
+  static __host__ __device__ int axis_count(int n, int p) { return (n + 1 - p) >> 1; }
+  __host__ __device__ int rows(int c) const {
+    return s.B * axis_count(s.D, c >> 2) * axis_count(s.H, c >> 1 & 1) * axis_count(s.W, c & 1);
   }
 };
 
-// dw partials: M = Co, N = Ci*27, K = B*outpos (split over blockIdx.z)
+// 64 rows of one parity class by NT columns; 128 threads, 4 warps of 16xNT
+// (NT = 16) or 32x(NT/2).  Only the columns k whose tap the class meets are
+// loaded: threads 0-63 a row of A each, threads 64-127 the rows of B; A's other
+// columns stay zero, and K steps of 16 without any are not multiplied.  The
+// next step's values are in registers while this one is multiplied.  The sums
+// take the terms over k in the order of a dense GEMM.  (As a dense implicit
+// GEMM over all 27 taps, rows in memory order, the three layers of a batch of
+// 64 took 121, 124 and 259 us, bound by the gather's instructions.)
+template <int NT>
+__global__ void __launch_bounds__(128) k_dgrad(const ConvDgrad p) {
+  __shared__ __align__(16) bf16 As[BM][BK + PAD];
+  __shared__ __align__(16) bf16 Bs[NT][BK + PAD];
+  __shared__ int tap[27];
+  constexpr int WX = NT == 16 ? 1 : 2;
+  constexpr int WM = BM / (4 / WX), WN = NT / WX;
+  constexpr int MI = WM / 16, NJ = WN / 8;
+  constexpr int kMost = 11;   // most columns of 32 that a class of 8 taps meets
+  const Shape &s = p.s;
+  int cls = 0, tile = blockIdx.x;
+  for (; cls < 7; ++cls) {
+    const int n = (p.rows(cls) + BM - 1) / BM;
+    if (tile < n) break;
+    tile -= n;
+  }
+  const int pd = cls >> 2, ph = cls >> 1 & 1, pw = cls & 1;
+  const int nd = ConvDgrad::axis_count(s.D, pd), nh = ConvDgrad::axis_count(s.H, ph), nw = ConvDgrad::axis_count(s.W, pw);
+  const int rows = p.rows(cls), row0 = tile * BM, n0 = blockIdx.y * NT;
+  const int K = s.Co * 27, op = s.out_pos(), ip = s.in_pos();
+  // the class's taps, as a bit per (kd, kh, kw), and three periods of them
+  const auto taps = [&](unsigned md, unsigned mh, unsigned mw) {
+    unsigned m = 0;
+    for (int t = 0; t < 27; ++t)
+      if ((md >> t / 9 & 1u) && (mh >> t / 3 % 3 & 1u) && (mw >> t % 3 & 1u)) m |= 1u << t;
+    return m;
+  };
+  const unsigned cmask = taps(pd ? 5u : 2u, ph ? 5u : 2u, pw ? 5u : 2u);
+  const unsigned long long period = cmask | (unsigned long long)cmask << 27 | (unsigned long long)cmask << 54;
+  if (threadIdx.x < 27) {
+    const int t = threadIdx.x;
+    tap[t] = -((((t / 9) >> 1) * s.Ho + ((t / 3 % 3) >> 1)) * s.Wo + ((t % 3) >> 1));
+  }
+  for (int i = threadIdx.x; i < BM * (BK + PAD) / 2; i += 128) ((unsigned *)As)[i] = 0u;
+  for (int i = threadIdx.x; i < NT * (BK + PAD) / 2; i += 128) ((unsigned *)Bs)[i] = 0u;
+  const bool loads_a = threadIdx.x < 64;
+  const int lr = threadIdx.x & 63;
+  // A: the row's base in dy and the taps that meet an output of it.  B: row
+  // lr % NT, every (64 / NT)-th column.
+  const bf16 *base = nullptr;
+  unsigned rmask = 0;
+  constexpr int BQ = 64 / NT;
+  const int bq = lr / NT, bn = n0 + lr % NT;
+  if (loads_a) {
+    const int q = row0 + lr;
+    if (q < rows) {
+      const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
+      const int fd = jd + pd, fh = jh + ph, fw = jw + pw;
+      const auto axis = [](int par, int f, int n) { return par ? (f < n ? 5u : 4u) : 2u; };
+      rmask = taps(axis(pd, fd, s.Do), axis(ph, fh, s.Ho), axis(pw, fw, s.Wo));
+      base = p.dy + (ptrdiff_t)b * s.Co * op + (fd * s.Ho + fh) * s.Wo + fw;
+    }
+  } else if (bn < s.Ci) {
+    rmask = cmask;
+    base = p.w + (size_t)bn * 27;
+  }
+  const size_t stride = loads_a ? (size_t)op : (size_t)s.Ci * 27;
+  __syncthreads();
+  const auto window = [&](int k0) {   // the columns of [k0, k0 + 32) the class meets
+    const unsigned w = (unsigned)(period >> (k0 % 27));
+    return K - k0 >= 32 ? w : w & ((1u << (K - k0)) - 1u);
+  };
+  bf16 v[kMost];
+  const auto load = [&](int k0) {
+    const int t0 = k0 % 27;
+    const bf16 *c = base + (size_t)(k0 / 27) * stride;
+    unsigned w = window(k0);
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+      if (!w) break;
+      int t = t0 + __ffs(w) - 1;
+      w &= w - 1;
+      const int over = (t >= 27) + (t >= 54);
+      t -= 27 * over;
+      v[i] = __float2bfloat16(0.0f);
+      if ((rmask >> t & 1u) && (loads_a || i % BQ == bq)) v[i] = c[over * stride + (loads_a ? tap[t] : t)];
+    }
+  };
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, tig = lane & 3;
+  const int wm = (warp / WX) * WM, wn = (warp % WX) * WN;
+  float acc[MI][NJ][4] = {};
+  unsigned last = 0;   // the columns of A's tile that are not zero
+  load(0);
+  for (int k0 = 0; k0 < K; k0 += BK) {
+    const unsigned now = window(k0);
+    if (loads_a) {
+      for (unsigned w = last & ~now; w; w &= w - 1) As[lr][__ffs(w) - 1] = __float2bfloat16(0.0f);
+    }
+    unsigned w = now;
+#pragma unroll
+    for (int i = 0; i < kMost; ++i) {
+      if (!w) break;
+      const int j = __ffs(w) - 1;
+      w &= w - 1;
+      if (loads_a) As[lr][j] = v[i];
+      else if (i % BQ == bq) Bs[lr % NT][j] = v[i];
+    }
+    last = now;
+    __syncthreads();
+    if (k0 + BK < K) load(k0 + BK);
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 16) {
+      if (!(now >> kk & 0xffffu)) continue;
+      unsigned af[MI][4], bfr[NJ][2];
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        const int r = wm + 16 * i + g;
+        af[i][0] = *(const unsigned *)&As[r][kk + 2 * tig];
+        af[i][1] = *(const unsigned *)&As[r + 8][kk + 2 * tig];
+        af[i][2] = *(const unsigned *)&As[r][kk + 2 * tig + 8];
+        af[i][3] = *(const unsigned *)&As[r + 8][kk + 2 * tig + 8];
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int c = wn + 8 * j + g;
+        bfr[j][0] = *(const unsigned *)&Bs[c][kk + 2 * tig];
+        bfr[j][1] = *(const unsigned *)&Bs[c][kk + 2 * tig + 8];
+      }
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int q = row0 + wm + 16 * i + g + 8 * h;
+      if (q >= rows) continue;
+      const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
+      const size_t at = (size_t)b * s.Ci * ip + ((2 * jd + pd) * s.H + 2 * jh + ph) * s.W + 2 * jw + pw;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int n = n0 + wn + 8 * j + 2 * tig + e;
+          if (n >= s.Ci) continue;
+          const size_t o = at + (size_t)n * ip;
+          p.dx[o] = relu_grad(acc[i][j][2 * h + e], p.x[o]);
+        }
+    }
+}
+
+// dw partials, and the bias gradient as one more column of ones: M = Co,
+// N = Ci*27 + 1, K = B*outpos (split over blockIdx.z)
 struct ConvWgrad {
   int M, N, K;
   Shape s;
-  const bf16 *x, *dy, *y;
-  float *part;   // [splits][Co][Ci*27]
-  int relu;
+  const bf16 *x, *dy;
+  float *part;   // [splits][Co][Ci*27 + 1]
   PosDiv pd;     // decomposition of a position index k into (b, od, oh, ow)
   struct ARow { int m; };
-  struct BRow { int ci, kd, kh, kw; };
+  struct BRow { int ci, kd, kh, kw; };   // ci = Ci: the column of ones
+  __device__ int tap(int) const { return 0; }
   __device__ ARow a_row(int m) const { return ARow{m}; }
-  __device__ bf16 a(const ARow &R, int k) const {
+  // an image's positions are a multiple of 8 (checked where the layers are
+  // laid out), so each half of a run lies in one image
+  __device__ void load_a(Vals &o, const ARow &R, const int *, int k, int nv) const {
     const int op = s.out_pos();
-    const int b = pd.op.q(k), r = k - b * op;
-    return __float2bfloat16(dact(dy, y, ((size_t)b * s.Co + R.m) * op + r, relu));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int kk = k + 8 * h;
+      uint4 q = make_uint4(0u, 0u, 0u, 0u);
+      if (8 * h < nv) {
+        const int b = pd.op.q(kk);
+        q = *(const uint4 *)(dy + ((size_t)b * s.Co + R.m) * op + (kk - b * op));
+      }
+      o.half(h, q);
+    }
   }
   __device__ BRow b_row(int n) const {
     const int ci = n / 27, t = n - ci * 27;
     return BRow{ci, t / 9 - 1, (t / 3) % 3 - 1, t % 3 - 1};
   }
-  __device__ bf16 b(const BRow &R, int k) const {
+  __device__ void load_b(Vals &o, const BRow &R, const int *, int k, int nv) const {
+    o.clear();
+    if (R.ci == s.Ci) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < nv) o.put(j, __float2bfloat16(1.0f));
+      return;
+    }
     const int op = s.out_pos();
-    const int bb = pd.op.q(k), r = k - bb * op;
-    const int od = pd.hw.q(r), r2 = r - od * s.Ho * s.Wo;
-    const int oh = pd.w.q(r2), ow = r2 - oh * s.Wo;
-    const int id = 2 * od + R.kd, ih = 2 * oh + R.kh, iw = 2 * ow + R.kw;
-    if (id < 0 || id >= s.D || ih < 0 || ih >= s.H || iw < 0 || iw >= s.W) return __float2bfloat16(0.0f);
-    return x[(((size_t)bb * s.Ci + R.ci) * s.D + id) * s.H * s.W + ih * s.W + iw];
+    const int b = pd.op.q(k), r = k - b * op;
+    int od = pd.hw.q(r);
+    const int r2 = r - od * s.Ho * s.Wo;
+    int oh = pd.w.q(r2), ow = r2 - oh * s.Wo;
+    const bf16 *img = x + ((size_t)b * s.Ci + R.ci) * s.in_pos();
+    const bf16 *row = img + ((2 * od + R.kd) * s.H + 2 * oh + R.kh) * s.W + R.kw;
+    bool in = (unsigned)(2 * od + R.kd) < (unsigned)s.D && (unsigned)(2 * oh + R.kh) < (unsigned)s.H;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (j < nv && in && (unsigned)(2 * ow + R.kw) < (unsigned)s.W) o.put(j, row[2 * ow]);
+      if (++ow == s.Wo) {
+        ow = 0;
+        if (++oh == s.Ho) {
+          oh = 0;
+          if (++od == s.Do) { od = 0; img += (size_t)s.Ci * s.in_pos(); }
+        }
+        row = img + ((2 * od + R.kd) * s.H + 2 * oh + R.kh) * s.W + R.kw;
+        in = (unsigned)(2 * od + R.kd) < (unsigned)s.D && (unsigned)(2 * oh + R.kh) < (unsigned)s.H;
+      }
+    }
   }
   __device__ void store(int m, int n, int z, float v) const { part[((size_t)z * M + m) * N + n] = v; }
 };
@@ -258,45 +498,87 @@ struct LinFwd {
   float *y;
   struct ARow { const bf16 *r; };
   struct BRow { const bf16 *r; };
+  __device__ int tap(int) const { return 0; }
   __device__ ARow a_row(int m) const { return ARow{x + (size_t)m * K}; }
-  __device__ bf16 a(const ARow &R, int k) const { return R.r[k]; }
+  __device__ void load_a(Vals &o, const ARow &R, const int *, int k, int nv) const {
+    load_run(o, R.r + k, nv, (((uintptr_t)x | (unsigned)K * 2u) & 15u) == 0);
+  }
   __device__ BRow b_row(int n) const { return BRow{w + (size_t)n * K}; }
-  __device__ bf16 b(const BRow &R, int k) const { return R.r[k]; }
+  __device__ void load_b(Vals &o, const BRow &R, const int *, int k, int nv) const {
+    load_run(o, R.r + k, nv, (((uintptr_t)w | (unsigned)K * 2u) & 15u) == 0);
+  }
   __device__ void store(int m, int n, int, float v) const { y[(size_t)m * N + n] = v + bias[n]; }
 };
-// dx = dy W: M = B, N = in, K = out
+// dx = dy W masked by the ReLU that made x: M = B, N = in, K = out
 struct LinDgrad {
   int M, N, K;
-  const bf16 *dy, *w;
+  const bf16 *dy, *x, *w;
   bf16 *dx;
   struct ARow { const bf16 *r; };
   struct BRow { int n; };
+  __device__ int tap(int) const { return 0; }
   __device__ ARow a_row(int m) const { return ARow{dy + (size_t)m * K}; }
-  __device__ bf16 a(const ARow &R, int k) const { return R.r[k]; }
+  __device__ void load_a(Vals &o, const ARow &R, const int *, int k, int nv) const {
+    load_run(o, R.r + k, nv, (((uintptr_t)dy | (unsigned)K * 2u) & 15u) == 0);
+  }
   __device__ BRow b_row(int n) const { return BRow{n}; }
-  __device__ bf16 b(const BRow &R, int k) const { return w[(size_t)k * N + R.n]; }
-  __device__ void store(int m, int n, int, float v) const { dx[(size_t)m * N + n] = __float2bfloat16(v); }
+  __device__ void load_b(Vals &o, const BRow &R, const int *, int k, int nv) const {
+    load_strided(o, w + (size_t)k * N + R.n, N, nv);
+  }
+  __device__ void store(int m, int n, int, float v) const {
+    const size_t i = (size_t)m * N + n;
+    dx[i] = relu_grad(v, x[i]);
+  }
 };
-// dW = dy^T x: M = out, N = in, K = B
+// dW = dy^T x, and the bias gradient as one more column of ones: M = out,
+// N = in + 1, K = B
 struct LinWgrad {
   int M, N, K;
   const bf16 *dy, *x;
   float *part;
   struct ARow { int m; };
   struct BRow { int n; };
+  __device__ int tap(int) const { return 0; }
   __device__ ARow a_row(int m) const { return ARow{m}; }
-  __device__ bf16 a(const ARow &R, int k) const { return dy[(size_t)k * M + R.m]; }
+  __device__ void load_a(Vals &o, const ARow &R, const int *, int k, int nv) const {
+    load_strided(o, dy + (size_t)k * M + R.m, M, nv);
+  }
   __device__ BRow b_row(int n) const { return BRow{n}; }
-  __device__ bf16 b(const BRow &R, int k) const { return x[(size_t)k * N + R.n]; }
+  __device__ void load_b(Vals &o, const BRow &R, const int *, int k, int nv) const {
+    if (R.n < N - 1) {
+      load_strided(o, x + (size_t)k * (N - 1) + R.n, N - 1, nv);
+    } else {
+      o.clear();
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < nv) o.put(j, __float2bfloat16(1.0f));
+    }
+  }
   __device__ void store(int m, int n, int z, float v) const { part[((size_t)z * M + m) * N + n] = v; }
 };
 
 // ------------------------------------------------------------------ small kernels
-__global__ void k_sum_splits(const float *part, int splits, int n, float *out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Weight and bias gradients from the partials of [M][N] sums, the last column
+// the bias: one warp per 32 entries, its lanes of a block's 8 warps taking every
+// eighth split in order, the eight sums added in order.
+__global__ void __launch_bounds__(256) k_sum_splits(const float *part, int splits, int M, int N, float *dw, float *db) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = M * N;
+  for (int i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {
+    const int i = i0 + lane;
     float s = 0.0f;
-    for (int z = 0; z < splits; ++z) s += part[(size_t)z * n + i];
-    out[i] = s;
+    if (i < n)
+      for (int z = warp; z < splits; z += 8) s += part[(size_t)z * n + i];
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < n) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) s += red[w][lane];
+      const int m = i / N, c = i - m * N;
+      if (c < N - 1) dw[(size_t)m * (N - 1) + c] = s;
+      else db[m] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -318,25 +600,6 @@ __global__ void k_finish(const P p, const float *part, int splits) {
     float s = 0.0f;
     for (int z = 0; z < splits; ++z) s += part[z * mn + i];
     p.store((int)(i / p.N), (int)(i % p.N), 0, s);
-  }
-}
-
-// bias gradient: sum of dy' over batch and positions, one block per channel
-__global__ void k_bias_grad(const bf16 *dy, const bf16 *y, int B, int C, int pos, int relu, float *db) {
-  const int c = blockIdx.x;
-  float s = 0.0f;
-  for (int i = threadIdx.x; i < B * pos; i += blockDim.x) {
-    const int b = i / pos, r = i - b * pos;
-    s += dact(dy, y, ((size_t)b * C + c) * pos + r, relu);
-  }
-  __shared__ float red[32];
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    db[c] = t;
   }
 }
 
@@ -380,8 +643,20 @@ __global__ void k_to_bf16(const float *a, int n, bf16 *b) {
 // ------------------------------------------------------------------ host side
 template <class P>
 cudaError_t run_gemm(const P &p, int splits, cudaStream_t st) {
-  dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN, splits);
-  k_igemm<P><<<grid, 128, 0, st>>>(p);
+  const int mb = (p.M + BM - 1) / BM;
+  if (p.N <= 16) k_igemm<P, 16><<<dim3(mb, 1, splits), 128, 0, st>>>(p);
+  // 32 columns also where 64-column tiles would leave most SMs without a block
+  else if (p.N <= 32 || (long long)mb * ((p.N + 63) / 64) * splits < 128)
+    k_igemm<P, 32><<<dim3(mb, (p.N + 31) / 32, splits), 128, 0, st>>>(p);
+  else k_igemm<P, 64><<<dim3(mb, (p.N + 63) / 64, splits), 128, 0, st>>>(p);
+  return cudaGetLastError();
+}
+
+inline cudaError_t run_dgrad(const ConvDgrad &p, cudaStream_t st) {
+  int tiles = 0;
+  for (int c = 0; c < 8; ++c) tiles += (p.rows(c) + BM - 1) / BM;
+  if (p.s.Ci <= 16) k_dgrad<16><<<dim3(tiles, (p.s.Ci + 15) / 16), 128, 0, st>>>(p);
+  else k_dgrad<32><<<dim3(tiles, (p.s.Ci + 31) / 32), 128, 0, st>>>(p);
   return cudaGetLastError();
 }
 
@@ -424,6 +699,8 @@ struct Layout {
       b[l] = o; o += kCh[l + 1];
       d = out_dim(d); h = out_dim(h); wd = out_dim(wd);
     }
+    static_assert(kIn[0] % 32 == 0 && kIn[1] % 32 == 0 && kIn[2] % 24 == 0,
+                  "every layer's output positions are a multiple of 8 (ConvWgrad)");
     w[kLayers] = o; o += (size_t)kOut * kFeat;
     b[kLayers] = o; o += kOut;
     total = o;
@@ -474,9 +751,12 @@ n4_status_t efail(n4_status_t s, const std::string &m) { return n4_record_error(
     cudaError_t e_ = (x);                                                                   \
     if (e_ != cudaSuccess) { cudaGetLastError(); return efail(N4_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); } \
   } while (0)
-constexpr int kSplitsMax = 128;
-
-int wgrad_splits(long long K) { return (int)std::min<long long>(kSplitsMax, std::max<long long>(1, K / 2048)); }
+// Splits of a weight gradient's sum over K positions: about four blocks per SM
+// (592) of at least four K steps each.
+int wgrad_splits(int M, int N, long long K) {
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  return (int)std::max<long long>(1, std::min<long long>(592 / tiles, K / (4 * BK)));
+}
 }  // namespace
 
 extern "C" {
@@ -515,10 +795,10 @@ n4_status_t n4_encoder_create(n4_encoder_t **out, int device, int max_batch) {
   // split-K partials: the largest weight gradient times the splits
   size_t need = 0;
   for (int l = 0; l < kLayers; ++l) {
-    const long long K = (long long)max_batch * L.s[l].out_pos();
-    need = std::max(need, (size_t)wgrad_splits(K) * L.s[l].Co * L.s[l].Ci * 27);
+    const int M = L.s[l].Co, N = L.s[l].Ci * 27 + 1;
+    need = std::max(need, (size_t)wgrad_splits(M, N, (long long)max_batch * L.s[l].out_pos()) * M * N);
   }
-  need = std::max(need, (size_t)wgrad_splits(max_batch) * kOut * kFeat);
+  need = std::max(need, (size_t)wgrad_splits(kOut, kFeat + 1, max_batch) * kOut * (kFeat + 1));
   // and the forward's split layers at every batch size up to max_batch
   const size_t unbounded = ~(size_t)0;
   for (int b = 1; b <= max_batch; ++b) {
@@ -605,31 +885,26 @@ n4_status_t n4_encoder_train_step(n4_encoder_t *e, const void *d_x, const float 
   n4_status_t s = forward(e, d_x, B, st);
   if (s != N4_OK) return s;
   Layout L(B);
-  k_mse<<<1, 256, 0, st>>>(e->out, d_target, B * kOut, e->loss, e->dout);
+  k_mse<<<1, 1024, 0, st>>>(e->out, d_target, B * kOut, e->loss, e->dout);
   ECK(cudaGetLastError());
   // linear head
   {
-    const int splits = wgrad_splits(B);
-    LinWgrad wg{kOut, kFeat, B, e->dout, e->act[kLayers], e->part};
+    const int N = kFeat + 1, splits = wgrad_splits(kOut, N, B);
+    LinWgrad wg{kOut, N, B, e->dout, e->act[kLayers], e->part};
     ECK(run_gemm(wg, splits, st));
-    k_sum_splits<<<64, 256, 0, st>>>(e->part, splits, kOut * kFeat, e->g + L.w[kLayers]);
-    // bias gradient = column sums of dout (positions = 1, no activation)
-    k_bias_grad<<<kOut, 256, 0, st>>>(e->dout, e->dout, B, kOut, 1, 0, e->g + L.b[kLayers]);
-    LinDgrad dg{B, kFeat, kOut, e->dout, e->pb + L.w[kLayers], e->dact_[kLayers]};
+    k_sum_splits<<<(kOut * N + 31) / 32, 256, 0, st>>>(e->part, splits, kOut, N, e->g + L.w[kLayers], e->g + L.b[kLayers]);
+    LinDgrad dg{B, kFeat, kOut, e->dout, e->act[kLayers], e->pb + L.w[kLayers], e->dact_[kLayers]};
     ECK(run_gemm(dg, 1, st));
   }
   for (int l = kLayers - 1; l >= 0; --l) {
     const Shape &sh = L.s[l];
     const long long K = (long long)B * sh.out_pos();
-    const int splits = wgrad_splits(K);
-    ConvWgrad wg{sh.Co, sh.Ci * 27, (int)K, sh, e->act[l], e->dact_[l + 1], e->act[l + 1], e->part, 1,
-                 PosDiv(sh.out_pos(), sh.Ho * sh.Wo, sh.Wo)};
+    const int N = sh.Ci * 27 + 1, splits = wgrad_splits(sh.Co, N, K);
+    ConvWgrad wg{sh.Co, N, (int)K, sh, e->act[l], e->dact_[l + 1], e->part, PosDiv(sh.out_pos(), sh.Ho * sh.Wo, sh.Wo)};
     ECK(run_gemm(wg, splits, st));
-    k_sum_splits<<<64, 256, 0, st>>>(e->part, splits, sh.Co * sh.Ci * 27, e->g + L.w[l]);
-    k_bias_grad<<<sh.Co, 256, 0, st>>>(e->dact_[l + 1], e->act[l + 1], B, sh.Co, sh.out_pos(), 1, e->g + L.b[l]);
+    k_sum_splits<<<(sh.Co * N + 31) / 32, 256, 0, st>>>(e->part, splits, sh.Co, N, e->g + L.w[l], e->g + L.b[l]);
     if (l > 0) {
-      ConvDgrad dg{B * sh.in_pos(), sh.Ci, sh.Co * 27, sh, e->dact_[l + 1], e->act[l + 1], e->pb + L.w[l], e->dact_[l], 1};
-      ECK(run_gemm(dg, 1, st));
+      ECK(run_dgrad(ConvDgrad{sh, e->dact_[l + 1], e->act[l], e->pb + L.w[l], e->dact_[l]}, st));
     }
   }
   ECK(cudaGetLastError());
