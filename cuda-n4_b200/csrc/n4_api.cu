@@ -112,6 +112,7 @@ struct TuneVal {
 
 constexpr int kStaticSmemReserve = 1024;
 constexpr int kSlots = 4;
+constexpr int kTableParts = 4;   // blocks per axis table
 constexpr int kMaxSub = 4;   // sub-batches of a pipelined batch
 constexpr int kHostLanes = 4;   // lanes of n4_run_batched_host
 
@@ -122,7 +123,10 @@ struct n4_context {
   int nsm = 0;
   int max_smem = 0;
   DevBuf imlog, tables, big, red, bar;
-  DevBuf s1, s2, s3, s4, s5;   // component scratch
+  DevBuf s1, s2, s4, s5;   // component scratch
+  DevBuf ticket;
+  void *pinned = nullptr;
+  size_t pinned_cap = 0;
   DevBuf warm_x, warm_lat;     // learned warm start: network inputs, predicted lattices
   DevBuf h_im, h_mask, h_out, h_lat, h_bias, h_warm;   // host-run staging
   // pipelined host batches: one stream and one device staging slot per lane
@@ -135,6 +139,7 @@ struct n4_context {
   int last_slot = -1;
   cudaStream_t last_stream = nullptr;
   cudaEvent_t last_done = nullptr;
+  bool any_done = false;   // last_done has been recorded
   std::map<TuneKey, TuneVal> tune;
   // standalone components: (fx, fy, fz, ncpt, field alignment) -> fit shape,
   // (fx, fy, fz, ncpt) -> evaluation (correction) tile shape
@@ -434,7 +439,6 @@ struct Upload {
   Slot *slot;
   int index;
   size_t off;
-  char *h() const { return slot->h; }
   template <class T> T *hp(size_t o) const { return (T *)(slot->h + o); }
   template <class T> T *dp(size_t o) const { return (T *)((char *)slot->d.p + o); }
 };
@@ -465,7 +469,7 @@ n4_status_t acquire_slot(n4_context *ctx, size_t bytes, Upload &u) {
 n4_status_t begin_run(n4_context *ctx, cudaStream_t st) {
   CK(cudaSetDevice(ctx->device));
   if (!ctx->last_done) CK(cudaEventCreateWithFlags(&ctx->last_done, cudaEventDisableTiming));
-  if (ctx->last_slot >= 0 && st != ctx->last_stream) CK(cudaStreamWaitEvent(st, ctx->last_done, 0));
+  if (ctx->any_done && st != ctx->last_stream) CK(cudaStreamWaitEvent(st, ctx->last_done, 0));
   return N4_OK;
 }
 
@@ -475,6 +479,16 @@ n4_status_t end_run(n4_context *ctx, cudaStream_t st, Upload &u) {
   u.slot->pending = true;
   ctx->last_slot = u.index;
   ctx->last_stream = st;
+  ctx->any_done = true;
+  return N4_OK;
+}
+
+// The end of a component call: later work of the context on other streams
+// waits for it.
+n4_status_t end_component(n4_context *ctx, cudaStream_t st) {
+  CK(cudaEventRecord(ctx->last_done, st));
+  ctx->last_stream = st;
+  ctx->any_done = true;
   return N4_OK;
 }
 
@@ -1001,18 +1015,23 @@ n4_status_t ensure_pipe(n4_context *ctx) {
 // and writes only its own volumes' buffers; st waits for all five streams.
 // k_correct over `tiles` tiles from t0 with tile shape `shape`.
 n4_status_t launch_correct(int shape, long long tiles, int ncz, cudaStream_t st, const CorrectVol *vols,
-                           const long long *tile_starts, int nvol, long long t0, float low, bool log_only = false) {
+                           const long long *tile_starts, int nvol, long long t0, float low) {
   if (tiles <= 0) return N4_OK;
   const CorrectShape cs = kCorrectShape[shape];
   const size_t smem = correct_smem_bytes(cs.rows, ncz);
   const unsigned g = (unsigned)tiles;
-  if (log_only) {
-    if (cs.threads == 512) k_correct<512, true><<<g, 512, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
-    else k_correct<256, true><<<g, 256, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
-  } else {
-    if (cs.threads == 512) k_correct<512, false><<<g, 512, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
-    else k_correct<256, false><<<g, 256, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
-  }
+  if (cs.threads == 512) k_correct<512><<<g, 512, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
+  else k_correct<256><<<g, 256, smem, st>>>(vols, tile_starts, nvol, t0, low, cs.rows);
+  CK(cudaGetLastError());
+  return N4_OK;
+}
+
+// The log field of one volume over `tiles` tiles of shape `shape`.
+n4_status_t launch_evaluate(int shape, long long tiles, const CorrectVol &vol, cudaStream_t st) {
+  const CorrectShape cs = kCorrectShape[shape];
+  const size_t smem = correct_smem_bytes(cs.rows, vol.ncz);
+  if (cs.threads == 512) k_evaluate<512><<<(unsigned)tiles, 512, smem, st>>>(vol, cs.rows);
+  else k_evaluate<256><<<(unsigned)tiles, 256, smem, st>>>(vol, cs.rows);
   CK(cudaGetLastError());
   return N4_OK;
 }
@@ -1030,7 +1049,7 @@ n4_status_t enqueue_pipelined(n4_context *ctx, const n4_params_t *p, const Prepa
   const int n = P.n;
   const long long *pst = B.hp<long long>(P.o_pst), *tst = B.hp<long long>(P.o_tst);
   int launches = 0;
-  k_axis_tables<<<3 * n, 256, 0, side>>>(B.dp<TableJob>(P.o_tab));
+  k_axis_tables<<<dim3(3 * n, kTableParts), 128, 0, side>>>(B.dp<TableJob>(P.o_tab));
   CK(cudaGetLastError());
   CK(cudaEventRecord(ev[1], side));
   CK(cudaStreamWaitEvent(corr, ev[1], 0));
@@ -1151,7 +1170,7 @@ n4_status_t enqueue_run(n4_context *ctx, const n4_params_t *p, const Prepared &P
     ++launches;
   }
   if (profile) TRY(prof_mark(ctx, 2, st));
-  k_axis_tables<<<3 * n, 256, 0, st>>>(B.dp<TableJob>(P.o_tab));
+  k_axis_tables<<<dim3(3 * n, kTableParts), 128, 0, st>>>(B.dp<TableJob>(P.o_tab));
   CK(cudaGetLastError());
   if (profile) TRY(prof_mark(ctx, 3, st));
   TRY(launch_correct(P.corr, P.tiles, P.NCZ, st, B.dp<CorrectVol>(P.o_cor), B.dp<long long>(P.o_tst), n, 0,
@@ -1197,7 +1216,12 @@ n4_status_t run_volumes(n4_context *ctx, const n4_params_t *p, const std::vector
 n4_status_t collect_slot(n4_context *ctx, int slot, n4_report_t *out, int n);
 
 n4_status_t collect(n4_context *ctx, n4_report_t *out, int n) {
-  if (ctx->last_slot < 0) return fail(N4_ERR_INVALID_ARG, "no run to synchronise with");
+  if (ctx->last_slot < 0) {
+    // component calls only: nothing to report, but their work is done
+    if (!ctx->any_done) return fail(N4_ERR_INVALID_ARG, "no run to synchronise with");
+    CK(cudaEventSynchronize(ctx->last_done));
+    return N4_OK;
+  }
   return collect_slot(ctx, ctx->last_slot, out, n);
 }
 
@@ -1300,10 +1324,10 @@ n4_status_t n4_create(n4_context_t **out, int device) {
   CK(cudaDeviceGetAttribute(&c->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   // the largest correction tile: 512 rows of kMaxNcz z control points
   const int corr_smem = (int)correct_smem_bytes(512, kMaxNcz);
-  if (cudaFuncSetAttribute(k_correct<256, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_correct<512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_correct<256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_correct<512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess) {
+  if (cudaFuncSetAttribute(k_correct<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_correct<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_evaluate<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_evaluate<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, corr_smem) != cudaSuccess) {
     cudaGetLastError();
     delete c;
     return fail(N4_ERR_CUDA, "cannot raise the correction kernel's shared-memory limit");
@@ -1316,10 +1340,11 @@ n4_status_t n4_destroy(n4_context_t *c) {
   if (!c) return N4_OK;
   cudaSetDevice(c->device);
   cudaDeviceSynchronize();
-  for (DevBuf *b : {&c->imlog, &c->tables, &c->big, &c->red, &c->bar, &c->s1, &c->s2, &c->s3, &c->s4,
+  for (DevBuf *b : {&c->imlog, &c->tables, &c->big, &c->red, &c->bar, &c->s1, &c->s2, &c->ticket, &c->s4,
                     &c->s5, &c->h_im, &c->h_mask, &c->h_out, &c->h_lat, &c->h_bias, &c->h_warm, &c->warm_x,
                     &c->warm_lat, &c->hb})
     b->release();
+  if (c->pinned) cudaFreeHost(c->pinned);
   for (cudaEvent_t e : c->hev)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->hclock)
@@ -1768,7 +1793,7 @@ n4_status_t n4_run_batched_host(n4_context_t *ctx, const n4_params_t *p, int n, 
     if (!e) CK(cudaEventCreate(&e));
   // every lane starts after the context's earlier work and after the clock
   cudaStream_t lane0 = ctx->hst[0];
-  if (ctx->last_done && ctx->last_slot >= 0) CK(cudaStreamWaitEvent(lane0, ctx->last_done, 0));
+  if (ctx->any_done) CK(cudaStreamWaitEvent(lane0, ctx->last_done, 0));
   CK(cudaEventRecord(ctx->hclock[0], lane0));
   for (int l = 1; l < L; ++l) CK(cudaStreamWaitEvent(ctx->hst[l], ctx->hclock[0], 0));
   const int nsb = (n + per - 1) / per;
@@ -1835,6 +1860,7 @@ n4_status_t n4_run_batched_host(n4_context_t *ctx, const n4_params_t *p, int n, 
   // later work of this context waits for the downloads
   CK(cudaEventRecord(ctx->last_done, lane0));
   ctx->last_stream = lane0;
+  ctx->any_done = true;
   for (int k = std::max(0, nsb - kSlots); k < nsb; ++k) TRY(harvest(k));
   CK(cudaEventSynchronize(ctx->hclock[1]));
   if (device_ms) CK(cudaEventElapsedTime(device_ms, ctx->hclock[0], ctx->hclock[1]));
@@ -1994,6 +2020,11 @@ n4_status_t n4_batch_graph_destroy(n4_batch_graph_t *g) {
 static bool fit_shape_ok(int k, const float *field, const float *mask, int Z) {
   const uintptr_t al = (uintptr_t)field | (uintptr_t)mask;
   const FitShape f = kFitShape[k];
+  // rows at any offset: field and mask off the boundary by the same amount;
+  // only where the aligned 8-voxel steps do not apply
+  if (k == kFitAnyRow8)
+    return Z <= kFitZMaxD && (!mask || (((uintptr_t)field ^ (uintptr_t)mask) & 31u) == 0) &&
+           !fit_shape_ok(kFitDefault8, field, mask, Z);
   if (f.step == 16) return Z % 16 == 0 && Z <= kFitZMaxD && (al & 63u) == 0;
   if (f.step == 8) return Z % 8 == 0 && Z <= kFitZMaxD && (al & 31u) == 0;
   if (f.step == 4) return Z % 4 == 0 && Z <= kFitZMaxD && (al & 15u) == 0;
@@ -2002,6 +2033,7 @@ static bool fit_shape_ok(int k, const float *field, const float *mask, int Z) {
 
 static int fit_default_shape(const float *field, const float *mask, int Z) {
   if (fit_shape_ok(kFitDefault8, field, mask, Z)) return kFitDefault8;
+  if (fit_shape_ok(kFitAnyRow8, field, mask, Z)) return kFitAnyRow8;
   if (fit_shape_ok(kFitDefault4, field, mask, Z)) return kFitDefault4;
   return kFitScalar;
 }
@@ -2019,11 +2051,11 @@ static std::vector<int> eval_key(unsigned fx, unsigned fy, unsigned fz, unsigned
 }
 
 extern "C++" {
-template <int S, int D, int R>
+template <int S, int D, int R, bool Any = false>
 static void fit_rows_as(const float *field, const float *mask, long long rows, int Z, const Axis &az, float *t1n,
                         float *t1d, cudaStream_t st) {
-  k_fit_rows_v5<S, D, R><<<(unsigned)((rows + R - 1) / R), R, kFitTableBytes(Z), st>>>(field, mask, rows, Z, az, t1n,
-                                                                                      t1d);
+  k_fit_rows_v5<S, D, R, Any><<<(unsigned)((rows + R - 1) / R), R, kFitTableBytes(Z, Any), st>>>(field, mask, rows, Z,
+                                                                                                 az, t1n, t1d);
 }
 }  // extern "C++"
 
@@ -2043,12 +2075,13 @@ static void launch_fit_rows(int k, const float *field, const float *mask, long l
     case 10: fit_rows_as<16, 2, 64>(field, mask, rows, Z, az, t1n, t1d, st); break;
     case 11: fit_rows_as<16, 2, 32>(field, mask, rows, Z, az, t1n, t1d, st); break;
     case 12: fit_rows_as<16, 2, 128>(field, mask, rows, Z, az, t1n, t1d, st); break;
+    case kFitAnyRow8: fit_rows_as<8, 3, 64, true>(field, mask, rows, Z, az, t1n, t1d, st); break;
     default:
       k_fit_rows<<<(unsigned)((rows + kFitRows - 1) / kFitRows), kFitRows, 0, st>>>(field, mask, rows, Z, az, t1n,
                                                                                      t1d);
   }
 }
-static_assert(kFitShapes == 13, "launch_fit_rows covers every fit shape");
+static_assert(kFitShapes == 14, "launch_fit_rows covers every fit shape");
 
 // Sizes a standalone fit accepts: every extent below 2^31 (the kernels take
 // them as int), at most 2^36 field voxels and 4096 control points per axis,
@@ -2068,18 +2101,12 @@ static n4_status_t component_tables(n4_context_t *ctx, unsigned fx, unsigned fy,
                                     unsigned nz, cudaStream_t st, Axis &ax, Axis &ay, Axis &az) {
   const size_t bx = align_up(axis_bytes(fx, nx - 3), 256), by = align_up(axis_bytes(fy, ny - 3), 256),
                bz = align_up(axis_bytes(fz, nz - 3), 256);
-  TRY(ctx->s5.ensure(bx + by + bz + sizeof(TableJob) * 3 + 256, "tables"));
+  TRY(ctx->s5.ensure(bx + by + bz, "tables"));
   char *base = ctx->s5.as<char>();
-  TableJob tj[3] = {{base, (int)fx, (int)nx}, {base + bx, (int)fy, (int)ny}, {base + bx + by, (int)fz, (int)nz}};
-  Upload u;
-  TRY(acquire_slot(ctx, sizeof(tj), u));
-  std::memcpy(u.h(), tj, sizeof(tj));
   TRY(begin_run(ctx, st));
-  CK(cudaMemcpyAsync(u.slot->d.p, u.slot->h, sizeof(tj), cudaMemcpyHostToDevice, st));
-  k_axis_tables<<<3, 256, 0, st>>>(u.dp<TableJob>(0));
+  k_axis_tables_of<<<dim3(3, kTableParts), 128, 0, st>>>(TableJob{base, (int)fx, (int)nx}, TableJob{base + bx, (int)fy, (int)ny},
+                                                        TableJob{base + bx + by, (int)fz, (int)nz});
   CK(cudaGetLastError());
-  u.slot->nrep = 0;
-  TRY(end_run(ctx, st, u));
   ax = axis_at(base, fx, nx);
   ay = axis_at(base + bx, fy, ny);
   az = axis_at(base + bx + by, fz, nz);
@@ -2107,10 +2134,11 @@ n4_status_t n4_fit_bspline3d(n4_context_t *ctx, const float *d_field, const floa
   if (prof) TRY(prof_mark(ctx, 0, st));
   launch_fit_rows(shape, d_field, d_mask, rows, fz, az, t1n, t1d, st);
   if (prof) TRY(prof_mark(ctx, 1, st));
-  k_fit_planes<<<(int)std::min<size_t>((t2 + 255) / 256, gb), 256, 0, st>>>(t1n, t1d, fx, fy, ay, ncpt_z, t2n, t2d);
+  k_fit_planes<<<(int)std::min<size_t>((t2 * 4 + 255) / 256, gb), 256, 0, st>>>(t1n, t1d, fx, fy, ay, ncpt_z, t2n, t2d);
   if (prof) TRY(prof_mark(ctx, 2, st));
-  const int nlat = ncpt_x * ncpt_y * ncpt_z;
-  k_fit_final<<<(nlat + 255) / 256, 256, 0, st>>>(t2n, t2d, fx, ax, ncpt_y, ncpt_z, eps, zero_den, d_lattice);
+  const long long nlat = (long long)ncpt_x * ncpt_y * ncpt_z;
+  k_fit_final<<<(int)std::min<long long>((nlat + 3) / 4, gb * 2), 128, 0, st>>>(t2n, t2d, fx, ax, ncpt_y, ncpt_z, eps, zero_den,
+                                                                              d_lattice);
   if (prof) { TRY(prof_mark(ctx, 3, st)); TRY(prof_mark(ctx, 4, st)); }
   CK(cudaGetLastError());
   ctx->prof_launches = 4;
@@ -2119,7 +2147,7 @@ n4_status_t n4_fit_bspline3d(n4_context_t *ctx, const float *d_field, const floa
   ctx->prof_fit_shape = shape;
   ctx->prof_corr_shape = -1;
   ctx->prof_valid = prof;
-  return N4_OK;
+  return end_component(ctx, st);
 }
 
 n4_status_t n4_evaluate_bspline3d(n4_context_t *ctx, const float *d_lattice, unsigned int ncpt_x, unsigned int ncpt_y,
@@ -2140,15 +2168,9 @@ n4_status_t n4_evaluate_bspline3d(n4_context_t *ctx, const float *d_lattice, uns
   if (it != ctx->eval_tune.end()) shape = it->second;
   const long long rt = kCorrectShape[shape].rows;
   const long long tiles = ((long long)fx * fy + rt - 1) / rt;
-  Upload u;
-  TRY(acquire_slot(ctx, sizeof(cv) + 16, u));
-  std::memcpy(u.h(), &cv, sizeof(cv));
-  TRY(begin_run(ctx, st));
-  CK(cudaMemcpyAsync(u.slot->d.p, u.slot->h, sizeof(cv) + 16, cudaMemcpyHostToDevice, st));
-  const size_t so = align_up(sizeof(cv), 16);
   const bool prof = ctx->profiling != 0;
   if (prof) TRY(prof_mark(ctx, 1, st));
-  TRY(launch_correct(shape, tiles, (int)ncpt_z, st, u.dp<CorrectVol>(0), u.dp<long long>(so), 1, 0, 0.0f, true));
+  TRY(launch_evaluate(shape, tiles, cv, st));
   if (prof) { TRY(prof_mark(ctx, 2, st)); TRY(prof_mark(ctx, 3, st)); TRY(prof_mark(ctx, 4, st)); }
   ctx->prof_launches = 2;
   ctx->prof_fit = 0;
@@ -2156,8 +2178,7 @@ n4_status_t n4_evaluate_bspline3d(n4_context_t *ctx, const float *d_lattice, uns
   ctx->prof_fit_shape = -1;
   ctx->prof_corr_shape = shape;
   ctx->prof_valid = prof;
-  u.slot->nrep = 0;
-  return end_run(ctx, st, u);
+  return end_component(ctx, st);
 }
 
 n4_status_t n4_autotune_components(n4_context_t *ctx, const float *d_field, const float *d_mask, unsigned int ncpt_x,
@@ -2222,25 +2243,16 @@ n4_status_t n4_autotune_components(n4_context_t *ctx, const float *d_field, cons
   // the evaluation candidates write d_out from the lattice the fit produces
   if (status == N4_OK)
     status = n4_fit_bspline3d(ctx, d_field, d_mask, ncpt_x, ncpt_y, ncpt_z, fx, fy, fz, 1e-3f, 0, d_lattice, stream);
-  Upload u;
-  if (status == N4_OK) status = acquire_slot(ctx, sizeof(CorrectVol) + 16, u);
   if (status == N4_OK) {
     CorrectVol cv{nullptr, d_out, nullptr, d_lattice, (char *)ax.s, (char *)ay.s, (char *)az.s,
                   (int)fx, (int)fy, (int)fz, (int)ncpt_x, (int)ncpt_y, (int)ncpt_z, 0,
                   vec4_ok((int)fz, nullptr, d_out, nullptr)};
-    std::memcpy(u.h(), &cv, sizeof(cv));
-    status = begin_run(ctx, st);
-    if (status == N4_OK && cudaMemcpyAsync(u.slot->d.p, u.slot->h, sizeof(cv) + 16, cudaMemcpyHostToDevice, st) !=
-                               cudaSuccess)
-      status = fail(N4_ERR_CUDA, "descriptor upload failed");
-    const size_t so = align_up(sizeof(cv), 16);
     for (int k = 0; k < kCorrectShapes && status == N4_OK; ++k) {
       const long long rt = kCorrectShape[k].rows;
       const long long tiles = ((long long)fx * fy + rt - 1) / rt;
       float ms = 0.0f;
       n4_status_t ls = N4_OK;
-      status = timed([&] { ls = launch_correct(k, tiles, (int)ncpt_z, st, u.dp<CorrectVol>(0),
-                                               u.dp<long long>(so), 1, 0, 0.0f, true); }, &ms);
+      status = timed([&] { ls = launch_evaluate(k, tiles, cv, st); }, &ms);
       if (status == N4_OK) status = ls;
       if (status != N4_OK) break;
       const int c = rep.eval_candidates++;
@@ -2249,8 +2261,7 @@ n4_status_t n4_autotune_components(n4_context_t *ctx, const float *d_field, cons
       rep.eval_ms[c] = ms;
       if (c == 0 || ms < rep.eval_ms[rep.eval_chosen]) { rep.eval_chosen = c; rep.eval_shape = k; }
     }
-    u.slot->nrep = 0;
-    if (status == N4_OK) status = end_run(ctx, st, u);
+    if (status == N4_OK) status = end_component(ctx, st);
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -2271,6 +2282,25 @@ n4_status_t n4_upsample_lattice3d(n4_context_t *ctx, const float *d_lattice, uns
   return N4_OK;
 }
 
+// Counter of the "last block" kernels, 0 between them.
+static n4_status_t ensure_ticket(n4_context *ctx) {
+  if (ctx->ticket.p) return N4_OK;
+  TRY(ctx->ticket.ensure(64, "ticket"));
+  CK(cudaMemset(ctx->ticket.p, 0, 64));
+  return N4_OK;
+}
+// Page-locked buffer for what a component call reads back.
+static n4_status_t ensure_pinned(n4_context *ctx, size_t bytes) {
+  if (bytes <= ctx->pinned_cap) return N4_OK;
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  ctx->pinned = nullptr;
+  ctx->pinned_cap = 0;
+  bytes = align_up(std::max<size_t>(bytes, 4096), 4096);
+  CK(cudaMallocHost(&ctx->pinned, bytes));
+  ctx->pinned_cap = bytes;
+  return N4_OK;
+}
+
 n4_status_t n4_sharpen_image(n4_context_t *ctx, const float *d_before, const float *d_mask, unsigned int n,
                              unsigned int bins, float wiener, float fwhm, float *d_after, float *bin_min,
                              float *bin_max, float *h_E) {
@@ -2278,31 +2308,41 @@ n4_status_t n4_sharpen_image(n4_context_t *ctx, const float *d_before, const flo
   if (bins < 2 || bins > 1024) return fail(N4_ERR_INVALID_ARG, "bins must be in [2, 1024]");
   CK(cudaSetDevice(ctx->device));
   cudaStream_t st = nullptr;
-  const int nb = std::min<int>((int)((n + 255) / 256), ctx->nsm * 8);
-  TRY(ctx->s1.ensure((size_t)nb * 8 + 64, "partials"));
-  TRY(ctx->s2.ensure((size_t)bins * 16 + 64, "histogram"));
-  TRY(ctx->s3.ensure(64, "statistics"));
+  // blocks of each pass: four voxels per thread and step, whole waves at most
+  const auto blocks = [&](int threads, int per_sm) {
+    return (int)std::min<long long>(((long long)n + threads * 4 - 1) / (threads * 4), (long long)ctx->nsm * per_sm);
+  };
+  const int nbm = blocks(256, 8), nbh = blocks(512, 2), nbr = blocks(512, 4);
+  const int vec = ((((uintptr_t)d_before | (uintptr_t)d_mask | (uintptr_t)d_after) & 15u) == 0) ? 1 : 0;
+  TRY(ctx->s1.ensure((size_t)nbm * 8 + 64, "partials"));
+  // histogram; residual table; then what the host reads: statistics and E
+  const size_t o_r = align_up((size_t)bins * 8, 16), o_st = o_r + (size_t)bins * 16, o_e = o_st + 32,
+               read = 32 + (size_t)bins * 8;
+  TRY(ctx->s2.ensure(o_e + (size_t)bins * 8, "histogram"));
+  TRY(ensure_ticket(ctx));
+  char *base = ctx->s2.as<char>();
   float *part = ctx->s1.as<float>();
-  double *stats = ctx->s3.as<double>();
-  unsigned long long *hist = ctx->s2.as<unsigned long long>();
-  double *E = (double *)(hist + bins);
-  k_minmax<<<nb, 256, 0, st>>>(d_before, d_mask, n, part);
-  k_minmax_final<<<1, 256, 0, st>>>(part, nb, bins, stats);
-  CK(cudaMemsetAsync(hist, 0, (size_t)bins * 8, st));
-  // one block sees at most (grid-stride trips) x 256 voxels
-  const int shift = hist_shift_for(((long long)n + (long long)nb * 256 - 1) / ((long long)nb * 256) * 256);
-  k_hist<<<nb, 256, bins * 4, st>>>(d_before, d_mask, n, stats, bins, shift, hist);
+  double *stats = (double *)(base + o_st), *E = (double *)(base + o_e);
+  unsigned long long *hist = (unsigned long long *)base;
+  float4 *R = (float4 *)(base + o_r);
+  unsigned *ticket = ctx->ticket.as<unsigned>();
   const int npad = npad_of(bins), hoff = (int)(0.5 * (npad - bins));
-  const int smem = npad * (16 * 3 + 8) + bins * 16;
-  CK(cudaFuncSetAttribute(k_sharpen, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k_sharpen<<<1, 512, smem, st>>>(hist, stats, bins, shift, npad, hoff, decimal_of(wiener), decimal_of(fwhm), E);
-  k_remap<<<nb, 256, 0, st>>>(d_before, d_mask, n, stats, E, bins, d_after);
+  const int smem = (int)hist_smem_bytes(bins, npad);
+  CK(cudaFuncSetAttribute(k_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_minmax<<<nbm, 256, 0, st>>>(d_before, d_mask, n, vec, part, bins, stats, hist, ticket);
+  // a histogram copy gets two of a block's 16 warps: its grid-stride steps of
+  // 4 x 64 voxels (and of 64 for the rest of the vector steps)
+  const long long lanes = (long long)nbh * 512;
+  const long long steps = vec ? ((n >> 2) + lanes - 1) / lanes * 4 + 1 : ((long long)n + lanes - 1) / lanes;
+  const int shift = hist_shift_for(steps * 64);
+  k_hist<<<nbh, 512, smem, st>>>(d_before, d_mask, n, vec, stats, bins, shift, hist, npad, hoff, decimal_of(wiener),
+                                 decimal_of(fwhm), E, R, ticket);
+  k_remap<<<nbr, 512, bins * 16, st>>>(d_before, d_mask, n, vec, stats, E, R, bins, d_after);
   CK(cudaGetLastError());
-  double hs[4];
-  std::vector<double> hE(bins);
-  CK(cudaMemcpyAsync(hs, stats, sizeof(hs), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(hE.data(), E, (size_t)bins * 8, cudaMemcpyDeviceToHost, st));
+  TRY(ensure_pinned(ctx, read));
+  CK(cudaMemcpyAsync(ctx->pinned, stats, read, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  const double *hs = (const double *)ctx->pinned, *hE = hs + 4;
   if (bin_min) *bin_min = (float)hs[0];
   if (bin_max) *bin_max = (float)hs[1];
   if (h_E) for (unsigned b = 0; b < bins; ++b) h_E[b] = (float)hE[b];
@@ -2315,13 +2355,16 @@ n4_status_t n4_convergence(n4_context_t *ctx, const float *d_field1, const float
   if (!ctx || !d_field1 || !d_field2 || !cv || n == 0) return fail(N4_ERR_INVALID_ARG, "bad arguments");
   CK(cudaSetDevice(ctx->device));
   const int nb = std::min<int>((int)((n + 255) / 256), ctx->nsm * 4);
-  TRY(ctx->s1.ensure((size_t)nb * 24, "partials"));
-  k_cv<<<nb, 256>>>(d_field1, d_field2, d_mask, n, ctx->s1.as<double>());
+  TRY(ctx->s1.ensure((size_t)nb * 24 + 32, "partials"));
+  TRY(ensure_ticket(ctx));
+  TRY(ensure_pinned(ctx, 24));
+  double *part = ctx->s1.as<double>();
+  k_cv<<<nb, 256>>>(d_field1, d_field2, d_mask, n, part, part + 3 * nb, ctx->ticket.as<unsigned>());
   CK(cudaGetLastError());
-  std::vector<double> part((size_t)nb * 3);
-  CK(cudaMemcpy(part.data(), ctx->s1.p, part.size() * 8, cudaMemcpyDeviceToHost));
-  double s0 = 0, s1 = 0, c = 0;
-  for (int b = 0; b < nb; ++b) { s0 += part[3 * b]; s1 += part[3 * b + 1]; c += part[3 * b + 2]; }
+  CK(cudaMemcpyAsync(ctx->pinned, part + 3 * nb, 24, cudaMemcpyDeviceToHost, nullptr));
+  CK(cudaStreamSynchronize(nullptr));
+  const double *sums = (const double *)ctx->pinned;
+  const double s0 = sums[0], s1 = sums[1], c = sums[2];
   if (c < 1.0) return fail(N4_ERR_EMPTY_MASK, "no voxel in the mask");
   const double m = s0 / c;
   double var = s1 / c - m * m;
@@ -2377,12 +2420,6 @@ n4_status_t current_context_id(unsigned long long *id) {
   return N4_OK;
 }
 
-// The three tables of one call, passed by value (no descriptor upload).
-__global__ void k_axis_tables_by_value(TableJob jx, TableJob jy, TableJob jz) {
-  const TableJob t = blockIdx.x == 0 ? jx : (blockIdx.x == 1 ? jy : jz);
-  build_axis(axis_at(t.base, t.n, t.nc));
-}
-
 }  // namespace
 
 extern "C" {
@@ -2424,16 +2461,17 @@ n4_status_t n4_fit_bspline3d_noalloc(const float *d_field, const float *d_mask, 
   cudaStream_t st = (cudaStream_t)stream;
   const TableJob jx{base, (int)fx, (int)ncpt_x}, jy{base + bx, (int)fy, (int)ncpt_y},
       jz{base + bx + by, (int)fz, (int)ncpt_z};
-  k_axis_tables_by_value<<<3, 256, 0, st>>>(jx, jy, jz);
+  k_axis_tables_of<<<dim3(3, kTableParts), 128, 0, st>>>(jx, jy, jz);
   const Axis ax = axis_at(jx.base, fx, ncpt_x), ay = axis_at(jy.base, fy, ncpt_y), az = axis_at(jz.base, fz, ncpt_z);
   float *t1n = (float *)(base + bx + by + bz), *t1d = t1n + t1;
   float *t2n = (float *)(base + bx + by + bz + align_up(t1 * 8, 256)), *t2d = t2n + t2;
   const long long rows = (long long)fx * fy;
   launch_fit_rows(fit_default_shape(d_field, d_mask, (int)fz), d_field, d_mask, rows, fz, az, t1n, t1d, st);
-  k_fit_planes<<<(int)std::min<size_t>((t2 + 255) / 256, 148 * 8), 256, 0, st>>>(t1n, t1d, fx, fy, ay, ncpt_z, t2n,
-                                                                                   t2d);
-  const int nlat = ncpt_x * ncpt_y * ncpt_z;
-  k_fit_final<<<(nlat + 255) / 256, 256, 0, st>>>(t2n, t2d, fx, ax, ncpt_y, ncpt_z, eps, zero_den, d_lattice);
+  k_fit_planes<<<(int)std::min<size_t>((t2 * 4 + 255) / 256, 148 * 8), 256, 0, st>>>(t1n, t1d, fx, fy, ay, ncpt_z, t2n,
+                                                                                       t2d);
+  const long long nlat = (long long)ncpt_x * ncpt_y * ncpt_z;
+  k_fit_final<<<(int)std::min<long long>((nlat + 3) / 4, 148 * 16), 128, 0, st>>>(t2n, t2d, fx, ax, ncpt_y, ncpt_z, eps,
+                                                                                zero_den, d_lattice);
   CK(cudaGetLastError());
   return N4_OK;
 }

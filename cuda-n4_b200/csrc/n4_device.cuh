@@ -92,31 +92,36 @@ __device__ __forceinline__ int axis_voxel(int i, double span, int nsp, float4 &w
   return s;
 }
 
-// Voxel range of every span by binary search on the monotone span index.
-__device__ __forceinline__ void axis_ranges(int n, int nsp, double span, int *lo_out, int *hi_out) {
-  for (int sp = threadIdx.x; sp < nsp; sp += blockDim.x) {
-    int lo = 0, hi = n;                // first voxel with span >= sp
-    while (lo < hi) { int m = (lo + hi) >> 1; if (span_of(m, span, nsp) >= sp) hi = m; else lo = m + 1; }
-    int l2 = lo, h2 = n;               // first voxel with span >= sp + 1
-    while (l2 < h2) { int m = (l2 + h2) >> 1; if (span_of(m, span, nsp) >= sp + 1) h2 = m; else l2 = m + 1; }
-    lo_out[sp] = lo;
-    hi_out[sp] = l2;
+// Voxel i's part of the spans' voxel ranges: lo[sp] is the first voxel of a
+// span >= sp (n if there is none) and hi[sp] = lo[sp + 1], so the voxel where
+// the span index s changes writes the spans up to its own.  (A binary search
+// per span took two FP64 divisions a step one after the other.)
+__device__ __forceinline__ void axis_range(int i, int s, int n, int nsp, double span, int *lo, int *hi) {
+  const int before = i > 0 ? span_of(i - 1, span, nsp) : -1;
+  for (int sp = before + 1; sp <= s; ++sp) {
+    lo[sp] = i;
+    if (sp > 0) hi[sp - 1] = i;
+  }
+  if (i == n - 1) {
+    hi[s] = n;
+    for (int sp = s + 1; sp < nsp; ++sp) lo[sp] = hi[sp] = n;
   }
 }
 
-// Fill one axis table with the CTA's threads (caller synchronises).
-__device__ void build_axis(const Axis &a) {
+// Fill voxels first, first + step, ... of one axis table (caller synchronises).
+__device__ __forceinline__ void build_axis(const Axis &a, int first, int step) {
   const double span = __ddiv_rn((double)a.n, (double)a.nsp);
-  for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
+  for (int i = first; i < a.n; i += step) {
     float4 w, p, q;
-    a.s[i] = axis_voxel(i, span, a.nsp, w, p, q);
+    const int s = axis_voxel(i, span, a.nsp, w, p, q);
+    a.s[i] = s;
     a.w[i] = w;
     a.p4[i] = p;
     a.q4[i] = q;
     a.p[0 * a.n + i] = p.x; a.p[1 * a.n + i] = p.y; a.p[2 * a.n + i] = p.z; a.p[3 * a.n + i] = p.w;
     a.q[0 * a.n + i] = q.x; a.q[1 * a.n + i] = q.y; a.q[2 * a.n + i] = q.z; a.q[3 * a.n + i] = q.w;
+    axis_range(i, s, a.n, a.nsp, span, a.lo, a.hi);
   }
-  axis_ranges(a.n, a.nsp, span, a.lo, a.hi);
 }
 
 // b = sum_j w_j g[j] with a fixed association (identical in every pass).
@@ -418,6 +423,7 @@ __device__ __forceinline__ float two_sum(float a, float b, float &err) {
 struct BinMap {
   double binMin, slope, inv_slope, top;
   float fmin, ih, il, ff_limit;
+  BinMap() = default;
   __device__ BinMap(double mn, double sl, int bins)
       : binMin(mn), slope(sl), inv_slope(1.0 / sl), top((double)bins - 1.5), fmin((float)mn),
         ih((float)inv_slope), il((float)(inv_slope - (double)ih)), ff_limit((float)(bins - 2)) {}
@@ -499,20 +505,6 @@ __host__ __device__ inline int hist_shift_for(long long n) {
   int s = kHistMaxShift;
   while (s > 0 && (unsigned long long)n << s > 0xffffffffull) --s;
   return s;
-}
-
-// Warp-aggregated add of one value into a shared 32-bit histogram.  All 32
-// lanes must call it (lanes without a value pass key < 0).
-__device__ __forceinline__ void hist_add_warp(unsigned *h, int bins, int key, unsigned qlo, unsigned qhi) {
-  const unsigned grp = __match_any_sync(kFull, key);
-  if (key >= 0) {
-    const unsigned slo = __reduce_add_sync(grp, qlo);
-    const unsigned shi = __reduce_add_sync(grp, qhi);
-    if ((threadIdx.x & 31) == (unsigned)(__ffs(grp) - 1)) {
-      atomicAdd(&h[key], slo);
-      if (shi && key + 1 < bins) atomicAdd(&h[key + 1], shi);
-    }
-  }
 }
 
 // Piecewise-linear remap through E (N4.py:107-113) from the FP64 bin

@@ -360,12 +360,13 @@ struct Engine {
     const double span = __ddiv_rn((double)a.n, (double)a.nsp);
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
       float4 w, p, q;
-      at<int>(a.o_s)[i] = axis_voxel(i, span, a.nsp, w, p, q);
+      const int s = axis_voxel(i, span, a.nsp, w, p, q);
+      at<int>(a.o_s)[i] = s;
       at<float4>(a.o_w)[i] = w;
       at<float4>(a.o_p)[i] = p;
       at<float4>(a.o_q)[i] = q;
+      axis_range(i, s, a.n, a.nsp, span, at<int>(a.o_lo), at<int>(a.o_hi));
     }
-    axis_ranges(a.n, a.nsp, span, at<int>(a.o_lo), at<int>(a.o_hi));
   }
 
   // ytab[m][sp]: first row of the CTA's list at or after the first voxel of

@@ -11,7 +11,7 @@
 //                     (cudaN4.cu:1697-1729, N4.py:329-330)
 //   k_fit_*           standalone separable B-spline fit (FitBspline3D)
 //   k_refine          lattice refinement (upsampleLattice3D_gpu)
-//   k_minmax/k_hist/k_sharpen/k_remap   standalone sharpenImage
+//   k_minmax/k_hist/k_remap   standalone sharpenImage
 //   k_cv              standalone convergence measurement
 #pragma once
 #include <cuda_bf16.h>
@@ -349,9 +349,16 @@ struct TableJob {
   int n, nc;
 };
 
+// One axis per blockIdx.x, its voxels over the blocks of blockIdx.y (a voxel's
+// weights are a chain of FP64 divisions: one per thread).
 __global__ void k_axis_tables(const TableJob *jobs) {
   const TableJob t = jobs[blockIdx.x];
-  build_axis(axis_at(t.base, t.n, t.nc));
+  build_axis(axis_at(t.base, t.n, t.nc), blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
+}
+// The same for the three axes of one call, given by value (no upload).
+__global__ void k_axis_tables_of(TableJob jx, TableJob jy, TableJob jz) {
+  const TableJob t = blockIdx.x == 0 ? jx : (blockIdx.x == 1 ? jy : jz);
+  build_axis(axis_at(t.base, t.n, t.nc), blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
 }
 
 // ------------------------------------------------------------------ final correction
@@ -607,14 +614,20 @@ __device__ __forceinline__ void correct_tile(const CorrectVol *vols, const long 
 
 // Tile t0 + blockIdx.x of a batch (numbered as in CorrectVol::tile0, tiles of
 // `rt` rows) of the volumes vols[0 .. nvol); dynamic shared memory
-// correct_smem_bytes(rt, ncz).  256 threads: 4 CTAs per SM for the log field
-// (64 registers), 3 for the correction, whose loads in flight need more.
-template <int NT, bool kLog>
-__global__ void __launch_bounds__(NT, NT <= 256 ? (kLog ? 4 : 3) : 1) k_correct(const CorrectVol *vols,
-                                                                   const long long *tile_starts, int nvol,
-                                                                   long long t0, float low, int rt) {
+// correct_smem_bytes(rt, ncz).  256 threads: 3 CTAs per SM (the loads in flight
+// need the registers); 4 for the log field alone (k_evaluate, 64 registers).
+template <int NT>
+__global__ void __launch_bounds__(NT, NT <= 256 ? 3 : 1) k_correct(const CorrectVol *vols, const long long *tile_starts,
+                                                                   int nvol, long long t0, float low, int rt) {
   extern __shared__ __align__(16) float correct_sm[];
-  correct_tile<kLog>(vols, tile_starts, nvol, t0 + blockIdx.x, low, rt, correct_sm + 2 * kLxMax, correct_sm);
+  correct_tile<false>(vols, tile_starts, nvol, t0 + blockIdx.x, low, rt, correct_sm + 2 * kLxMax, correct_sm);
+}
+
+// The log field of one volume (EvaluateBspline3D), its descriptor by value.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT <= 256 ? 4 : 1) k_evaluate(const __grid_constant__ CorrectVol vol, int rt) {
+  extern __shared__ __align__(16) float correct_sm[];
+  correct_tile<true>(&vol, nullptr, 1, blockIdx.x, 0.0f, rt, correct_sm + 2 * kLxMax, correct_sm);
 }
 
 // ------------------------------------------------------------------ standalone fit
@@ -702,12 +715,13 @@ constexpr int kFitZMaxD = 1024;
 struct FitShape {
   int step, depth, rows;
 };
-constexpr int kFitShapes = 13;
+constexpr int kFitShapes = 14;
 constexpr FitShape kFitShape[kFitShapes] = {{8, 3, 64},  {8, 2, 64},  {8, 4, 64},  {8, 3, 32},  {8, 3, 128},
                                             {8, 2, 128}, {4, 6, 64},  {4, 4, 64},  {4, 6, 128}, {0, 0, kFitRows},
-                                            {16, 2, 64}, {16, 2, 32}, {16, 2, 128}};
-constexpr int kFitDefault8 = 0, kFitDefault4 = 6, kFitScalar = 9;
-__host__ __device__ inline size_t kFitTableBytes(int Z) { return (size_t)Z * 36; }
+                                            {16, 2, 64}, {16, 2, 32}, {16, 2, 128}, {8, 3, 64}};
+constexpr int kFitDefault8 = 0, kFitDefault4 = 6, kFitScalar = 9, kFitAnyRow8 = 13;
+// z table of a fit; with `any` rows (k_fit_rows_v5) 8 entries more at each end
+__host__ __device__ inline size_t kFitTableBytes(int Z, bool any = false) { return (size_t)(Z + (any ? 16 : 0)) * 36; }
 
 template <int S> struct FitStep { float v[S]; };
 
@@ -787,39 +801,65 @@ struct FitWalk {
   }
 };
 
-__device__ __forceinline__ void fit_table(const Axis &az, int Z, char *tab) {
-  float4 *sp4 = (float4 *)tab, *sq4 = sp4 + Z;
-  int *ss = (int *)(sq4 + Z);
-  for (int i = threadIdx.x; i < Z; i += blockDim.x) {
-    sp4[i] = az.p4[i];
-    sq4[i] = az.q4[i];
-    ss[i] = az.s[i];
+// The z table of voxels -pad .. Z + pad - 1 (weights 0 and the row's first and
+// last span outside it), so that tab entries are indexed by z + pad.
+__device__ __forceinline__ void fit_table(const Axis &az, int Z, int pad, char *tab) {
+  const int n = Z + 2 * pad;
+  float4 *sp4 = (float4 *)tab, *sq4 = sp4 + n;
+  int *ss = (int *)(sq4 + n);
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int z = i - pad;
+    const bool in = z >= 0 && z < Z;
+    sp4[i] = in ? az.p4[z] : zero;
+    sq4[i] = in ? az.q4[z] : zero;
+    ss[i] = az.s[z < 0 ? 0 : (z < Z ? z : Z - 1)];
   }
 }
 
-template <int S, int D, int R>
+// `Any`: rows that do not start on the load's boundary (Z % S != 0, or field
+// and mask off it by the same amount).  A row's steps then start at the
+// boundary at or before its first voxel; what they hold of other rows is
+// taken as masked out (exact zeros), so the sums are bitwise those of aligned
+// rows.  Steps that reach beyond the field (its first and last) load voxel by
+// voxel.
+template <int S, int D, int R, bool Any>
 __global__ void __launch_bounds__(R, 512 / R) k_fit_rows_v5(const float *__restrict__ field,
                                                               const float *__restrict__ mask, long long rows, int Z,
                                                               Axis az, float *__restrict__ t1n,
                                                               float *__restrict__ t1d) {
   extern __shared__ __align__(16) char fit_tab[];
-  const float4 *sp4 = (const float4 *)fit_tab, *sq4 = sp4 + Z;
-  const int *ss = (const int *)(sq4 + Z);
+  constexpr int kPad = Any ? 8 : 0;
+  const float4 *sp4 = (const float4 *)fit_tab, *sq4 = sp4 + Z + 2 * kPad;
+  const int *ss = (const int *)(sq4 + Z + 2 * kPad);
+  sp4 += kPad; sq4 += kPad; ss += kPad;
   const long long row = (long long)blockIdx.x * R + threadIdx.x;
   const bool live = row < rows;
-  const int nq = Z / S;                             // steps per row
-  const float *fp = field + (live ? row : 0) * Z;
-  const float *mp = mask ? mask + (live ? row : 0) * Z : nullptr;
+  const long long first = (live ? row : 0) * Z;    // the row's first voxel
+  const int off = Any ? (int)(((uintptr_t)(field + first) >> 2) & (S - 1)) : 0;   // voxels from the boundary to it
+  const int nq = (Z + off + S - 1) / S;            // steps per row
+  const float *fp = field + first - off;
+  const float *mp = mask ? mask + first - off : nullptr;
   FitStep<S> F[D], M[D];
+  const auto load = [&](FitStep<S> &f, FitStep<S> &m, int q) {
+    if (Any && (first - off + (long long)q * S < 0 || first - off + (long long)q * S + S > rows * Z)) {
+#pragma unroll
+      for (int j = 0; j < S; ++j) {
+        const int z = q * S + j - off;
+        const bool in = z >= 0 && z < Z;
+        f.v[j] = in ? field[first + z] : 0.0f;
+        m.v[j] = in && mask ? mask[first + z] : 0.0f;
+      }
+      return;
+    }
+    fit_load(f, fp + q * S);
+    if (mp) fit_load(m, mp + q * S);
+  };
   // the first steps are requested before the table is built
 #pragma unroll
-  for (int k = 0; k < D; ++k) {
-    if (live && k < nq) {
-      fit_load(F[k], fp + k * S);
-      if (mp) fit_load(M[k], mp + k * S);
-    }
-  }
-  fit_table(az, Z, fit_tab);
+  for (int k = 0; k < D; ++k)
+    if (live && k < nq) load(F[k], M[k], k);
+  fit_table(az, Z, kPad, fit_tab);
   __syncthreads();
   if (!live) return;
   const int ncz = az.nc;
@@ -837,60 +877,81 @@ __global__ void __launch_bounds__(R, 512 / R) k_fit_rows_v5(const float *__restr
       for (int j = 0; j < S; ++j) {
         fa[j] = F[k].v[j];
         ma[j] = mp ? M[k].v[j] : 1.0f;
+        if (Any && (unsigned)(S * q + j - off) >= (unsigned)Z) ma[j] = 0.0f;   // of another row
       }
       // step q is in registers: request step q + D into its slot
-      if (q + D < nq) {
-        fit_load(F[k], fp + (q + D) * S);
-        if (mp) fit_load(M[k], mp + (q + D) * S);
-      }
-      w.step<S>(fa, ma, S * q, sp4, sq4, ss, az.hi);
+      if (q + D < nq) load(F[k], M[k], q + D);
+      w.step<S>(fa, ma, S * q - off, sp4, sq4, ss, az.hi);
     }
   }
   w.flush(ncz);
 }
 
-// T2[vx][cy][cz] from T1.
-__global__ void k_fit_planes(const float *t1n, const float *t1d, int X, int Y, Axis ay, int ncz,
-                             float *t2n, float *t2d) {
+// Sum over a group of `lanes` lanes (a power of two) of compensated sums, in
+// FP64, on all of them.
+__device__ __forceinline__ double kahan_lanes(const KahanSum &k, int lanes) {
+  double v = (double)k.s - (double)k.c;
+  for (int o = lanes >> 1; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
+
+// T2[vx][cy][cz] from T1: one lane per (entry, span that reaches it), its rows
+// compensated, the four spans added in FP64.  (One thread per entry walked
+// its four spans' rows one after the other: 27 us at 256x256x160 with 11
+// control points against 5.)
+__global__ void k_fit_planes(const float *__restrict__ t1n, const float *__restrict__ t1d, int X, int Y, Axis ay,
+                             int ncz, float *t2n, float *t2d) {
   const int ncy = ay.nc;
-  const long long ntask = (long long)X * ncy * ncz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < ntask;
+  const long long ntask = (long long)X * ncy * ncz, nlane = (ntask * 4 + 31) / 32 * 32;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nlane;
        t += (long long)gridDim.x * blockDim.x) {
-    const int cz = (int)(t % ncz), cy = (int)((t / ncz) % ncy);
-    const long long vx = t / ((long long)ncz * ncy);
+    const long long u = t >> 2;
+    const int j = (int)(t & 3);
+    const int cz = (int)(u % ncz), cy = (int)((u / ncz) % ncy);
+    const long long vx = u / ((long long)ncz * ncy);
+    const int sp = cy - j;
     KahanSum an, ad;
-    for (int j = 0; j < 4; ++j) {
-      const int sp = cy - j;
-      if (sp < 0 || sp >= ay.nsp) continue;
-      for (int vy = ay.lo[sp]; vy < ay.hi[sp]; ++vy) {
+    if (u < ntask && sp >= 0 && sp < ay.nsp) {
+      const float *py = ay.p + (size_t)j * Y, *qy = ay.q + (size_t)j * Y;
+      const int hi = ay.hi[sp];
+#pragma unroll 4
+      for (int vy = ay.lo[sp]; vy < hi; ++vy) {
         const long long i = (vx * Y + vy) * ncz + cz;
-        an.add_prod(ay.p[j * Y + vy], t1n[i]);
-        ad.add_prod(ay.q[j * Y + vy], t1d[i]);
+        an.add_prod(py[vy], t1n[i]);
+        ad.add_prod(qy[vy], t1d[i]);
       }
     }
-    t2n[t] = an.value();
-    t2d[t] = ad.value();
+    const double n = kahan_lanes(an, 4), d = kahan_lanes(ad, 4);
+    if (u < ntask && j == 0) {
+      t2n[u] = (float)n;
+      t2d[u] = (float)d;
+    }
   }
 }
 
-__global__ void k_fit_final(const float *t2n, const float *t2d, int X, Axis ax, int ncy, int ncz,
-                            float eps, int zero_den, float *lattice) {
-  const int ncx = ax.nc;
-  const int nlat = ncx * ncy * ncz;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nlat; c += gridDim.x * blockDim.x) {
-    const int cz = c % ncz, cy = (c / ncz) % ncy, cx = c / (ncz * ncy);
+// The lattice from T2: one warp per control point, its lanes over the
+// x-planes that reach it (24 us with one thread per control point, 4 so).
+__global__ void k_fit_final(const float *__restrict__ t2n, const float *__restrict__ t2d, int X, Axis ax, int ncy,
+                            int ncz, float eps, int zero_den, float *lattice) {
+  const int slice = ncy * ncz, nlat = ax.nc * slice;
+  const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+  for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < nlat; c += nw) {
+    const int cx = c / slice, cc = c - cx * slice;
     KahanSum sn, sd;
     for (int j = 0; j < 4; ++j) {
       const int sp = cx - j;
       if (sp < 0 || sp >= ax.nsp) continue;
-      for (int vx = ax.lo[sp]; vx < ax.hi[sp]; ++vx) {
-        const long long i = ((long long)vx * ncy + cy) * ncz + cz;
-        sn.add_prod(ax.p[j * X + vx], t2n[i]);
-        sd.add_prod(ax.q[j * X + vx], t2d[i]);
+      const float *px = ax.p + (size_t)j * X, *qx = ax.q + (size_t)j * X;
+      const int hi = ax.hi[sp];
+#pragma unroll 2
+      for (int vx = ax.lo[sp] + lane; vx < hi; vx += 32) {
+        const long long i = (long long)vx * slice + cc;
+        sn.add_prod(px[vx], t2n[i]);
+        sd.add_prod(qx[vx], t2d[i]);
       }
     }
-    const float an = sn.value(), ad = sd.value();
-    lattice[c] = zero_den ? (ad != 0.0f ? an / ad : 0.0f) : an / (ad + eps);
+    const float an = (float)kahan_lanes(sn, 32), ad = (float)kahan_lanes(sd, 32);
+    if (lane == 0) lattice[c] = zero_den ? (ad != 0.0f ? an / ad : 0.0f) : an / (ad + eps);
   }
 }
 
@@ -899,26 +960,64 @@ __global__ void k_refine(const float *in, int ncx, int ncy, int ncz, float *out)
 }
 
 // ------------------------------------------------------------------ standalone sharpen
-__global__ void k_minmax(const float *x, const float *mask, long long n, float *part) {
-  float vmin = INFINITY, vmax = -INFINITY;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (mask && mask[i] == 0.0f) continue;
-    vmin = fminf(vmin, x[i]);
-    vmax = fmaxf(vmax, x[i]);
+// Three launches: k_minmax (masked range; its last block forms the statistics
+// and clears the histogram), k_hist (fractional histogram; its last block
+// runs the sharpening map), k_remap.  All are bound by the read of image and
+// mask: 84 MB each at 256x256x160, partly from L2.  A block's last-ness comes
+// from a ticket that the last block sets back to 0.
+
+// True in the last block of the grid to get here; the block's earlier writes
+// are visible to it, and to the last block all the others'.
+__device__ __forceinline__ bool last_block(unsigned *ticket) {
+  __shared__ unsigned s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (s_last) *ticket = 0u;
   }
-  __shared__ double scratch[160];
-  double out[4];
-  block_reduce4(vmin, vmax, 0.0, 0.0, scratch + 8, out);
-  if (threadIdx.x == 0) { part[2 * blockIdx.x] = (float)out[0]; part[2 * blockIdx.x + 1] = (float)out[1]; }
+  __syncthreads();
+  __threadfence();
+  return s_last != 0;
 }
 
-// stats[0] = min, stats[1] = max, stats[2] = slope, stats[3] = 1 / slope (FP64)
-__global__ void k_minmax_final(const float *part, int nb, int bins, double *stats) {
+// body(x, i) for every masked voxel i of the grid's share: four at a time
+// through 16-byte loads where `vec` (x and mask on 16-byte boundaries).
+template <class Body>
+__device__ __forceinline__ void masked_voxels(const float *x, const float *mask, long long n, bool vec, Body &&body) {
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  const long long n4 = vec ? n >> 2 : 0;
+  for (long long q = first; q < n4; q += stride) {
+    const float4 v = __ldg((const float4 *)x + q);
+    const float4 m = mask ? __ldg((const float4 *)mask + q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (m.x != 0.0f) body(v.x);
+    if (m.y != 0.0f) body(v.y);
+    if (m.z != 0.0f) body(v.z);
+    if (m.w != 0.0f) body(v.w);
+  }
+  for (long long i = n4 * 4 + first; i < n; i += stride)
+    if (!mask || mask[i] != 0.0f) body(x[i]);
+}
+
+// stats[0] = min, stats[1] = max, stats[2] = slope, stats[3] = 1 / slope (FP64;
+// 0 where there is no bin range)
+__global__ void __launch_bounds__(256) k_minmax(const float *x, const float *mask, long long n, int vec, float *part,
+                                                int bins, double *stats, unsigned long long *hist, unsigned *ticket) {
   float vmin = INFINITY, vmax = -INFINITY;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) { vmin = fminf(vmin, part[2 * i]); vmax = fmaxf(vmax, part[2 * i + 1]); }
-  __shared__ double scratch[160];
+  masked_voxels(x, mask, n, vec != 0, [&](float v) { vmin = fminf(vmin, v); vmax = fmaxf(vmax, v); });
+  __shared__ double scratch[136];
   double out[4];
-  block_reduce4(vmin, vmax, 0.0, 0.0, scratch + 8, out);
+  block_reduce4(vmin, vmax, 0.0, 0.0, scratch, out);
+  if (threadIdx.x == 0) { part[2 * blockIdx.x] = (float)out[0]; part[2 * blockIdx.x + 1] = (float)out[1]; }
+  if (!last_block(ticket)) return;
+  vmin = INFINITY;
+  vmax = -INFINITY;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+    vmin = fminf(vmin, __ldcg(part + 2 * i));
+    vmax = fmaxf(vmax, __ldcg(part + 2 * i + 1));
+  }
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) hist[b] = 0ull;
+  block_reduce4(vmin, vmax, 0.0, 0.0, scratch, out);
   if (threadIdx.x == 0) {
     const double slope = (out[1] - out[0]) / (double)(bins - 1);
     stats[0] = out[0];
@@ -928,53 +1027,117 @@ __global__ void k_minmax_final(const float *part, int nb, int bins, double *stat
   }
 }
 
-__global__ void k_hist(const float *x, const float *mask, long long n, const double *stats, int bins, int shift,
-                       unsigned long long *hist) {
-  extern __shared__ unsigned hs[];
-  for (int i = threadIdx.x; i < bins; i += blockDim.x) hs[i] = 0u;
+// Dynamic shared memory: the histogram copies, then (last block) the FFT
+// buffers and E.  E_out[bins], R[bins]: the map and its residual form, from
+// which k_remap takes the values (FP64 form as two floats each: x - E(x) =
+// R.x + R.y + f (R.z + R.w) in bin b at fraction f).
+__host__ __device__ inline size_t hist_smem_bytes(int bins, int npad) {
+  const size_t copies = ((size_t)kHistCopies * bins * 4 + 15) / 16 * 16;
+  return copies + (size_t)npad * (16 * 3) + (size_t)(npad / 2 + 2) * 8 + (size_t)bins * 8;
+}
+__global__ void __launch_bounds__(512) k_hist(const float *x, const float *mask, long long n, int vec,
+                                              const double *stats, int bins, int shift, unsigned long long *hist,
+                                              int npad, int hoff, double wiener, double fwhm, double *E_out,
+                                              float4 *R_out, unsigned *ticket) {
+  extern __shared__ __align__(16) char hist_sm[];
+  __shared__ BinMap s_bm;
+  unsigned *copies = (unsigned *)hist_sm;
+  const bool live = stats[3] > 0.0;
+  for (int i = threadIdx.x; i < kHistCopies * bins; i += blockDim.x) copies[i] = 0u;
+  if (threadIdx.x == 0) s_bm = BinMap(stats[0], live ? stats[2] : 1.0, bins);
   __syncthreads();
-  const double inv = stats[3];
-  const BinMap bm(stats[0], inv > 0.0 ? stats[2] : 1.0, bins);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = blockIdx.x * (long long)blockDim.x; base < n; base += stride) {
-    const long long i = base + threadIdx.x;
-    int key = -1;
-    unsigned qlo = 0, qhi = 0;
-    if (i < n && inv > 0.0 && (!mask || mask[i] != 0.0f)) key = hist_bin(bm.coord(x[i]), bins, ldexp(1.0, shift), qlo, qhi);
-    hist_add_warp(hs, bins, key, qlo, qhi);
+  if (live) {
+    const float bmin = s_bm.fmin, ih = s_bm.ih, il = s_bm.il, lim = s_bm.ff_limit;
+    const double scale = ldexp(1.0, shift);
+    const float fscale = (float)scale;
+    const unsigned one = (unsigned)fscale;
+    unsigned *hc = copies + (threadIdx.x >> 5) % kHistCopies * bins;
+    masked_voxels(x, mask, n, vec != 0, [&](float v) {
+      int k;
+      float f;
+      if (coord_split(v, bmin, ih, il, lim, k, f)) {
+        const unsigned qhi = min(__float2uint_rn(__fmul_rn(f, fscale)), one);
+        atomicAdd(&hc[k], one - qhi);
+        atomicAdd(&hc[k + 1], qhi);
+      } else {
+        unsigned qlo = 0, qhi = 0;
+        const int key = hist_bin_top(&s_bm, v, bins, scale, qlo, qhi);
+        if (key >= 0) {
+          atomicAdd(&hc[key], qlo);
+          if (qhi) atomicAdd(&hc[key + 1], qhi);
+        }
+      }
+    });
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < bins; i += blockDim.x)
-    if (hs[i]) atomicAdd(&hist[i], (unsigned long long)hs[i]);
-}
-
-__global__ void k_sharpen(const unsigned long long *hist, const double *stats, int bins, int shift, int npad,
-                          int hoff, double wiener, double fwhm, double *E_out) {
-  extern __shared__ __align__(16) char sm[];
-  double2 *fa = (double2 *)sm, *fb = fa + npad, *tw = fb + npad;
-  double *Ff = (double *)(tw + npad);
-  double *E = Ff + npad;
-  fft_twiddles(tw, npad);
-  __syncthreads();
-  if (stats[3] > 0.0) {
-    SharpenBufs sb{fa, fb, tw, Ff};
-    const double inv = ldexp(1.0, -shift);
-    sharpen_map([=](int b) { return (double)hist[b] * inv; }, bins, npad, hoff, stats[0], stats[2], wiener,
-                gauss_of(stats[2], fwhm), sb, E);
-    for (int b = threadIdx.x; b < bins; b += blockDim.x) E_out[b] = E[b];
-  } else {
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) {
+    unsigned long long s = 0;
+#pragma unroll
+    for (int c = 0; c < kHistCopies; ++c) s += copies[c * bins + b];
+    if (s) atomicAdd(&hist[b], s);
+  }
+  if (!last_block(ticket)) return;
+  if (!live) {
     for (int b = threadIdx.x; b < bins; b += blockDim.x) E_out[b] = 0.0;
+    return;
+  }
+  double2 *fa = (double2 *)(hist_sm + ((size_t)kHistCopies * bins * 4 + 15) / 16 * 16), *fb = fa + npad, *tw = fb + npad;
+  double *Ff = (double *)(tw + npad);
+  double *E = Ff + npad / 2 + 2;
+  fft_twiddles(tw, npad);
+  const double inv = ldexp(1.0, -shift), binMin = s_bm.binMin, slope = s_bm.slope;
+  sharpen_map([=](int b) { return (double)__ldcg(hist + b) * inv; }, bins, npad, hoff, binMin, slope, wiener,
+              gauss_of(slope, fwhm), SharpenBufs{fa, fb, tw, Ff}, E);
+  for (int b = threadIdx.x; b < bins; b += blockDim.x) {
+    const double e = E[b];
+    E_out[b] = e;
+    if (b + 1 < bins) {
+      const double r = binMin + (double)b * slope - e, s = slope - (E[b + 1] - e);
+      const float rh = (float)r, sh = (float)s;
+      R_out[b] = make_float4(rh, (float)(r - (double)rh), sh, (float)(s - (double)sh));
+    }
   }
 }
 
-__global__ void k_remap(const float *x, const float *mask, long long n, const double *stats, const double *E,
-                        int bins, float *out) {
-  const double inv = stats[3];
-  const BinMap bm(stats[0], inv > 0.0 ? stats[2] : 1.0, bins);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (mask && mask[i] == 0.0f) { out[i] = 0.0f; continue; }
-    out[i] = inv > 0.0 ? (float)sharpened_value(bm.coord(x[i]), E, bins) : x[i];
+// x - (R + f S) with R and S as float pairs: the product and the sum of the
+// leading parts exact (Dekker, Knuth), so that the result is E(x) rounded
+// once but for ~2^-25 slope of the fraction.
+__device__ __forceinline__ float remap_value(float x, float f, const float4 t) {
+  const float p = __fmul_rn(f, t.z), pe = __fmaf_rn(f, t.z, -p);
+  float e1, e2;
+  const float s1 = two_sum(x, -t.x, e1), s2 = two_sum(s1, -p, e2);
+  const float low = __fsub_rn(__fadd_rn(e1, e2), __fadd_rn(pe, __fmaf_rn(f, t.w, t.y)));
+  return __fadd_rn(s2, low);
+}
+
+// Dynamic shared memory: R[bins].
+__global__ void __launch_bounds__(512) k_remap(const float *x, const float *mask, long long n, int vec,
+                                               const double *stats, const double *E, const float4 *R, int bins,
+                                               float *out) {
+  extern __shared__ __align__(16) float4 remap_sm[];
+  __shared__ BinMap s_bm;
+  const bool live = stats[3] > 0.0;
+  if (threadIdx.x == 0) s_bm = BinMap(stats[0], live ? stats[2] : 1.0, bins);
+  if (live)
+    for (int b = threadIdx.x; b + 1 < bins; b += blockDim.x) remap_sm[b] = R[b];
+  __syncthreads();
+  const float bmin = s_bm.fmin, ih = s_bm.ih, il = s_bm.il, lim = s_bm.ff_limit;
+  const auto value = [&](float v, float m) {
+    if (m == 0.0f) return 0.0f;
+    if (!live) return v;
+    int k;
+    float f;
+    if (coord_split(v, bmin, ih, il, lim, k, f)) return remap_value(v, f, remap_sm[k]);
+    return (float)sharpened_value(s_bm.coord(v), E, bins);
+  };
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  const long long n4 = vec ? n >> 2 : 0;
+  for (long long q = first; q < n4; q += stride) {
+    const float4 v = __ldg((const float4 *)x + q);
+    const float4 m = mask ? __ldg((const float4 *)mask + q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    __stcs((float4 *)out + q, make_float4(value(v.x, m.x), value(v.y, m.y), value(v.z, m.z), value(v.w, m.w)));
   }
+  for (long long i = n4 * 4 + first; i < n; i += stride) out[i] = value(x[i], mask ? mask[i] : 1.0f);
 }
 
 // ------------------------------------------------------------------ autotuner helper
@@ -991,25 +1154,38 @@ __global__ void k_read_evict(const float4 *p, long long n, float *sink) {
 }
 
 // ------------------------------------------------------------------ standalone convergence
-__global__ void k_cv(const float *f1, const float *f2, const float *mask, long long n, double *part) {
+// Sums of y, y^2 and 1 over the masked voxels, y = exp(f1 - f2) - 1; the last
+// block adds the blocks' sums into sums[0..2].
+__global__ void __launch_bounds__(256) k_cv(const float *f1, const float *f2, const float *mask, long long n,
+                                            double *part, double *sums, unsigned *ticket) {
   double s0 = 0.0, s1 = 0.0, c = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     if (mask && mask[i] == 0.0f) continue;
     const double y = (double)expm1f(__fsub_rn(f1[i], f2[i]));
     s0 += y; s1 += y * y; c += 1.0;
   }
-  s0 = warp_sum(s0); s1 = warp_sum(s1); c = warp_sum(c);
   __shared__ double ws[3][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { ws[0][wid] = s0; ws[1][wid] = s1; ws[2][wid] = c; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0, d = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += ws[0][w]; b += ws[1][w]; d += ws[2][w]; }
-    part[3 * blockIdx.x] = a;
-    part[3 * blockIdx.x + 1] = b;
-    part[3 * blockIdx.x + 2] = d;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const auto block_sum = [&](double *out) {
+    s0 = warp_sum(s0); s1 = warp_sum(s1); c = warp_sum(c);
+    if (lane == 0) { ws[0][wid] = s0; ws[1][wid] = s1; ws[2][wid] = c; }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+      double a = 0.0;
+      for (int w = 0; w < nw; ++w) a += ws[threadIdx.x][w];
+      out[threadIdx.x] = a;
+    }
+    __syncthreads();
+  };
+  block_sum(part + 3 * blockIdx.x);
+  if (!last_block(ticket)) return;
+  s0 = s1 = c = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+    s0 += __ldcg(part + 3 * b);
+    s1 += __ldcg(part + 3 * b + 1);
+    c += __ldcg(part + 3 * b + 2);
   }
+  block_sum(sums);
 }
 
 }  // namespace n4
