@@ -1027,9 +1027,9 @@ n4_status_t launch_correct(int shape, long long tiles, int ncz, cudaStream_t st,
 }
 
 // The log field of one volume over `tiles` tiles of shape `shape`.
-n4_status_t launch_evaluate(int shape, long long tiles, const CorrectVol &vol, cudaStream_t st) {
+n4_status_t launch_evaluate(int shape, long long tiles, const CorrectVol *vol, int ncz, cudaStream_t st) {
   const CorrectShape cs = kCorrectShape[shape];
-  const size_t smem = correct_smem_bytes(cs.rows, vol.ncz);
+  const size_t smem = correct_smem_bytes(cs.rows, ncz);
   if (cs.threads == 512) k_evaluate<512><<<(unsigned)tiles, 512, smem, st>>>(vol, cs.rows);
   else k_evaluate<256><<<(unsigned)tiles, 256, smem, st>>>(vol, cs.rows);
   CK(cudaGetLastError());
@@ -2097,15 +2097,26 @@ static n4_status_t check_fit_sizes(unsigned ncpt_x, unsigned ncpt_y, unsigned nc
   return N4_OK;
 }
 
+// The axis tables of a component call and, for an evaluation (out != null), the
+// descriptor k_evaluate reads, at *vol on the device.
 static n4_status_t component_tables(n4_context_t *ctx, unsigned fx, unsigned fy, unsigned fz, unsigned nx, unsigned ny,
-                                    unsigned nz, cudaStream_t st, Axis &ax, Axis &ay, Axis &az) {
+                                    unsigned nz, cudaStream_t st, Axis &ax, Axis &ay, Axis &az,
+                                    const float *lattice = nullptr, float *out = nullptr, CorrectVol **vol = nullptr) {
   const size_t bx = align_up(axis_bytes(fx, nx - 3), 256), by = align_up(axis_bytes(fy, ny - 3), 256),
                bz = align_up(axis_bytes(fz, nz - 3), 256);
-  TRY(ctx->s5.ensure(bx + by + bz, "tables"));
+  TRY(ctx->s5.ensure(bx + by + bz + sizeof(CorrectVol), "tables"));
   char *base = ctx->s5.as<char>();
   TRY(begin_run(ctx, st));
-  k_axis_tables_of<<<dim3(3, kTableParts), 128, 0, st>>>(TableJob{base, (int)fx, (int)nx}, TableJob{base + bx, (int)fy, (int)ny},
-                                                        TableJob{base + bx + by, (int)fz, (int)nz});
+  const TableJob jx{base, (int)fx, (int)nx}, jy{base + bx, (int)fy, (int)ny}, jz{base + bx + by, (int)fz, (int)nz};
+  const dim3 grid(3, kTableParts);
+  if (out) {
+    *vol = (CorrectVol *)(base + bx + by + bz);
+    k_evaluate_tables<<<grid, 128, 0, st>>>(
+        jx, jy, jz, CorrectVol{nullptr, out, nullptr, lattice, jx.base, jy.base, jz.base, (int)fx, (int)fy, (int)fz,
+                               (int)nx, (int)ny, (int)nz, 0, vec4_ok((int)fz, nullptr, out, nullptr)}, *vol);
+  } else {
+    k_axis_tables_of<<<grid, 128, 0, st>>>(jx, jy, jz);
+  }
   CK(cudaGetLastError());
   ax = axis_at(base, fx, nx);
   ay = axis_at(base + bx, fy, ny);
@@ -2159,10 +2170,8 @@ n4_status_t n4_evaluate_bspline3d(n4_context_t *ctx, const float *d_lattice, uns
   cudaStream_t st = (cudaStream_t)stream;
   Axis ax, ay, az;
   if (ctx->profiling) TRY(prof_mark(ctx, 0, st));
-  TRY(component_tables(ctx, fx, fy, fz, ncpt_x, ncpt_y, ncpt_z, st, ax, ay, az));
-  CorrectVol cv{nullptr, d_fitted, nullptr, d_lattice, (char *)ax.s, (char *)ay.s, (char *)az.s,
-                (int)fx, (int)fy, (int)fz, (int)ncpt_x, (int)ncpt_y, (int)ncpt_z, 0,
-                vec4_ok((int)fz, nullptr, d_fitted, nullptr)};
+  CorrectVol *cv = nullptr;
+  TRY(component_tables(ctx, fx, fy, fz, ncpt_x, ncpt_y, ncpt_z, st, ax, ay, az, d_lattice, d_fitted, &cv));
   int shape = kCorrectDefault;
   auto it = ctx->eval_tune.find(eval_key(fx, fy, fz, ncpt_x, ncpt_y, ncpt_z));
   if (it != ctx->eval_tune.end()) shape = it->second;
@@ -2170,7 +2179,7 @@ n4_status_t n4_evaluate_bspline3d(n4_context_t *ctx, const float *d_lattice, uns
   const long long tiles = ((long long)fx * fy + rt - 1) / rt;
   const bool prof = ctx->profiling != 0;
   if (prof) TRY(prof_mark(ctx, 1, st));
-  TRY(launch_evaluate(shape, tiles, cv, st));
+  TRY(launch_evaluate(shape, tiles, cv, (int)ncpt_z, st));
   if (prof) { TRY(prof_mark(ctx, 2, st)); TRY(prof_mark(ctx, 3, st)); TRY(prof_mark(ctx, 4, st)); }
   ctx->prof_launches = 2;
   ctx->prof_fit = 0;
@@ -2244,15 +2253,14 @@ n4_status_t n4_autotune_components(n4_context_t *ctx, const float *d_field, cons
   if (status == N4_OK)
     status = n4_fit_bspline3d(ctx, d_field, d_mask, ncpt_x, ncpt_y, ncpt_z, fx, fy, fz, 1e-3f, 0, d_lattice, stream);
   if (status == N4_OK) {
-    CorrectVol cv{nullptr, d_out, nullptr, d_lattice, (char *)ax.s, (char *)ay.s, (char *)az.s,
-                  (int)fx, (int)fy, (int)fz, (int)ncpt_x, (int)ncpt_y, (int)ncpt_z, 0,
-                  vec4_ok((int)fz, nullptr, d_out, nullptr)};
+    CorrectVol *cv = nullptr;
+    status = component_tables(ctx, fx, fy, fz, ncpt_x, ncpt_y, ncpt_z, st, ax, ay, az, d_lattice, d_out, &cv);
     for (int k = 0; k < kCorrectShapes && status == N4_OK; ++k) {
       const long long rt = kCorrectShape[k].rows;
       const long long tiles = ((long long)fx * fy + rt - 1) / rt;
       float ms = 0.0f;
       n4_status_t ls = N4_OK;
-      status = timed([&] { ls = launch_evaluate(k, tiles, cv, st); }, &ms);
+      status = timed([&] { ls = launch_evaluate(k, tiles, cv, (int)ncpt_z, st); }, &ms);
       if (status == N4_OK) status = ls;
       if (status != N4_OK) break;
       const int c = rep.eval_candidates++;
@@ -2312,7 +2320,7 @@ n4_status_t n4_sharpen_image(n4_context_t *ctx, const float *d_before, const flo
   const auto blocks = [&](int threads, int per_sm) {
     return (int)std::min<long long>(((long long)n + threads * 4 - 1) / (threads * 4), (long long)ctx->nsm * per_sm);
   };
-  const int nbm = blocks(256, 8), nbh = blocks(512, 2), nbr = blocks(512, 4);
+  const int nbm = blocks(256, 8), nbh = blocks(512, 3), nbr = blocks(512, 3);
   const int vec = ((((uintptr_t)d_before | (uintptr_t)d_mask | (uintptr_t)d_after) & 15u) == 0) ? 1 : 0;
   TRY(ctx->s1.ensure((size_t)nbm * 8 + 64, "partials"));
   // histogram; residual table; then what the host reads: statistics and E

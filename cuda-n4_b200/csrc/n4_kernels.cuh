@@ -15,6 +15,7 @@
 //   k_cv              standalone convergence measurement
 #pragma once
 #include <cuda_bf16.h>
+#include <type_traits>
 
 #include "n4_engine.cuh"
 
@@ -401,15 +402,12 @@ __host__ __device__ inline size_t correct_smem_bytes(int rows, int ncz) {
 // I/O.  HBM traffic: read im, write out (+ bias).
 constexpr int kCorrectPre = 3;   // rows of input float4s a thread loads per step (two steps in flight)
 
-// Tile `tile` of a batch (numbered as in CorrectVol::tile0) of the volumes
-// vols[0 .. nvol); Gs and Lx in shared memory.  kLog: every volume's im is
-// null and the log field is the output (its own instantiation: no input
-// registers held).
+// Tile `tile` of volume C (numbered as in CorrectVol::tile0); Gs and Lx in
+// shared memory.  kLog: im is null and the log field is the output (its own
+// instantiation: no input registers held).
 template <bool kLog>
-__device__ __forceinline__ void correct_tile(const CorrectVol *vols, const long long *tile_starts, int nvol,
-                                             long long tile, float low, int rt, float *Gs, float *Lx) {
-  const int v = find_volume(tile_starts, nvol, tile);
-  const CorrectVol &C = vols[v];
+__device__ __forceinline__ void correct_tile(const CorrectVol &C, long long tile, float low, int rt, float *Gs,
+                                             float *Lx) {
   const Axis ax = axis_at(C.tx, C.FX, C.ncx), ay = axis_at(C.ty, C.FY, C.ncy), az = axis_at(C.tz, C.FZ, C.ncz);
   const long long rows = (long long)C.FX * C.FY;
   const long long row0 = (tile - C.tile0) * (long long)rt;
@@ -620,14 +618,26 @@ template <int NT>
 __global__ void __launch_bounds__(NT, NT <= 256 ? 3 : 1) k_correct(const CorrectVol *vols, const long long *tile_starts,
                                                                    int nvol, long long t0, float low, int rt) {
   extern __shared__ __align__(16) float correct_sm[];
-  correct_tile<false>(vols, tile_starts, nvol, t0 + blockIdx.x, low, rt, correct_sm + 2 * kLxMax, correct_sm);
+  const long long tile = t0 + blockIdx.x;
+  correct_tile<false>(vols[find_volume(tile_starts, nvol, tile)], tile, low, rt, correct_sm + 2 * kLxMax, correct_sm);
 }
 
-// The log field of one volume (EvaluateBspline3D), its descriptor by value.
+// The log field of one volume (EvaluateBspline3D).
 template <int NT>
-__global__ void __launch_bounds__(NT, NT <= 256 ? 4 : 1) k_evaluate(const __grid_constant__ CorrectVol vol, int rt) {
+__global__ void __launch_bounds__(NT, NT <= 256 ? 4 : 1) k_evaluate(const CorrectVol *vol, int rt) {
   extern __shared__ __align__(16) float correct_sm[];
-  correct_tile<true>(&vol, nullptr, 1, blockIdx.x, 0.0f, rt, correct_sm + 2 * kLxMax, correct_sm);
+  correct_tile<true>(*vol, blockIdx.x, 0.0f, rt, correct_sm + 2 * kLxMax, correct_sm);
+}
+
+// The tables of one evaluation's three axes, and its descriptor, from its
+// parameters into memory: k_evaluate reads it from there (as a parameter of
+// k_evaluate its fields took registers: spills, 60 instead of 57 us at
+// 512x512x320; uploaded, a copy before every call).
+__global__ void k_evaluate_tables(TableJob jx, TableJob jy, TableJob jz, const __grid_constant__ CorrectVol vol,
+                                  CorrectVol *out) {
+  const TableJob t = blockIdx.x == 0 ? jx : (blockIdx.x == 1 ? jy : jz);
+  build_axis(axis_at(t.base, t.n, t.nc), blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
+  if (blockIdx.x + blockIdx.y + threadIdx.x == 0) *out = vol;
 }
 
 // ------------------------------------------------------------------ standalone fit
@@ -981,22 +991,27 @@ __device__ __forceinline__ bool last_block(unsigned *ticket) {
   return s_last != 0;
 }
 
-// body(x, i) for every masked voxel i of the grid's share: four at a time
-// through 16-byte loads where `vec` (x and mask on 16-byte boundaries).
-template <class Body>
-__device__ __forceinline__ void masked_voxels(const float *x, const float *mask, long long n, bool vec, Body &&body) {
+// quad(q, x, m) for every four voxels 4q .. 4q + 3 of the grid's share and
+// one(i, x, m) for single voxels: 16-byte loads where `vec` (x and mask on
+// 16-byte boundaries).  The mask is read first, and x only where it has a voxel
+// (elsewhere x is a NaN): most of a head's box is background.  One quad per
+// thread in flight: four took 64 registers, half the warps, and 124 instead of
+// 112 us for the whole call at 256x256x160.
+template <class Quad, class One>
+__device__ __forceinline__ void voxel_quads(const float *x, const float *mask, long long n, bool vec, Quad &&quad,
+                                            One &&one) {
   const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
   const long long n4 = vec ? n >> 2 : 0;
   for (long long q = first; q < n4; q += stride) {
-    const float4 v = __ldg((const float4 *)x + q);
     const float4 m = mask ? __ldg((const float4 *)mask + q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    if (m.x != 0.0f) body(v.x);
-    if (m.y != 0.0f) body(v.y);
-    if (m.z != 0.0f) body(v.z);
-    if (m.w != 0.0f) body(v.w);
+    float4 v = make_float4(kNaN, kNaN, kNaN, kNaN);
+    if (m.x != 0.0f || m.y != 0.0f || m.z != 0.0f || m.w != 0.0f) v = __ldg((const float4 *)x + q);
+    quad(q, v, m);
   }
-  for (long long i = n4 * 4 + first; i < n; i += stride)
-    if (!mask || mask[i] != 0.0f) body(x[i]);
+  for (long long i = n4 * 4 + first; i < n; i += stride) {
+    const float m = mask ? mask[i] : 1.0f;
+    one(i, m != 0.0f ? x[i] : kNaN, m);
+  }
 }
 
 // stats[0] = min, stats[1] = max, stats[2] = slope, stats[3] = 1 / slope (FP64;
@@ -1004,7 +1019,15 @@ __device__ __forceinline__ void masked_voxels(const float *x, const float *mask,
 __global__ void __launch_bounds__(256) k_minmax(const float *x, const float *mask, long long n, int vec, float *part,
                                                 int bins, double *stats, unsigned long long *hist, unsigned *ticket) {
   float vmin = INFINITY, vmax = -INFINITY;
-  masked_voxels(x, mask, n, vec != 0, [&](float v) { vmin = fminf(vmin, v); vmax = fmaxf(vmax, v); });
+  const auto take = [&](float v, float m) {
+    v = m != 0.0f ? v : kNaN;   // a NaN operand is passed over
+    vmin = fminf(vmin, v);
+    vmax = fmaxf(vmax, v);
+  };
+  voxel_quads(
+      x, mask, n, vec != 0,
+      [&](long long, const float4 &v, const float4 &m) { take(v.x, m.x); take(v.y, m.y); take(v.z, m.z); take(v.w, m.w); },
+      [&](long long, float v, float m) { take(v, m); });
   __shared__ double scratch[136];
   double out[4];
   block_reduce4(vmin, vmax, 0.0, 0.0, scratch, out);
@@ -1035,7 +1058,7 @@ __host__ __device__ inline size_t hist_smem_bytes(int bins, int npad) {
   const size_t copies = ((size_t)kHistCopies * bins * 4 + 15) / 16 * 16;
   return copies + (size_t)npad * (16 * 3) + (size_t)(npad / 2 + 2) * 8 + (size_t)bins * 8;
 }
-__global__ void __launch_bounds__(512) k_hist(const float *x, const float *mask, long long n, int vec,
+__global__ void __launch_bounds__(512, 3) k_hist(const float *x, const float *mask, long long n, int vec,
                                               const double *stats, int bins, int shift, unsigned long long *hist,
                                               int npad, int hoff, double wiener, double fwhm, double *E_out,
                                               float4 *R_out, unsigned *ticket) {
@@ -1052,22 +1075,38 @@ __global__ void __launch_bounds__(512) k_hist(const float *x, const float *mask,
     const float fscale = (float)scale;
     const unsigned one = (unsigned)fscale;
     unsigned *hc = copies + (threadIdx.x >> 5) % kHistCopies * bins;
-    masked_voxels(x, mask, n, vec != 0, [&](float v) {
-      int k;
-      float f;
-      if (coord_split(v, bmin, ih, il, lim, k, f)) {
-        const unsigned qhi = min(__float2uint_rn(__fmul_rn(f, fscale)), one);
-        atomicAdd(&hc[k], one - qhi);
-        atomicAdd(&hc[k + 1], qhi);
-      } else {
-        unsigned qlo = 0, qhi = 0;
-        const int key = hist_bin_top(&s_bm, v, bins, scale, qlo, qhi);
-        if (key >= 0) {
-          atomicAdd(&hc[key], qlo);
-          if (qhi) atomicAdd(&hc[key + 1], qhi);
+    // N voxels, their coordinates formed together
+    const auto add = [&](auto N, const float *v, const float *m) {
+      constexpr int kN = decltype(N)::value;
+      int k[kN];
+      float f[kN];
+      bool in[kN];
+#pragma unroll
+      for (int u = 0; u < kN; ++u) in[u] = coord_split(v[u], bmin, ih, il, lim, k[u], f[u]) && m[u] != 0.0f;
+#pragma unroll
+      for (int u = 0; u < kN; ++u) {
+        if (in[u]) {
+          const unsigned qhi = min(__float2uint_rn(__fmul_rn(f[u], fscale)), one);
+          atomicAdd(&hc[k[u]], one - qhi);
+          atomicAdd(&hc[k[u] + 1], qhi);
+        } else if (m[u] != 0.0f) {
+          unsigned qlo = 0, qhi = 0;
+          const int key = hist_bin_top(&s_bm, v[u], bins, scale, qlo, qhi);
+          if (key >= 0) {
+            atomicAdd(&hc[key], qlo);
+            if (qhi) atomicAdd(&hc[key + 1], qhi);
+          }
         }
       }
-    });
+    };
+    voxel_quads(
+        x, mask, n, vec != 0,
+        [&](long long, const float4 &v, const float4 &m) {
+          if (m.x == 0.0f && m.y == 0.0f && m.z == 0.0f && m.w == 0.0f) return;
+          const float va[4] = {v.x, v.y, v.z, v.w}, ma[4] = {m.x, m.y, m.z, m.w};
+          add(std::integral_constant<int, 4>(), va, ma);
+        },
+        [&](long long, float v, float m) { add(std::integral_constant<int, 1>(), &v, &m); });
   }
   __syncthreads();
   for (int b = threadIdx.x; b < bins; b += blockDim.x) {
@@ -1111,33 +1150,51 @@ __device__ __forceinline__ float remap_value(float x, float f, const float4 t) {
 }
 
 // Dynamic shared memory: R[bins].
-__global__ void __launch_bounds__(512) k_remap(const float *x, const float *mask, long long n, int vec,
+__global__ void __launch_bounds__(512, 3) k_remap(const float *x, const float *mask, long long n, int vec,
                                                const double *stats, const double *E, const float4 *R, int bins,
                                                float *out) {
   extern __shared__ __align__(16) float4 remap_sm[];
   __shared__ BinMap s_bm;
   const bool live = stats[3] > 0.0;
   if (threadIdx.x == 0) s_bm = BinMap(stats[0], live ? stats[2] : 1.0, bins);
-  if (live)
-    for (int b = threadIdx.x; b + 1 < bins; b += blockDim.x) remap_sm[b] = R[b];
+  for (int b = threadIdx.x; b < bins; b += blockDim.x)
+    remap_sm[b] = live && b + 1 < bins ? R[b] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   __syncthreads();
   const float bmin = s_bm.fmin, ih = s_bm.ih, il = s_bm.il, lim = s_bm.ff_limit;
-  const auto value = [&](float v, float m) {
-    if (m == 0.0f) return 0.0f;
-    if (!live) return v;
-    int k;
-    float f;
-    if (coord_split(v, bmin, ih, il, lim, k, f)) return remap_value(v, f, remap_sm[k]);
-    return (float)sharpened_value(s_bm.coord(v), E, bins);
+  // N voxels' values, 0 outside the mask
+  const auto values = [&](auto N, float *v, const float *m) {
+    constexpr int kN = decltype(N)::value;
+    unsigned top = 0;
+#pragma unroll
+    for (int u = 0; u < kN; ++u) {
+      int k;
+      float f;
+      const bool in = coord_split(v[u], bmin, ih, il, lim, k, f);
+      if (!in && m[u] != 0.0f) top |= 1u << u;
+      const float r = remap_value(v[u], f, remap_sm[k]);
+      v[u] = m[u] == 0.0f ? 0.0f : (live && in ? r : v[u]);
+    }
+    if (live && top) {
+#pragma unroll
+      for (int u = 0; u < kN; ++u)
+        if (top >> u & 1u) v[u] = (float)sharpened_value(s_bm.coord(v[u]), E, bins);
+    }
   };
-  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-  const long long n4 = vec ? n >> 2 : 0;
-  for (long long q = first; q < n4; q += stride) {
-    const float4 v = __ldg((const float4 *)x + q);
-    const float4 m = mask ? __ldg((const float4 *)mask + q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    __stcs((float4 *)out + q, make_float4(value(v.x, m.x), value(v.y, m.y), value(v.z, m.z), value(v.w, m.w)));
-  }
-  for (long long i = n4 * 4 + first; i < n; i += stride) out[i] = value(x[i], mask ? mask[i] : 1.0f);
+  voxel_quads(
+      x, mask, n, vec != 0,
+      [&](long long q, const float4 &v, const float4 &m) {
+        float va[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (m.x != 0.0f || m.y != 0.0f || m.z != 0.0f || m.w != 0.0f) {
+          const float ma[4] = {m.x, m.y, m.z, m.w};
+          va[0] = v.x; va[1] = v.y; va[2] = v.z; va[3] = v.w;
+          values(std::integral_constant<int, 4>(), va, ma);
+        }
+        __stcs((float4 *)out + q, make_float4(va[0], va[1], va[2], va[3]));
+      },
+      [&](long long i, float v, float m) {
+        values(std::integral_constant<int, 1>(), &v, &m);
+        out[i] = v;
+      });
 }
 
 // ------------------------------------------------------------------ autotuner helper
