@@ -271,9 +271,10 @@ __device__ __forceinline__ void stockham_pass(const In &in, double2 *y, int N, i
 // Forward FFT (length N = 2^m, 4 <= N <= 4096) of in(0..N): radix 4, the last
 // pass radix 2 where N is no power of 4; the first pass goes to a, the others
 // ping-pong a and b, each ending with a CTA barrier.  Returns the buffer that
-// holds the result.  (Radix 8 needs more registers than the engine's kernels
-// have left.)  NC: N where it is known at compile time (512, up to 256 bins:
-// the passes' strides and twiddle steps become constants), else 0.
+// holds the result.  NC: N where it is known at compile time (512, up to 256
+// bins: the passes' strides and twiddle steps become constants), else 0.
+// (Three radix-8 passes of 64 threads took 11.0k instead of 12.0k cycles for
+// the map, but round differently, and N4 on a small volume follows every bit.)
 template <int NC, class In>
 __device__ __forceinline__ double2 *fft_from(const In &in, double2 *a, double2 *b, int N, const double2 *tw) {
   auto from = [](const double2 *x) { return [x](int i) { return x[i]; }; };
@@ -436,23 +437,23 @@ struct BinMap {
 
 // The same coordinate in float-float arithmetic, from the map's fields fmin,
 // ih + il and ff_limit: the bin k and the fraction f of x, or false within
-// two bins of the top and for a NaN (k = 0, f = 0: in range of every table).
-// Branch-free, so that several voxels' chains overlap.
+// two bins of the top and for a NaN (then k = 0, in range of every table, and
+// f is of no use).  Branch-free, so that several voxels' chains overlap, and
+// without conversions, which go at a quarter of the rate: adding 2^23 rounded
+// down leaves floor(p) in the low bits.
 __device__ __forceinline__ bool coord_split(float x, float fmin, float ih, float il, float limit, int &k, float &f) {
+  constexpr float kMagic = 8388608.0f;   // 2^23
   float dl;
   const float dh = two_sum(x, -fmin, dl);                  // x - binMin = dh + dl exactly
   const float p = __fmul_rn(dh, ih);
   const float pe = __fmaf_rn(dh, ih, -p);                  // p + pe = dh * ih exactly
   const float cl = __fadd_rn(pe, __fmaf_rn(dh, il, __fmul_rn(dl, ih)));
   const bool in = p < limit;                               // not near the top bin (or NaN)
-  const float kf = floorf(p);
-  float fr = __fadd_rn(__fsub_rn(p, kf), cl);              // p - kf is exact
-  int kk = (int)kf;
-  if (fr < 0.0f) { fr = __fadd_rn(fr, 1.0f); --kk; }
-  else if (fr >= 1.0f) { fr = __fsub_rn(fr, 1.0f); ++kk; }
-  const bool ok = in && kk >= 0;                           // x >= binMin: only rounding gives kk < 0
-  k = ok ? kk : 0;
-  f = ok ? fr : 0.0f;
+  const float t = __fadd_rd(p, kMagic);                    // 2^23 + floor(p), for 0 <= p < 2^22
+  const float fr = __fadd_rn(__fsub_rn(p, __fsub_rn(t, kMagic)), cl);   // p - floor(p) is exact
+  const float step = fr < 0.0f ? 1.0f : (fr >= 1.0f ? -1.0f : 0.0f);
+  f = __fadd_rn(fr, step);
+  k = in ? max(__float_as_int(__fsub_rn(t, step)) - __float_as_int(kMagic), 0) : 0;   // x >= binMin: never below 0
   return in;
 }
 
@@ -580,34 +581,34 @@ __device__ void refine_lattice(const float *L, int ncx, int ncy, int ncz, float 
 
 // ---------------------------------------------------------------- grid barrier
 // Barrier over all CTAs of a cooperative launch: arrivals are counted up
-// from zero, and a CTA waits until the count reaches the end of its own
-// round.  One release-add and one acquire-poll per CTA and round.  Every wait
-// is bounded: on timeout (or when another CTA already failed) it records
-// N4_ERR_TIMEOUT in *err and returns false.
+// from zero, and a CTA waits until the count reaches the end of its round
+// (counted by thread 0).  One release-add and one acquire-poll per CTA and
+// round: the CTA's barriers on both sides extend them to its other threads,
+// which read what other CTAs wrote past L1 (__ldcg).  Every wait is bounded:
+// on timeout (or when another CTA already failed) it records N4_ERR_TIMEOUT in
+// *err and returns false.
 struct GridBarrier {
   unsigned *count;
   int *err;
   unsigned nblocks;
+  unsigned target;   // arrivals at the end of this CTA's last round; starts at 0
 
-  __device__ bool sync() const {
+  __device__ bool sync() {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-      unsigned t;
-      __threadfence();
-      asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(count) : "memory");
-      const unsigned end = t / nblocks * nblocks + nblocks;   // the round this arrival belongs to
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+      target += nblocks;
       unsigned long long spins = 0;
       int ok = 1;
       for (;;) {
         unsigned c;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-        if ((int)(c - end) >= 0) break;
+        if ((int)(c - target) >= 0) break;
         ++spins;
         if ((spins & 255u) == 0 && *(volatile int *)err != 0) { ok = 0; break; }
         if (spins > kSpinLimit) { atomicExch(err, (int)N4_ERR_TIMEOUT); ok = 0; break; }
       }
-      __threadfence();
       s_ok = ok;
     }
     __syncthreads();

@@ -149,8 +149,8 @@ struct ClusterGroup {
 
 // Accumulators of the whole-GPU path in global memory, zero at launch: three
 // sets used in turn (one is cleared while the next is in use), each `len`
-// words for the histogram or the lattice sums, the last word a count of
-// partials that are not numbers.
+// words for the range, the histogram or the lattice sums, the last word a
+// count of partials that are not numbers.
 struct GridGroup {
   GridBarrier bar;
   char *big_base;      // per-CTA big regions, stride big_stride
@@ -160,7 +160,7 @@ struct GridGroup {
   unsigned *ext;       // [X*Y] row ranges z0 | z1 << 16 (0: no masked voxel)
   __device__ int rank() const { return (int)blockIdx.x; }
   __device__ int size() const { return (int)gridDim.x; }
-  __device__ bool sync() const { return bar.sync(); }
+  __device__ bool sync() { return bar.sync(); }
   template <class T> __device__ const T *peer(const T *p, int r) const {
     const char *mine = big_base + (size_t)blockIdx.x * big_stride;
     return (const T *)(big_base + (size_t)r * big_stride + ((const char *)p - mine));
@@ -274,24 +274,40 @@ struct Engine {
   __device__ __forceinline__ float *slotC() const { return at<float>(pl.sm_bytes + pl.b_slotC); }   // cluster path
 
   // ---- rows.  Row r of the CTA: its voxels [z0, z1), voxel z at p[z]; its
-  // plane m and y.
+  // plane m and y.  A pass takes the row map by value before its loops: read
+  // through the Engine, its fields would be loaded again after every store.
   struct Row {
     int z0, z1, m, vy;
     float *p;
   };
-  __device__ __forceinline__ Row row(int r) const {
-    Row o;
-    if constexpr (Group::kGrid) {
-      const int4 d = rowsp[r];
-      o.z0 = d.y & 0xffff; o.z1 = (int)((unsigned)d.y >> 16); o.m = d.z; o.vy = d.w;
-      o.p = (d.x + o.z1 <= slab_cap ? at<float>(slab_off) : slab_g) + d.x;
-    } else {
-      const uint2 d = at<uint2>(pl.o_rows)[r];
+  struct ClusterRows {
+    int rows, slab, Y, Z;   // byte offsets of the list and of the slab
+    __device__ __forceinline__ Row operator()(int r) const {
+      const uint2 d = at<uint2>(rows)[r];
+      Row o;
       o.z0 = (int)(d.x & 0xffffu); o.z1 = (int)(d.x >> 16);
       o.m = (int)(d.y >> 16); o.vy = (int)(d.y & 0xffffu);
-      o.p = at<float>(pl.sm_bytes + pl.b_imlog) + (o.m * Y + o.vy) * Z;
+      o.p = at<float>(slab) + (o.m * Y + o.vy) * Z;
+      return o;
     }
-    return o;
+    __device__ __forceinline__ int vy(int r) const { return (int)(at<uint2>(rows)[r].y & 0xffffu); }
+  };
+  struct GridRows {
+    const int4 *rows;
+    int slab, cap;          // byte offset of the shared slab, its floats
+    float *slab_g;          // where rows beyond it are
+    __device__ __forceinline__ Row operator()(int r) const {
+      const int4 d = rows[r];
+      Row o;
+      o.z0 = d.y & 0xffff; o.z1 = (int)((unsigned)d.y >> 16); o.m = d.z; o.vy = d.w;
+      o.p = (d.x + o.z1 <= cap ? at<float>(slab) : slab_g) + d.x;
+      return o;
+    }
+    __device__ __forceinline__ int vy(int r) const { return rows[r].w; }
+  };
+  __device__ __forceinline__ auto row_map() const {
+    if constexpr (Group::kGrid) return GridRows{rowsp, slab_off, slab_cap, slab_g};
+    else return ClusterRows{pl.o_rows, pl.sm_bytes + pl.b_imlog, Y, Z};
   }
   __device__ __forceinline__ int plane_vx(int m) const { return Group::kGrid ? vx0 + m : rank + m * K; }
   __device__ __forceinline__ const float *src_row(const Row &r) const {
@@ -374,13 +390,14 @@ struct Engine {
   // rows of a plane are ytab[m][sp] .. ytab[m][sp + 1] - 1.
   __device__ void build_ytab(int m0, int cnt) {
     const int w = ay.nsp + 1;
+    const auto rm = row_map();
     for (int t = threadIdx.x; t < cnt * w; t += blockDim.x) {
       const int m = m0 + t / w, sp = t % w;
       const int vy = sp < ay.nsp ? at<int>(ay.o_lo)[sp] : Y;
       int lo = 0, hi = nact;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        const Row r = row(mid);
+        const Row r = rm(mid);
         if (r.m > m || (r.m == m && r.vy >= vy)) hi = mid;
         else lo = mid + 1;
       }
@@ -393,10 +410,11 @@ struct Engine {
   __device__ void rowtab(const float *lat) {
     const int lsh = ncz_log2();
     float *Gt = Gd();
+    const auto rm = row_map();
     for (int t = threadIdx.x; t < (nact << lsh); t += blockDim.x) {
       const int r = t >> lsh, cz = t & ((1 << lsh) - 1);
       if (cz >= ncz) continue;
-      const Row o = row(r);
+      const Row o = rm(r);
       const int vx = plane_vx(o.m);
       const int sx = at<int>(ax.o_s)[vx], sy = at<int>(ay.o_s)[o.vy];
       const float4 wx = at<float4>(ax.o_w)[vx], wy = at<float4>(ay.o_w)[o.vy];
@@ -436,18 +454,22 @@ struct Engine {
       Xp[t] = __fmaf_rn(wx.w, pa[3 * slice], a);
     }
     __syncthreads();
-    const int lsh = ncz_log2();
+    const int lsh = ncz_log2(), nc = ncz, n = nact << lsh, cz = threadIdx.x & ((1 << lsh) - 1);
     float *Gt = Gd();
-    for (int t = threadIdx.x; t < (nact << lsh); t += blockDim.x) {
-      const int r = t >> lsh, cz = t & ((1 << lsh) - 1);
-      if (cz >= ncz) continue;
-      const Row o = row(r);
-      const float4 wy = at<float4>(ay.o_w)[o.vy];
-      const float *xa = Xp + o.m * slice + at<int>(ay.o_s)[o.vy] * ncz + cz;
-      float a = __fmul_rn(wy.x, xa[0]);
-      a = __fmaf_rn(wy.y, xa[ncz], a);
-      a = __fmaf_rn(wy.z, xa[2 * ncz], a);
-      Gt[r * ncz + cz] = __fmaf_rn(wy.w, xa[3 * ncz], a);
+    const auto rm = row_map();
+    const float4 *W = at<float4>(ay.o_w);
+    const int *S = at<int>(ay.o_s);
+    if (cz < nc) {   // blockDim is a multiple of 2^lsh: a thread keeps its cz
+      for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const int r = t >> lsh;
+        const Row o = rm(r);
+        const float4 wy = W[o.vy];
+        const float *xa = Xp + o.m * slice + S[o.vy] * nc + cz;
+        float a = __fmul_rn(wy.x, xa[0]);
+        a = __fmaf_rn(wy.y, xa[nc], a);
+        a = __fmaf_rn(wy.z, xa[2 * nc], a);
+        Gt[r * nc + cz] = __fmaf_rn(wy.w, xa[3 * nc], a);
+      }
     }
   }
 
@@ -457,19 +479,18 @@ struct Engine {
   template <class Body>
   __device__ __forceinline__ void span_pass(Body &&body) const {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int l = lane & ((1 << sg) - 1), sub = lane >> sg, rs = 5 - sg;
-    const int per = (1 << sg) >> sh;   // spans per round
-    const int ntask = (nact + (1 << rs) - 1) >> rs;
-    for (int sp0 = 0; sp0 < az.nsp; sp0 += per) {
-      const int sp = sp0 + (l >> sh), h = l & ((1 << sh) - 1);
-      const bool on = sp < az.nsp;
-      const int lo = on ? at<int>(az.o_lo)[sp] : 0, hi = on ? at<int>(az.o_hi)[sp] : 0;
-      for (int task = warp; task < ntask; task += nw) {
-        const int r = (task << rs) + sub;
-        if (r >= nact) continue;
-        const Row o = row(r);
+    const int sh_ = sh, l = lane & ((1 << sg) - 1), sub = lane >> sg, rs = 5 - sg, n = nact, nsp = az.nsp;
+    const int per = (1 << sg) >> sh_;   // spans per round
+    const auto rm = row_map();
+    const int *Lo = at<int>(az.o_lo), *Hi = at<int>(az.o_hi);
+    for (int sp0 = 0; sp0 < nsp; sp0 += per) {
+      const int sp = sp0 + (l >> sh_), h = l & ((1 << sh_) - 1);
+      const bool on = sp < nsp;
+      const int lo = on ? Lo[sp] : 0, hi = on ? Hi[sp] : 0;
+      for (int r = (warp << rs) + sub; r < n; r += nw << rs) {
+        const Row o = rm(r);
         int a, b;
-        piece(o, lo, hi, h, sh, a, b);
+        piece(o, lo, hi, h, sh_, a, b);
         body(o, r, a, b, sp);
       }
     }
@@ -484,14 +505,18 @@ struct Engine {
     rowtab(lat);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s;
-    for (int r = (warp << rs) + sub; r < nact; r += nw << rs) {
-      const Row o = row(r);
+    const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s, n = nact, nc = ncz;
+    const auto rm = row_map();
+    const float *Gp = Gd();
+    const float4 *W = at<float4>(az.o_w);
+    const int *S = at<int>(az.o_s);
+    for (int r = (warp << rs) + sub; r < n; r += nw << rs) {
+      const Row o = rm(r);
       const float *im = staged ? o.p : src_row(o);
-      const float *g0 = Gd() + r * ncz;
+      const float *g0 = Gp + r * nc;
       for (int z = o.z0 + l; z < o.z1; z += 1 << s) {
         const float v = im[z];
-        o.p[z] = isnan(v) ? v : __fsub_rn(v, dot4(at<float4>(az.o_w)[z], g0 + at<int>(az.o_s)[z]));
+        o.p[z] = isnan(v) ? v : __fsub_rn(v, dot4(W[z], g0 + S[z]));
       }
     }
     __syncthreads();
@@ -499,14 +524,21 @@ struct Engine {
 
   // ---- group reductions
   // Masked min/max and the convergence sums of the group, then what the
-  // iteration takes from them (Iter), the same in every CTA.  idle() runs on
-  // the CTA's other warps while the first one reduces.
+  // iteration takes from them (Iter), the same in every CTA.
   static __device__ __forceinline__ int fkey(float v) {   // order of floats as order of ints (an involution)
     const int k = __float_as_int(v);
     return k ^ ((k >> 31) & 0x7fffffff);
   }
   static __device__ __forceinline__ float funkey(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
 
+  // unsigned keys in the floats' order, 0 below all of them
+  static __device__ __forceinline__ unsigned long long ukey(float v) { return (unsigned)fkey(v) ^ 0x80000000u; }
+  static __device__ __forceinline__ float unukey(unsigned long long k) { return funkey((int)((unsigned)k ^ 0x80000000u)); }
+
+  // Warp 0 takes the range and forms the bin map, warp 1 the sums and the
+  // convergence value (chains of FP64 divisions), the others run idle().
+  // Whole-GPU path: the range by atomics on the accumulator set, the sums in
+  // CTA order from the CTAs' slots.
   template <class Idle>
   __device__ bool reduce_stats(float vmin, float vmax, double s0, double s1, bool need_cv, Idle &&idle) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -516,49 +548,83 @@ struct Engine {
     if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
     if (lane == 0) { sc[warp] = vmin; sc[32 + warp] = vmax; sc[64 + warp] = s0; sc[96 + warp] = s1; }
     __syncthreads();
+    const bool in = lane < nw;
     if (warp == 0) {
-      const bool in = lane < nw;
       vmin = funkey(__reduce_min_sync(kFull, fkey(in ? (float)sc[lane] : INFINITY)));
       vmax = funkey(__reduce_max_sync(kFull, fkey(in ? (float)sc[32 + lane] : -INFINITY)));
-      s0 = in ? sc[64 + lane] : 0.0;
-      s1 = in ? sc[96 + lane] : 0.0;
-      if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
-      if (lane == 0) { Stats *a = slotA(); a->v[0] = vmin; a->v[1] = vmax; a->v[2] = s0; a->v[3] = s1; }
+      if (lane == 0) {
+        if constexpr (Group::kGrid) {
+          atomicMax(acc_set(seq), ~ukey(vmin) & 0xffffffffull);
+          atomicMax(acc_set(seq) + 1, ukey(vmax));
+        } else {
+          slotA()->v[0] = vmin;
+          slotA()->v[1] = vmax;
+        }
+      }
+    } else if (warp == 1 && need_cv) {
+      s0 = warp_sum(in ? sc[64 + lane] : 0.0);
+      s1 = warp_sum(in ? sc[96 + lane] : 0.0);
+      if (lane == 0) { slotA()->v[2] = s0; slotA()->v[3] = s1; }
     }
     N4_MARK(PH_A_LOOP);
     if (!g.sync()) return false;
+    Iter &it = iter();
     if (warp == 0) {
       float mn = INFINITY, mx = -INFINITY;
-      s0 = 0.0;
-      s1 = 0.0;
-      for (int k = lane; k < K; k += 32) {
-        const Stats *p = g.peer(slotA(), k);
-        double v[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = Group::kGrid ? __ldcg(&p->v[i]) : p->v[i];
-        mn = fminf(mn, (float)v[0]);
-        mx = fmaxf(mx, (float)v[1]);
-        s0 += v[2];
-        s1 += v[3];
+      if constexpr (Group::kGrid) {
+        mn = unukey(~__ldcg(acc_set(seq)) & 0xffffffffull);
+        mx = unukey(__ldcg(acc_set(seq) + 1));
+      } else if (lane < K) {
+        const Stats *p = g.peer(slotA(), lane);
+        mn = (float)p->v[0];
+        mx = (float)p->v[1];
       }
-      mn = funkey(__reduce_min_sync(kFull, fkey(mn)));
-      mx = funkey(__reduce_max_sync(kFull, fkey(mx)));
-      if (need_cv) { s0 = warp_sum(s0); s1 = warp_sum(s1); }
+      if constexpr (!Group::kGrid) {
+        mn = funkey(__reduce_min_sync(kFull, fkey(mn)));
+        mx = funkey(__reduce_max_sync(kFull, fkey(mx)));
+      }
       if (lane == 0) {
-        Iter &it = iter();
-        it.st[0] = mn; it.st[1] = mx; it.st[2] = s0; it.st[3] = s1;
+        it.st[0] = mn; it.st[1] = mx;
         // bin range of the masked logU (N4.py:14-15); st holds FP32 values
         const double slope = ((double)mx - (double)mn) / (double)(pr.bins - 1);
         it.degenerate = !(slope > 0.0) || !isfinite(slope);
         it.bm = BinMap(mn, it.degenerate ? 1.0 : slope, pr.bins);
         it.scale = ldexp(1.0, hshift);
-        it.gauss = gauss_of(it.bm.slope, pr.fwhm);
-        if (need_cv) it.cv = cv_from(it.st);
+      }
+    } else if (warp == 1) {
+      if (need_cv) {
+        s0 = s1 = 0.0;
+        if constexpr (Group::kGrid) {
+          // eight slots' loads in flight
+          for (int k0 = lane; k0 < K; k0 += 256) {
+            double a[8], b[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const Stats *p = g.peer(slotA(), min(k0 + 32 * u, K - 1));
+              a[u] = __ldcg(&p->v[2]);
+              b[u] = __ldcg(&p->v[3]);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              if (k0 + 32 * u < K) { s0 += a[u]; s1 += b[u]; }
+          }
+        } else if (lane < K) {
+          const Stats *p = g.peer(slotA(), lane);
+          s0 = p->v[2];
+          s1 = p->v[3];
+        }
+        s0 = warp_sum(s0);
+        s1 = warp_sum(s1);
+        if (lane == 0) {
+          it.st[2] = s0; it.st[3] = s1;
+          it.cv = cv_from(it.st);
+        }
       }
     } else {
       idle();
     }
-    __syncthreads();
+    if constexpr (Group::kGrid) acc_clear();
+    acc_next();
     return true;
   }
 
@@ -600,10 +666,10 @@ struct Engine {
       }
     }
   }
+  // The next sum's set; read again only after further barriers of the CTA.
   __device__ __forceinline__ void acc_next() {
     __syncthreads();
-    if (writer()) ++seq;
-    publish();
+    if (Group::kGrid && threadIdx.x == 0) ++seq;
   }
 
   // Fixed-point scale of the lattice sums of the whole-GPU path: `bound` is at
@@ -633,22 +699,28 @@ struct Engine {
     const bool degenerate = Num && it.degenerate;
     {
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-      const int l = lane & ((1 << sz) - 1), rs = 5 - sz, d = 1 << szh;
-      const int per = (1 << sz) >> szh;   // spans per round: all of them, up to 32
-      const int ntask = (nact + (1 << rs) - 1) >> rs;
-      for (int sp0 = 0; sp0 < az.nsp; sp0 += per) {
-        const int k = l >> szh, sp = sp0 + k, h = l & (d - 1);
-        const bool in = sp < az.nsp;
-        const int lo = in ? at<int>(az.o_lo)[sp] : 0, hi = in ? at<int>(az.o_hi)[sp] : 0;
+      const int l = lane & ((1 << sz) - 1), rs = 5 - sz, d = 1 << (Group::kGrid ? szh : 0);
+      const int sub = lane >> sz, hh = Group::kGrid ? szh : 0;
+      const int per = (1 << sz) >> hh;   // spans per round: all of them, up to 32
+      const int n = nact, nsp = az.nsp, nc = ncz, ntask = (n + (1 << rs) - 1) >> rs;
+      const auto rm = row_map();
+      const int *Lo = at<int>(az.o_lo), *Hi = at<int>(az.o_hi);
+      const SpanSums<Num> sums = span_sums<Num>();
+      for (int sp0 = 0; sp0 < nsp; sp0 += per) {
+        const int k = l >> hh, sp = sp0 + k, h = l & (d - 1);
+        const bool in = sp < nsp;
+        const int lo = in ? Lo[sp] : 0, hi = in ? Hi[sp] : 0;
         for (int task = warp; task < ntask; task += nw) {
-          const int r = (task << rs) + (lane >> sz);
-          const bool on = in && r < nact;
+          const int r = (task << rs) + sub;
+          const bool on = in && r < n;
           float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           if (on && !degenerate) {
-            const Row o = row(r);
+            const Row o = rm(r);
             int a, b;
-            piece(o, lo, hi, h, szh, a, b);
-            span_sums<Num>(o.p, a, b, s);
+            piece(o, lo, hi, h, hh, a, b);
+            if constexpr (Group::kGrid) sums.template add<2>(o.p, a, b, s);
+            else if (nsp > 2) sums.template add<3>(o.p, a, b, s);
+            else sums.template add<4>(o.p, a, b, s);
           }
           for (int w = d >> 1; w; w >>= 1) {
             s.x += __shfl_xor_sync(kFull, s.x, w); s.y += __shfl_xor_sync(kFull, s.y, w);
@@ -659,7 +731,7 @@ struct Engine {
                       w1 = __shfl_up_sync(kFull, s.w, d), z2 = __shfl_up_sync(kFull, s.z, 2 * d),
                       w2 = __shfl_up_sync(kFull, s.w, 2 * d), w3 = __shfl_up_sync(kFull, s.w, 3 * d);
           if (on && h == 0) {
-            float *t1 = T1 + r * ncz + sp;
+            float *t1 = T1 + r * nc + sp;
             const bool p1 = k >= 1, p2 = k >= 2, p3 = k >= 3;
             // targets in the order of span mod 4; a round finds the last
             // three targets of the one before open
@@ -668,7 +740,7 @@ struct Engine {
               t1[i] = sp0 > 0 && k + i < 3 ? t1[i] + x : x;
             };
             put(0, s.x, p1 ? y1 : 0.0f, p2 ? z2 : 0.0f, p3 ? w3 : 0.0f);
-            if (k == per - 1 || sp == az.nsp - 1) {
+            if (k == per - 1 || sp == nsp - 1) {
               put(1, s.y, p1 ? z1 : 0.0f, p2 ? w2 : 0.0f, 0.0f);
               put(2, s.z, p1 ? w1 : 0.0f, 0.0f, 0.0f);
               put(3, s.w, 0.0f, 0.0f, 0.0f);
@@ -764,48 +836,67 @@ struct Engine {
   // The four targets' sums of voxels [a, b) of a row, in voxel order: weights
   // times the residual R = logU - E(logU) (Num), or the weights of the masked
   // voxels.  Voxels outside the mask add zeros.  The residuals of U voxels are
-  // formed together, without branches.
+  // formed together, without branches: 4 on the cluster path's long spans, 3 on
+  // its short ones (5 or 6 voxels: two steps, 6 slots instead of 8; 26.0k
+  // against 28.3k cycles at 8 spans of 44 voxels on 6 CTAs), 2 on the whole-GPU
+  // path (fewer registers: 1024 threads).
   template <bool Num>
-  __device__ __forceinline__ void span_sums(const float *p, int a, int b, float4 &s) const {
-    constexpr int U = Group::kGrid ? 2 : 4;   // measured best on each path
-    const Iter &it = iter();
-    const float bmin = it.bm.fmin, ih = it.bm.ih, il = it.bm.il, lim = it.bm.ff_limit;
-    const float4 *W = at<float4>(Num ? az.o_p : az.o_q);
-    for (int z = a; z < b; z += U) {
-      float v[U], x[U];
+  struct SpanSums {
+    float bmin, ih, il, lim;
+    const float4 *W;
+    const float2 *R2;
+    const BinMap *bm;
+    const double *E;
+    int bins;
+    template <int U>
+    __device__ __forceinline__ void add(const float *p, int a, int b, float4 &s) const {
+      for (int z = a; z < b; z += U) {
+        float v[U], x[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = z + u < b ? p[z + u] : kNaN;
-      unsigned top = 0;
+        for (int u = 0; u < U; ++u) v[u] = z + u < b ? p[z + u] : kNaN;
+        unsigned top = 0;
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if constexpr (Num) {
-          int k;
-          float f;
-          const bool in = coord_split(v[u], bmin, ih, il, lim, k, f);
-          x[u] = in ? residual_lin(k, f, R2()) : 0.0f;
-          if (!in && !isnan(v[u])) top |= 1u << u;
-        } else {
-          x[u] = isnan(v[u]) ? 0.0f : 1.0f;
+        for (int u = 0; u < U; ++u) {
+          if constexpr (Num) {
+            int k;
+            float f;
+            const bool in = coord_split(v[u], bmin, ih, il, lim, k, f);
+            x[u] = in ? residual_lin(k, f, R2) : 0.0f;
+            if (!in && !isnan(v[u])) top |= 1u << u;
+          } else {
+            x[u] = isnan(v[u]) ? 0.0f : 1.0f;
+          }
+        }
+        if (Num && top) {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (top >> u & 1u) x[u] = residual_top(bm, v[u], E, bins);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const float4 w = W[z + u];   // past the row: finite, times zero
+          s.x = __fmaf_rn(w.x, x[u], s.x); s.y = __fmaf_rn(w.y, x[u], s.y);
+          s.z = __fmaf_rn(w.z, x[u], s.z); s.w = __fmaf_rn(w.w, x[u], s.w);
         }
       }
-      if (Num && top) {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (top >> u & 1u) x[u] = residual_top(&it.bm, v[u], E(), pr.bins);
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float4 w = W[min(z + u, b - 1)];
-        s.x = __fmaf_rn(w.x, x[u], s.x); s.y = __fmaf_rn(w.y, x[u], s.y);
-        s.z = __fmaf_rn(w.z, x[u], s.z); s.w = __fmaf_rn(w.w, x[u], s.w);
-      }
     }
+  };
+  template <bool Num>
+  __device__ __forceinline__ SpanSums<Num> span_sums() const {
+    const Iter &it = iter();
+    return SpanSums<Num>{it.bm.fmin, it.bm.ih, it.bm.il, it.bm.ff_limit, at<float4>(Num ? az.o_p : az.o_q), R2(), &it.bm,
+                         E(), pr.bins};
   }
 
-  // T2[m][cy][cz] of `cnt` x-planes.  Cluster path: one thread per entry over
-  // its four spans' rows, Kahan in two chains (rows at even and at odd
-  // distance from the span's start); rows before and after the plane's listed
-  // ones add zeros, which a chain need take only once.  Whole-GPU path, whose
+  // T2[m][cy][cz] of `cnt` x-planes.  Cluster path: Kahan in two chains per
+  // entry (rows at even and at odd distance from the span's start); rows before
+  // and after the plane's listed ones add zeros, which a chain need take only
+  // once.  One thread per entry over its four spans where there are at least
+  // four and the entries are one round of the CTA; else one thread per (plane,
+  // cz) that walks the plane once for all its entries (per iteration, 16 CTAs,
+  // 64x64x48: 1 span 4.1k cycles against 6.4k, 8 spans 6.9k against 4.4k; 6
+  // CTAs, 64x64x44: 4.7k against 8.0k and 8.3k against 11.2k).  Same terms in
+  // the same order either way.  Whole-GPU path, whose
   // CTAs hold two or three planes: one lane per span, the four sums added in
   // FP64.
   template <bool Num>
@@ -813,31 +904,86 @@ struct Engine {
     float *T2p = T2();
     const int *yt = ytab();
     const float *PY = at<float>(Num ? ay.o_p : ay.o_q);
-    const int n = cnt * ncy * ncz, w = ay.nsp + 1;
+    const int nc = ncz, ny = ncy, nsp = ay.nsp, n = cnt * ny * nc, w = nsp + 1;
+    const auto rm = row_map();
+    const int *Lo = at<int>(ay.o_lo), *Hi = at<int>(ay.o_hi);
     if constexpr (!Group::kGrid) {
+      if (nsp < 4 || n > 512) {
+      // one thread per (plane, cz): spans from the last to the first, the four
+      // targets a span reaches open in registers
+      for (int u = threadIdx.x; u < cnt * nc; u += blockDim.x) {
+        const int m = u / nc, cz = u - m * nc;
+        float *out = T2p + m * ny * nc + cz;
+        KahanSum a[4], b[4];   // target sp + j: rows at even and at odd distance
+        for (int sp = nsp - 1; sp >= 0; --sp) {
+          const int lo = Lo[sp], hi = Hi[sp];
+          const int r0 = yt[m * w + sp], k = yt[m * w + sp + 1] - r0;
+          const int va = k > 0 ? rm.vy(r0) : hi, vb = va + k;
+          if (va > lo) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              a[j].add(0.0f);
+              if (va > lo + 1) b[j].add(0.0f);
+            }
+          }
+          const float *t1 = T1 + r0 * nc + cz;
+          const float4 *py = (const float4 *)PY + va;
+          int i = 0;
+          const auto take = [&](KahanSum (&s)[4]) {
+            const float4 p = py[i];
+            const float x = t1[i * nc];
+            s[0].add_prod(p.x, x); s[1].add_prod(p.y, x); s[2].add_prod(p.z, x); s[3].add_prod(p.w, x);
+            ++i;
+          };
+          if (k > 0 && ((va - lo) & 1)) take(b);
+          while (i + 1 < k) { take(a); take(b); }
+          if (i < k) take(a);
+          if (k > 0 && vb < hi) {
+            const bool odd = (vb - lo) & 1, both = vb + 1 < hi;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (!odd || both) a[j].add(0.0f);
+              if (odd || both) b[j].add(0.0f);
+            }
+          }
+          a[3].merge(b[3]);
+          out[(sp + 3) * nc] = a[3].value();
+#pragma unroll
+          for (int j = 3; j > 0; --j) { a[j] = a[j - 1]; b[j] = b[j - 1]; }
+          a[0] = KahanSum();
+          b[0] = KahanSum();
+        }
+#pragma unroll
+        for (int j = 1; j < 4; ++j) {   // targets 0, 1, 2
+          a[j].merge(b[j]);
+          out[(j - 1) * nc] = a[j].value();
+        }
+      }
+      return;
+      }
       for (int u = threadIdx.x; u < n; u += blockDim.x) {
-        const int q = u / ncz, cz = u - q * ncz;
-        const int m = q / ncy, cy = q - m * ncy;
+        const int q = u / nc, cz = u - q * nc;
+        const int m = q / ny, cy = q - m * ny;
         KahanSum acc, acc2;
         for (int j = 0; j < 4; ++j) {
           const int sp = cy - j;
-          if (sp < 0 || sp >= ay.nsp) continue;
-          const int lo = at<int>(ay.o_lo)[sp], hi = at<int>(ay.o_hi)[sp];
+          if (sp < 0 || sp >= nsp) continue;
+          const int lo = Lo[sp], hi = Hi[sp];
           const int r0 = yt[m * w + sp], r1 = yt[m * w + sp + 1];
-          const int va = r0 < r1 ? row_vy(r0) : hi, vb = va + (r1 - r0);
+          const int va = r0 < r1 ? rm.vy(r0) : hi, vb = va + (r1 - r0);
           if (va > lo) acc.add(0.0f);
           if (va > lo + 1) acc2.add(0.0f);
-          const float *t1 = T1 + r0 * ncz + cz, *py = PY + va * 4 + j;
+          const float *t1 = T1 + r0 * nc + cz, *py = PY + va * 4 + j;
           int k = r1 - r0;
           if (k > 0 && ((va - lo) & 1)) {
             acc2.add_prod(py[0], t1[0]);
-            t1 += ncz;
+            t1 += nc;
             py += 4;
             --k;
           }
-          for (; k > 1; k -= 2, t1 += 2 * ncz, py += 8) {
+          for (; k > 1; k -= 2, t1 += 2 * nc, py += 8) {
             acc.add_prod(py[0], t1[0]);
-            acc2.add_prod(py[4], t1[ncz]);
+            acc2.add_prod(py[4], t1[nc]);
           }
           if (k > 0) acc.add_prod(py[0], t1[0]);
           if (r0 < r1 && vb < hi) {
@@ -854,18 +1000,18 @@ struct Engine {
     const int nt = (n * 4 + 31) & ~31;   // whole warps: the lanes of an entry exchange their sums
     for (int t = threadIdx.x; t < nt; t += blockDim.x) {
       const int u = t >> 2, j = t & 3;
-      const int q = u / ncz, cz = u - q * ncz;
-      const int m = q / ncy, cy = q - m * ncy, sp = cy - j;
+      const int q = u / nc, cz = u - q * nc;
+      const int m = q / ny, cy = q - m * ny, sp = cy - j;
       double s = 0.0;
-      if (u < n && sp >= 0 && sp < ay.nsp) {
+      if (u < n && sp >= 0 && sp < nsp) {
         KahanSum acc, acc2;
         int r = yt[m * w + sp];
         const int end = yt[m * w + sp + 1];
         for (; r + 1 < end; r += 2) {
-          acc.add_prod(PY[row_vy(r) * 4 + j], T1[r * ncz + cz]);
-          acc2.add_prod(PY[row_vy(r + 1) * 4 + j], T1[(r + 1) * ncz + cz]);
+          acc.add_prod(PY[rm.vy(r) * 4 + j], T1[r * nc + cz]);
+          acc2.add_prod(PY[rm.vy(r + 1) * 4 + j], T1[(r + 1) * nc + cz]);
         }
-        if (r < end) acc.add_prod(PY[row_vy(r) * 4 + j], T1[r * ncz + cz]);
+        if (r < end) acc.add_prod(PY[rm.vy(r) * 4 + j], T1[r * nc + cz]);
         s = ((double)acc.s - (double)acc.c) + ((double)acc2.s - (double)acc2.c);
       }
       s += __shfl_xor_sync(kFull, s, 1);
@@ -873,11 +1019,6 @@ struct Engine {
       if (u < n && j == 0) T2p[u] = (float)s;
     }
   }
-  __device__ __forceinline__ int row_vy(int r) const {
-    if constexpr (Group::kGrid) return rowsp[r].w;
-    else return (int)(at<uint2>(pl.o_rows)[r].y & 0xffffu);
-  }
-
   // ---- pass A: the previous update's convergence sums from eval(Gd) (when
   // need_cv), applied to logU (when apply: logU -= eval(Gd)), and the masked
   // min/max of logU; clears the histogram copies
@@ -886,12 +1027,13 @@ struct Engine {
     double sy = 0.0, syy = 0.0;
     const float *Gp = Gd();
     const float4 *W4 = at<float4>(az.o_w);
+    const int nc = ncz;
     span_pass(
         [&](const Row &o, int r, int a, int b, int sp) {
           if (a >= b) return;
           constexpr int U = 2;
           if (need_cv) {
-            const float *gp = Gp + r * ncz + sp;
+            const float *gp = Gp + r * nc + sp;
             const float g[4] = {gp[0], gp[1], gp[2], gp[3]};
             for (int z = a; z < b; z += U) {
               float v[U], ed[U], y[U];
@@ -899,7 +1041,7 @@ struct Engine {
               for (int u = 0; u < U; ++u) v[u] = z + u < b ? o.p[z + u] : kNaN;
 #pragma unroll
               for (int u = 0; u < U; ++u) {
-                ed[u] = dot4(W4[min(z + u, b - 1)], g);
+                ed[u] = dot4(W4[z + u], g);   // past the row: finite, not used
                 y[u] = expm1_conv(-ed[u]);
               }
 #pragma unroll
@@ -927,7 +1069,7 @@ struct Engine {
     const bool ok = reduce_stats(vmin, vmax, sy, syy, need_cv, [&] {
       // the copies lie in the Gd region, which every thread has read by now
       unsigned *h = hist();
-      for (int i = (int)threadIdx.x - 32; i < kHistCopies * pr.bins; i += (int)blockDim.x - 32) h[i] = 0u;
+      for (int i = (int)threadIdx.x - 64; i < kHistCopies * pr.bins; i += (int)blockDim.x - 64) h[i] = 0u;
     });
     N4_MARK(PH_A_RED);
     return ok;
@@ -936,7 +1078,9 @@ struct Engine {
   // ---- pass B + sharpening: histogram of logU over the group, then E
   __device__ bool pass_b() {
     const int bins = pr.bins;
-    const Iter &it = iter();
+    Iter &it = iter();
+    // for the sharpening, beside the first voxels
+    if (threadIdx.x == blockDim.x - 1) it.gauss = gauss_of(it.bm.slope, pr.fwhm);
     {
       const float bmin = it.bm.fmin, ih = it.bm.ih, il = it.bm.il, lim = it.bm.ff_limit;
       const float scale = (float)it.scale;
@@ -944,8 +1088,10 @@ struct Engine {
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
       const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s;
       unsigned *hc = hist() + (warp % kHistCopies) * bins;
-      for (int r = (warp << rs) + sub; r < nact; r += nw << rs) {
-        const Row o = row(r);
+      const auto rm = row_map();
+      const int n = nact;
+      for (int r = (warp << rs) + sub; r < n; r += nw << rs) {
+        const Row o = rm(r);
         constexpr int U = 2;
         for (int z = o.z0 + l; z < o.z1; z += U << s) {
           float v[U], f[U];
@@ -1227,8 +1373,9 @@ struct Engine {
     if (threadIdx.x < kHistCopies) copies[threadIdx.x] = 0;
     __syncthreads();
     const int rs = 5 - row_lanes_log2(Z);
+    const auto rm = row_map();
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-      const Row o = row(r);
+      const Row o = rm(r);
       atomicAdd(&copies[(r >> rs) % kHistCopies], o.z1 - o.z0);
     }
     __syncthreads();
@@ -1356,10 +1503,10 @@ struct Engine {
       if (threadIdx.x == 0) { rep->status = N4_OK; rep->device_end_ns = global_ns(); }
     }
 #ifdef N4_PHASE_TIMERS
-    if (lead)
-      printf("N4PHASE K=%d nt=%d setup=%lld A=%lld Aloop=%lld Ared=%lld Bloop=%lld Bmerge=%lld Bred=%lld "
+    if (threadIdx.x == 0 && (rank == 0 || rank == K / 4 || rank == K / 2))
+      printf("N4PHASE K=%d nt=%d rank=%d rows=%d setup=%lld A=%lld Aloop=%lld Ared=%lld Bloop=%lld Bmerge=%lld Bred=%lld "
              "sharp=%lld T1=%lld T2=%lld P=%lld Fred=%lld update=%lld\n",
-             K, (int)blockDim.x, ph_acc[PH_SETUP], ph_acc[PH_A], ph_acc[PH_A_LOOP], ph_acc[PH_A_RED],
+             K, (int)blockDim.x, rank, nact, ph_acc[PH_SETUP], ph_acc[PH_A], ph_acc[PH_A_LOOP], ph_acc[PH_A_RED],
              ph_acc[PH_B_LOOP], ph_acc[PH_B_MERGE], ph_acc[PH_B_RED], ph_acc[PH_SHARP], ph_acc[PH_F_T1],
              ph_acc[PH_F_T2], ph_acc[PH_F_P], ph_acc[PH_F_RED], ph_acc[PH_UPDATE]);
 #endif
