@@ -216,6 +216,7 @@ struct Engine {
   int hshift;          // fixed-point scale of this volume's histogram
   int seq;             // whole-GPU path: group sums so far
   double nfg;          // masked voxels of the volume
+  float denmax;        // whole-GPU path: the level's largest fit denominator
   const float *src;    // the job's log volume (global memory), read by reset
   // level
   int ncx, ncy, ncz, nlat;
@@ -754,8 +755,12 @@ struct Engine {
     N4_MARK(PH_F_T1);
     double scale = 1.0;
     if constexpr (Group::kGrid) {
+      // den: weights below 1.  num: with w <= 2/3 and sum w^2 >= 0.46 per axis,
+      // w^3/sum w^2 <= 1.45 w^2, so an entry's terms sum to at most 3.1 times
+      // its den times the largest residual; E lies within 4 ranges of the data
+      // or is 0.
       const double range = it.st[1] - it.st[0];
-      scale = ldexp(1.0, sum_shift(Num ? nfg * (5.0 * range + fabs(it.st[0]) + fabs(it.st[1])) : nfg));
+      scale = ldexp(1.0, sum_shift(Num ? 4.0 * denmax * (5.0 * range + fabs(it.st[0]) + fabs(it.st[1])) : nfg));
     }
     const int slice = ncy * ncz;
     for (int m0 = 0; m0 < np || m0 == 0; m0 += tp) {
@@ -1445,7 +1450,19 @@ struct Engine {
       // logU of this level's lattice, then the constant denominator of the fit
       reset(L(), level == 0 && !Group::kGrid);
       float *dn = den();
-      if (!contract<false>([=](int c, float v) { dn[c] = v; })) goto timeout;
+      float dmax = 0.0f;
+      if (!contract<false>([=, &dmax](int c, float v) { dn[c] = v; dmax = fmaxf(dmax, v); })) goto timeout;
+      if constexpr (Group::kGrid) {
+        dmax = funkey(__reduce_max_sync(kFull, fkey(dmax)));
+        float *sc = (float *)red();
+        if ((threadIdx.x & 31) == 0) sc[threadIdx.x >> 5] = dmax;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          denmax = 0.0f;
+          for (int w = 0; w < (int)(blockDim.x >> 5); ++w) denmax = fmaxf(denmax, sc[w]);
+        }
+        __syncthreads();
+      }
       const int maxIt = pr.iters[level];
       int it = 0;
       float cv = 1e10f;
