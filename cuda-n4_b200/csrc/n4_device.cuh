@@ -231,12 +231,26 @@ __device__ __forceinline__ void dft4(double2 &v0, double2 &v1, double2 &v2, doub
   double2 t0 = cadd(v0, v2), t1 = csub(v0, v2), t2 = cadd(v1, v3), t3 = mul_mi(csub(v1, v3));
   v0 = cadd(t0, t2); v2 = csub(t0, t2); v1 = cadd(t1, t3); v3 = csub(t1, t3);
 }
-// tw[m] = exp(-2 pi i m / N), m in [0, N).
+// FFT buffers keep value i at sw(i): a radix-4 pass stores every fourth value,
+// which in order would lie in two of the eight 16-byte banks.
+__device__ __forceinline__ int sw(int i) { return i ^ ((i >> 3) & 7); }
+
+// Twiddles exp(-2 pi i m / N): m in [0, N) in order, or, for N = 512, the passes'
+// own sequences one after the other, so that a warp's loads are consecutive
+// (in the table of all m a pass's stride put eight of them into one bank: 410
+// cycles per pass): radix-4 passes of Ns = 4, 16, 64 at 0, 12 and 60 as
+// [r - 1][k], the radix-2 pass of Ns = 256 at 252.
 __device__ void fft_twiddles(double2 *tw, int N) {
-  for (int m = threadIdx.x; m < N; m += blockDim.x) {
+  for (int t = threadIdx.x; t < N; t += blockDim.x) {
+    int m = t;
+    if (N == 512) {
+      const int Ns = t < 12 ? 4 : (t < 60 ? 16 : (t < 252 ? 64 : 256)), u = t - (t < 12 ? 0 : (t < 60 ? 12 : (t < 252 ? 60 : 252)));
+      if (Ns == 256) m = u & 255;
+      else m = (u / Ns + 1) * (u % Ns) * (N / (Ns * 4));
+    }
     double s, c;
     sincospi(-2.0 * (double)m / (double)N, &s, &c);
-    tw[m] = make_double2(c, s);
+    tw[t] = make_double2(c, s);
   }
 }
 
@@ -245,25 +259,25 @@ template <> __device__ __forceinline__ void dft_r<2>(double2 *v) { dft2(v); }
 template <> __device__ __forceinline__ void dft_r<4>(double2 *v) { dft4(v[0], v[1], v[2], v[3]); }
 
 // One Stockham pass of radix R (Govindaraju et al., SC'08, "High performance
-// discrete Fourier transforms on graphics processors"): in(0..N) -> y.  The
-// input is a function, so that an elementwise step before an FFT can be part
-// of its first pass (Ns = 1, where every twiddle is 1).
-template <int R, class In>
-__device__ __forceinline__ void stockham_pass(const In &in, double2 *y, int N, int Ns, const double2 *tw) {
+// discrete Fourier transforms on graphics processors"): in(0..N) -> y, with
+// twiddle(r, k) for r in [1, R), k in [0, Ns).  The input is a function, so that
+// an elementwise step before an FFT can be part of its first pass (Ns = 1, where
+// every twiddle is 1).
+template <int R, class In, class Tw>
+__device__ __forceinline__ void stockham_pass(const In &in, double2 *y, int N, int Ns, const Tw &twiddle) {
   const int T = N / R;
-  const int tstep = N / (Ns * R);
   for (int j = threadIdx.x; j < T; j += blockDim.x) {
     const int k = j & (Ns - 1);
     double2 v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       v[r] = in(j + r * T);
-      if (r && Ns > 1) v[r] = cmul(v[r], tw[(r * k * tstep) & (N - 1)]);
+      if (r && Ns > 1) v[r] = cmul(v[r], twiddle(r, k));
     }
     dft_r<R>(v);
     const int base = (j - k) * R + k;
 #pragma unroll
-    for (int r = 0; r < R; ++r) y[base + r * Ns] = v[r];
+    for (int r = 0; r < R; ++r) y[sw(base + r * Ns)] = v[r];
   }
   __syncthreads();
 }
@@ -271,28 +285,31 @@ __device__ __forceinline__ void stockham_pass(const In &in, double2 *y, int N, i
 // Forward FFT (length N = 2^m, 4 <= N <= 4096) of in(0..N): radix 4, the last
 // pass radix 2 where N is no power of 4; the first pass goes to a, the others
 // ping-pong a and b, each ending with a CTA barrier.  Returns the buffer that
-// holds the result.  NC: N where it is known at compile time (512, up to 256
-// bins: the passes' strides and twiddle steps become constants), else 0.
-// (Three radix-8 passes of 64 threads took 11.0k instead of 12.0k cycles for
-// the map, but round differently, and N4 on a small volume follows every bit.)
+// holds the result (value i at sw(i)).  NC: N where it is known at compile time
+// (512, up to 256 bins: the passes' strides become constants), else 0.
+// (Three radix-8 passes of 64 threads round differently, and N4 on a small
+// volume follows every bit; the last two passes in one of 64 threads, the
+// values in registers between them, took as long as the two.)
 template <int NC, class In>
 __device__ __forceinline__ double2 *fft_from(const In &in, double2 *a, double2 *b, int N, const double2 *tw) {
-  auto from = [](const double2 *x) { return [x](int i) { return x[i]; }; };
+  auto from = [](const double2 *x) { return [x](int i) { return x[sw(i)]; }; };
   if constexpr (NC == 512) {
-    stockham_pass<4>(in, a, 512, 1, tw);
-    stockham_pass<4>(from(a), b, 512, 4, tw);
-    stockham_pass<4>(from(b), a, 512, 16, tw);
-    stockham_pass<4>(from(a), b, 512, 64, tw);
-    stockham_pass<2>(from(b), a, 512, 256, tw);
+    auto packed = [tw](int at, int Ns) { return [=](int r, int k) { return tw[at + (r - 1) * Ns + k]; }; };
+    stockham_pass<4>(in, a, 512, 1, packed(0, 1));
+    stockham_pass<4>(from(a), b, 512, 4, packed(0, 4));
+    stockham_pass<4>(from(b), a, 512, 16, packed(12, 16));
+    stockham_pass<4>(from(a), b, 512, 64, packed(60, 64));
+    stockham_pass<2>(from(b), a, 512, 256, packed(252, 256));
     return a;
   } else {
+    auto plain = [=](int step) { return [=](int r, int k) { return tw[(r * k * step) & (N - 1)]; }; };
     const int R0 = N % 4 == 0 ? 4 : 2;
-    if (R0 == 4) stockham_pass<4>(in, a, N, 1, tw);
-    else stockham_pass<2>(in, a, N, 1, tw);
+    if (R0 == 4) stockham_pass<4>(in, a, N, 1, plain(0));
+    else stockham_pass<2>(in, a, N, 1, plain(0));
     for (int Ns = R0, rem = N / R0; rem > 1;) {
       const int R = rem % 4 == 0 ? 4 : 2;
-      if (R == 4) stockham_pass<4>(from(a), b, N, Ns, tw);
-      else stockham_pass<2>(from(a), b, N, Ns, tw);
+      if (R == 4) stockham_pass<4>(from(a), b, N, Ns, plain(N / (Ns * 4)));
+      else stockham_pass<2>(from(a), b, N, Ns, plain(N / (Ns * 2)));
       double2 *t = a; a = b; b = t;
       Ns *= R;
       rem /= R;
@@ -348,21 +365,21 @@ __device__ __forceinline__ void sharpen_map_n(const HistF &hv, int bins, int N, 
   // Ff real; conj(Uf), so that the forward FFT inverts
   for (int k = threadIdx.x; k <= N / 2; k += blockDim.x) {
     const int kn = (N - k) & (N - 1);
-    const double2 zk = Z[k], zn = Z[kn];
+    const double2 zk = Z[sw(k)], zn = Z[sw(kn)];
     const double2 Vf = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
     const double Ff = 0.5 * (zk.y + zn.y);
     const double g = Ff / (Ff * Ff + wiener);
     sb.Ff[k] = Ff;
-    W[kn] = make_double2(Vf.x * g, Vf.y * g);
-    W[k] = make_double2(Vf.x * g, -Vf.y * g);
+    W[sw(kn)] = make_double2(Vf.x * g, Vf.y * g);
+    W[sw(k)] = make_double2(Vf.x * g, -Vf.y * g);
   }
   __syncthreads();
-  double2 *Y = fft_from<NC>([&](int k) { return W[k]; }, Z, W, N, sb.tw);
+  double2 *Y = fft_from<NC>([&](int k) { return W[sw(k)]; }, Z, W, N, sb.tw);
   double2 *Y2 = (Y == W) ? Z : W;
   // U = max(Re(ifft(Uf)), 0); pack the numerator c_i U_i (real) and U (imaginary)
   double2 *P = fft_from<NC>(
       [&](int i) {
-        const double U = fmax(Y[i].x * invN, 0.0);
+        const double U = fmax(Y[sw(i)].x * invN, 0.0);
         const double c = binMin + (double)(i - off) * slope;
         return make_double2(c * U, U);
       },
@@ -371,13 +388,13 @@ __device__ __forceinline__ void sharpen_map_n(const HistF &hv, int bins, int N, 
   // Gaussian smoothing of both: multiply by the (real) Ff, inverse transform
   double2 *S = fft_from<NC>(
       [&](int k) {
-        const double2 v = P[k];
+        const double2 v = P[sw(k)];
         const double f = sb.Ff[k <= N / 2 ? k : N - k];
         return make_double2(v.x * f, -v.y * f);
       },
       P2, P, N, sb.tw);
   for (int b = threadIdx.x; b < bins; b += blockDim.x) {
-    const double2 v = S[off + b];
+    const double2 v = S[sw(off + b)];
     const double nu = v.x * invN, de = -v.y * invN;
     E[b] = (de != 0.0) ? nu / de : 0.0;
   }
