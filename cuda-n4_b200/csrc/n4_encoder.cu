@@ -272,23 +272,89 @@ struct ConvDgrad {
   }
 };
 
-// 64 rows of one parity class by NT columns; 128 threads, 4 warps of 16xNT
-// (NT = 16) or 32x(NT/2).  Only the columns k whose tap the class meets are
-// loaded: threads 0-63 a row of A each, threads 64-127 the rows of B; A's other
-// columns stay zero, and K steps of 16 without any are not multiplied.  The
-// next step's values are in registers while this one is multiplied.  The sums
-// take the terms over k in the order of a dense GEMM.  (As a dense implicit
-// GEMM over all 27 taps, rows in memory order, the three layers of a batch of
-// 64 took 121, 124 and 259 us, bound by the gather's instructions.)
+// 64 rows of one parity class by NT columns; 256 threads, 8 warps of 16 x NT/2.
+// Sixteen channels are staged at a time: 432 dense columns k = 27 c + t, which
+// are 27 whole K steps of 16.  A class meets the same columns of every group,
+// so the others are cleared once per block, a group's loads are only those of
+// the class's T taps (all in flight while the group before is multiplied), the
+// fragments come by ldmatrix and nothing is synchronised between the 27 steps;
+// steps without a tap are not multiplied.  Terms, their order and their
+// grouping by 16 are those of the dense GEMM over all 27 taps.  The row stride
+// of 440 puts the eight rows of a matrix on different banks, and a warp stages
+// 8 rows of 4 channels for the same reason.  Bound by the gathers' lines in L1.
+// The three layers of a batch of 64 take 29, 49 and 88 us; 98, 105 and 142 us
+// when each step of 32 dense columns loaded its own few columns between two
+// barriers, 39, 56 and 136 us with only the T columns staged and the fragments
+// picked from them through a table.
+constexpr int kDgCols = 432, kDgLd = kDgCols + 8;
+constexpr size_t dgrad_smem(int NT) { return (size_t)(BM + NT) * kDgLd * sizeof(bf16); }
+
+template <int T, int NT>
+__device__ __forceinline__ void dgrad_rows(const ConvDgrad &p, bf16 *As, bf16 *Bs, const int *off, const int *tap,
+                                           const bf16 *arow, unsigned amask, int n0, unsigned long long period,
+                                           float (&acc)[NT / 16][4]) {
+  constexpr int NJ = NT / 16, PARTS = 256 / NT, NA = 4 * T, NB = 16 * T / PARTS;
+  const Shape &s = p.s;
+  const int op = s.out_pos();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane >> 3;
+  const int bn = (lane & 7) + 8 * (warp % (NT / 8)), bpart = sub + 4 * (warp / (NT / 8));
+  const bool b_ok = n0 + bn < s.Ci;
+  const bf16 *bw = p.w + (size_t)(b_ok ? n0 + bn : 0) * 27;
+  bf16 *const ato = As + ((lane & 7) + 8 * warp) * kDgLd + 27 * sub;
+  bf16 *const bto = Bs + bn * kDgLd + 27 * bpart;
+  const bf16 zero = __float2bfloat16(0.0f);
+  bf16 va[NA], vb[NB];
+  const auto load = [&](int c0) {
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const int c = c0 + i / T * 4 + sub, t = i % T;
+      va[i] = zero;
+      if (c < s.Co && (amask >> tap[t] & 1u)) va[i] = arow[(ptrdiff_t)c * op + off[t]];
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int c = c0 + i / T * PARTS + bpart, t = i % T;
+      vb[i] = zero;
+      if (b_ok && c < s.Co) vb[i] = bw[(size_t)c * s.Ci * 27 + tap[t]];
+    }
+  };
+  const unsigned a_at = (unsigned)__cvta_generic_to_shared(As + ((warp >> 1) * 16 + (lane & 15)) * kDgLd + (lane >> 4) * 8);
+  const unsigned b_at = (unsigned)__cvta_generic_to_shared(
+      Bs + ((warp & 1) * (NT / 2) + (NJ == 2 ? (lane >> 4) * 8 : 0) + (lane & 7)) * kDgLd + (lane >> 3 & 1) * 8);
+  load(0);
+  for (int c0 = 0; c0 < s.Co; c0 += 16) {
+    if (c0 > 0) __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NA; ++i) ato[i / T * 4 * 27 + tap[i % T]] = va[i];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) bto[i / T * PARTS * 27 + tap[i % T]] = vb[i];
+    __syncthreads();
+    if (c0 + 16 < s.Co) load(c0 + 16);
+#pragma unroll
+    for (int k = 0; k < 27; ++k) {
+      if (!((unsigned)(period >> (16 * k % 27)) & 0xffffu)) continue;
+      unsigned af[4], bfr[2 * NJ];
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(af[0]), "=r"(af[1]), "=r"(af[2]), "=r"(af[3]) : "r"(a_at + 32 * k) : "memory");
+      if constexpr (NJ == 2)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(bfr[0]), "=r"(bfr[1]), "=r"(bfr[2]), "=r"(bfr[3]) : "r"(b_at + 32 * k) : "memory");
+      else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+                     : "=r"(bfr[0]), "=r"(bfr[1]) : "r"(b_at + 32 * k) : "memory");
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) mma_bf16(acc[j], af, bfr + 2 * j);
+    }
+  }
+}
+
 template <int NT>
-__global__ void __launch_bounds__(128) k_dgrad(const ConvDgrad p) {
-  __shared__ __align__(16) bf16 As[BM][BK + PAD];
-  __shared__ __align__(16) bf16 Bs[NT][BK + PAD];
-  __shared__ int tap[27];
-  constexpr int WX = NT == 16 ? 1 : 2;
-  constexpr int WM = BM / (4 / WX), WN = NT / WX;
-  constexpr int MI = WM / 16, NJ = WN / 8;
-  constexpr int kMost = 11;   // most columns of 32 that a class of 8 taps meets
+__global__ void __launch_bounds__(256) k_dgrad(const ConvDgrad p) {
+  constexpr int NJ = NT / 16;
+  extern __shared__ __align__(16) bf16 stage[];
+  bf16 *As = stage, *Bs = stage + BM * kDgLd;
+  __shared__ int tap[8], off[8];            // the class's taps, ascending; their offsets in dy
   const Shape &s = p.s;
   int cls = 0, tile = blockIdx.x;
   for (; cls < 7; ++cls) {
@@ -299,131 +365,58 @@ __global__ void __launch_bounds__(128) k_dgrad(const ConvDgrad p) {
   const int pd = cls >> 2, ph = cls >> 1 & 1, pw = cls & 1;
   const int nd = ConvDgrad::axis_count(s.D, pd), nh = ConvDgrad::axis_count(s.H, ph), nw = ConvDgrad::axis_count(s.W, pw);
   const int rows = p.rows(cls), row0 = tile * BM, n0 = blockIdx.y * NT;
-  const int K = s.Co * 27, op = s.out_pos(), ip = s.in_pos();
-  // the class's taps, as a bit per (kd, kh, kw), and three periods of them
-  const auto taps = [&](unsigned md, unsigned mh, unsigned mw) {
-    unsigned m = 0;
-    for (int t = 0; t < 27; ++t)
-      if ((md >> t / 9 & 1u) && (mh >> t / 3 % 3 & 1u) && (mw >> t % 3 & 1u)) m |= 1u << t;
-    return m;
+  const int op = s.out_pos(), ip = s.in_pos();
+  // a bit per tap (kd, kh, kw) from the axes' bits, and two periods of the class's
+  const auto taps = [](unsigned md, unsigned mh, unsigned mw) {
+    return mw * ((mh & 1u) | (mh & 2u) << 2 | (mh & 4u) << 4) * ((md & 1u) | (md & 2u) << 8 | (md & 4u) << 16);
   };
   const unsigned cmask = taps(pd ? 5u : 2u, ph ? 5u : 2u, pw ? 5u : 2u);
-  const unsigned long long period = cmask | (unsigned long long)cmask << 27 | (unsigned long long)cmask << 54;
-  if (threadIdx.x < 27) {
-    const int t = threadIdx.x;
-    tap[t] = -((((t / 9) >> 1) * s.Ho + ((t / 3 % 3) >> 1)) * s.Wo + ((t % 3) >> 1));
+  const unsigned long long period = cmask | (unsigned long long)cmask << 27;
+  if (threadIdx.x < 27 && (cmask >> threadIdx.x & 1u)) {
+    const int t = threadIdx.x, i = __popc(cmask & ((1u << t) - 1u));
+    tap[i] = t;
+    off[i] = -((((t / 9) >> 1) * s.Ho + ((t / 3 % 3) >> 1)) * s.Wo + ((t % 3) >> 1));
   }
-  for (int i = threadIdx.x; i < BM * (BK + PAD) / 2; i += 128) ((unsigned *)As)[i] = 0u;
-  for (int i = threadIdx.x; i < NT * (BK + PAD) / 2; i += 128) ((unsigned *)Bs)[i] = 0u;
-  const bool loads_a = threadIdx.x < 64;
-  const int lr = threadIdx.x & 63;
-  // A: the row's base in dy and the taps that meet an output of it.  B: row
-  // lr % NT, every (64 / NT)-th column.
-  const bf16 *base = nullptr;
-  unsigned rmask = 0;
-  constexpr int BQ = 64 / NT;
-  const int bq = lr / NT, bn = n0 + lr % NT;
-  if (loads_a) {
-    const int q = row0 + lr;
+  for (int i = threadIdx.x; i < (BM + NT) * kDgLd / 8; i += 256) ((uint4 *)stage)[i] = make_uint4(0u, 0u, 0u, 0u);
+  // the staged row's base in dy and the taps that meet an output of it
+  const bf16 *arow = p.dy;
+  unsigned amask = 0;
+  {
+    const int q = row0 + (threadIdx.x & 7) + 8 * (threadIdx.x >> 5);
     if (q < rows) {
       const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
       const int fd = jd + pd, fh = jh + ph, fw = jw + pw;
       const auto axis = [](int par, int f, int n) { return par ? (f < n ? 5u : 4u) : 2u; };
-      rmask = taps(axis(pd, fd, s.Do), axis(ph, fh, s.Ho), axis(pw, fw, s.Wo));
-      base = p.dy + (ptrdiff_t)b * s.Co * op + (fd * s.Ho + fh) * s.Wo + fw;
+      amask = taps(axis(pd, fd, s.Do), axis(ph, fh, s.Ho), axis(pw, fw, s.Wo));
+      arow = p.dy + (ptrdiff_t)b * s.Co * op + (fd * s.Ho + fh) * s.Wo + fw;
     }
-  } else if (bn < s.Ci) {
-    rmask = cmask;
-    base = p.w + (size_t)bn * 27;
   }
-  const size_t stride = loads_a ? (size_t)op : (size_t)s.Ci * 27;
   __syncthreads();
-  const auto window = [&](int k0) {   // the columns of [k0, k0 + 32) the class meets
-    const unsigned w = (unsigned)(period >> (k0 % 27));
-    return K - k0 >= 32 ? w : w & ((1u << (K - k0)) - 1u);
-  };
-  bf16 v[kMost];
-  const auto load = [&](int k0) {
-    const int t0 = k0 % 27;
-    const bf16 *c = base + (size_t)(k0 / 27) * stride;
-    unsigned w = window(k0);
-#pragma unroll
-    for (int i = 0; i < kMost; ++i) {
-      if (!w) break;
-      int t = t0 + __ffs(w) - 1;
-      w &= w - 1;
-      const int over = (t >= 27) + (t >= 54);
-      t -= 27 * over;
-      v[i] = __float2bfloat16(0.0f);
-      if ((rmask >> t & 1u) && (loads_a || i % BQ == bq)) v[i] = c[over * stride + (loads_a ? tap[t] : t)];
-    }
-  };
+  float acc[NJ][4] = {};
+  switch (__popc(cmask)) {
+    case 8: dgrad_rows<8, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
+    case 4: dgrad_rows<4, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
+    case 2: dgrad_rows<2, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
+    default: dgrad_rows<1, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
-  const int wm = (warp / WX) * WM, wn = (warp % WX) * WN;
-  float acc[MI][NJ][4] = {};
-  unsigned last = 0;   // the columns of A's tile that are not zero
-  load(0);
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    const unsigned now = window(k0);
-    if (loads_a) {
-      for (unsigned w = last & ~now; w; w &= w - 1) As[lr][__ffs(w) - 1] = __float2bfloat16(0.0f);
-    }
-    unsigned w = now;
 #pragma unroll
-    for (int i = 0; i < kMost; ++i) {
-      if (!w) break;
-      const int j = __ffs(w) - 1;
-      w &= w - 1;
-      if (loads_a) As[lr][j] = v[i];
-      else if (i % BQ == bq) Bs[lr % NT][j] = v[i];
-    }
-    last = now;
-    __syncthreads();
-    if (k0 + BK < K) load(k0 + BK);
+  for (int h = 0; h < 2; ++h) {
+    const int q = row0 + (warp >> 1) * 16 + g + 8 * h;
+    if (q >= rows) continue;
+    const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
+    const size_t at = (size_t)b * s.Ci * ip + ((2 * jd + pd) * s.H + 2 * jh + ph) * s.W + 2 * jw + pw;
 #pragma unroll
-    for (int kk = 0; kk < BK; kk += 16) {
-      if (!(now >> kk & 0xffffu)) continue;
-      unsigned af[MI][4], bfr[NJ][2];
+    for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int i = 0; i < MI; ++i) {
-        const int r = wm + 16 * i + g;
-        af[i][0] = *(const unsigned *)&As[r][kk + 2 * tig];
-        af[i][1] = *(const unsigned *)&As[r + 8][kk + 2 * tig];
-        af[i][2] = *(const unsigned *)&As[r][kk + 2 * tig + 8];
-        af[i][3] = *(const unsigned *)&As[r + 8][kk + 2 * tig + 8];
+      for (int e = 0; e < 2; ++e) {
+        const int n = n0 + (warp & 1) * (NT / 2) + 8 * j + 2 * tig + e;
+        if (n >= s.Ci) continue;
+        const size_t o = at + (size_t)n * ip;
+        p.dx[o] = relu_grad(acc[j][2 * h + e], p.x[o]);
       }
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int c = wn + 8 * j + g;
-        bfr[j][0] = *(const unsigned *)&Bs[c][kk + 2 * tig];
-        bfr[j][1] = *(const unsigned *)&Bs[c][kk + 2 * tig + 8];
-      }
-#pragma unroll
-      for (int i = 0; i < MI; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
-    }
-    __syncthreads();
   }
-#pragma unroll
-  for (int i = 0; i < MI; ++i)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int q = row0 + wm + 16 * i + g + 8 * h;
-      if (q >= rows) continue;
-      const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
-      const size_t at = (size_t)b * s.Ci * ip + ((2 * jd + pd) * s.H + 2 * jh + ph) * s.W + 2 * jw + pw;
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int n = n0 + wn + 8 * j + 2 * tig + e;
-          if (n >= s.Ci) continue;
-          const size_t o = at + (size_t)n * ip;
-          p.dx[o] = relu_grad(acc[i][j][2 * h + e], p.x[o]);
-        }
-    }
 }
 
 // dw partials, and the bias gradient as one more column of ones: M = Co,
@@ -652,12 +645,17 @@ cudaError_t run_gemm(const P &p, int splits, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <int NT>
+cudaError_t run_dgrad_nt(const ConvDgrad &p, int tiles, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_dgrad<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dgrad_smem(NT));
+  if (e != cudaSuccess) return e;
+  k_dgrad<NT><<<dim3(tiles, (p.s.Ci + NT - 1) / NT), 256, dgrad_smem(NT), st>>>(p);
+  return cudaGetLastError();
+}
 inline cudaError_t run_dgrad(const ConvDgrad &p, cudaStream_t st) {
   int tiles = 0;
   for (int c = 0; c < 8; ++c) tiles += (p.rows(c) + BM - 1) / BM;
-  if (p.s.Ci <= 16) k_dgrad<16><<<dim3(tiles, (p.s.Ci + 15) / 16), 128, 0, st>>>(p);
-  else k_dgrad<32><<<dim3(tiles, (p.s.Ci + 31) / 32), 128, 0, st>>>(p);
-  return cudaGetLastError();
+  return p.s.Ci <= 16 ? run_dgrad_nt<16>(p, tiles, st) : run_dgrad_nt<32>(p, tiles, st);
 }
 
 // Splits of a forward GEMM: enough blocks for about two per SM, at least two
