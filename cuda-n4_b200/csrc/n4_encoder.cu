@@ -264,6 +264,7 @@ struct ConvDgrad {
   Shape s;
   const bf16 *dy, *x, *w;
   bf16 *dx;
+  int first[8];   // first block of a class
   // positions of one axis with parity p, and rows of class c (parities of d,
   // h, w in bits 2, 1, 0) over the batch
   static __host__ __device__ int axis_count(int n, int p) { return (n + 1 - p) >> 1; }
@@ -281,56 +282,62 @@ struct ConvDgrad {
 // steps without a tap are not multiplied.  Terms, their order and their
 // grouping by 16 are those of the dense GEMM over all 27 taps.  The row stride
 // of 440 puts the eight rows of a matrix on different banks, and a warp stages
-// 8 rows of 4 channels for the same reason.  Bound by the gathers' lines in L1.
-// The three layers of a batch of 64 take 29, 49 and 88 us; 98, 105 and 142 us
-// when each step of 32 dense columns loaded its own few columns between two
-// barriers, 39, 56 and 136 us with only the T columns staged and the fragments
-// picked from them through a table.
+// 8 rows of 4 channels for the same reason.  Bound by the instructions of the
+// gathers (one per value) and, where a layer has few rows, by the latency of
+// its groups.  The three layers of a batch of 64 take 19, 37 and 70 us; 29, 49
+// and 88 us when every thread divided its rows' indices and read the taps from
+// shared memory at each load, 98, 105 and 142 us when each step of 32 dense
+// columns loaded its own few columns between two barriers.
 constexpr int kDgCols = 432, kDgLd = kDgCols + 8;
 constexpr size_t dgrad_smem(int NT) { return (size_t)(BM + NT) * kDgLd * sizeof(bf16); }
 
 template <int T, int NT>
-__device__ __forceinline__ void dgrad_rows(const ConvDgrad &p, bf16 *As, bf16 *Bs, const int *off, const int *tap,
-                                           const bf16 *arow, unsigned amask, int n0, unsigned long long period,
-                                           float (&acc)[NT / 16][4]) {
+__device__ __forceinline__ void dgrad_rows(const ConvDgrad &p, bf16 *As, bf16 *Bs, const int *tap, int at, unsigned amask,
+                                           int n0, unsigned long long period, float (&acc)[NT / 16][4]) {
   constexpr int NJ = NT / 16, PARTS = 256 / NT, NA = 4 * T, NB = 16 * T / PARTS;
   const Shape &s = p.s;
-  const int op = s.out_pos();
+  const int op = s.out_pos(), cw = s.Ci * 27;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane >> 3;
   const int bn = (lane & 7) + 8 * (warp % (NT / 8)), bpart = sub + 4 * (warp / (NT / 8));
-  const bool b_ok = n0 + bn < s.Ci;
-  const bf16 *bw = p.w + (size_t)(b_ok ? n0 + bn : 0) * 27;
   bf16 *const ato = As + ((lane & 7) + 8 * warp) * kDgLd + 27 * sub;
   bf16 *const bto = Bs + bn * kDgLd + 27 * bpart;
+  // the taps, their offsets in dy, and a bit per tap that meets an output of the row
+  int tp[T], of[T];
+  unsigned ok = 0;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    tp[t] = tap[t];
+    of[t] = -((((tp[t] / 9) >> 1) * s.Ho + ((tp[t] / 3 % 3) >> 1)) * s.Wo + ((tp[t] % 3) >> 1));
+    ok |= (amask >> tp[t] & 1u) << t;
+  }
   const bf16 zero = __float2bfloat16(0.0f);
   bf16 va[NA], vb[NB];
-  const auto load = [&](int c0) {
+  at += sub * op;
+  int wat = min(n0 + bn, s.Ci - 1) * 27 + bpart * cw;   // a column past Ci repeats the last and is not stored
+  const auto load = [&]() {   // the next 16 channels
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
-      const int c = c0 + i / T * 4 + sub, t = i % T;
       va[i] = zero;
-      if (c < s.Co && (amask >> tap[t] & 1u)) va[i] = arow[(ptrdiff_t)c * op + off[t]];
+      if (ok & 1u << i % T) va[i] = p.dy[at + i / T * 4 * op + of[i % T]];
     }
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      const int c = c0 + i / T * PARTS + bpart, t = i % T;
-      vb[i] = zero;
-      if (b_ok && c < s.Co) vb[i] = bw[(size_t)c * s.Ci * 27 + tap[t]];
-    }
+    for (int i = 0; i < NB; ++i) vb[i] = p.w[wat + i / T * PARTS * cw + tp[i % T]];
+    at += 16 * op;
+    wat += 16 * cw;
   };
   const unsigned a_at = (unsigned)__cvta_generic_to_shared(As + ((warp >> 1) * 16 + (lane & 15)) * kDgLd + (lane >> 4) * 8);
   const unsigned b_at = (unsigned)__cvta_generic_to_shared(
       Bs + ((warp & 1) * (NT / 2) + (NJ == 2 ? (lane >> 4) * 8 : 0) + (lane & 7)) * kDgLd + (lane >> 3 & 1) * 8);
-  load(0);
+  load();
   for (int c0 = 0; c0 < s.Co; c0 += 16) {
     if (c0 > 0) __syncthreads();
 #pragma unroll
-    for (int i = 0; i < NA; ++i) ato[i / T * 4 * 27 + tap[i % T]] = va[i];
+    for (int i = 0; i < NA; ++i) ato[i / T * 4 * 27 + tp[i % T]] = va[i];
 #pragma unroll
-    for (int i = 0; i < NB; ++i) bto[i / T * PARTS * 27 + tap[i % T]] = vb[i];
+    for (int i = 0; i < NB; ++i) bto[i / T * PARTS * 27 + tp[i % T]] = vb[i];
     __syncthreads();
-    if (c0 + 16 < s.Co) load(c0 + 16);
+    if (c0 + 16 < s.Co) load();
 #pragma unroll
     for (int k = 0; k < 27; ++k) {
       if (!((unsigned)(period >> (16 * k % 27)) & 0xffffu)) continue;
@@ -354,66 +361,60 @@ __global__ void __launch_bounds__(256) k_dgrad(const ConvDgrad p) {
   constexpr int NJ = NT / 16;
   extern __shared__ __align__(16) bf16 stage[];
   bf16 *As = stage, *Bs = stage + BM * kDgLd;
-  __shared__ int tap[8], off[8];            // the class's taps, ascending; their offsets in dy
+  __shared__ int tap[8];                    // the class's taps, ascending
+  __shared__ int row_dy[BM], row_dx[BM];    // a row's element of channel 0 in dy and dx (-1: no row)
+  __shared__ unsigned row_taps[BM];         // the taps that meet an output of it
   const Shape &s = p.s;
-  int cls = 0, tile = blockIdx.x;
-  for (; cls < 7; ++cls) {
-    const int n = (p.rows(cls) + BM - 1) / BM;
-    if (tile < n) break;
-    tile -= n;
-  }
+  int cls = 0, first = 0;
+#pragma unroll
+  for (int c = 1; c < 8; ++c)
+    if ((int)blockIdx.x >= p.first[c]) cls = c, first = p.first[c];
+  const int row0 = ((int)blockIdx.x - first) * BM, n0 = blockIdx.y * NT;
   const int pd = cls >> 2, ph = cls >> 1 & 1, pw = cls & 1;
-  const int nd = ConvDgrad::axis_count(s.D, pd), nh = ConvDgrad::axis_count(s.H, ph), nw = ConvDgrad::axis_count(s.W, pw);
-  const int rows = p.rows(cls), row0 = tile * BM, n0 = blockIdx.y * NT;
-  const int op = s.out_pos(), ip = s.in_pos();
+  const int ip = s.in_pos();
   // a bit per tap (kd, kh, kw) from the axes' bits, and two periods of the class's
   const auto taps = [](unsigned md, unsigned mh, unsigned mw) {
     return mw * ((mh & 1u) | (mh & 2u) << 2 | (mh & 4u) << 4) * ((md & 1u) | (md & 2u) << 8 | (md & 4u) << 16);
   };
   const unsigned cmask = taps(pd ? 5u : 2u, ph ? 5u : 2u, pw ? 5u : 2u);
   const unsigned long long period = cmask | (unsigned long long)cmask << 27;
-  if (threadIdx.x < 27 && (cmask >> threadIdx.x & 1u)) {
-    const int t = threadIdx.x, i = __popc(cmask & ((1u << t) - 1u));
-    tap[i] = t;
-    off[i] = -((((t / 9) >> 1) * s.Ho + ((t / 3 % 3) >> 1)) * s.Wo + ((t % 3) >> 1));
+  if (threadIdx.x < 27 && (cmask >> threadIdx.x & 1u)) tap[__popc(cmask & ((1u << threadIdx.x) - 1u))] = threadIdx.x;
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + BM) {
+    const int r = threadIdx.x - 64, q = row0 + r;
+    const int nd = ConvDgrad::axis_count(s.D, pd), nh = ConvDgrad::axis_count(s.H, ph), nw = ConvDgrad::axis_count(s.W, pw);
+    const int qh = q / nw, qd = qh / nh, b = qd / nd;
+    const int jw = q - qh * nw, jh = qh - qd * nh, jd = qd - b * nd;
+    const int fd = jd + pd, fh = jh + ph, fw = jw + pw;
+    const auto axis = [](int par, int f, int n) { return par ? (f < n ? 5u : 4u) : 2u; };
+    const bool in = b < s.B;
+    row_taps[r] = in ? taps(axis(pd, fd, s.Do), axis(ph, fh, s.Ho), axis(pw, fw, s.Wo)) : 0u;
+    row_dy[r] = b * s.Co * s.out_pos() + (fd * s.Ho + fh) * s.Wo + fw;
+    row_dx[r] = in ? b * s.Ci * ip + ((2 * jd + pd) * s.H + 2 * jh + ph) * s.W + 2 * jw + pw : -1;
   }
   for (int i = threadIdx.x; i < (BM + NT) * kDgLd / 8; i += 256) ((uint4 *)stage)[i] = make_uint4(0u, 0u, 0u, 0u);
-  // the staged row's base in dy and the taps that meet an output of it
-  const bf16 *arow = p.dy;
-  unsigned amask = 0;
-  {
-    const int q = row0 + (threadIdx.x & 7) + 8 * (threadIdx.x >> 5);
-    if (q < rows) {
-      const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
-      const int fd = jd + pd, fh = jh + ph, fw = jw + pw;
-      const auto axis = [](int par, int f, int n) { return par ? (f < n ? 5u : 4u) : 2u; };
-      amask = taps(axis(pd, fd, s.Do), axis(ph, fh, s.Ho), axis(pw, fw, s.Wo));
-      arow = p.dy + (ptrdiff_t)b * s.Co * op + (fd * s.Ho + fh) * s.Wo + fw;
-    }
-  }
   __syncthreads();
   float acc[NJ][4] = {};
+  const int mine = (threadIdx.x & 7) + 8 * (threadIdx.x >> 5), at = row_dy[mine];
+  const unsigned amask = row_taps[mine];
   switch (__popc(cmask)) {
-    case 8: dgrad_rows<8, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
-    case 4: dgrad_rows<4, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
-    case 2: dgrad_rows<2, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
-    default: dgrad_rows<1, NT>(p, As, Bs, off, tap, arow, amask, n0, period, acc); break;
+    case 8: dgrad_rows<8, NT>(p, As, Bs, tap, at, amask, n0, period, acc); break;
+    case 4: dgrad_rows<4, NT>(p, As, Bs, tap, at, amask, n0, period, acc); break;
+    case 2: dgrad_rows<2, NT>(p, As, Bs, tap, at, amask, n0, period, acc); break;
+    default: dgrad_rows<1, NT>(p, As, Bs, tap, at, amask, n0, period, acc); break;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tig = lane & 3;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int q = row0 + (warp >> 1) * 16 + g + 8 * h;
-    if (q >= rows) continue;
-    const int jw = q % nw, jh = q / nw % nh, jd = q / (nw * nh) % nd, b = q / (nw * nh * nd);
-    const size_t at = (size_t)b * s.Ci * ip + ((2 * jd + pd) * s.H + 2 * jh + ph) * s.W + 2 * jw + pw;
+    const int dx0 = row_dx[(warp >> 1) * 16 + g + 8 * h];
+    if (dx0 < 0) continue;
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int n = n0 + (warp & 1) * (NT / 2) + 8 * j + 2 * tig + e;
         if (n >= s.Ci) continue;
-        const size_t o = at + (size_t)n * ip;
+        const int o = dx0 + n * ip;
         p.dx[o] = relu_grad(acc[j][2 * h + e], p.x[o]);
       }
   }
@@ -652,9 +653,15 @@ cudaError_t run_dgrad_nt(const ConvDgrad &p, int tiles, cudaStream_t st) {
   k_dgrad<NT><<<dim3(tiles, (p.s.Ci + NT - 1) / NT), 256, dgrad_smem(NT), st>>>(p);
   return cudaGetLastError();
 }
-inline cudaError_t run_dgrad(const ConvDgrad &p, cudaStream_t st) {
+// whole groups of channels, and 32-bit element offsets at every batch size
+static_assert(kCh[2] % 16 == 0 && kCh[3] % 16 == 0 && kCh[4] % 16 == 0 &&
+              4096ll * 16 * 16 * 16 * 12 < (1ll << 31), "k_dgrad");
+inline cudaError_t run_dgrad(ConvDgrad p, cudaStream_t st) {
   int tiles = 0;
-  for (int c = 0; c < 8; ++c) tiles += (p.rows(c) + BM - 1) / BM;
+  for (int c = 0; c < 8; ++c) {
+    p.first[c] = tiles;
+    tiles += (p.rows(c) + BM - 1) / BM;
+  }
   return p.s.Ci <= 16 ? run_dgrad_nt<16>(p, tiles, st) : run_dgrad_nt<32>(p, tiles, st);
 }
 
