@@ -44,9 +44,14 @@ namespace n4 {
 #define kNaN __int_as_float(0x7fc00000)
 
 // Work of one row in the whole-GPU path's partition: its voxels and what it
-// costs beside them.  The floor keeps a CTA of many short rows within the
+// costs beside them (its entries of the row tables, its share of the y
+// contraction).  Half a row of voxels: with an eighth the CTAs of the short
+// rows at the volume's ends took 66k cycles for the contractions of an
+// iteration where the others took 49k (512x512x320 at half resolution, 148
+// CTAs: 162k cycles an iteration with Z/8, 154k with Z/4 and Z/2; 181x217x181:
+// 128k, 124k and 121k).  The floor keeps a CTA of many short rows within the
 // row buffers (grid_rows_bound).
-__host__ __device__ inline int grid_row_overhead(int Z) { return Z / 8 > 16 ? Z / 8 : 16; }
+__host__ __device__ inline int grid_row_overhead(int Z) { return Z / 2 > 16 ? Z / 2 : 16; }
 // Most rows, and most voxels, the partition gives one of K CTAs.
 __host__ __device__ inline long long grid_rows_bound(long long rows, int Z, int K) {
   const int c = grid_row_overhead(Z);
