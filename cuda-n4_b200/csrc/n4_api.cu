@@ -2300,6 +2300,7 @@ static n4_status_t ensure_ticket(n4_context *ctx) {
   if (ctx->ticket.p) return N4_OK;
   TRY(ctx->ticket.ensure(64, "ticket"));
   CK(cudaMemset(ctx->ticket.p, 0, 64));
+  CK(cudaStreamSynchronize(nullptr));   // the caller's stream may not wait for the default one
   return N4_OK;
 }
 // Page-locked buffer for what a component call reads back.
