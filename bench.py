@@ -195,7 +195,7 @@ def cpu_baseline_single(seconds=12.0):
 def measure_components(dev, ctx, hbm_peak, reps=10):
     """Standalone HBM-bound kernels at the 512x512x320 scale: the fit's z
     contraction (k_fit_rows_v5) on the 256x256x160 fitting grid (reads field
-    4 B + float mask 4 B per voxel) and the dense evaluation (k_correct) at
+    4 B + float mask 4 B per voxel) and the dense evaluation (k_evaluate) at
     full resolution (writes 4 B per voxel); device time of the kernel alone
     from the library's stage events, mean of `reps` calls, L2 evicted before
     each."""
@@ -246,7 +246,7 @@ def measure_components(dev, ctx, hbm_peak, reps=10):
         "upsample_gbs": {"value": ups, "frac": ups / hbm_peak, "ms": ms_eval,
                          "shape": {"rows_per_tile": te["correct_rows"], "threads": te["correct_threads"]},
                          "tuner_candidates_ms": tune_eval["evaluate"],
-                         "workload": "EvaluateBspline3D dense evaluation (k_correct) of an 11^3 lattice at "
+                         "workload": "EvaluateBspline3D dense evaluation (k_evaluate) of an 11^3 lattice at "
                                      "512x512x320 (4 B per voxel written)"},
     }
 

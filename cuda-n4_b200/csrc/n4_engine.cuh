@@ -174,10 +174,10 @@ struct GridGroup {
 };
 
 // ------------------------------------------------------------------ phase timers
-// Compile with -DN4_PHASE_TIMERS to print, per volume, the cycles thread 0
-// of the first CTA spends between phase marks (measurement builds only).  The
-// counters live in shared memory, so that the timed build allocates the
-// kernel's registers as the product build does.
+// Compile with -DN4_PHASE_TIMERS to print, per volume, the cycles thread 0 of
+// the first and of the middle CTA spends between phase marks (measurement
+// builds only).  The counters live in shared memory, so that the timed build
+// allocates the kernel's registers as the product build does.
 #ifdef N4_PHASE_TIMERS
 #define N4_MARK(k)                                                     \
   do {                                                                 \

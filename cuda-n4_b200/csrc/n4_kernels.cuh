@@ -9,6 +9,7 @@
 //   k_correct         final dense evaluation at full resolution fused with
 //                     im / exp(b) and the optional exp(b) output
 //                     (cudaN4.cu:1697-1729, N4.py:329-330)
+//   k_evaluate        the final evaluation alone (EvaluateBspline3D)
 //   k_fit_*           standalone separable B-spline fit (FitBspline3D)
 //   k_refine          lattice refinement (upsampleLattice3D_gpu)
 //   k_minmax/k_hist/k_remap   standalone sharpenImage

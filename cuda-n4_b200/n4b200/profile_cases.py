@@ -5,7 +5,7 @@ each (run from the repository root)::
     PYTHONPATH=cuda-n4_b200 python -m n4b200.profile_cases c2x4     # k_n4_cluster, k_prologue, k_correct
     PYTHONPATH=cuda-n4_b200 python -m n4b200.profile_cases encoder  # enc::k_igemm
     PYTHONPATH=cuda-n4_b200 python -m n4b200.profile_cases fit      # k_fit_rows_v5
-    PYTHONPATH=cuda-n4_b200 python -m n4b200.profile_cases evaluate # k_correct (log field only)
+    PYTHONPATH=cuda-n4_b200 python -m n4b200.profile_cases evaluate # k_evaluate
 
 * ``c3``: one 512x512x320 phantom (0.5 mm, 8^3-grid bias N(0, 0.25^2),
   Rician 0.02) through ``n4_run`` at shrink 2 (256x256x160 fitting grid,

@@ -60,6 +60,7 @@ typedef enum {
  * sub-batch's prologue, warm start and correction overlapping the other
  * sub-batches' N4 iterations on the SMs the clusters leave free (1 = one
  * pass, no overlap; 0 = choose: one sub-batch per two waves of clusters, at
+ * least 2 if the volumes do not all fit at once and there is no encoder, at
  * most 4).  Every volume's result is the same either way. */
 #define N4_FLAG_SUB_BATCHES(k)  (((unsigned int)(k) & 7u) << 16)
 /* Bits 19-23: with two or more sub-batches, each sub-batch runs on the
