@@ -792,7 +792,8 @@ n4_status_t n4_encoder_create(n4_encoder_t **out, int device, int max_batch) {
   cudaMemset(e->pb, 0, n * 2);
   for (int l = 0; l <= kLayers; ++l) {
     const size_t sz = l == 0 ? (size_t)max_batch * L.s[0].in_pos() : (size_t)max_batch * L.s[l - 1].Co * L.s[l - 1].out_pos();
-    if ((err = cudaMalloc(&e->act[l], sz * 2)) || (err = cudaMalloc(&e->dact_[l], sz * 2))) return fail_free(err);
+    if ((err = cudaMalloc(&e->act[l], sz * 2))) return fail_free(err);
+    if (l > 0 && (err = cudaMalloc(&e->dact_[l], sz * 2))) return fail_free(err);   // the input has no gradient
   }
   if ((err = cudaMalloc(&e->out, (size_t)max_batch * kOut * 4)) || (err = cudaMalloc(&e->tgt, (size_t)max_batch * kOut * 4)) ||
       (err = cudaMalloc(&e->loss, 16)) || (err = cudaMalloc(&e->dout, (size_t)max_batch * kOut * 2)))
