@@ -1549,6 +1549,9 @@ struct Engine {
           if (!fit_step(false)) goto timeout;
           if (!pass_a(true, false)) goto timeout;   // the update's CV; logU not advanced
           cvs[arm] = iter().cv;
+          // the next pass A writes the CTAs' sums again: not before every CTA
+          // has read them (a CTA that read others would take the other arm)
+          if (!g.sync()) goto timeout;
           if (arm == 0) {   // keep the warm result in aux, its update in tmp
             for (int c = threadIdx.x; c < nlat; c += blockDim.x) { aux()[c] = L()[c]; tmp()[c] = D()[c]; }
           }
