@@ -283,7 +283,7 @@ Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool 
   auto take = [&](size_t bytes) { size_t r = o; o = align_up(o + bytes, 16); return (int)r; };
   pl.o_ax = take(eaxis_bytes(pl.Xmax, pl.NCX - 3));
   pl.o_ay = take(eaxis_bytes(pl.Ymax, pl.NCY - 3));
-  pl.o_az = take(eaxis_bytes(pl.Zmax, pl.NCZ - 3));
+  pl.o_az = take(eaxis_bytes(pl.Zmax, pl.NCZ - 3, kWeightTail));
   pl.o_L = take((size_t)pl.NLAT * 4);
   pl.o_D = take((size_t)pl.NLAT * 4);
   pl.o_den = take((size_t)pl.NLAT * 4);

@@ -68,21 +68,27 @@ __host__ __device__ inline int row_lanes_log2(int Z) { return Z <= 64 ? 3 : (Z <
 // One axis of the fitting grid at one level, in the CTA's dynamic shared
 // memory: byte offsets of the span index and the weights of every voxel
 // (B0..B3, the fit's numerator weights w^3 / sum w^2 and denominator weights
-// w^2) and of the spans' voxel ranges.
+// w^2) and of the spans' voxel ranges.  The z contraction's lanes step over
+// several voxels at once and read weights up to 7 entries past the row's last
+// voxel, for terms that are zero: `tail` zero entries after the last table keep
+// those reads in memory that has been written (zero times a NaN left there by
+// an earlier kernel is a NaN).
 struct EAxis {
   int n, nc, nsp;
-  int o_s, o_w, o_p, o_q, o_lo, o_hi;
+  int o_s, o_w, o_p, o_q, o_tail, o_lo, o_hi;
 };
-__host__ __device__ inline size_t eaxis_bytes(int n, int nsp) {
-  return ((size_t)n * 4 + 15) / 16 * 16 + (size_t)n * 48 + ((size_t)nsp * 8 + 15) / 16 * 16;
+constexpr int kWeightTail = 8;   // of the z axis
+__host__ __device__ inline size_t eaxis_bytes(int n, int nsp, int tail = 0) {
+  return ((size_t)n * 4 + 15) / 16 * 16 + (size_t)n * 48 + (size_t)tail * 16 + ((size_t)nsp * 8 + 15) / 16 * 16;
 }
-__host__ __device__ inline EAxis eaxis_at(int off, int n, int nc) {
+__host__ __device__ inline EAxis eaxis_at(int off, int n, int nc, int tail = 0) {
   EAxis a;
   a.n = n; a.nc = nc; a.nsp = nc - 3;
   a.o_w = off;
   a.o_p = a.o_w + n * 16;
   a.o_q = a.o_p + n * 16;
-  a.o_s = a.o_q + n * 16;
+  a.o_tail = a.o_q + n * 16;
+  a.o_s = a.o_tail + tail * 16;
   a.o_lo = a.o_s + (n * 4 + 15) / 16 * 16;
   a.o_hi = a.o_lo + a.nsp * 4;
   return a;
@@ -339,7 +345,7 @@ struct Engine {
       nlat = ncx * ncy * ncz;
       ax = eaxis_at(pl.o_ax, X, ncx);
       ay = eaxis_at(pl.o_ay, Y, ncy);
-      az = eaxis_at(pl.o_az, Z, ncz);
+      az = eaxis_at(pl.o_az, Z, ncz, kWeightTail);
       // lanes per row: 8, or enough for one per span (16 or 32 lanes of a
       // 160-voxel row hold too little each: the z contraction at 512x512x320
       // took 68k and 109k cycles per iteration against 48k)
@@ -377,6 +383,7 @@ struct Engine {
       else if (t < X + Y) build_voxel(ay, t - X);
       else build_voxel(az, t - X - Y);
     }
+    if (threadIdx.x < kWeightTail) at<float4>(az.o_tail)[threadIdx.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     __syncthreads();
     if (np <= tp) build_ytab(0, np);
     __syncthreads();
@@ -893,7 +900,7 @@ struct Engine {
         terms(v, x);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const float4 w = W[z + u];   // past the row: finite, times zero
+          const float4 w = W[z + u];   // past the row: the next table or its tail, times zero
           s.x = __fmaf_rn(w.x, x[u], s.x); s.y = __fmaf_rn(w.y, x[u], s.y);
           s.z = __fmaf_rn(w.z, x[u], s.z); s.w = __fmaf_rn(w.w, x[u], s.w);
         }
@@ -946,7 +953,7 @@ struct Engine {
           v[u] = z < b ? p[z] : kNaN;
         }
         sums.terms(v, x);
-        const float *w = Wj + 4 * min(a + q, zmax);   // past the row: finite, times zero
+        const float *w = Wj + 4 * min(a + q, zmax);   // past the row: the next table or its tail, times zero
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
