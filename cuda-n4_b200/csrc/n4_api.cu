@@ -236,6 +236,7 @@ Params make_dev_params(const n4_params_t *p) {
   r.thr = decimal_of(p->ConvergenceThreshold);
   r.eps = p->FitEpsilon;
   r.zero_den = (p->flags & N4_FLAG_FIT_ZERO_DEN) ? 1 : 0;
+  r.sum_words = sum_words(r.eps, r.zero_den);
   r.ddof1 = (p->flags & N4_FLAG_CV_DDOF1) ? 1 : 0;
   for (unsigned l = 0; l < N4_MAX_LEVELS; ++l)
     r.iters[l] = l < p->NumberOfFittingLevels ? (int)p->MaximumNumberOfIterations[l] : 0;
@@ -511,7 +512,7 @@ struct RunVol {
 };
 
 // Words of one accumulator set of the whole-GPU path.
-int grid_acc_len(const Plan &pl) { return std::max(pl.bins, pl.NLAT) + 1; }
+int grid_acc_len(const Plan &pl, const Params &pr) { return std::max(pl.bins, pl.NLAT * pr.sum_words) + 1; }
 
 // Workspaces of the whole-GPU path for one volume (sized before any capture):
 // the CTAs' slices; the accumulator sets and the barrier, zero at launch;
@@ -520,7 +521,7 @@ n4_status_t ensure_grid_workspace(n4_context *ctx, const n4_params_t *p, const D
   std::vector<Dims> one{d};
   Plan pl = make_plan(p, ctx->nsm, one, true, ctx->max_smem);
   TRY(ctx->big.ensure((size_t)pl.big_bytes * ctx->nsm, "grid workspace"));
-  TRY(ctx->red.ensure((size_t)3 * grid_acc_len(pl) * 8 + 64, "grid reduction"));
+  TRY(ctx->red.ensure((size_t)3 * grid_acc_len(pl, make_dev_params(p)) * 8 + 64, "grid reduction"));
   TRY(ctx->bar.ensure((size_t)d.X * d.Y * 4, "grid rows"));
   return N4_OK;
 }
@@ -547,7 +548,7 @@ n4_status_t launch_grid_path(n4_context *ctx, const n4_params_t *p, const Params
   if (((long long)rv.d.X * rv.d.Y + nblk - 1) / nblk * rv.d.Z >= (1ll << 22))
     return fail(N4_ERR_TOO_LARGE, "fitting grid too large for one GPU (raise ShrinkFactor)");
   TRY(ensure_grid_workspace(ctx, p, rv.d));
-  const size_t acc_bytes = (size_t)3 * grid_acc_len(pl) * 8;
+  const size_t acc_bytes = (size_t)3 * grid_acc_len(pl, pr) * 8;
   CK(cudaMemsetAsync(ctx->red.p, 0, acc_bytes + 64, st));
   GridArgs a{};
   a.pl = pl;
@@ -556,7 +557,7 @@ n4_status_t launch_grid_path(n4_context *ctx, const n4_params_t *p, const Params
   a.big_base = ctx->big.as<char>();
   a.big_stride = pl.big_bytes;
   a.acc = ctx->red.as<unsigned long long>();
-  a.acc_len = grid_acc_len(pl);
+  a.acc_len = grid_acc_len(pl, pr);
   a.bar.count = (unsigned *)(ctx->red.as<char>() + acc_bytes);
   a.bar.err = (int *)(a.bar.count + 8);
   a.bar.nblocks = nblk;

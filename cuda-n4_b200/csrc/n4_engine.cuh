@@ -117,11 +117,24 @@ struct Plan {
   int a_fa, a_fb, a_hist, a_ff;
 };
 
+// The whole-GPU path adds the CTAs' parts of a lattice sum as integers: one
+// word, whose unit is 2^-60 of a bound on the level's sums (sum_shift).  That
+// is an absolute unit, nothing beside FitEpsilon's default; without an epsilon
+// of that size (or with N4_FLAG_FIT_ZERO_DEN) a control point that few voxels
+// reach is the quotient of two sums far below the largest, and each part takes
+// kSumWords words, each of 2^-40 of the unit before it: 120 bits more, every
+// digit of a float at any size.  With one word such a lattice was 3e-5 off the
+// FP64 oracle where sums of floats are 1e-6 off.
+constexpr int kSumWords = 4;
+constexpr double kSumWordUnit = 1.0 / 1099511627776.0;   // 2^-40
+inline int sum_words(float eps, int zero_den) { return zero_den || eps < 1e-3f ? kSumWords : 1; }
+
 struct Params {
   int bins;
   double wiener, fwhm, thr;   // decimal values of the float parameters
   float eps;
   int zero_den, ddof1;
+  int sum_words;              // whole-GPU path: words of a lattice sum (kSumWords)
   int iters[N4_MAX_LEVELS];
 };
 
@@ -137,7 +150,7 @@ struct VolJob {
 struct Stats { double v[4]; };
 
 // What the passes of one iteration need from the statistics, in the CTA's
-// shared memory (o_red, after the reduction scratch).
+// shared memory (o_red, after 144 words of reduction scratch).
 struct Iter {
   double st[4];     // group min, max, sum y, sum y^2
   BinMap bm;
@@ -146,6 +159,7 @@ struct Iter {
   int degenerate;   // no bin range: nothing to fit
   float cv;
 };
+static_assert(sizeof(Iter) <= (160 - 144) * 8, "Iter lies in the o_red words behind the scratch");
 
 // ------------------------------------------------------------------ groups
 struct ClusterGroup {
@@ -160,8 +174,8 @@ struct ClusterGroup {
 
 // Accumulators of the whole-GPU path in global memory, zero at launch: three
 // sets used in turn (one is cleared while the next is in use), each `len`
-// words for the range, the histogram or the lattice sums, the last word a
-// count of partials that are not numbers.
+// words for the range, the histogram or the lattice sums (word k of entry c at
+// k NLAT + c), the last word a count of partials that are not numbers.
 struct GridGroup {
   GridBarrier bar;
   char *big_base;      // per-CTA big regions, stride big_stride
@@ -689,7 +703,9 @@ struct Engine {
 
   // Fixed-point scale of the lattice sums of the whole-GPU path: `bound` is at
   // least the sum of the magnitudes of all terms, so that the 64-bit integer
-  // sum cannot overflow; integer sums are exact and the same in any order.
+  // sum stays below 2^62, whichever CTAs the terms are in (a mask of nearly
+  // empty rows leaves most of them to one); integer sums are exact and the same
+  // in any order.
   static __device__ __forceinline__ int sum_shift(double bound) {
     return min(61 - ilogb(fmin(fmax(bound, 1e-30), 1e300)), 52);
   }
@@ -773,10 +789,8 @@ struct Engine {
     if constexpr (Group::kGrid) {
       // den: weights below 1.  num: with w <= 2/3 and sum w^2 >= 0.46 per axis,
       // w^3/sum w^2 <= 1.45 w^2, so an entry's terms sum to at most 3.1 times
-      // its den times the largest residual; E lies within 4 ranges of the data
-      // or is 0.
-      const double range = it.st[1] - it.st[0];
-      scale = ldexp(1.0, sum_shift(Num ? 4.0 * denmax * (5.0 * range + fabs(it.st[0]) + fabs(it.st[1])) : nfg));
+      // its den times the largest residual.
+      scale = ldexp(1.0, sum_shift(Num ? 4.0 * denmax * (degenerate ? 0.0f : residual_bound()) : nfg));
     }
     const int slice = ncy * ncz;
     for (int m0 = 0; m0 < np || m0 == 0; m0 += tp) {
@@ -815,11 +829,15 @@ struct Engine {
         }
         if constexpr (Group::kGrid) {
           if (any) {
-            const double v = ((double)acc.s - (double)acc.c) * scale;
-            if (!isfinite(v)) atomicAdd(acc_set(seq) + g.len - 1, 1ull);
+            double v = ((double)acc.s - (double)acc.c) * scale;
+            // a part beyond the bound is one of a map that is not finite
+            if (!(fabs(v) < 4611686018427387904.0)) atomicAdd(acc_set(seq) + g.len - 1, 1ull);
             else if (v != 0.0) {
-              const double lim = 4611686018427387904.0 / K;   // 2^62: the sum of K terms cannot wrap
-              atomicAdd(acc_set(seq) + c, (unsigned long long)__double2ll_rn(fmin(fmax(v, -lim), lim)));
+              atomicAdd(acc_set(seq) + c, (unsigned long long)__double2ll_rn(v));
+              for (int k = 1; k < pr.sum_words; ++k) {
+                v = (v - rint(v)) / kSumWordUnit;   // exact
+                atomicAdd(acc_set(seq) + k * pl.NLAT + c, (unsigned long long)__double2ll_rn(v));
+              }
             }
           }
         } else {
@@ -834,8 +852,14 @@ struct Engine {
       const unsigned long long *a = acc_set(seq);
       const bool nan = __ldcg(a + g.len - 1) != 0;
       const double inv = 1.0 / scale;
-      for (int c = threadIdx.x; c < nlat; c += blockDim.x)
-        fin(c, nan ? kNaN : (float)((double)(long long)__ldcg(a + c) * inv));
+      for (int c = threadIdx.x; c < nlat; c += blockDim.x) {
+        double s = (double)(long long)__ldcg(a + c), unit = 1.0;
+        for (int k = 1; k < pr.sum_words; ++k) {
+          unit *= kSumWordUnit;
+          s += (double)(long long)__ldcg(a + k * pl.NLAT + c) * unit;
+        }
+        fin(c, nan ? kNaN : (float)(s * inv));
+      }
       acc_clear();
       acc_next();
     } else {
@@ -844,6 +868,27 @@ struct Engine {
     }
     N4_MARK(PH_F_RED);
     return true;
+  }
+
+  // The largest residual x - E(x) of the map (whole-GPU path): it is linear
+  // within a bin, so the bins' ends hold it, whatever values E takes in bins
+  // that no voxel fills.  One value per warp, from the bins its threads have
+  // just tabulated; read after the z contraction's barrier.  Every CTA has the
+  // same map.
+  __device__ __forceinline__ float *rmax() const { return (float *)(red() + 128); }
+  __device__ __forceinline__ void residual_max() const {
+    const float2 *t = R2();
+    if ((int)(threadIdx.x & ~31u) + 1 >= pr.bins) return;
+    float m = 0.0f;
+    for (int b = threadIdx.x; b + 1 < pr.bins; b += blockDim.x) m = fmaxf(m, fmaxf(fabsf(t[b].x), fabsf(t[b].x + t[b].y)));
+    m = __int_as_float(__reduce_max_sync(kFull, __float_as_int(m)));
+    if ((threadIdx.x & 31) == 0) rmax()[threadIdx.x >> 5] = m;
+  }
+  __device__ __forceinline__ float residual_bound() const {
+    const int n = (min((int)blockDim.x, pr.bins - 1) + 31) >> 5;
+    float m = 0.0f;
+    for (int w = 0; w < n; ++w) m = fmaxf(m, rmax()[w]);
+    return m;
   }
 
   // x0 + x1 + x2 + x3, the sums of spans s, s - 1, s - 2, s - 3, added in the
@@ -1230,6 +1275,7 @@ struct Engine {
     SharpenBufs sb{at<double2>(a0 + pl.a_fa), at<double2>(a0 + pl.a_fb), at<double2>(pl.o_tw), at<double>(a0 + pl.a_ff)};
     sharpen_map([=](int b) { return (double)h64[b] * inv; }, bins, pl.npad, pl.hoff, it.bm.binMin, it.bm.slope,
                 pr.wiener, it.gauss, sb, E(), R2());
+    if constexpr (Group::kGrid) residual_max();
     N4_MARK(PH_SHARP);
     return true;
   }

@@ -67,3 +67,71 @@ def test_leftovers_in_shared_memory_do_not_matter(cuda, fill_shared_memory, shap
         out, lat = O.N4(im, np.ones(shape, np.float32), low_value=0, maximumNumberOfLevels=1,
                         maximumNumberOfIterations=[1], ConvergenceThreshold=0.0)
         assert nrel(c.lattice, lat) < TOL and nrel(c.im_normalized, out) < TOL
+
+
+def log_volume(shape, seed):
+    return (np.abs(make_phantom(shape, seed=seed, sigma=0.03, grid=4, coeff_std=0.15).im) + 0.3).astype(np.float32)
+
+
+def thin_rows_and_solid_planes(shape):
+    """Rows of two voxels, and two x-planes of whole rows in one CTA's share:
+    one CTA of the whole-GPU path has a third of the volume's voxels."""
+    m = np.zeros(shape, np.float32)
+    m[:, :, 0] = m[:, :, -1] = 1
+    m[shape[0] // 2:shape[0] // 2 + 2] = 1
+    return m
+
+
+def hollow_box(shape):
+    m = np.zeros(shape, np.float32)
+    m[[0, -1]] = 1
+    m[:, [0, -1]] = 1
+    m[:, :, [0, -1]] = 1
+    return m
+
+
+def one_row(shape, n):
+    m = np.zeros(shape, np.float32)
+    m[shape[0] // 2, 10:10 + n] = 1
+    return m
+
+
+@pytest.mark.parametrize("shape,mask,levels", [
+    ((256, 256, 160), thin_rows_and_solid_planes, 2),
+    ((100, 400, 400), hollow_box, 1),
+    ((24, 24, 1000), lambda s: one_row(s, 10), 1),
+])
+def test_masks_that_leave_most_voxels_to_one_cta(cuda, shape, mask, levels):
+    """The lattice sums of the whole-GPU path hold the whole volume's terms in
+    any one CTA.  (Of 10,000 voxels one more or less in the top bin moves the
+    lattice by 5e-5 a step: one iteration there, two on the large masks.)"""
+    im, m = log_volume(shape, 5), mask(shape)
+    iters = [2] * levels if m.sum() > 20_000 else [1]
+    p = run(cuda, im, m, levels, iters, flags=0x8)
+    out, lat = O.N4(im, m, low_value=0, maximumNumberOfLevels=levels, maximumNumberOfIterations=iters,
+                    ConvergenceThreshold=0.0)
+    assert p.report["status"] == "N4_OK" and p.report["path"] == "grid"
+    assert nrel(p.lattice, lat) < TOL and nrel(p.im_normalized, out) < TOL
+
+
+@pytest.mark.parametrize("force", [0x8, 0])
+@pytest.mark.parametrize("flags,eps", [(0x2, 1e-3), (0, 0.0), (0, 1e-9)])
+def test_control_points_almost_without_voxels(cuda, flags, eps, force):
+    """A mask in one corner of one span: the denominators of the far control
+    points are 1e-8 to 1e-24 of the largest, and without an epsilon the lattice
+    there is a quotient of such sums.  Bound 1e-5: the sums along z are plain
+    FP32 over at most 52 voxels of a row, 52 * 2^-24 = 3e-6 for numerator and
+    denominator each, the other sums compensated, and one voxel in the top bin
+    (174720 voxels) 3e-6."""
+    import n4b200
+    shape = (128, 120, 112)
+    im = log_volume(shape, 5)
+    m = np.zeros(shape, np.float32)
+    m[2:62, 2:58, 2:54] = 1
+    p = n4b200.N4Param(NumberOfFittingLevels=1, MaximumNumberOfIterations=[2], ConvergenceThreshold=0.0, low_value=0.0,
+                       flags=flags | force, FitEpsilon=eps)
+    res = n4b200.N4(cuda.tensor(im, device="cuda"), cuda.tensor(m, device="cuda"), p)
+    out, lat = O.N4(im, m, low_value=0, maximumNumberOfLevels=1, maximumNumberOfIterations=[2],
+                    ConvergenceThreshold=0.0, fit_eps=eps, fit_zero_den=bool(flags & 2))
+    assert res.report["status"] == "N4_OK"
+    assert nrel(res.lattice, lat) < 1e-5 and nrel(res.im_normalized, out) < 1e-5
