@@ -29,8 +29,10 @@
 // have one (an ellipsoid mask leaves 36 % of the rows out and fills 60 % of
 // the others).  2^sg lanes share a row; in the passes that follow the
 // lattice's spans along z, a lane takes one span of the row or, with fewer
-// spans than lanes, an equal part of it, so that a row's voxels are taken a
-// few per lane instead of one after the other in one thread.
+// spans than lanes, a part of it, so that a row's voxels are taken a few per
+// lane instead of one after the other in one thread: an equal piece (pass A on
+// the cluster path), or every 2^szh-th voxel (whole-GPU path, whose rows are
+// long and may lie in global memory).
 #pragma once
 #include <cooperative_groups.h>
 #include <new>
@@ -362,7 +364,7 @@ struct Engine {
       az = eaxis_at(pl.o_az, Z, ncz, kWeightTail);
       // lanes per row: 8, or enough for one per span (16 or 32 lanes of a
       // 160-voxel row hold too little each: the z contraction at 512x512x320
-      // took 68k and 109k cycles per iteration against 48k)
+      // in equal pieces took 68k and 109k cycles per iteration against 48k)
       sg = 3;
       while (sg < 5 && (1 << sg) < az.nsp) ++sg;
       sh = 0;
@@ -713,10 +715,14 @@ struct Engine {
   // ---- separable fit contraction of the rows into the group's lattice sums
   // num: the residuals with weights w^3/sum w^2; den: the mask with weights
   // w^2 (N4.py:224-236).
-  //   T1[row][cz]   z contraction: the lane of a (row, span) piece accumulates
-  //                 the span's 4 targets in registers; the pieces of a span
-  //                 are added by shuffles, and target t takes its sums from
-  //                 spans t-3 .. t by shuffles too
+  //   T1[row][cz]   z contraction: the lane of a (row, span) part accumulates
+  //                 the span's 4 targets in registers; the parts of a span
+  //                 (every 2^szh-th voxel each, so that a span's lanes read
+  //                 consecutive voxels and weights; equal pieces of 32 voxels
+  //                 met in one shared-memory bank: 320x320x256 without a mask,
+  //                 9.2M cycles over 18 iterations against 4.3M) are added by
+  //                 shuffles, and target t takes its sums from spans t-3 .. t
+  //                 by shuffles too
   //   T2[m][cy][cz] y contraction over the CTA's rows of each x-plane
   //   lattice       x contraction (the CTA's partial lattice)
   // then the group's sum of the partial lattices, fin(c, sum) per entry.  The
@@ -750,10 +756,11 @@ struct Engine {
           if (on && !degenerate) {
             const Row o = rm(r);
             int a, b;
-            piece(o, lo, hi, h, hh, a, b);
-            if constexpr (Group::kGrid) sums.template add<2>(o.p, a, b, s);
-            else if (nsp > 2) sums.template add<3>(o.p, a, b, s);
-            else sums.template add<4>(o.p, a, b, s);
+            a = max(lo, o.z0);
+            b = min(hi, o.z1);
+            if constexpr (Group::kGrid) sums.template add<2>(o.p, a + h, b, d, s);
+            else if (nsp > 2) sums.template add<3>(o.p, a, b, 1, s);
+            else sums.template add<4>(o.p, a, b, 1, s);
           }
           for (int w = d >> 1; w; w >>= 1) {
             s.x += __shfl_xor_sync(kFull, s.x, w); s.y += __shfl_xor_sync(kFull, s.y, w);
@@ -899,9 +906,9 @@ struct Engine {
     return __fadd_rn(__fadd_rn(__fadd_rn(t0, t1), t2), t3);
   }
 
-  // The four targets' sums of voxels [a, b) of a row, in voxel order: weights
-  // times the residual R = logU - E(logU) (Num), or the weights of the masked
-  // voxels.  Voxels outside the mask add zeros.  The residuals of U voxels are
+  // The four targets' sums of every d-th voxel of [a, b) of a row, in voxel
+  // order: weights times the residual R = logU - E(logU) (Num), or the weights
+  // of the masked voxels.  Voxels outside the mask add zeros.  The residuals of U voxels are
   // formed together, without branches: 4 on the cluster path's long spans, 3 on
   // its short ones (5 or 6 voxels: two steps, 6 slots instead of 8; 26.0k
   // against 28.3k cycles at 8 spans of 44 voxels on 6 CTAs), 2 on the whole-GPU
@@ -937,15 +944,15 @@ struct Engine {
       }
     }
     template <int U>
-    __device__ __forceinline__ void add(const float *p, int a, int b, float4 &s) const {
-      for (int z = a; z < b; z += U) {
+    __device__ __forceinline__ void add(const float *p, int a, int b, int d, float4 &s) const {
+      for (int z = a; z < b; z += U * d) {
         float v[U], x[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = z + u < b ? p[z + u] : kNaN;
+        for (int u = 0; u < U; ++u) v[u] = z + u * d < b ? p[z + u * d] : kNaN;
         terms(v, x);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const float4 w = W[z + u];   // past the row: the next table or its tail, times zero
+          const float4 w = W[z + u * d];   // past the row: the next table or its tail, times zero
           s.x = __fmaf_rn(w.x, x[u], s.x); s.y = __fmaf_rn(w.y, x[u], s.y);
           s.z = __fmaf_rn(w.z, x[u], s.z); s.w = __fmaf_rn(w.w, x[u], s.w);
         }
@@ -1154,44 +1161,90 @@ struct Engine {
     const float *Gp = Gd();
     const float4 *W4 = at<float4>(az.o_w);
     const int nc = ncz;
-    span_pass(
-        [&](const Row &o, int r, int a, int b, int sp) {
-          if (a >= b) return;
-          constexpr int U = 2;
+    if constexpr (Group::kGrid) {
+      // a row's lanes take consecutive voxels: bound by the shared-memory reads
+      // of the rows held there and by the lines of the others.  With a piece of
+      // the row per lane, whose four values of Gd stay in registers, the lanes'
+      // weights met in the same banks and every line of a row in global memory
+      // came several times: 12.5M cycles over 18 iterations of 320x320x256
+      // without a mask against 2.8M so, 1.83M against 0.85M at 256x256x160.
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+      const int s = row_lanes_log2(Z), l = lane & ((1 << s) - 1), sub = lane >> s, rs = 5 - s, n = nact;
+      const auto rm = row_map();
+      const int *S = at<int>(az.o_s);
+      for (int r = (warp << rs) + sub; r < n; r += nw << rs) {
+        const Row o = rm(r);
+        const float *g0 = Gp + r * nc;
+        constexpr int U = 2;
+        for (int z0 = o.z0 + l; z0 < o.z1; z0 += U << s) {
+          float v[U], ed[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) v[u] = z0 + (u << s) < o.z1 ? o.p[z0 + (u << s)] : kNaN;
           if (need_cv) {
-            const float *gp = Gp + r * nc + sp;
-            const float g[4] = {gp[0], gp[1], gp[2], gp[3]};
-            for (int z = a; z < b; z += U) {
-              float v[U], ed[U], y[U];
 #pragma unroll
-              for (int u = 0; u < U; ++u) v[u] = z + u < b ? o.p[z + u] : kNaN;
-#pragma unroll
-              for (int u = 0; u < U; ++u) {
-                ed[u] = dot4(W4[z + u], g);   // past the row: finite, not used
-                y[u] = expm1_conv(-ed[u]);
-              }
-#pragma unroll
-              for (int u = 0; u < U; ++u) {
-                const bool in = !isnan(v[u]);
-                const double yd = in ? (double)y[u] : 0.0;
-                sy += yd;
-                syy += yd * yd;
-                if (apply) {
-                  v[u] = __fsub_rn(v[u], ed[u]);
-                  if (in) o.p[z + u] = v[u];
-                }
-                vmin = fminf(vmin, v[u]);   // a NaN operand is passed over
-                vmax = fmaxf(vmax, v[u]);
-              }
+            for (int u = 0; u < U; ++u) {
+              const int z = min(z0 + (u << s), o.z1 - 1);
+              ed[u] = dot4(W4[z], g0 + S[z]);
             }
-          } else {
-            for (int z = a; z < b; ++z) {
-              const float v = o.p[z];
-              vmin = fminf(vmin, v);
-              vmax = fmaxf(vmax, v);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const bool in = !isnan(v[u]);
+              const double yd = in ? (double)expm1_conv(-ed[u]) : 0.0;
+              sy += yd;
+              syy += yd * yd;
+              if (apply) {
+                v[u] = __fsub_rn(v[u], ed[u]);
+                if (in) o.p[z0 + (u << s)] = v[u];
+              }
             }
           }
-        });
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            vmin = fminf(vmin, v[u]);   // a NaN operand is passed over
+            vmax = fmaxf(vmax, v[u]);
+          }
+        }
+      }
+    } else {
+      span_pass(
+          [&](const Row &o, int r, int a, int b, int sp) {
+            if (a >= b) return;
+            constexpr int U = 2;
+            if (need_cv) {
+              const float *gp = Gp + r * nc + sp;
+              const float g[4] = {gp[0], gp[1], gp[2], gp[3]};
+              for (int z = a; z < b; z += U) {
+                float v[U], ed[U], y[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = z + u < b ? o.p[z + u] : kNaN;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                  ed[u] = dot4(W4[z + u], g);   // past the row: finite, not used
+                  y[u] = expm1_conv(-ed[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                  const bool in = !isnan(v[u]);
+                  const double yd = in ? (double)y[u] : 0.0;
+                  sy += yd;
+                  syy += yd * yd;
+                  if (apply) {
+                    v[u] = __fsub_rn(v[u], ed[u]);
+                    if (in) o.p[z + u] = v[u];
+                  }
+                  vmin = fminf(vmin, v[u]);   // a NaN operand is passed over
+                  vmax = fmaxf(vmax, v[u]);
+                }
+              }
+            } else {
+              for (int z = a; z < b; ++z) {
+                const float v = o.p[z];
+                vmin = fminf(vmin, v);
+                vmax = fmaxf(vmax, v);
+              }
+            }
+          });
+    }
     const bool ok = reduce_stats(vmin, vmax, sy, syy, need_cv, [&] {
       // the copies lie in the Gd region, which every thread has read by now
       unsigned *h = hist();

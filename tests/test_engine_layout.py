@@ -44,8 +44,9 @@ def engine(tmp_path_factory):
 
 def test_every_weight_read_lies_in_a_table_or_its_zero_tail(engine):
     """The z contraction reads the numerator weights and the denominator weights
-    in steps of 8 voxels (four lanes per span, from a start of at most Z - 1) or
-    of 2, 3 or 4 (one lane), pass A the cubic weights in steps of 2.  What a step
+    in steps of 8 voxels (four lanes per span, from a start of at most Z - 1), of
+    2, 3 or 4 (one lane) or of 2 that are 1, 2, 4 or 8 voxels apart (a span's
+    lanes on the whole-GPU path), pass A the cubic weights in steps of 2.  What a step
     holds past the row has to be one of the tables (filled for every voxel) or
     the zero entries behind them."""
     ask = [("axis", Z, nc, lv) for Z in range(1, 200) for nc, lv in ((4, 4), (5, 4), (11, 4), (19, 7), (64, 64))]
@@ -57,6 +58,7 @@ def test_every_weight_read_lies_in_a_table_or_its_zero_tail(engine):
         for start in range(Z):
             last.add(start + 7)                          # quad_rows: min(a + q, Z - 1) + 7
             last.update(start + u - 1 for u in (2, 3, 4))   # SpanSums::add
+            last.update(start + d for d in (1, 2, 4, 8))    # its lanes on the whole-GPU path
         reads = {o + 16 * z for o in (op, oq) for z in range(max(last) + 1)}
         reads |= {ow + 16 * z for z in range(Z + 1)}     # pass A
         assert reads <= written
