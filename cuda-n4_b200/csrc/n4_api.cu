@@ -1222,13 +1222,10 @@ n4_status_t run_volumes(n4_context *ctx, const n4_params_t *p, const std::vector
 n4_status_t collect_slot(n4_context *ctx, int slot, n4_report_t *out, int n);
 
 n4_status_t collect(n4_context *ctx, n4_report_t *out, int n) {
-  if (ctx->last_slot < 0) {
-    // component calls only: nothing to report, but their work is done
-    if (!ctx->any_done) return fail(N4_ERR_INVALID_ARG, "no run to synchronise with");
-    CK(cudaEventSynchronize(ctx->last_done));
-    return N4_OK;
-  }
-  return collect_slot(ctx, ctx->last_slot, out, n);
+  if (!ctx->any_done) return fail(N4_ERR_INVALID_ARG, "no run to synchronise with");
+  // the context's last work, a component call after the last run among it
+  CK(cudaEventSynchronize(ctx->last_done));
+  return ctx->last_slot < 0 ? N4_OK : collect_slot(ctx, ctx->last_slot, out, n);
 }
 
 n4_status_t collect_slot(n4_context *ctx, int slot, n4_report_t *out, int n) {

@@ -185,7 +185,8 @@ n4_status_t n4_run_batched_host(n4_context_t *ctx, const n4_params_t *p, int n,
 n4_status_t n4_run_batched(n4_context_t *ctx, const n4_params_t *p, int n,
                            const n4_volume_t *vols, void *stream, n4_report_t *reports);
 
-/* Wait for the context's last asynchronous run and fill its reports. */
+/* Wait for the context's last asynchronous call (a run, a fit, an evaluation)
+ * and fill the reports of its last run. */
 n4_status_t n4_sync(n4_context_t *ctx, n4_report_t *reports, int n);
 
 /* A batched run recorded once as a CUDA graph (no counterpart in the
