@@ -2326,6 +2326,7 @@ n4_status_t n4_sharpen_image(n4_context_t *ctx, const float *d_before, const flo
   };
   const int nbm = blocks(256, 8), nbh = blocks(512, 3), nbr = blocks(512, 3);
   const int vec = ((((uintptr_t)d_before | (uintptr_t)d_mask | (uintptr_t)d_after) & 15u) == 0) ? 1 : 0;
+  TRY(begin_run(ctx, st));   // a fit on another stream may still use the scratch
   TRY(ctx->s1.ensure((size_t)nbm * 8 + 64, "partials"));
   // histogram; residual table; then what the host reads: statistics and E
   const size_t o_r = align_up((size_t)bins * 8, 16), o_st = o_r + (size_t)bins * 16, o_e = o_st + 32,
@@ -2367,6 +2368,7 @@ n4_status_t n4_convergence(n4_context_t *ctx, const float *d_field1, const float
   if (!ctx || !d_field1 || !d_field2 || !cv || n == 0) return fail(N4_ERR_INVALID_ARG, "bad arguments");
   CK(cudaSetDevice(ctx->device));
   const int nb = std::min<int>((int)((n + 255) / 256), ctx->nsm * 4);
+  TRY(begin_run(ctx, nullptr));   // a fit on another stream may still use the scratch
   TRY(ctx->s1.ensure((size_t)nb * 24 + 32, "partials"));
   TRY(ensure_ticket(ctx));
   TRY(ensure_pinned(ctx, 24));

@@ -27,3 +27,34 @@ def test_sync_waits_for_a_component_call_after_a_run(cuda):
         _lib.check(_lib.load().n4_sync(ctx.handle, rep, 1))
         assert s.query()
     assert rep[0].status == 0 and rep[0].levels == 1
+
+
+@pytest.mark.parametrize("call", ["sharpen", "convergence"])
+def test_default_stream_calls_wait_for_a_fit_on_another_stream(cuda, call):
+    """A fit on a non-blocking stream keeps its row and plane sums in the scratch
+    that sharpening and the convergence value use on the default stream, which
+    does not wait for that stream by itself: the fit's lattice has the same bits
+    as alone, at every distance between the calls."""
+    import n4b200
+    from n4b200 import _lib
+    lib = _lib.load()
+    shape, nc = (256, 256, 200), (7, 7, 7)
+    field = cuda.rand(shape, device="cuda")
+    x = cuda.rand(4096, device="cuda")
+    y = cuda.rand(4096, device="cuda")
+    out = cuda.empty_like(x)
+    E, cv = np.zeros(200, np.float32), ctypes.c_double()
+    want = n4b200.FitBspline3D(field, None, nc)
+    cuda.cuda.synchronize()
+    ctx = n4b200.Context(0)
+    s = cuda.cuda.Stream()
+    for _ in range(20):
+        with cuda.cuda.stream(s):
+            got = n4b200.FitBspline3D(field, None, nc, ctx=ctx)
+        if call == "sharpen":
+            _lib.check(lib.n4_sharpen_image(ctx.handle, x.data_ptr(), None, 4096, 200, 0.01, 0.15, out.data_ptr(), None,
+                                            None, E.ctypes.data))
+        else:
+            _lib.check(lib.n4_convergence(ctx.handle, x.data_ptr(), y.data_ptr(), None, 4096, 0, ctypes.byref(cv)))
+        s.synchronize()
+        assert cuda.equal(got, want)
