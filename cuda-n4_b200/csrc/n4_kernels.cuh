@@ -1212,16 +1212,45 @@ __global__ void k_read_evict(const float4 *p, long long n, float *sink) {
 }
 
 // ------------------------------------------------------------------ standalone convergence
+// Voxels a thread takes at a time (their loads in flight together).  Bound by
+// the reads, and by the mask's where voxels in it and out of it alternate: 60
+// million voxels without a mask 124 us (3.9 TB/s), with 40 % of them at random
+// 197 us; one at a time 282 and 459, four 135 and 218.
+constexpr int kCvVoxels = 8;
+
 // Sums of y, y^2 and 1 over the masked voxels, y = exp(f1 - f2) - 1; the last
 // block adds the blocks' sums into sums[0..2].
 __global__ void __launch_bounds__(256) k_cv(const float *f1, const float *f2, const float *mask, long long n,
                                             double *part, double *sums, unsigned *ticket) {
   double s0 = 0.0, s1 = 0.0, c = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (mask && mask[i] == 0.0f) continue;
-    const double y = (double)expm1f(__fsub_rn(f1[i], f2[i]));
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  const auto add = [&](float a, float b) {
+    const double y = (double)expm1f(__fsub_rn(a, b));
     s0 += y; s1 += y * y; c += 1.0;
-  }
+  };
+  const auto sum = [&](auto masked) {
+    constexpr bool kMask = decltype(masked)::value;
+    constexpr int U = kCvVoxels;
+    long long i = first;
+    for (; i + (U - 1) * stride < n; i += U * stride) {
+      float a[U], b[U];
+      bool on[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) on[u] = !kMask || mask[i + u * stride] != 0.0f;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        a[u] = on[u] ? f1[i + u * stride] : 0.0f;
+        b[u] = on[u] ? f2[i + u * stride] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (on[u]) add(a[u], b[u]);
+    }
+    for (; i < n; i += stride)
+      if (!kMask || mask[i] != 0.0f) add(f1[i], f2[i]);
+  };
+  if (mask) sum(std::true_type());
+  else sum(std::false_type());
   __shared__ double ws[3][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const auto block_sum = [&](double *out) {
