@@ -307,10 +307,16 @@ Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool 
   if (grid) {
     // Gd: 24 KB hold the rows of a CTA's share of a 256x256x160 grid (280 of
     // 11 control points); T2 of six 11x11 planes; both fall back to global
-    // memory.  The row list and the volume take the rest.
+    // memory.  The row list and the volume take the rest.  Beside a lattice
+    // that leaves no room for them only the work buffers of the sharpening
+    // remain of them.
     pl.gd_bytes = (int)align_up(std::max<size_t>(alias_bytes, 24 << 10), 128);
-    pl.o_gd = take(pl.gd_bytes);
     pl.t2_bytes = 4 << 10;
+    if ((long long)o + pl.gd_bytes + 2 * pl.t2_bytes + 128 > max_smem - kStaticSmemReserve) {
+      pl.gd_bytes = (int)align_up(alias_bytes, 16);
+      pl.t2_bytes = 0;
+    }
+    pl.o_gd = take(pl.gd_bytes);
     pl.o_t2 = take(pl.t2_bytes);
     pl.o_ytab = take(pl.t2_bytes);
     o = align_up(o, 128);

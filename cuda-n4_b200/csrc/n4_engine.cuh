@@ -1466,7 +1466,8 @@ struct Engine {
         *slotB() = (unsigned long long)weight;
       }
       if (!g.sync()) return false;
-      long long *prefix = at<long long>(pl.o_gd);   // K + 1 words, free before the first level
+      // K + 1 words, in the five lattices (1280 bytes at least), free before the first level
+      long long *prefix = at<long long>(pl.o_L);
       for (int k = threadIdx.x; k < K; k += blockDim.x) prefix[k + 1] = (long long)__ldcg(g.peer(slotB(), k));
       __syncthreads();
       if (threadIdx.x == 0) {

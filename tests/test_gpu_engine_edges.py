@@ -135,3 +135,23 @@ def test_control_points_almost_without_voxels(cuda, flags, eps, force):
                     ConvergenceThreshold=0.0, fit_eps=eps, fit_zero_den=bool(flags & 2))
     assert res.report["status"] == "N4_OK"
     assert nrel(res.lattice, lat) < 1e-5 and nrel(res.im_normalized, out) < 1e-5
+
+
+@pytest.mark.parametrize("shape,nc,levels,bins", [
+    ((117, 27, 18), (22, 20, 20), 1, 200),   # 176 KB of lattices in shared memory
+    ((90, 60, 24), (7, 6, 4), 4, 32),        # 35 x 27 x 11 control points, 208 KB
+])
+def test_lattices_that_fill_the_shared_memory(cuda, shape, nc, levels, bins):
+    """A lattice beside which the whole-GPU path has no room for its row and
+    plane buffers in shared memory runs with them in global memory."""
+    import n4b200
+    im = log_volume(shape, 5)
+    p = n4b200.N4Param(NumberOfFittingLevels=levels, MaximumNumberOfIterations=[2] * levels, ConvergenceThreshold=0.0,
+                       low_value=0.0, flags=0x8, NumberOfControlPoints_x=nc[0], NumberOfControlPoints_y=nc[1],
+                       NumberOfControlPoints_z=nc[2], NumberOfHistogramBins=bins)
+    res = n4b200.N4(cuda.tensor(im, device="cuda"), None, p)
+    out, lat = O.N4(im, np.ones(shape, np.float32), low_value=0, maximumNumberOfLevels=levels,
+                    maximumNumberOfIterations=[2] * levels, ConvergenceThreshold=0.0, numberOfControlPoints=nc,
+                    numberOfHistogramBins=bins)
+    assert res.report["status"] == "N4_OK" and res.report["path"] == "grid"
+    assert nrel(res.lattice, lat) < TOL and nrel(res.im_normalized, out) < TOL
