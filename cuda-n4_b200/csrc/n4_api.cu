@@ -244,9 +244,10 @@ Params make_dev_params(const n4_params_t *p) {
 }
 
 // Workspace layout for a group of K CTAs over the given fitting grids;
-// max_smem: shared memory per CTA (whole-GPU path, whose volume takes what is
-// left beside the tables).
-Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool grid, int max_smem = 0) {
+// max_smem: shared memory per CTA (the whole-GPU path's volume takes what is
+// left beside the tables; a cluster the caller asks for works without its row
+// lists where they do not fit).
+Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool grid, int max_smem) {
   Plan pl{};
   pl.levels = (int)p->NumberOfFittingLevels;
   pl.nc0x = (int)p->NumberOfControlPoints_x;
@@ -324,7 +325,9 @@ Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool 
     const long long rest = (long long)max_smem - kStaticSmemReserve - (long long)o;
     pl.pool_bytes = (int)std::max<long long>(0, rest / 128 * 128);
     o += pl.pool_bytes;
-  } else {
+  }
+  const size_t o_lists = o;
+  if (!grid) {
     pl.o_rows = take((size_t)pl.rows_max * 8);
     pl.o_ytab = take(yt);
   }
@@ -343,6 +346,15 @@ Plan make_plan(const n4_params_t *p, int K, const std::vector<Dims> &vols, bool 
     pl.b_slotC = take((size_t)pl.NLAT * 4);
   }
   pl.big_bytes = (int)align_up(o, 128);
+  // Rows of a few voxels: 8 bytes of list per row are much of what the row has
+  // (172x172x16 on 16 CTAs).  Where the path is ours to choose such a volume
+  // takes the whole GPU (0.66 ms for 3 levels of 6 iterations against 1.79 on
+  // a cluster without lists before there were any).
+  const bool asked = ((p->flags >> 8) & 31u) != 0 || (p->flags & N4_FLAG_FORCE_CLUSTER);
+  if (!grid && asked && (long long)pl.sm_bytes + pl.big_bytes + kStaticSmemReserve > max_smem) {
+    pl.whole_rows = 1;
+    pl.sm_bytes = (int)align_up(o_lists, 128);
+  }
   return pl;
 }
 
@@ -355,26 +367,26 @@ bool cluster_fits(const n4_context *ctx, const Plan &pl) {
 // record is process-wide too and the grant only ever grows.
 constexpr int kMaxDev = 64;
 std::mutex g_attr_mu;
-int g_attr_smem[kMaxDev][3];   // per thread count: 512, 768, 1024
+int g_attr_smem[kMaxDev][4];   // per thread count: 512, 768, 1024; 512 without row lists
 
-template <int NT>
+template <int NT, bool kListed>
 n4_status_t grant_cluster_smem(n4_context *ctx, int smem) {
   static_assert(NT == 512 || NT == 768 || NT == 1024, "engine thread counts");
   if (ctx->device < 0 || ctx->device >= kMaxDev) return fail(N4_ERR_INVALID_ARG, "device ordinal out of range");
   std::lock_guard<std::mutex> lock(g_attr_mu);
-  int &granted = g_attr_smem[ctx->device][NT == 512 ? 0 : (NT == 768 ? 1 : 2)];
+  int &granted = g_attr_smem[ctx->device][!kListed ? 3 : (NT == 512 ? 0 : (NT == 768 ? 1 : 2))];
   if (smem > granted) {
-    CK(cudaFuncSetAttribute(k_n4_cluster<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CK(cudaFuncSetAttribute(k_n4_cluster<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    CK(cudaFuncSetAttribute(k_n4_cluster<NT, kListed>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CK(cudaFuncSetAttribute(k_n4_cluster<NT, kListed>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     granted = smem;
   }
   return N4_OK;
 }
 
-template <int NT>
+template <int NT, bool kListed>
 n4_status_t cluster_capacity(n4_context *ctx, int K, int smem, int *nclusters) {
-  auto kern = k_n4_cluster<NT>;
-  TRY(grant_cluster_smem<NT>(ctx, smem));
+  auto kern = k_n4_cluster<NT, kListed>;
+  TRY((grant_cluster_smem<NT, kListed>(ctx, smem)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(K);
   cfg.blockDim = dim3(NT);
@@ -392,12 +404,16 @@ n4_status_t cluster_capacity(n4_context *ctx, int K, int smem, int *nclusters) {
   return N4_OK;
 }
 
-n4_status_t capacity(n4_context *ctx, int nt, int K, int smem, int *n) {
-  const auto key = std::make_tuple(nt, K, smem);
+// Clusters of K CTAs of nt threads with layout `pl` that fit at once.
+n4_status_t capacity(n4_context *ctx, int nt, int K, const Plan &pl, int *n) {
+  const int smem = pl.sm_bytes + pl.big_bytes;
+  const auto key = std::make_tuple(pl.whole_rows ? 0 : nt, K, smem);
   auto it = ctx->cluster_cap.find(key);
   if (it != ctx->cluster_cap.end()) { *n = it->second; return N4_OK; }
-  TRY(nt == 1024 ? cluster_capacity<1024>(ctx, K, smem, n)
-                  : nt == 768 ? cluster_capacity<768>(ctx, K, smem, n) : cluster_capacity<512>(ctx, K, smem, n));
+  if (pl.whole_rows) TRY((cluster_capacity<512, false>(ctx, K, smem, n)));
+  else if (nt == 1024) TRY((cluster_capacity<1024, true>(ctx, K, smem, n)));
+  else if (nt == 768) TRY((cluster_capacity<768, true>(ctx, K, smem, n)));
+  else TRY((cluster_capacity<512, true>(ctx, K, smem, n)));
   ctx->cluster_cap[key] = *n;
   return N4_OK;
 }
@@ -407,10 +423,10 @@ n4_status_t choose_cluster(n4_context *ctx, const n4_params_t *p, const std::vec
                            int *K_out) {
   *K_out = 0;
   for (int K : {16, 12, 8, 6, 4, 2, 1}) {
-    Plan pl = make_plan(p, K, vols, false);
+    Plan pl = make_plan(p, K, vols, false, ctx->max_smem);
     if (!cluster_fits(ctx, pl)) continue;
     int n = 0;
-    TRY(capacity(ctx, nt, K, pl.sm_bytes + pl.big_bytes, &n));
+    TRY(capacity(ctx, nt, K, pl, &n));
     if (n > 0) { *K_out = K; return N4_OK; }
   }
   return N4_OK;
@@ -429,7 +445,7 @@ std::vector<int> cluster_subset(const n4_context *ctx, const n4_params_t *p, con
   std::vector<Dims> sub;
   for (int i : order) {
     sub.push_back(dims[i]);
-    if (cluster_fits(ctx, make_plan(p, K, sub, false))) {
+    if (cluster_fits(ctx, make_plan(p, K, sub, false, ctx->max_smem))) {
       fit.push_back(i);
     } else {
       sub.pop_back();
@@ -574,11 +590,11 @@ n4_status_t launch_grid_path(n4_context *ctx, const n4_params_t *p, const Params
   return launch_grid_kernel<512>(a, nblk, smem, st);
 }
 
-template <int NT>
+template <int NT, bool kListed>
 n4_status_t launch_cluster_kernel(n4_context *ctx, const ClusterArgs &a, int K, int nclusters, int smem,
                                   cudaStream_t st) {
-  auto kern = k_n4_cluster<NT>;
-  TRY(grant_cluster_smem<NT>(ctx, smem));
+  auto kern = k_n4_cluster<NT, kListed>;
+  TRY((grant_cluster_smem<NT, kListed>(ctx, smem)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(K * nclusters);
   cfg.blockDim = dim3(NT);
@@ -642,9 +658,9 @@ n4_status_t choose_path(n4_context *ctx, const n4_params_t *p, const std::vector
   const int forced_k = (int)((p->flags >> 8) & 31u);
   if (forced_k) {
     if (p->flags & N4_FLAG_FORCE_GRID) return fail(N4_ERR_INVALID_ARG, "cluster size given with FORCE_GRID");
-    Plan pl = make_plan(p, forced_k, vols, false);
+    Plan pl = make_plan(p, forced_k, vols, false, ctx->max_smem);
     int cap = 0;
-    if (cluster_fits(ctx, pl)) TRY(capacity(ctx, c.nt, forced_k, pl.sm_bytes + pl.big_bytes, &cap));
+    if (cluster_fits(ctx, pl)) TRY(capacity(ctx, c.nt, forced_k, pl, &cap));
     if (cap < 1) return fail(N4_ERR_TOO_LARGE, "a volume does not fit a cluster of the requested size");
     c.K = forced_k;
     return N4_OK;
@@ -753,9 +769,9 @@ n4_status_t plan_run(n4_context *ctx, const n4_params_t *p, const std::vector<Ru
     if (!P.in_cluster.empty()) {
       std::vector<Dims> sub;
       for (int i : P.in_cluster) sub.push_back(dims[i]);
-      const Plan pl = make_plan(p, 16, sub, false);
+      const Plan pl = make_plan(p, 16, sub, false, ctx->max_smem);
       int cap = 0;
-      TRY(capacity(ctx, 512, 16, pl.sm_bytes + pl.big_bytes, &cap));
+      TRY(capacity(ctx, 512, 16, pl, &cap));
       if (cap > 0) {
         ch.grid = false;
         ch.nt = 512;
@@ -792,9 +808,9 @@ n4_status_t plan_run(n4_context *ctx, const n4_params_t *p, const std::vector<Ru
   if (P.in_grid.empty() && n > 1 && want_sub != 1) {
     int S = want_sub ? want_sub : ch.nsub;
     if (S == 0) {
-      const Plan pl = make_plan(p, ch.K, dims, false);
+      const Plan pl = make_plan(p, ch.K, dims, false, ctx->max_smem);
       int cap = 0;
-      TRY(capacity(ctx, ch.nt, ch.K, pl.sm_bytes + pl.big_bytes, &cap));
+      TRY(capacity(ctx, ch.nt, ch.K, pl, &cap));
       S = cap > 0 ? n / (2 * cap) : 1;
       if (cap > 0 && n > cap && !enc) S = std::max(S, 2);
     }
@@ -829,9 +845,9 @@ n4_status_t plan_run(n4_context *ctx, const n4_params_t *p, const std::vector<Ru
       int Kk = 0;
       for (int K : {2, 4, 6, 8, 12, 16}) {
         if (K < ch.adapt) continue;
-        const Plan pl = make_plan(p, K, sub, false);
+        const Plan pl = make_plan(p, K, sub, false, ctx->max_smem);
         int cap = 0;
-        if (cluster_fits(ctx, pl)) TRY(capacity(ctx, ch.nt, K, pl.sm_bytes + pl.big_bytes, &cap));
+        if (cluster_fits(ctx, pl)) TRY(capacity(ctx, ch.nt, K, pl, &cap));
         if (cap > 0) { Kk = K; break; }
       }
       P.subK.push_back(Kk > 0 ? Kk : ch.K);
@@ -984,10 +1000,10 @@ n4_status_t launch_engine(n4_context *ctx, const n4_params_t *p, const Prepared 
   } else {
     for (int i : P.in_cluster) sub.push_back(P.dims[i]);
   }
-  Plan pl = make_plan(p, K, sub, false);
+  Plan pl = make_plan(p, K, sub, false, ctx->max_smem);
   const int smem = pl.sm_bytes + pl.big_bytes;
   int cap = 0;
-  TRY(capacity(ctx, P.ch.nt, K, smem, &cap));
+  TRY(capacity(ctx, P.ch.nt, K, pl, &cap));
   if (cap < 1) return fail(N4_ERR_TOO_LARGE, "no cluster of this size fits on the device");
   ClusterArgs a{};
   a.pl = pl;
@@ -998,9 +1014,10 @@ n4_status_t launch_engine(n4_context *ctx, const n4_params_t *p, const Prepared 
   a.queue = B.dp<int>(P.o_q) + 4 * q;
   a.use_tma = 1;
   const int ncl = std::min<int>(cap, njobs);
-  if (P.ch.nt == 1024) TRY(launch_cluster_kernel<1024>(ctx, a, K, ncl, smem, st));
-  else if (P.ch.nt == 768) TRY(launch_cluster_kernel<768>(ctx, a, K, ncl, smem, st));
-  else TRY(launch_cluster_kernel<512>(ctx, a, K, ncl, smem, st));
+  if (pl.whole_rows) TRY((launch_cluster_kernel<512, false>(ctx, a, K, ncl, smem, st)));
+  else if (P.ch.nt == 1024) TRY((launch_cluster_kernel<1024, true>(ctx, a, K, ncl, smem, st)));
+  else if (P.ch.nt == 768) TRY((launch_cluster_kernel<768, true>(ctx, a, K, ncl, smem, st)));
+  else TRY((launch_cluster_kernel<512, true>(ctx, a, K, ncl, smem, st)));
   return N4_OK;
 }
 
@@ -1541,10 +1558,10 @@ n4_status_t n4_autotune(n4_context_t *ctx, const n4_params_t *p, int n, const n4
     if (fit.empty() || fit.size() < most) continue;
     std::vector<Dims> sub;
     for (int i : fit) sub.push_back(dims[i]);
-    Plan pl = make_plan(p, K, sub, false);
+    Plan pl = make_plan(p, K, sub, false, ctx->max_smem);
     for (int nt : {1024, 768, 512}) {
       int cap = 0;
-      TRY(capacity(ctx, nt, K, pl.sm_bytes + pl.big_bytes, &cap));
+      TRY(capacity(ctx, nt, K, pl, &cap));
       if (cap > 0) cand.push_back(Choice{false, K, nt});
     }
   }

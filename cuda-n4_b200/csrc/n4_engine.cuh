@@ -100,6 +100,7 @@ __host__ __device__ inline EAxis eaxis_at(int off, int n, int nc, int tail = 0) 
 // "b_" offsets in dynamic shared memory behind sm_bytes (cluster path) or in
 // a per-CTA slice of global memory (whole-GPU path).
 struct Plan {
+  int whole_rows;      // cluster path without row lists
   // limits
   int levels, nc0x, nc0y, nc0z, NCX, NCY, NCZ, NLAT;
   int Xmax, Ymax, Zmax, slab_floats, rows_max, nvxl;
@@ -164,6 +165,10 @@ struct Iter {
 static_assert(sizeof(Iter) <= (160 - 144) * 8, "Iter lies in the o_red words behind the scratch");
 
 // ------------------------------------------------------------------ groups
+// kListed: the CTA's rows are listed in shared memory; else it works on all rows
+// of its planes from end to end (volumes of short rows whose list would not fit,
+// where the caller asks for the cluster path).
+template <bool kListed>
 struct ClusterGroup {
   __device__ int rank() const { return (int)cg::this_cluster().block_rank(); }
   __device__ int size() const { return (int)cg::this_cluster().num_blocks(); }
@@ -171,7 +176,7 @@ struct ClusterGroup {
   template <class T> __device__ const T *peer(const T *p, int r) const {
     return cg::this_cluster().map_shared_rank(const_cast<T *>(p), r);
   }
-  static constexpr bool kGrid = false;
+  static constexpr bool kGrid = false, kRowList = kListed;
 };
 
 // Accumulators of the whole-GPU path in global memory, zero at launch: three
@@ -192,7 +197,7 @@ struct GridGroup {
     const char *mine = big_base + (size_t)blockIdx.x * big_stride;
     return (const T *)(big_base + (size_t)r * big_stride + ((const char *)p - mine));
   }
-  static constexpr bool kGrid = true;
+  static constexpr bool kGrid = true, kRowList = true;
 };
 
 // ------------------------------------------------------------------ phase timers
@@ -320,6 +325,16 @@ struct Engine {
     }
     __device__ __forceinline__ int vy(int r) const { return (int)(at<uint2>(rows)[r].y & 0xffffu); }
   };
+  struct WholeRows {
+    int slab, Y, Z;         // byte offset of the slab
+    __device__ __forceinline__ Row operator()(int r) const {
+      Row o;
+      o.z0 = 0; o.z1 = Z; o.m = r / Y; o.vy = r - o.m * Y;
+      o.p = at<float>(slab) + r * Z;
+      return o;
+    }
+    __device__ __forceinline__ int vy(int r) const { return r % Y; }
+  };
   struct GridRows {
     const int4 *rows;
     int slab, cap;          // byte offset of the shared slab, its floats
@@ -335,7 +350,8 @@ struct Engine {
   };
   __device__ __forceinline__ auto row_map() const {
     if constexpr (Group::kGrid) return GridRows{rowsp, slab_off, slab_cap, slab_g};
-    else return ClusterRows{pl.o_rows, pl.sm_bytes + pl.b_imlog, Y, Z};
+    else if constexpr (Group::kRowList) return ClusterRows{pl.o_rows, pl.sm_bytes + pl.b_imlog, Y, Z};
+    else return WholeRows{pl.sm_bytes + pl.b_imlog, Y, Z};
   }
   __device__ __forceinline__ int plane_vx(int m) const { return Group::kGrid ? vx0 + m : rank + m * K; }
   __device__ __forceinline__ const float *src_row(const Row &r) const {
@@ -401,7 +417,8 @@ struct Engine {
     }
     if (threadIdx.x < kWeightTail) at<float4>(az.o_tail)[threadIdx.x] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     __syncthreads();
-    if (np <= tp) build_ytab(0, np);
+    if constexpr (Group::kRowList)
+      if (np <= tp) build_ytab(0, np);
     __syncthreads();
   }
 
@@ -1040,6 +1057,11 @@ struct Engine {
     const int nc = ncz, ny = ncy, nsp = ay.nsp, n = cnt * ny * nc, w = nsp + 1;
     const auto rm = row_map();
     const int *Lo = at<int>(ay.o_lo), *Hi = at<int>(ay.o_hi);
+    const int yy = Y;
+    const auto first_row = [=](int m, int sp) {   // of span sp in plane m
+      if constexpr (Group::kRowList) return yt[m * w + sp];
+      else return m * yy + (sp < nsp ? Lo[sp] : yy);
+    };
     if constexpr (!Group::kGrid) {
       if (nsp < 4 || n > 512) {
       // one thread per (plane, cz): spans from the last to the first, the four
@@ -1050,7 +1072,7 @@ struct Engine {
         KahanSum a[4], b[4];   // target sp + j: rows at even and at odd distance
         for (int sp = nsp - 1; sp >= 0; --sp) {
           const int lo = Lo[sp], hi = Hi[sp];
-          const int r0 = yt[m * w + sp], k = yt[m * w + sp + 1] - r0;
+          const int r0 = first_row(m, sp), k = first_row(m, sp + 1) - r0;
           const int va = k > 0 ? rm.vy(r0) : hi, vb = va + k;
           if (va > lo) {
 #pragma unroll
@@ -1102,7 +1124,7 @@ struct Engine {
           const int sp = cy - j;
           if (sp < 0 || sp >= nsp) continue;
           const int lo = Lo[sp], hi = Hi[sp];
-          const int r0 = yt[m * w + sp], r1 = yt[m * w + sp + 1];
+          const int r0 = first_row(m, sp), r1 = first_row(m, sp + 1);
           const int va = r0 < r1 ? rm.vy(r0) : hi, vb = va + (r1 - r0);
           if (va > lo) acc.add(0.0f);
           if (va > lo + 1) acc2.add(0.0f);
@@ -1138,8 +1160,8 @@ struct Engine {
       double s = 0.0;
       if (u < n && sp >= 0 && sp < nsp) {
         KahanSum acc, acc2;
-        int r = yt[m * w + sp];
-        const int end = yt[m * w + sp + 1];
+        int r = first_row(m, sp);
+        const int end = first_row(m, sp + 1);
         for (; r + 1 < end; r += 2) {
           acc.add_prod(PY[rm.vy(r) * 4 + j], T1[r * nc + cz]);
           acc2.add_prod(PY[rm.vy(r + 1) * 4 + j], T1[(r + 1) * nc + cz]);
@@ -1522,27 +1544,30 @@ struct Engine {
         if (lane == 0) ext[i] = e;
         cnt += n;
       }
-      // a plane's rows are listed from its first to its last row with a masked
-      // voxel, empty ones between them as the empty range [1, 1)
-      int *ya = at<int>(pl.sm_bytes + pl.b_T2), *yb = ya + nplane;
-      for (int m = threadIdx.x; m < nplane; m += blockDim.x) { ya[m] = Y; yb[m] = -1; }
-      __syncthreads();
-      const int yy = Y;
-      for (int i = threadIdx.x; i < nrow; i += blockDim.x)
-        if (ext[i]) {
-          atomicMin(&ya[i / yy], i % yy);
-          atomicMax(&yb[i / yy], i % yy);
-        }
-      __syncthreads();
-      uint2 *out = at<uint2>(pl.o_rows);
-      auto range = [=](int i) {
-        const unsigned e = ext[i];
-        return e || i % yy < ya[i / yy] || i % yy > yb[i / yy] ? e : 0x10001u;
-      };
-      rows = list_rows(nrow, range, [=](int r, int, int i, unsigned e) {
-        const int m = i / yy;
-        out[r] = make_uint2(e, (unsigned)m << 16 | (unsigned)(i - m * yy));
-      });
+      rows = nrow;
+      if constexpr (Group::kRowList) {
+        // a plane's rows are listed from its first to its last row with a masked
+        // voxel, empty ones between them as the empty range [1, 1)
+        int *ya = at<int>(pl.sm_bytes + pl.b_T2), *yb = ya + nplane;
+        for (int m = threadIdx.x; m < nplane; m += blockDim.x) { ya[m] = Y; yb[m] = -1; }
+        __syncthreads();
+        const int yy = Y;
+        for (int i = threadIdx.x; i < nrow; i += blockDim.x)
+          if (ext[i]) {
+            atomicMin(&ya[i / yy], i % yy);
+            atomicMax(&yb[i / yy], i % yy);
+          }
+        __syncthreads();
+        uint2 *out = at<uint2>(pl.o_rows);
+        auto range = [=](int i) {
+          const unsigned e = ext[i];
+          return e || i % yy < ya[i / yy] || i % yy > yb[i / yy] ? e : 0x10001u;
+        };
+        rows = list_rows(nrow, range, [=](int r, int, int i, unsigned e) {
+          const int m = i / yy;
+          out[r] = make_uint2(e, (unsigned)m << 16 | (unsigned)(i - m * yy));
+        });
+      }
       nact = rows;
       np = nplane;
       vx0 = 0;
@@ -1556,8 +1581,15 @@ struct Engine {
     const int rs = 5 - row_lanes_log2(Z);
     const auto rm = row_map();
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-      const Row o = rm(r);
-      atomicAdd(&copies[(r >> rs) % kHistCopies], o.z1 - o.z0);
+      int len;
+      if constexpr (Group::kRowList) {
+        const Row o = rm(r);
+        len = o.z1 - o.z0;
+      } else {
+        const unsigned e = at<unsigned>(pl.sm_bytes + pl.b_Gd)[r];
+        len = (int)(e >> 16) - (int)(e & 0xffffu);
+      }
+      atomicAdd(&copies[(r >> rs) % kHistCopies], len);
     }
     __syncthreads();
     int most = 0;

@@ -274,7 +274,7 @@ struct ClusterArgs {
   int use_tma;
 };
 
-template <int NT>
+template <int NT, bool kListed>
 __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ ClusterArgs a) {
   extern __shared__ __align__(128) char smem[];
   __shared__ Plan s_pl;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ Cl
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  ClusterGroup g;
+  ClusterGroup<kListed> g;
   unsigned phase = 0;
   for (;;) {
     if (g.rank() == 0 && threadIdx.x == 0) s_job = atomicAdd(a.queue, 1);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(NT, 1) k_n4_cluster(const __grid_constant__ Cl
       if (!ok) mbar_wait(&s_mbar, phase ^ 1u);
       break;
     }
-    Engine<ClusterGroup> e(g, s_pl, s_pr, nullptr);
+    Engine<ClusterGroup<kListed>> e(g, s_pl, s_pr, nullptr);
     e.run(job);   // the slab holds the staged rows
   }
 }

@@ -155,3 +155,22 @@ def test_lattices_that_fill_the_shared_memory(cuda, shape, nc, levels, bins):
                     numberOfHistogramBins=bins)
     assert res.report["status"] == "N4_OK" and res.report["path"] == "grid"
     assert nrel(res.lattice, lat) < TOL and nrel(res.im_normalized, out) < TOL
+
+
+@pytest.mark.parametrize("shape,levels,k", [((28, 152, 17), 2, 2), ((220, 220, 6), 3, 16), ((320, 320, 1), 1, 16)])
+@pytest.mark.parametrize("kind", ["full", "holes"])
+def test_forced_clusters_of_short_rows(cuda, shape, levels, k, kind):
+    """Volumes of short rows that fit a cluster of the requested size only
+    without the list of their rows."""
+    im = log_volume(shape, 5)
+    m = np.ones(shape, np.float32)
+    if kind == "holes":
+        m = (np.random.default_rng(7).random(shape) < 0.5).astype(np.float32)
+        m[:, 20:25] = 0
+        m[3] = 0
+    for flags in (k << 8, 0x10) if k == 16 else (k << 8,):
+        res = run(cuda, im, m, levels, [2] * levels, flags=flags)
+        out, lat = O.N4(im, m, low_value=0, maximumNumberOfLevels=levels, maximumNumberOfIterations=[2] * levels,
+                        ConvergenceThreshold=0.0)
+        assert res.report["status"] == "N4_OK" and res.report["path"] == "cluster" and res.report["cluster_size"] == k
+        assert nrel(res.lattice, lat) < TOL and nrel(res.im_normalized, out) < TOL
