@@ -3,6 +3,7 @@ program that includes csrc/n4_engine.cuh prints what its functions return."""
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 from conftest import ROOT
@@ -21,6 +22,9 @@ int main(int argc, char **argv) {
       const n4::EAxis e = n4::eaxis_at(0, (int)a, (int)c, n4::kWeightTail);
       std::printf("%d %d %d %d %d %d %d %d %zu\n", e.o_w, e.o_p, e.o_q, e.o_tail, e.o_s, e.o_lo, e.o_hi,
                   n4::kWeightTail, n4::eaxis_bytes((int)a, (int)b - 3, n4::kWeightTail));
+    } else if (!std::strcmp(what, "share")) {   // rows, voxels of a row, CTAs
+      std::printf("%d %lld %lld\n", n4::grid_row_overhead((int)b), n4::grid_rows_bound(a, (int)b, (int)c),
+                  n4::grid_voxels_bound(a, (int)b, (int)c));
     }
   }
 }
@@ -63,3 +67,45 @@ def test_every_weight_read_lies_in_a_table_or_its_zero_tail(engine):
         reads |= {ow + 16 * z for z in range(Z + 1)}     # pass A
         assert reads <= written
         assert max(written) + 16 <= os_ and os_ + 4 * Z <= olo and olo + 4 * (lv - 3) == ohi and ohi + 4 * (lv - 3) <= size
+
+
+def shares(lens, K, c):
+    """First row of each CTA's share, as the whole-GPU path deals rows out whose
+    masked ranges are `lens` voxels long (0: none): a row weighs its range and c,
+    the CTAs add up even shares of the rows, and a CTA's share begins at the
+    first row with its part of the total before it."""
+    w = np.where(lens > 0, lens + c, 0).astype(np.int64)
+    n = w.size
+    cut = [n * k // K for k in range(K + 1)]
+    before = np.concatenate(([0], np.cumsum(w)))
+
+    def boundary(target):
+        k = max(q for q in range(K) if before[cut[q]] <= target)
+        rows = np.arange(cut[k], cut[k + 1])
+        hit = rows[before[rows] >= target]
+        return int(hit[0]) if hit.size else cut[k + 1]
+
+    return [boundary(int(before[-1]) * r // K) for r in range(K)] + [n], w
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_shares_of_the_rows_lie_within_their_buffers(engine, seed):
+    """The row list and the slab of a CTA are sized by grid_rows_bound and
+    grid_voxels_bound of the code and filled without further checks."""
+    rng = np.random.default_rng(seed)
+    Z = int(rng.choice([1, 2, 5, 31, 32, 33, 60, 160, 181, 700, 1024]))
+    n, K = int(rng.integers(1, 4000)), int(rng.choice([1, 7, 148]))
+    lens = rng.integers(0, Z + 1, n)
+    kind = seed % 4
+    if kind == 1:
+        lens[rng.random(n) < 0.95] = 0
+    if kind == 2:
+        lens = np.where(rng.random(n) < 0.5, 1, Z)              # short rows beside full ones
+    if kind == 3:
+        lens = np.where(np.arange(n) < n // 2, 1, Z)            # all short ones first
+    ((c, rows_bound, voxels_bound),) = engine([("share", n, Z, K)])
+    b, w = shares(lens, K, c)
+    assert not w[:b[0]].any() and all(x <= y for x, y in zip(b, b[1:]))   # every row once
+    for r in range(K):
+        part = lens[b[r]:b[r + 1]]
+        assert (part > 0).sum() <= rows_bound and part.sum() <= voxels_bound
