@@ -228,3 +228,21 @@ def test_encoder_gradients_of_ragged_batches(cuda, batch):
         g, r = got[at:at + k], ref[at:at + k]
         assert np.abs(g - r).max() <= 2e-2 * np.abs(r).max(), name
         at += k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(40, 30, 4), (40, 30, 44), (20, 30, 92), (20, 30, 108), (12, 9, 1020)])
+def test_fit_rows_on_16_byte_boundaries(cuda, shape):
+    """Rows of 4 k voxels, k odd: steps of 4 voxels or of 8 from any offset, by
+    their length; bitwise the same as off the boundary, and the oracle's."""
+    import n4b200
+    rng = np.random.default_rng(33)
+    n, nc = int(np.prod(shape)), (5, 4, 6)
+    f, m = rng.normal(0, 0.3, n).astype(np.float32), (rng.random(n) < 0.6).astype(np.float32)
+    lats = []
+    for off in (0, 4, 1):
+        fb, mb = cuda.zeros(n + 8, device="cuda"), cuda.zeros(n + 8, device="cuda")
+        fb[off:off + n], mb[off:off + n] = cuda.tensor(f, device="cuda"), cuda.tensor(m, device="cuda")
+        lats.append(n4b200.FitBspline3D(fb[off:off + n].view(shape), mb[off:off + n].view(shape), nc))
+    assert cuda.equal(lats[0], lats[1]) and cuda.equal(lats[0], lats[2])
+    assert nrel(lats[0], O.FitBspline3D(f.reshape(shape).astype(np.float64), m.reshape(shape), nc)) < 1e-5
