@@ -17,7 +17,6 @@
 
 namespace n4 {
 
-constexpr int kMaxThreads = 1024;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kHistCopies = 8;                   // shared histogram copies per CTA
 constexpr int kHistMaxShift = 24;                // fixed-point weight 2^shift, shift <= 24
@@ -155,10 +154,6 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 __device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_sumf(float v) {
   for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
   return v;
 }

@@ -986,9 +986,10 @@ struct Engine {
   // The z contraction with four lanes per (row, span): each forms the terms of
   // every fourth voxel, then, in voxel order, the sum of one of the span's four
   // targets.  The same sums as one lane per (row, span), with four times the
-  // lanes, for CTAs whose (row, span)s are half their threads or fewer (16
-  // CTAs, 64x64x48, 152 rows of one span: 7.8k cycles per iteration against
-  // 10.5k; 304 (row, span)s: 8.3k against 7.7k).
+  // lanes, for CTAs of 256 (row, span)s or fewer, half of the cluster path's
+  // default 512 threads, with which the line was drawn (16 CTAs, 64x64x48, 152
+  // rows of one span: 7.8k cycles per iteration against 10.5k; 304 (row, span)s:
+  // 8.3k against 7.7k).
   static constexpr int kQuadLanes = 256;
   template <bool Num>
   __device__ __forceinline__ void quad_rows(float *T1, bool degenerate) const {
@@ -1042,13 +1043,13 @@ struct Engine {
   // entry (rows at even and at odd distance from the span's start); rows before
   // and after the plane's listed ones add zeros, which a chain need take only
   // once.  One thread per entry over its four spans where there are at least
-  // four and the entries are one round of the CTA; else one thread per (plane,
-  // cz) that walks the plane once for all its entries (per iteration, 16 CTAs,
-  // 64x64x48: 1 span 4.1k cycles against 6.4k, 8 spans 6.9k against 4.4k; 6
-  // CTAs, 64x64x44: 4.7k against 8.0k and 8.3k against 11.2k).  Same terms in
-  // the same order either way.  Whole-GPU path, whose
-  // CTAs hold two or three planes: one lane per span, the four sums added in
-  // FP64.
+  // four and the entries are no more than the default 512 threads, with which
+  // the line was drawn; else one thread per (plane, cz) that walks the plane
+  // once for all its entries (per iteration, 16 CTAs, 64x64x48: 1 span 4.1k
+  // cycles against 6.4k, 8 spans 6.9k against 4.4k; 6 CTAs, 64x64x44: 4.7k
+  // against 8.0k and 8.3k against 11.2k).  Same terms in the same order either
+  // way.  Whole-GPU path, whose CTAs hold two or three planes: one lane per
+  // span, the four sums added in FP64.
   template <bool Num>
   __device__ void plane_sums(const float *T1, int cnt) {
     float *T2p = T2();
@@ -1174,6 +1175,7 @@ struct Engine {
       if (u < n && j == 0) T2p[u] = (float)s;
     }
   }
+
   // ---- pass A: the previous update's convergence sums from eval(Gd) (when
   // need_cv), applied to logU (when apply: logU -= eval(Gd)), and the masked
   // min/max of logU; clears the histogram copies
