@@ -894,17 +894,28 @@ struct Engine {
     return true;
   }
 
-  // The largest residual x - E(x) of the map (whole-GPU path): it is linear
-  // within a bin, so the bins' ends hold it, whatever values E takes in bins
-  // that no voxel fills.  One value per warp, from the bins its threads have
-  // just tabulated; read after the z contraction's barrier.  Every CTA has the
-  // same map.
+  // A bound on the voxels' residuals x - E(x) (whole-GPU path), which are linear
+  // within a bin: the larger of the bin's ends that hold weight in the
+  // histogram.  Bins without any have no voxel, and E there, a quotient of two
+  // sums that are rounding errors, may be anything: with them in the bound, the
+  // unit of the lattice sums grew to 2^-32 in a volume with one voxel of 1e12
+  // (lattice 3e-5 off the FP64 oracle instead of 1e-6).  At an end without
+  // weight a voxel lies within half a unit of the histogram of the other end;
+  // the last bin's may be one that the histogram drops.  One value per warp,
+  // from the bins its threads have just tabulated; read after the z
+  // contraction's barrier.  Every CTA has the same map.
   __device__ __forceinline__ float *rmax() const { return (float *)(red() + 128); }
   __device__ __forceinline__ void residual_max() const {
-    const float2 *t = R2();
     if ((int)(threadIdx.x & ~31u) + 1 >= pr.bins) return;
+    const float2 *t = R2();
+    const unsigned long long *h = H64();
+    const float unit = (float)(1.0 / iter().scale);
     float m = 0.0f;
-    for (int b = threadIdx.x; b + 1 < pr.bins; b += blockDim.x) m = fmaxf(m, fmaxf(fabsf(t[b].x), fabsf(t[b].x + t[b].y)));
+    for (int b = threadIdx.x; b + 1 < pr.bins; b += blockDim.x) {
+      const bool lo = h[b] != 0, hi = h[b + 1] != 0 || b + 2 == pr.bins;
+      const float e = fmaxf(lo ? fabsf(t[b].x) : 0.0f, hi ? fabsf(t[b].x + t[b].y) : 0.0f);
+      if (lo || hi) m = fmaxf(m, lo && hi ? e : e + fabsf(t[b].y) * unit);
+    }
     m = __int_as_float(__reduce_max_sync(kFull, __float_as_int(m)));
     if ((threadIdx.x & 31) == 0) rmax()[threadIdx.x >> 5] = m;
   }

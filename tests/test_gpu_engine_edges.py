@@ -174,3 +174,20 @@ def test_forced_clusters_of_short_rows(cuda, shape, levels, k, kind):
                         ConvergenceThreshold=0.0)
         assert res.report["status"] == "N4_OK" and res.report["path"] == "cluster" and res.report["cluster_size"] == k
         assert nrel(res.lattice, lat) < TOL and nrel(res.im_normalized, out) < TOL
+
+
+@pytest.mark.parametrize("seed", [6, 7])
+@pytest.mark.parametrize("force", [0, 0x8])
+def test_a_bright_voxel_leaves_the_sums_their_digits(cuda, seed, force):
+    """One voxel of 1e12: all others lie in a few of the histogram's bins, and
+    the map's values in the bins between, quotients of rounding errors, must not
+    set the scale of the whole-GPU path's lattice sums.  Bound 1e-5: FP32 sums
+    over at most 56 voxels of a row, 56 * 2^-24 = 3e-6, and one of 98,000 voxels
+    in the top bin, 5e-6."""
+    shape = (72, 64, 56)
+    ph = make_phantom(shape, seed=seed, sigma=0.03, grid=4, coeff_std=0.15)
+    im, m = (np.abs(ph.im) + 0.3).astype(np.float32), ph.mask.astype(np.float32)
+    im[20, 20, 15] = 1e12
+    res = run(cuda, im, m, 1, [1], flags=force)
+    _, lat = O.N4(im, m, low_value=0, maximumNumberOfLevels=1, maximumNumberOfIterations=[1], ConvergenceThreshold=0.0)
+    assert res.report["status"] == "N4_OK" and nrel(res.lattice, lat) < 1e-5
