@@ -50,8 +50,9 @@ namespace n4 {
 // contraction).  Half a row of voxels: with an eighth the CTAs of the short
 // rows at the volume's ends took 66k cycles for the contractions of an
 // iteration where the others took 49k (512x512x320 at half resolution, 148
-// CTAs: 162k cycles an iteration with Z/8, 154k with Z/4 and Z/2; 181x217x181:
-// 128k, 124k and 121k).  The floor keeps a CTA of many short rows within the
+// CTAs: 162k cycles an iteration with Z/8, 154k with Z/4 and Z/2, when pass A
+// took pieces of rows; 142k with Z/2 now; 181x217x181: 128k, 124k and 121k).
+// The floor keeps a CTA of many short rows within the
 // row buffers (grid_rows_bound).
 __host__ __device__ inline int grid_row_overhead(int Z) { return Z / 2 > 16 ? Z / 2 : 16; }
 // Most rows, and most voxels, the partition gives one of K CTAs.
