@@ -162,6 +162,7 @@ struct Iter {
   Gauss gauss;
   int degenerate;   // no bin range: nothing to fit
   float cv;
+  float rmax;       // whole-GPU path: bound on the residuals of the map
 };
 static_assert(sizeof(Iter) <= (160 - 144) * 8, "Iter lies in the o_red words behind the scratch");
 
@@ -815,7 +816,7 @@ struct Engine {
       // den: weights below 1.  num: with w <= 2/3 and sum w^2 >= 0.46 per axis,
       // w^3/sum w^2 <= 1.45 w^2, so an entry's terms sum to at most 3.1 times
       // its den times the largest residual.
-      scale = ldexp(1.0, sum_shift(Num ? 4.0 * denmax * (degenerate ? 0.0f : residual_bound()) : nfg));
+      scale = ldexp(1.0, sum_shift(Num ? 4.0 * denmax * (degenerate ? 0.0f : it.rmax) : nfg));
     }
     const int slice = ncy * ncz;
     for (int m0 = 0; m0 < np || m0 == 0; m0 += tp) {
@@ -902,29 +903,23 @@ struct Engine {
   // unit of the lattice sums grew to 2^-32 in a volume with one voxel of 1e12
   // (lattice 3e-5 off the FP64 oracle instead of 1e-6).  At an end without
   // weight a voxel lies within half a unit of the histogram of the other end;
-  // the last bin's may be one that the histogram drops.  One value per warp,
-  // from the bins its threads have just tabulated; read after the z
-  // contraction's barrier.  Every CTA has the same map.
-  __device__ __forceinline__ float *rmax() const { return (float *)(red() + 128); }
-  __device__ __forceinline__ void residual_max() const {
+  // the last bin's may be one that the histogram drops.  From the bins a thread
+  // has just tabulated; read after the z contraction's barrier.  Every CTA has
+  // the same map.  (One value per warp and a loop over them in every thread took
+  // 10 of 1366 us at 181x217x181.)
+  __device__ __forceinline__ void residual_max() {
     if ((int)(threadIdx.x & ~31u) + 1 >= pr.bins) return;
     const float2 *t = R2();
     const unsigned long long *h = H64();
-    const float unit = (float)(1.0 / iter().scale);
+    const float unit = __int_as_float((127 - hshift) << 23);   // 2^-hshift
     float m = 0.0f;
     for (int b = threadIdx.x; b + 1 < pr.bins; b += blockDim.x) {
       const bool lo = h[b] != 0, hi = h[b + 1] != 0 || b + 2 == pr.bins;
       const float e = fmaxf(lo ? fabsf(t[b].x) : 0.0f, hi ? fabsf(t[b].x + t[b].y) : 0.0f);
       if (lo || hi) m = fmaxf(m, lo && hi ? e : e + fabsf(t[b].y) * unit);
     }
-    m = __int_as_float(__reduce_max_sync(kFull, __float_as_int(m)));
-    if ((threadIdx.x & 31) == 0) rmax()[threadIdx.x >> 5] = m;
-  }
-  __device__ __forceinline__ float residual_bound() const {
-    const int n = (min((int)blockDim.x, pr.bins - 1) + 31) >> 5;
-    float m = 0.0f;
-    for (int w = 0; w < n; ++w) m = fmaxf(m, rmax()[w]);
-    return m;
+    const int k = __reduce_max_sync(kFull, __float_as_int(m));
+    if ((threadIdx.x & 31) == 0) atomicMax((int *)&iter().rmax, k);
   }
 
   // x0 + x1 + x2 + x3, the sums of spans s, s - 1, s - 2, s - 3, added in the
@@ -1295,7 +1290,10 @@ struct Engine {
     const int bins = pr.bins;
     Iter &it = iter();
     // for the sharpening, beside the first voxels
-    if (threadIdx.x == blockDim.x - 1) it.gauss = gauss_of(it.bm.slope, pr.fwhm);
+    if (threadIdx.x == blockDim.x - 1) {
+      it.gauss = gauss_of(it.bm.slope, pr.fwhm);
+      it.rmax = 0.0f;
+    }
     {
       const float bmin = it.bm.fmin, ih = it.bm.ih, il = it.bm.il, lim = it.bm.ff_limit;
       const float scale = (float)it.scale;
